@@ -250,13 +250,15 @@ static int alloc_weight(rq_ctx* ctx, int type, int64_t rows, int64_t cols, rq_we
     if (e != cudaSuccess) { delete w; return rq_fail(RQ_ERR_ALLOC, "weight of %lld bytes: %s", (long long)w->bytes, cudaGetErrorString(e)); }
     w->main = base;
     w->scale = scale_bytes ? (uint16_t*)(base + main_padded) : nullptr;
+    const int rc = rq_make_tile_map(w);
+    if (rc) { rq_weight_free(ctx, w); return rc; }
     *out = w;
     return RQ_OK;
 }
 
 int rq_make_tile_map(rq_weight* w) {
     w->has_tile_map = 0;
-    if ((w->type != RQ_Q4_K && w->type != RQ_Q6_K) || w->cols % 256) return RQ_OK;
+    if (!rq_type_has_fast_path(w->type)) return RQ_OK;
     typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                     CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static EncodeTiled encode = nullptr;
@@ -267,13 +269,17 @@ int rq_make_tile_map(rq_weight* w) {
             return rq_fail(RQ_ERR_CUDA, "the driver does not export cuTensorMapEncodeTiled");
         encode = (EncodeTiled)fn;
     }
-    const cuuint64_t unit = w->type == RQ_Q4_K ? 144 : 208, row_bytes = (cuuint64_t)(w->cols / 256) * unit;
+    // bytes of one row of a tile: a superblock of the K-quants, 128 bytes (128 values, 256 values) of Q8_0 and Q4_0. Tiles of 128-byte
+    // rows land swizzled, so that threads on adjacent rows read different banks; 144 and 208 bytes are odd counts of sixteen.
+    const bool kquant = w->type == RQ_Q4_K || w->type == RQ_Q6_K;
+    const cuuint64_t unit = w->type == RQ_Q4_K ? 144 : (w->type == RQ_Q6_K ? 208 : 128);
+    const cuuint64_t row_bytes = kquant ? (cuuint64_t)(w->cols / 256) * unit : (cuuint64_t)(w->type == RQ_Q8_0 ? w->cols : w->cols / 2);
     const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)w->rows};
-    const cuuint64_t strides[1] = {row_bytes};          // bytes between rows: a multiple of 16 (144 = 9 x 16, 208 = 13 x 16)
-    const cuuint32_t box[2] = {(cuuint32_t)unit, 128};  // one superblock of 128 rows; rows past the end arrive as zeros
+    const cuuint64_t strides[1] = {row_bytes};          // bytes between rows: a multiple of 16 (144 = 9 x 16, 208 = 13 x 16, blocks of 32 and 16)
+    const cuuint32_t box[2] = {(cuuint32_t)unit, 128};  // one tile of 128 rows; rows and bytes past the end arrive as zeros
     const cuuint32_t elem[2] = {1, 1};
     const CUresult rc = encode(&w->tile_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, w->main, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                               kquant ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (rc != CUDA_SUCCESS) return rq_fail(RQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d for a %lld x %lld weight", (int)rc, (long long)w->rows, (long long)w->cols);
     w->has_tile_map = 1;
     return RQ_OK;
@@ -296,7 +302,6 @@ extern "C" int rq_weight_prepare_device(rq_ctx* ctx, int type, const void* dev_b
     rc = alloc_weight(ctx, type, rows, cols, &w);
     if (rc) return rc;
     rc = rq_launch_repack(w, (const uint8_t*)dev_blocks, (cudaStream_t)stream);
-    if (!rc) rc = rq_make_tile_map(w);
     if (rc) { rq_weight_free(ctx, w); return rc; }
     *out = w;
     return RQ_OK;
@@ -431,17 +436,13 @@ extern "C" int rq_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_
     if (rc) return rc;
     if (sk <= 0 || yn <= 0 || (tokens > 1 && (st <= 0 || yt <= 0))) return rq_fail(RQ_ERR_INVALID, "rq_matmul: strides must be positive");
     DeviceGuard guard(ctx->device);
-    // K-quant weights: the integer-operand tensor-core kernel, for fp32 activations and for int8 windows of twelve and more
-    // positions (measured: below that the matvec kernel's exact integer dots, four tokens a pass, are faster)
+    // the tensor-core kernel, for fp32 activations and for int8 windows of twelve and more positions (below that the matvec kernel's
+    // exact integer dots, four tokens a pass, are faster)
     if (act_mode == RQ_ACT_FLOAT || (act_mode == RQ_ACT_INT8 && tokens >= 12)) {
-        rc = rq_launch_matmul_kq(ctx, w, x, sk, st, tokens, y, yn, yt, act_mode, step, (cudaStream_t)stream);
+        rc = rq_launch_matmul(ctx, w, x, sk, st, tokens, y, yn, yt, act_mode, step, (cudaStream_t)stream);
         if (rc != RQ_ERR_UNSUPPORTED) return rc;
     }
-    if (act_mode == RQ_ACT_FLOAT) {
-        rc = rq_launch_matmul(ctx, w, x, sk, st, tokens, y, yn, yt, (cudaStream_t)stream);
-        if (rc != RQ_ERR_UNSUPPORTED) return rc;
-    }
-    // int8 activations over the 32-value formats and odd widths go through the matvec kernels, four tokens a pass
+    // short int8 windows and the other formats go through the matvec kernels
     return rq_launch_gemv(ctx, w, x, sk, st, tokens, y, yn, yt, act_mode, step, (cudaStream_t)stream);
 }
 

@@ -28,8 +28,8 @@ struct rq_weight {
     uint16_t* scale; // fp16 d plane (null for Q4_K)
     int64_t bytes;   // total device bytes
     int device;
-    // K-quant weights of whole superblocks: a TMA descriptor of the main plane as a [rows][row bytes] byte matrix, fetched in
-    // tiles of 128 rows x one superblock (144 / 208 bytes) by the batched kernel
+    // the four formats with kernels of their own: a TMA descriptor of the main plane as a [rows][row bytes] byte matrix, fetched
+    // by the batched kernel in tiles of 128 rows x one superblock (144 / 208 bytes; 128 bytes of Q8_0 and Q4_0)
     alignas(64) CUtensorMap tile_map;
     int has_tile_map;
 };
@@ -97,7 +97,7 @@ int rq_launch_export(const rq_weight* w, uint8_t* dev_blocks, cudaStream_t s);
 int rq_launch_dequant(const rq_weight* w, float* out, cudaStream_t s);
 int rq_launch_gemv_generic(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s);
 int rq_launch_gather(const rq_weight* w, const int32_t* ids, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s);
-// fills w->tile_map for Q4_K / Q6_K weights (no-op for the others)
+// fills w->tile_map for the four formats with kernels of their own (no-op for the others)
 int rq_make_tile_map(rq_weight* w);
 int rq_launch_requant_q8_0(const rq_weight* src, rq_weight* dst, cudaStream_t s);
 int rq_launch_requant_q4_1(const rq_weight* src, rq_weight* dst, cudaStream_t s);
@@ -109,16 +109,11 @@ int rq_launch_gemv(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, 
 int rq_launch_gemv_multi(rq_ctx* ctx, int n, const rq_weight* const* ws, const float* x, int64_t sk, int64_t st, int tokens,
                          float* const* ys, int64_t yn, int64_t yt, int act_mode, int step, cudaStream_t s);
 int rq_launch_gemv_tiled_int8(rq_ctx* ctx, const rq_weight* w, int tokens, float* y, int64_t yn, int64_t yt, const uint8_t* act, cudaStream_t s);
-// RQ_ERR_UNSUPPORTED (no error text) = width not served by the tensor-core kernel
-int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s);
-// The K-quant batched product with integer weight operands (rq_matmul_kq.cu): FLOAT or INT8 activations.
-// RQ_ERR_UNSUPPORTED (no error text) = not a Q4_K / Q6_K weight.
-int rq_launch_matmul_kq(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int act_mode,
-                        int step, cudaStream_t s);
-size_t rq_matmul_kq_scratch_bytes(const rq_ctx* ctx, int type, int64_t rows, int64_t cols, int tokens);
-// y[row][token] = the splits' partial sums ([split][token][row]) added in split order
-int rq_launch_sum_splits(const float* partial, int splits, int64_t rows, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s);
-// scratch bytes rq_launch_matmul takes for a weight of this shape and this many tokens (its activation image and split-K sums)
+// The batched product with integer weight operands (rq_matmul_tc.cu): FLOAT or INT8 activations.
+// RQ_ERR_UNSUPPORTED (no error text) = not one of the four formats it serves.
+int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int act_mode,
+                     int step, cudaStream_t s);
+// scratch bytes that are enough for rq_launch_matmul over any weight of up to this shape and up to this many tokens (its activation image and shared tiles' sums)
 size_t rq_matmul_scratch_bytes(const rq_ctx* ctx, int64_t rows, int64_t cols, int tokens);
 int rq_launch_quantize(int type, const float* values, int64_t count, uint8_t* blocks, cudaStream_t s);
 // A run of virtual output rows of the streaming kernel (see rq_gemv_stream.cu).
