@@ -1,32 +1,302 @@
 // Matrix-vector product over the stored formats that have no streaming kernel of their own (Q4_1, Q5_0, Q5_1, Q5_K,
-// IQ4_NL, Q8_1, Q2_K, Q3_K, Q8_K, IQ4_XS): fp32 activations against per-value decoded weights, the reference's run
-// decoders (recipe.rs:7826-7917: one fused-multiply-add chain per unit of 32 values in index order; the units of a row
-// add up, ll:3451-3492; here the additions are regrouped, within the 1e-3 band). A warp owns a row and walks it in units
-// of 32 values, lane l taking value l of every unit, so that a unit's activations are one coalesced line and its weight
-// bytes one block; the lanes' sums meet in a fixed xor tree, so every run gives the same bits. `.int(8)` never reaches
-// these formats: the reference re-encodes them to Q8_0 at load (rq_weight_requantize), and that weight takes the
-// streaming kernel. `.int(4)` stores Q4_1 and dots it with int8 activation records: rq_gemv_q41_int8_kernel below.
+// IQ4_NL, Q8_1, Q2_K, Q3_K, Q8_K, IQ4_XS): fp32 activations against the decoded weights, the reference's run decoders
+// (recipe.rs:7826-7917: one fused-multiply-add chain per unit of 32 values; the units of a row add up, ll:3451-3492; here
+// the additions are regrouped, within the 1e-3 band). A LANE owns a group of 32 values: it fetches the group's bytes in
+// words, turns them into eight words of byte codes whatever the format, dots the codes with 32 inputs it holds in registers
+// and applies the scale and offset of each sixteen once. `.int(8)` never reaches these formats: the reference re-encodes
+// them to Q8_0 at load (rq_weight_requantize), and that weight takes the streaming kernel. `.int(4)` stores Q4_1 and dots it
+// with int8 activation records: rq_gemv_q41_int8_kernel below.
 #include "rq_decode.cuh"
 
 namespace {
 
 constexpr int kWarps = 8;  // rows per CTA
 
-template <int TYPE>
-__global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t cols, const float* __restrict__ x,
+constexpr int kChunkGroups = 256;          // 32-value groups of x in shared memory at a time: 8192 inputs
+constexpr int kGroupFloats = 36;           // a group's 32 inputs, padded: 144 bytes, so that eight lanes on adjacent groups read eight bank groups
+
+// N words from a 2-byte aligned address (blocks of 18, 22 and 110 bytes): the aligned words around it, shifted together. Nothing past
+// the last wanted byte's word is touched.
+template <int N>
+__device__ __forceinline__ void load_words2(const uint8_t* p, uint32_t* w) {
+    const uintptr_t a = (uintptr_t)p;
+    const uint32_t* q = (const uint32_t*)(a & ~(uintptr_t)3);
+    const uint32_t shift = (a & 2) ? 16u : 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __ldg(q + i);
+    const uint32_t last = shift ? __ldg(q + N) : 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(w[i], i + 1 < N ? w[i + 1] : last, shift);
+}
+template <int N>
+__device__ __forceinline__ void load_words4(const uint8_t* p, uint32_t* w) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __ldg((const uint32_t*)p + i);
+}
+__device__ __forceinline__ void load_line(const uint8_t* p, uint32_t* w) {
+    const uint4 v = __ldg((const uint4*)p);
+    w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+}
+
+// Four fifth bits (the low four of n) as bytes 0x10 / 0x00: bit i moves to 8 i + 4.
+__device__ __forceinline__ uint32_t fifth_bits(uint32_t n) { return ((n & 15u) * 0x02040810u) & 0x10101010u; }
+// The IQ4 levels of the eight nibbles of a word, biased by 128: bytes of the low nibbles (values 4 j ..) and of the high ones. The
+// sixteen levels (recipe.rs:15211) are four words; a byte permute looks four nibbles up in eight levels at a time.
+__device__ __forceinline__ void iq4_levels(uint32_t w, uint32_t& low, uint32_t& high) {
+    constexpr uint32_t k0 = 0xBFAD9881u ^ 0x80808080u, k1 = 0xF6EADDCFu ^ 0x80808080u, k2 = 0x26190D01u ^ 0x80808080u, k3 = 0x71594535u ^ 0x80808080u;
+    uint32_t v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // nibbles low0 high0 low1 high1 of half h
+        const uint32_t n = h ? w >> 16 : w & 0xffffu;
+        const uint32_t below = __byte_perm(k0, k1, n & 0x7777u), above = __byte_perm(k2, k3, n & 0x7777u);
+        const uint32_t pick = __byte_perm(0x0000FF00u, 0u, (n >> 3) & 0x1111u);
+        v[h] = (above & pick) | (below & ~pick);
+    }
+    low = __byte_perm(v[0], v[1], 0x6420);
+    high = __byte_perm(v[0], v[1], 0x7531);
+}
+
+// A group's stored bytes in registers, and what they stand for: value v = scale[v / 16] * (code[v] - bias) + offset[v / 16], codes
+// as the bytes of eight words in value order.
+template <int TYPE> struct GroupBytes;
+template <> struct GroupBytes<RQ_Q4_1> {
+    static constexpr int bias = 0;
+    uint32_t w[5];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<5>(row + (int64_t)g * 20, w); }
+    __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        scale[0] = scale[1] = rq_h2f((uint16_t)(w[0] & 0xffff));
+        offset[0] = offset[1] = rq_h2f((uint16_t)(w[0] >> 16));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { c[j] = w[1 + j] & 0x0F0F0F0Fu; c[4 + j] = (w[1 + j] >> 4) & 0x0F0F0F0Fu; }
+    }
+};
+template <> struct GroupBytes<RQ_Q5_0> {
+    static constexpr int bias = 16;
+    uint32_t w[6];  // d | high bits 0..15, high bits 16..31 | nibbles, ..: the fields straddle words
+    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+        const uint8_t* blk = row + (int64_t)g * 22;
+        w[0] = *(const uint16_t*)blk;
+        load_words2<5>(blk + 2, w + 1);
+    }
+    __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        scale[0] = scale[1] = rq_h2f((uint16_t)w[0]);
+        offset[0] = offset[1] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            c[j] = (w[2 + j] & 0x0F0F0F0Fu) | fifth_bits(w[1] >> (4 * j));
+            c[4 + j] = ((w[2 + j] >> 4) & 0x0F0F0F0Fu) | fifth_bits(w[1] >> (16 + 4 * j));
+        }
+    }
+};
+template <> struct GroupBytes<RQ_Q5_1> {
+    static constexpr int bias = 0;
+    uint32_t w[6];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<6>(row + (int64_t)g * 24, w); }
+    __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        scale[0] = scale[1] = rq_h2f((uint16_t)(w[0] & 0xffff));
+        offset[0] = offset[1] = rq_h2f((uint16_t)(w[0] >> 16));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            c[j] = (w[2 + j] & 0x0F0F0F0Fu) | fifth_bits(w[1] >> (4 * j));
+            c[4 + j] = ((w[2 + j] >> 4) & 0x0F0F0F0Fu) | fifth_bits(w[1] >> (16 + 4 * j));
+        }
+    }
+};
+template <> struct GroupBytes<RQ_Q5_K> {
+    static constexpr int bias = 0;
+    uint32_t hdr[4], qh[8], qs[8];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+        const uint8_t* blk = row + (int64_t)(g >> 3) * 176;  // eleven lines of sixteen bytes
+        load_line(blk, hdr);
+        load_line(blk + 16, qh);
+        load_line(blk + 32, qh + 4);
+        load_line(blk + 48 + 32 * ((g & 7) >> 1), qs);
+        load_line(blk + 64 + 32 * ((g & 7) >> 1), qs + 4);
+    }
+    __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        const int sub = g & 7;
+        int sc, mn;
+        rq_q4k_scale_min(hdr[1], hdr[2], hdr[3], sub, sc, mn);
+        scale[0] = scale[1] = __fmul_rn(rq_h2f((uint16_t)(hdr[0] & 0xffff)), (float)sc);
+        offset[0] = offset[1] = -__fmul_rn(rq_h2f((uint16_t)(hdr[0] >> 16)), (float)mn);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = ((qs[j] >> (4 * (sub & 1))) & 0x0F0F0F0Fu) | (((qh[j] >> sub) & 0x01010101u) << 4);
+    }
+};
+template <> struct GroupBytes<RQ_IQ4_NL> {
+    static constexpr int bias = 128;
+    uint32_t d, w[4];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+        const uint8_t* blk = row + (int64_t)g * 18;
+        d = *(const uint16_t*)blk;
+        load_words2<4>(blk + 2, w);
+    }
+    __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        scale[0] = scale[1] = rq_h2f((uint16_t)d);
+        offset[0] = offset[1] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) iq4_levels(w[j], c[j], c[4 + j]);
+    }
+};
+template <> struct GroupBytes<RQ_IQ4_XS> {
+    static constexpr int bias = 128;
+    uint32_t hdr[2], w[4];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+        const uint8_t* blk = row + (int64_t)(g >> 3) * 136;
+        load_words4<2>(blk, hdr);
+        load_words4<4>(blk + 8 + 16 * (g & 7), w);
+    }
+    __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        const int b = g & 7, high = (hdr[0] >> (16 + 2 * b)) & 3, low = (hdr[1] >> (4 * b)) & 15;
+        scale[0] = scale[1] = __fmul_rn(rq_h2f((uint16_t)(hdr[0] & 0xffff)), (float)((low | (high << 4)) - 32));
+        offset[0] = offset[1] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) iq4_levels(w[j], c[j], c[4 + j]);
+    }
+};
+template <> struct GroupBytes<RQ_Q8_1> {
+    static constexpr int bias = 128;
+    uint32_t w[9];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<9>(row + (int64_t)g * 36, w); }
+    __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        scale[0] = scale[1] = rq_h2f((uint16_t)(w[0] & 0xffff));
+        offset[0] = offset[1] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = w[1 + j] ^ 0x80808080u;
+    }
+};
+template <> struct GroupBytes<RQ_Q8_K> {
+    static constexpr int bias = 128;
+    uint32_t d, w[8];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+        const uint8_t* blk = row + (int64_t)(g >> 3) * 292;
+        d = __ldg((const uint32_t*)blk);
+        load_words4<8>(blk + 4 + 32 * (g & 7), w);
+    }
+    __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        scale[0] = scale[1] = __uint_as_float(d);
+        offset[0] = offset[1] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = w[j] ^ 0x80808080u;
+    }
+};
+template <> struct GroupBytes<RQ_Q2_K> {
+    static constexpr int bias = 0;
+    uint32_t meta, dd, w[8];
+    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+        const uint8_t* blk = row + (int64_t)(g >> 3) * 84;
+        meta = *(const uint16_t*)(blk + 2 * (g & 7));
+        load_words4<8>(blk + 16 + 32 * ((g & 7) >> 2), w);
+        dd = __ldg((const uint32_t*)(blk + 80));
+    }
+    __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        const float d = rq_h2f((uint16_t)(dd & 0xffff)), dmin = rq_h2f((uint16_t)(dd >> 16));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int m = (meta >> (8 * h)) & 0xff;
+            scale[h] = __fmul_rn(d, (float)(m & 15));
+            offset[h] = -__fmul_rn(dmin, (float)(m >> 4));
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = (w[j] >> (2 * (g & 3))) & 0x03030303u;
+    }
+};
+template <> struct GroupBytes<RQ_Q3_K> {
+    static constexpr int bias = 4;  // a clear mask bit takes four off the code
+    uint32_t mask[8], w[8], sc[3], d;
+    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+        const uint8_t* blk = row + (int64_t)(g >> 3) * 110;
+        load_words2<8>(blk, mask);
+        load_words2<8>(blk + 32 + 32 * ((g & 7) >> 2), w);
+        load_words2<3>(blk + 96, sc);
+        d = *(const uint16_t*)(blk + 108);
+    }
+    __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
+        const int sub = g & 7;
+        const float df = rq_h2f((uint16_t)d);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int b = 2 * sub + h, at = b & 7;
+            const int low = ((at < 4 ? sc[0] : sc[1]) >> (8 * (at & 3) + (b < 8 ? 0 : 4))) & 15, high = (sc[2] >> (8 * (b & 3) + 2 * (b >> 2))) & 3;
+            scale[h] = __fmul_rn(df, (float)((low | (high << 4)) - 32));
+            offset[h] = 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = ((w[j] >> (2 * (sub & 3))) & 0x03030303u) | (((mask[j] >> sub) & 0x01010101u) << 2);
+    }
+};
+
+// A warp owns ROWS rows, its lanes the groups g, g + 32, ..: a lane reads its group's 32 inputs from shared memory once and uses them
+// for all of its rows, whose bytes are all in flight before the first is decoded. What bounds it is instruction issue (per four
+// weights: two or three to isolate the codes, eight to make them floats, four products); the kernel it replaces decoded value by
+// value, every header field once per value, and took ten times as long.
+template <int TYPE, int ROWS>
+__global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* __restrict__ x,
                                                                         int64_t sk, int64_t st, float* __restrict__ y, int64_t yn, int64_t yt) {
+    extern __shared__ __align__(16) float xs[];
+    constexpr bool kOffset = TYPE == RQ_Q4_1 || TYPE == RQ_Q5_1 || TYPE == RQ_Q5_K || TYPE == RQ_Q2_K;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, token = blockIdx.y;
     const float* xt = x + (int64_t)token * st;
-    const int64_t units = cols >> 5;
-    for (int64_t row = (int64_t)blockIdx.x * kWarps + warp; row < rows; row += (int64_t)gridDim.x * kWarps) {
-        // lane l takes value l of every unit: the warp's activation loads are one line, its weight bytes one block
-        float sum = 0.f;
-        const int64_t first = row * cols + lane;
-#pragma unroll 4
-        for (int64_t u = 0; u < units; ++u) sum = fmaf(rq_decode_value<TYPE>(main_plane, nullptr, first + (u << 5), cols), __ldg(xt + ((u << 5) + lane) * sk), sum);
+    const int64_t row0 = ((int64_t)blockIdx.x * kWarps + warp) * ROWS;
+    const uint8_t* base[ROWS];
+    float sum[ROWS];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-        if (lane == 0) y[row * yn + (int64_t)token * yt] = sum;
+    for (int r = 0; r < ROWS; ++r) {
+        base[r] = main_plane + (row0 + r < rows ? row0 + r : rows - 1) * row_bytes;  // rows past the end are computed and dropped
+        sum[r] = 0.f;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int g0 = 0; g0 < groups; g0 += kChunkGroups) {
+        const int here = min(kChunkGroups, groups - g0);
+        if (g0) __syncthreads();
+        for (int k = threadIdx.x; k < here * 32; k += kWarps * 32) xs[(k >> 5) * kGroupFloats + (k & 31)] = __ldg(xt + ((int64_t)g0 * 32 + k) * sk);
+        __syncthreads();
+        for (int i = lane; i < here; i += 32) {
+            const int g = g0 + i;
+            GroupBytes<TYPE> raw[ROWS];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) raw[r].load(base[r], g);
+            float v[32], half_sum[2] = {0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) *(float4*)(v + 4 * j) = *(const float4*)(xs + i * kGroupFloats + 4 * j);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) half_sum[j >> 4] += v[j];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                uint32_t c[8];
+                float scale[2], offset[2];
+                raw[r].decode(g, c, scale, offset);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float a = 0.f, b = 0.f;
+#pragma unroll
+                    for (int j = 4 * h; j < 4 * h + 4; ++j) {
+                        // 0x4B0000cc is 2^23 + code: the subtraction leaves the code less its bias, exactly
+                        constexpr float kOff = 8388608.0f + (float)GroupBytes<TYPE>::bias;
+                        a = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7650)) - kOff, v[4 * j], a);
+                        b = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7651)) - kOff, v[4 * j + 1], b);
+                        a = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7652)) - kOff, v[4 * j + 2], a);
+                        b = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7653)) - kOff, v[4 * j + 3], b);
+                    }
+                    if (!kOffset || fabsf(half_sum[h]) <= 3.402823466e38f) {
+                        sum[r] = fmaf(scale[h], a + b, sum[r]);
+                        if (kOffset) sum[r] = fmaf(offset[h], half_sum[h], sum[r]);
+                    } else {
+                        // an infinite input (or a NaN): scale and offset taken apart would meet as inf - inf
+                        const int64_t first = ((row0 + r < rows ? row0 + r : rows - 1) * groups + g) * 32 + 16 * h;
+#pragma unroll 1
+                        for (int j = 0; j < 16; ++j) sum[r] = fmaf(rq_decode_value<TYPE>(main_plane, nullptr, first + j, 0), xs[i * kGroupFloats + 16 * h + j], sum[r]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], off);
+        if (lane == 0 && row0 + r < rows) y[(row0 + r) * yn + (int64_t)token * yt] = sum[r];
     }
 }
 
@@ -100,14 +370,30 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_q41_int8_kernel(const uin
     }
 }
 
+template <int TYPE, int ROWS>
+int launch_generic_rows(const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((w->rows + kWarps * ROWS - 1) / (kWarps * ROWS)), (unsigned)tokens);
+    cfg.blockDim = dim3(kWarps * 32);
+    const int groups = (int)(w->cols >> 5);
+    cfg.dynamicSmemBytes = (size_t)(groups < kChunkGroups ? groups : kChunkGroups) * kGroupFloats * 4;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int64_t row_bytes = w->cols / rq_block_values(TYPE) * rq_block_bytes(TYPE);
+    RQ_CUDA(cudaLaunchKernelEx(&cfg, rq_gemv_generic_kernel<TYPE, ROWS>, (const uint8_t*)w->main, w->rows, row_bytes, groups, x, sk, st, y, yn, yt));
+    return RQ_OK;
+}
 template <int TYPE>
 int launch_generic(const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int sm_count, cudaStream_t s) {
-    const int64_t ctas = (w->rows + kWarps - 1) / kWarps;
-    const int64_t cap = (int64_t)sm_count * 8;  // eight resident CTAs of 256 threads per SM
-    dim3 grid((unsigned)(ctas < cap ? ctas : cap), (unsigned)tokens);
-    rq_gemv_generic_kernel<TYPE><<<grid, kWarps * 32, 0, s>>>(w->main, w->rows, w->cols, x, sk, st, y, yn, yt);
-    RQ_CUDA(cudaGetLastError());
-    return RQ_OK;
+    // rows per warp: as many as leave every SM two CTAs (a row's sums do not depend on it)
+    const int64_t warps = (int64_t)sm_count * 2 * kWarps / (tokens < 8 ? tokens : 8);
+    if (w->rows >= 4 * warps) return launch_generic_rows<TYPE, 4>(w, x, sk, st, tokens, y, yn, yt, s);
+    if (w->rows >= 2 * warps) return launch_generic_rows<TYPE, 2>(w, x, sk, st, tokens, y, yn, yt, s);
+    return launch_generic_rows<TYPE, 1>(w, x, sk, st, tokens, y, yn, yt, s);
 }
 
 }  // namespace
