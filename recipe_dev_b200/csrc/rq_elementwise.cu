@@ -12,24 +12,61 @@
 
 namespace {
 
-__global__ void __launch_bounds__(256) rq_rmsnorm_kernel(const float* __restrict__ x, int64_t sk, int64_t st, int64_t n, const float* __restrict__ gain,
-                                                          float epsilon, float* __restrict__ y, int64_t yk, int64_t yt) {
+// One CTA per position, a chain of latencies from end to end (the launch sits between two projections of a decode layer): HELD values
+// per thread are loaded at once and kept for the second pass, the tree has one barrier (every warp adds the 256 partial sums up
+// for itself: the pairs t, t + 128, then t, t + 64, .. of a tree in shared memory, the last five steps by shuffles, the same
+// bits). HELD = 0: rows beyond 8192 values are read twice.
+// x is what the kernel before this one wrote, and this one may start before that one has ended: its loads are spelled __ldcg and the
+// pointers carry no __restrict__, or the compiler may take them for loads of constants and move them ahead of the wait.
+template <int HELD>
+__global__ void __launch_bounds__(256) rq_rmsnorm_kernel(const float* x, int64_t sk, int64_t st, int64_t n, const float* gain,
+                                                          float epsilon, float* y, int64_t yk, int64_t yt) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     __shared__ float red[256];
-    const int t = blockIdx.x, tid = threadIdx.x;
+    const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const float* xt = x + (int64_t)t * st;
+    float* yo = y + (int64_t)t * yt;
+    float held[HELD ? HELD : 1], factor[HELD ? HELD : 1];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     float acc = 0.0f;
-    for (int64_t k = tid; k < n; k += 256) { const float v = xt[k * sk]; acc = __fadd_rn(acc, __fmul_rn(v, v)); }
+    if (HELD) {
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) held[i] = tid + 256 * i < n ? __ldcg(xt + (int64_t)(tid + 256 * i) * sk) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) factor[i] = gain && tid + 256 * i < n ? __ldcg(gain + tid + 256 * i) : 1.0f;  // in flight with x
+#pragma unroll
+        for (int i = 0; i < HELD; ++i)
+            if (tid + 256 * i < n) acc = __fadd_rn(acc, __fmul_rn(held[i], held[i]));
+    } else {
+#pragma unroll 8
+        for (int64_t k = tid; k < n; k += 256) { const float v = __ldcg(xt + k * sk); acc = __fadd_rn(acc, __fmul_rn(v, v)); }
+    }
     red[tid] = acc;
     __syncthreads();
-    for (int off = 128; off > 0; off >>= 1) { if (tid < off) red[tid] = __fadd_rn(red[tid], red[tid + off]); __syncthreads(); }
-    const float variance = __fdiv_rn(red[0], (float)n);
+    float part[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) part[i] = red[lane + 32 * i];
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+        for (int i = 0; i < off; ++i) part[i] = __fadd_rn(part[i], part[i + off]);
+    float total = part[0];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) total = __fadd_rn(total, __shfl_xor_sync(0xffffffffu, total, off));
+    const float variance = __fdiv_rn(total, (float)n);
     const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(variance, epsilon)));
-    float* yo = y + (int64_t)t * yt;
-    for (int64_t k = tid; k < n; k += 256) {
-        const float v = __fmul_rn(xt[k * sk], scale);
-        yo[k * yk] = gain ? __fmul_rn(v, gain[k]) : v;
+    if (HELD) {
+#pragma unroll
+        for (int i = 0; i < HELD; ++i) {
+            const int64_t k = tid + 256 * i;
+            if (k < n) { const float v = __fmul_rn(held[i], scale); yo[k * yk] = gain ? __fmul_rn(v, factor[i]) : v; }
+        }
+    } else {
+#pragma unroll 4
+        for (int64_t k = tid; k < n; k += 256) {
+            const float v = __fmul_rn(__ldcg(xt + k * sk), scale);
+            yo[k * yk] = gain ? __fmul_rn(v, __ldcg(gain + k)) : v;
+        }
     }
 }
 
@@ -110,7 +147,8 @@ extern "C" int rq_rmsnorm(rq_ctx* ctx, const float* x, int64_t x_k_stride, int64
     if (n <= 0 || tokens <= 0 || x_k_stride <= 0 || y_k_stride <= 0) return rq_fail(RQ_ERR_INVALID, "rq_rmsnorm: n, tokens and strides must be positive");
     if (!(epsilon >= 0.0f)) return rq_fail(RQ_ERR_INVALID, "rq_rmsnorm: epsilon must be non-negative");
     DeviceGuard guard(ctx->device);
-    return launch_pdl(rq_rmsnorm_kernel, (unsigned)tokens, (cudaStream_t)stream, x, x_k_stride, x_t_stride, n, gain, epsilon, y, y_k_stride, y_t_stride);
+    auto kernel = n <= 256 * 8 ? rq_rmsnorm_kernel<8> : (n <= 256 * 16 ? rq_rmsnorm_kernel<16> : (n <= 256 * 32 ? rq_rmsnorm_kernel<32> : rq_rmsnorm_kernel<0>));
+    return launch_pdl(kernel, (unsigned)tokens, (cudaStream_t)stream, x, x_k_stride, x_t_stride, n, gain, epsilon, y, y_k_stride, y_t_stride);
 }
 
 extern "C" int rq_add(rq_ctx* ctx, const float* a, const float* b, int64_t n, float* y, void* stream) {

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint
     for (int g0 = 0; g0 < groups; g0 += kChunkGroups) {
         const int here = min(kChunkGroups, groups - g0);
         if (g0) __syncthreads();
-        for (int k = threadIdx.x; k < here * 32; k += kWarps * 32) xs[(k >> 5) * kGroupFloats + (k & 31)] = __ldg(xt + ((int64_t)g0 * 32 + k) * sk);
+        for (int k = threadIdx.x; k < here * 32; k += kWarps * 32) xs[(k >> 5) * kGroupFloats + (k & 31)] = __ldcg(xt + ((int64_t)g0 * 32 + k) * sk);
         __syncthreads();
         for (int i = lane; i < here; i += 32) {
             const int g = g0 + i;
