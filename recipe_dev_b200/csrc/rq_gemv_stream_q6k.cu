@@ -1,0 +1,7 @@
+// The streaming matrix-vector kernel over Q6_K weights.
+#include "rq_gemv_stream.cuh"
+
+template <>
+int rqstream::dispatch_type<RQ_Q6_K>(StreamParams& p, bool is_float, int sm_count, int vectors_per_launch, cudaStream_t s) {
+    return is_float ? dispatch_stream<RQ_Q6_K, RQ_ACT_FLOAT>(p, sm_count, vectors_per_launch, s) : dispatch_stream<RQ_Q6_K, RQ_ACT_INT8>(p, sm_count, vectors_per_launch, s);
+}

@@ -78,7 +78,7 @@ struct DeviceGuard {
 // Other widths use three planes: codes [cols] int8 | d [cols/32] fp32 | sum16 [cols/16] int16.
 // d = the step of a 32-value group, sum16 = the sum of the 16 codes of a slice.
 #define RQ_ACT_RECORD_INT8 336
-#define RQ_ACT_RECORD_FLOAT 1104
+#define RQ_ACT_RECORD_FLOAT 976
 __host__ __device__ inline bool rq_act_unit_layout(int64_t cols) { return cols % 256 == 0; }
 __host__ __device__ inline size_t rq_act_token_bytes(int64_t cols) {
     return rq_act_unit_layout(cols) ? (size_t)(cols / 256) * RQ_ACT_RECORD_INT8

@@ -1,0 +1,59 @@
+"""fp32 activations in the matvec kernel: inputs as 24-bit integers of their 32-input group, in three digit planes. Accuracy against
+64 bits over every format and row layout, inputs at the ends of the range, gated pairs against the two projections. GPU only (-m gpu)."""
+import numpy as np
+import pytest
+
+from tests import oracle_lib as ol
+from tests.test_gpu_parity import torch_cuda
+
+pytestmark = pytest.mark.gpu
+TYPES = [ol.Q4_K, ol.Q6_K, ol.Q8_0, ol.Q4_0]
+
+
+def _setup(rq_ctx, oracle, t, rows, cols):
+    blocks = oracle.quantize(t, oracle.normal(81, t + cols, rows * cols, 0.02))
+    return rq_ctx.weight_from_host(t, blocks, rows, cols), oracle.dequantize(t, blocks).astype(np.float64).reshape(rows, cols)
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("cols", [256, 768, 2048, 2560, 4096, 14336, 16384])  # one warp a row, padded groups, 5, 7 and 8 warps a row, partial sums
+@pytest.mark.parametrize("spread", [0.0, 1.0, 6.0])
+def test_accuracy_against_64_bits(rq_ctx, oracle, t, cols, spread):
+    rows = 65
+    w, exact = _setup(rq_ctx, oracle, t, rows, cols)
+    x = (oracle.normal(82, cols, cols, 1.0) * np.exp(spread * oracle.normal(82, cols + 1, cols, 1.0))).astype(np.float32)
+    y = rq_ctx.matvec(w, torch_cuda(x)).cpu().numpy()
+    # an input's rounding is at most 2^-24 of its group's largest magnitude; a row's sum of 32 such errors a group, weighted, stays
+    # below 2^-23 of sum |w| * (that magnitude); fp32 additions of the groups are covered by the factor of two
+    top = np.repeat(np.abs(x).reshape(-1, 32).max(1), 32).astype(np.float64)
+    bound = 2.0**-22 * (np.abs(exact) @ top)
+    assert np.all(np.abs(y - exact @ x.astype(np.float64)) <= bound)
+    if spread <= 1.0:
+        assert np.linalg.norm(y - exact @ x.astype(np.float64)) <= 4e-7 * np.linalg.norm(exact @ x.astype(np.float64))
+    # a window of positions gives each the bits of its own call
+    xs = np.stack([x, x[::-1], 2 * x, x, np.roll(x, 7)]).astype(np.float32)
+    ys = rq_ctx.matvec(w, torch_cuda(xs)).cpu().numpy()
+    for i in range(5):
+        assert np.array_equal(ys[i], rq_ctx.matvec(w, torch_cuda(xs[i])).cpu().numpy())
+    rq_ctx.check()
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_inputs_at_the_ends_of_the_range(rq_ctx, oracle, t):
+    rows, cols = 33, 1024
+    w, exact = _setup(rq_ctx, oracle, t, rows, cols)
+    base = oracle.normal(83, t, cols, 1.0)
+    for scale in (1e-30, 1e-34, 1e30):
+        x = (base.astype(np.float64) * scale).astype(np.float32)
+        y, want = rq_ctx.matvec(w, torch_cuda(x)).cpu().numpy().astype(np.float64), exact @ x.astype(np.float64)
+        # a step below 2^-126 is subnormal: off by up to 2^-150, and an input, 2^23 steps at most, by 2^-127
+        assert np.all(np.abs(y - want) <= 1e-6 * np.max(np.abs(want)) + 2.0**-126 * np.sum(np.abs(exact), axis=1))
+    assert np.array_equal(rq_ctx.matvec(w, torch_cuda(np.zeros(cols, np.float32))).cpu().numpy(), np.zeros(rows, np.float32))
+    for bad in (np.nan, np.inf, -np.inf):
+        x = base.copy()
+        x[100] = bad
+        y = rq_ctx.matvec(w, torch_cuda(x)).cpu().numpy()
+        assert not np.any(np.isfinite(y))
+    strided = torch_cuda(np.ascontiguousarray(np.stack([base, base]).T))  # every second float: the scalar loads
+    assert np.array_equal(rq_ctx.matvec(w, strided[:, 0]).cpu().numpy(), rq_ctx.matvec(w, torch_cuda(base)).cpu().numpy())
+    rq_ctx.check()
