@@ -189,6 +189,12 @@ extern "C" int rq_matvec_glu(rq_ctx* ctx, const rq_weight* gate, const rq_weight
     if (act_mode == RQ_ACT_INT8) {
         rc = rq_ensure_act_scratch(ctx, rq_act_token_bytes(gate->cols) * (size_t)tokens, s);
         if (rc) return rc;
+        if (rq_int8_fuses(tokens, gate->cols)) {
+            // one launch: it quantises x in its prologue and leaves the records for INT8_CACHED calls
+            rc = rq_launch_stream(ctx, gate->type, gate->cols, nullptr, &seg, 1, 2, RQ_EPI_GLU, gate->rows, x, sk, st, tokens, 0, yn, yt, act_mode, ctx->act_scratch, step, ctx->act_scratch, s);
+            if (rc == RQ_OK) { ctx->act_cols = gate->cols; ctx->act_tokens = tokens; ctx->act_step = step; }
+            if (rc != RQ_ERR_UNSUPPORTED) return rc;
+        }
         rc = rq_launch_act_quant(x, sk, st, gate->cols, tokens, step, ctx->act_scratch, nullptr, s);
         if (rc) return rc;
         ctx->act_cols = gate->cols; ctx->act_tokens = tokens; ctx->act_step = step;

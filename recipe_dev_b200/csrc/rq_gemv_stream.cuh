@@ -960,8 +960,9 @@ __device__ inline float rq_tanh_portable(float xf) {
 __device__ __forceinline__ float rq_sigmoid_portable(float x) { return __fmul_rn(0.5f, __fadd_rn(rq_tanh_portable(__fmul_rn(0.5f, x)), 1.0f)); }
 __device__ __forceinline__ float rq_silu_portable(float x) { return __fmul_rn(x, rq_sigmoid_portable(x)); }
 
-// R = rows a thread takes per stage in the warp scheme (its weight registers): 2 only where the launch uses two.
-template <int TYPE, int MODE, int T, int NW, int R>
+// R = rows a thread takes per stage in the warp scheme (its weight registers): 2 only where the launch uses two. GATED: the two are
+// the gate row and the up row of one virtual row
+template <int TYPE, int MODE, int T, int NW, int R, bool GATED>
 __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW <= 7 ? 2 : 1)) rq_gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr int kConsumers = NW * 32;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1372,6 +1373,17 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
             const size_t my_off = (size_t)row_in_pass * row_bytes + (size_t)my_u * p.unit_bytes;
             const size_t pass_bytes = (size_t)rows_per_pass * row_bytes;
             const bool writer = (lane & (group - 1)) == 0;
+            // Gated launches: the sums of a virtual row's gate and up rows wait in the warp's lanes, one virtual row a lane, until the lanes are full or the rows are over: silu goes through double precision,
+            // a long chain that one lane would otherwise walk for every row by itself.
+            constexpr bool gated = GATED;
+            int pending = 0;
+            float held_gate = 0.f, held_up = 0.f;
+            float* held_y = nullptr;
+            auto flush = [&]() {
+                if (held_y) *held_y = rq_silu_portable(held_gate) * held_up;
+                held_y = nullptr;
+                pending = 0;
+            };
             while (true) {
                 if (!mbar_wait(&full_bar[2 * slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); dead = true; }
                 if (dead) break;
@@ -1382,14 +1394,20 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                 bool have[R];
 #pragma unroll
                 for (int k = 0; k < R; ++k) {
-                    const int lr = row_in_pass + k * rows_per_pass;
+                    const int lr = row_in_pass + (gated ? 0 : k * rows_per_pass);
                     // the second pass's rows are the stage's second piece
                     if (k == 1 && p.pieces == 2 && !dead && !mbar_wait(&full_bar[2 * slot + 1], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); dead = true; }
                     have[k] = lr < info.x && act_owner;
                     if (have[k]) {
                         const uint16_t* sc = nullptr;
-                        if (TYPE != RQ_Q4_K) sc = (const uint16_t*)(stage + p.sub_main_bytes + info.w) + ((size_t)lr * p.units + my_u) * p.scales_per_unit;
-                        wr[k].load(stage + my_off + k * pass_bytes, sc, my_h, my_u);
+                        if (TYPE != RQ_Q4_K) {
+                            const uint8_t* plane = stage + (gated ? 2 : 1) * p.sub_main_bytes + info.w;
+                            // the up rows' d values: their copy starts at an offset of its own
+                            if (gated && k == 1)
+                                plane = stage + 2 * p.sub_main_bytes + p.sub_scale_bytes + (((uintptr_t)table[info.y].scale[1] + (uintptr_t)((int64_t)info.z * row_scales * 2)) & 15);
+                            sc = (const uint16_t*)plane + ((size_t)lr * p.units + my_u) * p.scales_per_unit;
+                        }
+                        wr[k].load(stage + my_off + (gated ? k * p.sub_main_bytes : k * pass_bytes), sc, my_h, my_u);
                     }
                 }
                 // the warp holds its weights in registers: the producer may refill the slot
@@ -1416,7 +1434,18 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                             for (int k = 0; k < R; ++k) v[j][k] += __shfl_xor_sync(0xffffffffu, v[j][k], off);
                     }
                 }
-                if (!split) {
+                if (!split && gated) {
+                    // every lane of a row's group holds its sums: lanes pending .. pending + warp_rows - 1 take the pass's rows
+                    const int mine = (lane - pending) & (p.warp_rows - 1), src = mine * group;
+                    const float g = __shfl_sync(0xffffffffu, v[0][0], src), u = __shfl_sync(0xffffffffu, v[0][R - 1], src);
+                    const int live = __shfl_sync(0xffffffffu, have[0] ? 1 : 0, src);
+                    if (lane >= pending && lane < pending + p.warp_rows && live) {
+                        held_gate = g; held_up = u;
+                        held_y = table[info.y].y + (int64_t)(info.z + warp * p.warp_rows + mine) * p.yn + (int64_t)tok0 * p.yt;
+                    }
+                    pending += p.warp_rows;
+                    if (pending == 32) flush();
+                } else if (!split) {
                     if (writer) {
                         float* yb = table[info.y].y;
 #pragma unroll
@@ -1449,6 +1478,12 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                             float out = 0.f;
 #pragma unroll
                             for (int w = 0; w < NW; ++w) out += *(volatile float*)&cross_sum[cross_buf][j][row][w];
+                            if (gated) {
+                                float up = 0.f;
+#pragma unroll
+                                for (int w = 0; w < NW; ++w) up += *(volatile float*)&cross_sum[cross_buf][j][(row + rows_per_pass) & 7][w];
+                                out = rq_silu_portable(out) * up;
+                            }
                             table[info.y].y[(int64_t)(info.z + row) * p.yn + (int64_t)(tok0 + j) * p.yt] = out;
                         }
                         __syncwarp();
@@ -1457,6 +1492,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                     if (++cross_buf > kMaxStages) cross_buf = 0;
                 }
             }
+            if (gated) flush();
         } else if (R == 2) {
             // two-row instantiations serve the warp scheme only
         } else if (MODE == RQ_ACT_INT8 && T == 1 && p.act_regs) {
@@ -1572,9 +1608,9 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
     }
 }
 
-template <int TYPE, int MODE, int T, int NW, int R>
+template <int TYPE, int MODE, int T, int NW, int R, bool GATED = false>
 int launch_stream(const StreamParams& p, int grid_x, size_t smem, cudaStream_t s) {
-    auto kernel = rq_gemv_stream_kernel<TYPE, MODE, T, NW, R>;
+    auto kernel = rq_gemv_stream_kernel<TYPE, MODE, T, NW, R, GATED>;
     static bool configured[64] = {};  // per instantiation and device: the opt-in to large dynamic shared memory
     int dev = 0;
     RQ_CUDA(cudaGetDevice(&dev));
@@ -1662,26 +1698,29 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     p.warp_rows = 0; p.rows_per_thread = 0;
     p.row_warps = 1;
     p.sum_group = 0; p.sum_chunks = 1;
-    const bool warp_shape = vectors_per_launch == 0 && p.table == nullptr && p.plan == nullptr && p.subs == 1 && p.epilogue == RQ_EPI_PLAIN;
+    // Gated pairs (a gate row and an up row of one vector: the dense feed-forward's first half, an expert bank's) run it as well,
+    // the two rows in one thread.
+    const bool gated_shape = p.subs == 2 && p.epilogue == RQ_EPI_GLU && vectors_per_launch <= 1 && p.table == nullptr;
+    const bool warp_shape = gated_shape || (vectors_per_launch == 0 && p.table == nullptr && p.plan == nullptr && p.subs == 1 && p.epilogue == RQ_EPI_PLAIN);
     // launches that run a warp scheme: int8 with register activations, fp32 with the token's record in shared memory
     const bool warp_launch = warp_shape && (p.act_regs || (MODE == RQ_ACT_FLOAT && t == 1));
     int layout_group = 0, layout_chunks = 1;
-    row_layout(ipr, &layout_group, &layout_chunks);
+    row_layout(2 * p.units, &layout_group, &layout_chunks);
     const bool split_shape = layout_chunks > 1 && layout_chunks == NW;
     if (warp_shape && layout_group) { p.sum_group = layout_group; p.sum_chunks = layout_chunks; }
     if (warp_launch && layout_group && layout_chunks == 1) {
         const int group = layout_group;
         p.warp_rows = 32 / group;
         const int pass_rows = NW * p.warp_rows;
-        p.rows_per_thread = (int64_t)2 * pass_rows * row_bytes <= 34 * 1024 && rows_per_cta > pass_rows ? 2 : 1;
-        stage_rows = pass_rows * p.rows_per_thread;
+        p.rows_per_thread = gated_shape || ((int64_t)2 * pass_rows * row_bytes <= 34 * 1024 && rows_per_cta > pass_rows) ? 2 : 1;
+        stage_rows = gated_shape ? pass_rows : pass_rows * p.rows_per_thread;
     } else if (warp_launch && split_shape) {
         // longer rows whose items split evenly over the warps, a power of two of lanes each (14336 inputs: 7 x 16)
         const int group = layout_group;
         p.warp_rows = 32 / group;
         p.row_warps = NW;
-        p.rows_per_thread = (int64_t)2 * p.warp_rows * row_bytes <= 34 * 1024 && rows_per_cta > p.warp_rows && 2 * p.warp_rows <= 8 ? 2 : 1;
-        stage_rows = p.warp_rows * p.rows_per_thread;
+        p.rows_per_thread = gated_shape || ((int64_t)2 * p.warp_rows * row_bytes <= 34 * 1024 && rows_per_cta > p.warp_rows && 2 * p.warp_rows <= 8) ? 2 : 1;
+        stage_rows = gated_shape ? p.warp_rows : p.warp_rows * p.rows_per_thread;
     }
     if (token_pairs) {
         if (!p.warp_rows) return RQ_ERR_UNSUPPORTED;  // pairs run a warp scheme or not at all
@@ -1689,7 +1728,7 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     }
     p.stage_rows = stage_rows;
     p.pieces = 1; p.piece_rows = stage_rows;
-    if (p.warp_rows && p.rows_per_thread == 2) { p.pieces = 2; p.piece_rows = stage_rows / 2; }
+    if (p.warp_rows && p.rows_per_thread == 2 && !gated_shape) { p.pieces = 2; p.piece_rows = stage_rows / 2; }
     {
         // in flight per CTA: about 32 KB (two CTAs per SM: some 9 MB on the whole GPU, the memory latency at full bandwidth), two pieces at least
         const int64_t piece_bytes = (int64_t)p.piece_rows * row_bytes * p.subs;
@@ -1723,6 +1762,9 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
         if (token_pairs) return launch_stream<TYPE, MODE, 2, NW, 1>(p, grid_x, smem, s);
     }
     if (t == 4) return launch_stream<TYPE, MODE, 4, NW, 1>(p, grid_x, smem, s);
+    if constexpr (NW != 5) {
+        if (p.warp_rows && gated_shape) return launch_stream<TYPE, MODE, 1, NW, 2, true>(p, grid_x, smem, s);
+    }
     if (p.rows_per_thread == 2) return launch_stream<TYPE, MODE, 1, NW, 2>(p, grid_x, smem, s);
     return launch_stream<TYPE, MODE, 1, NW, 1>(p, grid_x, smem, s);
 }

@@ -85,6 +85,10 @@ __host__ __device__ inline size_t rq_act_token_bytes(int64_t cols) {
                                     : (size_t)cols + (size_t)(cols / 32) * 4 + (size_t)(cols / 16) * 2;
 }
 
+// Whether an INT8 call quantises inside the matvec launch. Every CTA of such a launch reads all of x: beyond 8192 inputs that
+// traffic (some 300 CTAs x 4 bytes x inputs) costs more than the quantiser launch it saves.
+inline bool rq_int8_fuses(int tokens, int64_t cols) { return tokens == 1 && cols % 256 == 0 && cols <= 8192; }
+
 // Orders this call's use of the context's work areas after the previous call's when the two were given different streams.
 int rq_order_work_areas(rq_ctx* ctx, cudaStream_t s);
 // Makes the activation scratch at least `bytes` large (growing it synchronises the device: rq_reserve does that ahead of

@@ -57,3 +57,31 @@ def test_inputs_at_the_ends_of_the_range(rq_ctx, oracle, t):
     strided = torch_cuda(np.ascontiguousarray(np.stack([base, base]).T))  # every second float: the scalar loads
     assert np.array_equal(rq_ctx.matvec(w, strided[:, 0]).cpu().numpy(), rq_ctx.matvec(w, torch_cuda(base)).cpu().numpy())
     rq_ctx.check()
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("rows,cols", [(1, 256), (50, 768), (333, 2048), (1000, 4096), (40, 14336)])
+@pytest.mark.parametrize("mode,step", [(0, 32), (1, 32), (1, 256)])
+def test_gated_pairs_equal_the_two_projections(rq_ctx, oracle, t, rows, cols, mode, step):
+    import torch
+
+    g, _ = _setup(rq_ctx, oracle, t, rows, cols)
+    u = rq_ctx.weight_from_host(t, oracle.quantize(t, oracle.normal(84, t, rows * cols, 0.02)), rows, cols)
+    x = torch_cuda(oracle.normal(84, 5, 5 * cols, 1.0).reshape(5, cols))
+    for tokens in (1, 5):
+        xt = x[:tokens]
+        y = rq_ctx.matvec_glu(g, u, xt, act_mode=mode, step=step).cpu().numpy()
+        gd, ud = (rq_ctx.matvec(w, xt, act_mode=mode, step=step).cpu().numpy() for w in (g, u))
+        want = oracle.glu(gd.reshape(-1), ud.reshape(-1)).reshape(tokens, rows)
+        # the same sums in the same order wherever the rows have a lane layout; elsewhere to fp32 rounding of the sums
+        assert np.max(np.abs(y - want)) <= 2e-6 * np.max(np.abs(want))
+        first = rq_ctx.matvec_glu(g, u, x[0], act_mode=mode, step=step)
+        assert torch.equal(first, torch.from_numpy(y[0]).cuda())
+    if mode == 1:  # the fused launch leaves the records a cached call may use
+        y1 = rq_ctx.matvec_glu(g, u, x[0], act_mode=1, step=step)
+        cached, plain = torch.empty(rows, device="cuda"), rq_ctx.matvec(g, x[0], act_mode=1, step=step)
+        rq_ctx.matvec_glu(g, u, x[0], y=y1, act_mode=1, step=step)
+        s = torch.cuda.current_stream().cuda_stream
+        assert rq_ctx.lib.rq_matvec(rq_ctx.handle, g.handle, x.data_ptr(), 1, cols, 1, cached.data_ptr(), 1, rows, 2, step, s) == 0
+        assert torch.equal(cached, plain)
+    rq_ctx.check()
