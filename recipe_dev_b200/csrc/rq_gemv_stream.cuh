@@ -316,155 +316,12 @@ __device__ __forceinline__ float item_dot(const uint8_t* __restrict__ w, const u
 //   sum of slice s (s < 16), int16           at 1152 + 8 s + 2 t
 //   sum of group g, int16                    at 1280 + 8 g + 2 t
 // 1360 bytes = 85 sixteen-byte lines, an odd count: the loads of eight threads on adjacent units fall
-// in eight different bank groups. A weight word is masked once and dotted with four tokens; every
-// token's float operations are those of item_dot, in its order, so the sums are bit for bit the same.
+// in eight different bank groups.
 // ------------------------------------------------------------------------------------------
 constexpr int kRecord4 = 1360;
 __device__ __forceinline__ uint32_t lane_of(const uint4& v, int t) { return t == 0 ? v.x : (t == 1 ? v.y : (t == 2 ? v.z : v.w)); }
 __device__ __forceinline__ float lane_of(const float4& v, int t) { return t == 0 ? v.x : (t == 1 ? v.y : (t == 2 ? v.z : v.w)); }
 __device__ __forceinline__ int short_of(const uint2& v, int t) { return (int)(int16_t)((t < 2 ? v.x : v.y) >> (16 * (t & 1))); }
-
-template <int TYPE>
-__device__ __forceinline__ void item_dot_tok4(const uint8_t* __restrict__ w, const uint16_t* __restrict__ sc, const uint8_t* __restrict__ rec, const int h, const int u, float (&out)[4]) {
-    const uint4* codes = (const uint4*)rec + 32 * h;              // the half's 32 code words, four tokens each
-    const float4* steps = (const float4*)(rec + 1024) + 4 * h;    // its four group steps
-    const uint2* sum16 = (const uint2*)(rec + 1152) + 8 * h;      // its eight slice sums
-    const uint2* sum32 = (const uint2*)(rec + 1280) + 4 * h;      // its four group sums
-    if (TYPE == RQ_Q4_K) {
-        const uint4 hdr = *(const uint4*)w;
-        const float d = rq_h2f((uint16_t)(hdr.x & 0xffff)), dmin = rq_h2f((uint16_t)(hdr.x >> 16));
-        const uint32_t scw = h == 0 ? (hdr.y & 0x3f3f3f3fu) : ((hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u));
-        const uint32_t mnw = h == 0 ? (hdr.z & 0x3f3f3f3fu) : (((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u));
-        float acc_s[4] = {0.f, 0.f, 0.f, 0.f}, acc_m[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int pp = 0; pp < 2; ++pp) {
-            const uint8_t* qp = w + 16 + 64 * h + 32 * pp;
-            const uint4 q0 = *(const uint4*)qp, q1 = *(const uint4*)(qp + 16);
-            const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-            const int sc_lo = (scw >> (16 * pp)) & 0xff, sc_hi = (scw >> (16 * pp + 8)) & 0xff;
-            const int mn_lo = (mnw >> (16 * pp)) & 0xff, mn_hi = (mnw >> (16 * pp + 8)) & 0xff;
-            int dl[4] = {0, 0, 0, 0}, dh[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t lo = qw[j] & 0x0F0F0F0Fu, hi = qw[j] & 0xF0F0F0F0u;
-                const uint4 al = codes[16 * pp + j], ah = codes[16 * pp + 8 + j];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    dl[t] = dp4a_us(lo, lane_of(al, t), dl[t]);
-                    dh[t] = dp4a_us(hi, lane_of(ah, t), dh[t]);  // sixteen times the high-nibble dot
-                }
-            }
-            const float4 d_lo = steps[2 * pp], d_hi = steps[2 * pp + 1];
-            const uint2 g_lo = sum32[2 * pp], g_hi = sum32[2 * pp + 1];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                acc_s[t] = fmaf(lane_of(d_lo, t), (float)(sc_lo * dl[t]), acc_s[t]);
-                acc_s[t] = fmaf(lane_of(d_hi, t), (float)(sc_hi * (dh[t] >> 4)), acc_s[t]);
-                acc_m[t] = fmaf(__fmul_rn(lane_of(d_lo, t), (float)short_of(g_lo, t)), (float)mn_lo, acc_m[t]);
-                acc_m[t] = fmaf(__fmul_rn(lane_of(d_hi, t), (float)short_of(g_hi, t)), (float)mn_hi, acc_m[t]);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t) out[t] = diff_of_products(d, acc_s[t], dmin, acc_m[t]);
-    } else if (TYPE == RQ_Q6_K) {
-        const float d = rq_h2f(sc[0]);
-        const uint2 s2 = *(const uint2*)(w + 192 + 8 * h);
-        const uint32_t scales[2] = {s2.x, s2.y};
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int wh = 0; wh < 2; ++wh) {
-            const uint4 qh4 = *(const uint4*)(w + 128 + 32 * h + 16 * wh);
-            const uint32_t qh[4] = {qh4.x, qh4.y, qh4.z, qh4.w};
-#pragma unroll
-            for (int gl = 0; gl < 2; ++gl) {
-                const uint4 ql4 = *(const uint4*)(w + 64 * h + 32 * gl + 16 * wh);
-                const uint32_t ql[4] = {ql4.x, ql4.y, ql4.z, ql4.w};
-                const int s_lo = 2 * gl + wh, s_hi = s_lo + 4;
-                const int sc_lo = (int)(int8_t)(scales[s_lo >> 2] >> (8 * (s_lo & 3)));
-                const int sc_hi = (int)(int8_t)(scales[s_hi >> 2] >> (8 * (s_hi & 3)));
-                const int k_lo = 32 * gl + 16 * wh, k_hi = k_lo + 64;
-                constexpr uint32_t kPairLo = 0x03030303u, kPairHi = 0x30303030u;
-                int nl[4] = {0, 0, 0, 0}, nh[4] = {0, 0, 0, 0}, pl[4] = {0, 0, 0, 0}, ph[4] = {0, 0, 0, 0};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t m_nl = ql[j] & 0x0F0F0F0Fu, m_nh = ql[j] & 0xF0F0F0F0u;
-                    const uint32_t m_pl = qh[j] & (kPairLo << (2 * gl)), m_ph = qh[j] & (kPairHi << (2 * gl));
-                    const uint4 al = codes[(k_lo >> 2) + j], ah = codes[(k_hi >> 2) + j];
-#pragma unroll
-                    for (int t = 0; t < 4; ++t) {
-                        nl[t] = dp4a_us(m_nl, lane_of(al, t), nl[t]);
-                        nh[t] = dp4a_us(m_nh, lane_of(ah, t), nh[t]);
-                        pl[t] = dp4a_us(m_pl, lane_of(al, t), pl[t]);
-                        ph[t] = dp4a_us(m_ph, lane_of(ah, t), ph[t]);
-                    }
-                }
-                const float4 d_lo = steps[k_lo >> 5], d_hi = steps[k_hi >> 5];
-                const uint2 a_lo = sum16[k_lo >> 4], a_hi = sum16[k_hi >> 4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const int dl = nl[t] + ((pl[t] >> (2 * gl)) << 4) - 32 * short_of(a_lo, t);
-                    const int dh = (nh[t] >> 4) + (ph[t] >> (2 * gl)) - 32 * short_of(a_hi, t);
-                    acc[t] = fmaf(lane_of(d_lo, t), (float)(sc_lo * dl), acc[t]);
-                    acc[t] = fmaf(lane_of(d_hi, t), (float)(sc_hi * dh), acc[t]);
-                }
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t) out[t] = d * acc[t];
-    } else if (TYPE == RQ_Q8_0) {
-        const uint2 dd = *(const uint2*)(sc + 4 * h);
-        const uint32_t dw[2] = {dd.x, dd.y};
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const float d = rq_h2f((uint16_t)(dw[b >> 1] >> (16 * (b & 1))));
-            const uint4 q0 = *(const uint4*)(w + 16 * ((8 * h + 2 * b) ^ (u & 7))), q1 = *(const uint4*)(w + 16 * ((8 * h + 2 * b + 1) ^ (u & 7)));
-            const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-            int dot[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint4 a = codes[8 * b + j];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) dot[t] = dp4a_ss(qw[j], lane_of(a, t), dot[t]);
-            }
-            const float4 d8 = steps[b];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) acc[t] = fmaf(__fmul_rn(lane_of(d8, t), d), (float)dot[t], acc[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t) out[t] = acc[t];
-    } else {  // Q4_0
-        const uint2 dd = *(const uint2*)(sc + 4 * h);
-        const uint32_t dw[2] = {dd.x, dd.y};
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const float d = rq_h2f((uint16_t)(dw[b >> 1] >> (16 * (b & 1))));
-            const uint4 q = *(const uint4*)(w + 16 * ((4 * h + b) ^ (u & 7)));
-            const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
-            int dl[4] = {0, 0, 0, 0}, dh[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t lo = qw[j] & 0x0F0F0F0Fu, hi = qw[j] & 0xF0F0F0F0u;
-                const uint4 al = codes[8 * b + j], ah = codes[8 * b + 4 + j];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    dl[t] = dp4a_us(lo, lane_of(al, t), dl[t]);
-                    dh[t] = dp4a_us(hi, lane_of(ah, t), dh[t]);
-                }
-            }
-            const float4 d8 = steps[b];
-            const uint2 g = sum32[b];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                const int dot = dl[t] + (dh[t] >> 4) - 8 * short_of(g, t);
-                acc[t] = fmaf(__fmul_rn(lane_of(d8, t), d), (float)dot, acc[t]);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 4; ++t) out[t] = acc[t];
-    }
-}
 
 // ------------------------------------------------------------------------------------------
 // Register-resident items (single-token INT8 launches): a thread copies its item's weights out
@@ -620,6 +477,189 @@ __device__ __forceinline__ float dot_regs(const ItemRegs<RQ_Q4_0>& r, const ActH
         acc = fmaf(a.d8[b] * d, (float)dot, acc);
     }
     return acc;
+}
+
+// ------------------------------------------------------------------------------------------
+// Four int8 tokens in the warp schemes: the weights of the thread's R rows in registers, the tokens' codes from the interleaved
+// records (kRecord4): a 128-bit load brings a word of all four tokens and serves R rows. Q6_K codes are assembled here (three
+// instructions per four codes, then one dp4a a token, where the bit fields would take two); the integers are the same, and per
+// token and row the float operations and their order are dot_regs', so every position gets the bits of its own call.
+// ------------------------------------------------------------------------------------------
+template <int R>
+__device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q4_K> (&r)[R], const uint8_t* __restrict__ rec, const int h, float (&out)[4][R]) {
+    const uint4* codes = (const uint4*)rec + 32 * h;
+    const float4* steps = (const float4*)(rec + 1024) + 4 * h;
+    const uint2* sum32 = (const uint2*)(rec + 1280) + 4 * h;
+    float acc_s[4][R], acc_m[4][R];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int k = 0; k < R; ++k) acc_s[t][k] = acc_m[t][k] = 0.f;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {  // sub-block 4 h + g: low (even) or high (odd) nibbles of the 32 bytes of pair g / 2
+        int dot[4][R];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int k = 0; k < R; ++k) dot[t][k] = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint4 a = codes[8 * g + j];
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const uint4 q = r[k].q[2 * (g >> 1) + (j >> 2)];
+                const uint32_t w = (j & 3) == 0 ? q.x : ((j & 3) == 1 ? q.y : ((j & 3) == 2 ? q.z : q.w));
+                const uint32_t m = w & (g & 1 ? 0xF0F0F0F0u : 0x0F0F0F0Fu);  // high nibbles in place: sixteen times their dot
+#pragma unroll
+                for (int t = 0; t < 4; ++t) dot[t][k] = dp4a_us(m, lane_of(a, t), dot[t][k]);
+            }
+        }
+        const float4 d8 = steps[g];
+        const uint2 gs = sum32[g];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const uint4 hdr = r[k].hdr;
+            const uint32_t scw = h == 0 ? (hdr.y & 0x3f3f3f3fu) : ((hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u));
+            const uint32_t mnw = h == 0 ? (hdr.z & 0x3f3f3f3fu) : (((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u));
+            const int sc = (scw >> (8 * g)) & 0xff;
+            const float mn = small_int_to_float((mnw >> (8 * g)) & 0xff);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                acc_s[t][k] = fmaf(lane_of(d8, t), small_int_to_float(sc * (g & 1 ? dot[t][k] >> 4 : dot[t][k])), acc_s[t][k]);
+                acc_m[t][k] = fmaf(__fmul_rn(lane_of(d8, t), small_int_to_float(short_of(gs, t))), mn, acc_m[t][k]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+        const float d = rq_h2f((uint16_t)(r[k].hdr.x & 0xffff)), dmin = rq_h2f((uint16_t)(r[k].hdr.x >> 16));
+#pragma unroll
+        for (int t = 0; t < 4; ++t) out[t][k] = diff_of_products(d, acc_s[t][k], dmin, acc_m[t][k]);
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q6_K> (&r)[R], const uint8_t* __restrict__ rec, const int h, float (&out)[4][R]) {
+    const uint4* codes = (const uint4*)rec + 32 * h;
+    const float4* steps = (const float4*)(rec + 1024) + 4 * h;
+    const uint2* sum16 = (const uint2*)(rec + 1152) + 8 * h;
+    float acc[4][R];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int k = 0; k < R; ++k) acc[t][k] = 0.f;
+#pragma unroll
+    for (int o = 0; o < 8; ++o) {  // the order of dot_regs: half lines, ql line, low nibbles before high
+        const int wh = o >> 2, g = ((o >> 1) & 1) + 2 * (o & 1), at = 2 * g + wh;  // group of 32 in the chunk, slice 2 g + wh
+        int dot[4][R];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int k = 0; k < R; ++k) dot[t][k] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint4 a = codes[8 * g + 4 * wh + j];
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const uint4 ql4 = r[k].ql[2 * (g & 1) + wh], qh4 = r[k].qh[wh];
+                const uint32_t ql = j == 0 ? ql4.x : (j == 1 ? ql4.y : (j == 2 ? ql4.z : ql4.w)), qh = j == 0 ? qh4.x : (j == 1 ? qh4.y : (j == 2 ? qh4.z : qh4.w));
+                const uint32_t low = g < 2 ? ql & 0x0F0F0F0Fu : (ql >> 4) & 0x0F0F0F0Fu;
+                const uint32_t high = g == 0 ? qh << 4 : (g == 1 ? qh << 2 : (g == 2 ? qh : qh >> 2));
+                const uint32_t c = low | (high & 0x30303030u);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) dot[t][k] = dp4a_us(c, lane_of(a, t), dot[t][k]);
+            }
+        }
+        const float4 d8 = steps[g];
+        const uint2 ss = sum16[at];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const int sc = (int)(int8_t)((at < 4 ? r[k].sc.x : r[k].sc.y) >> (8 * (at & 3)));
+#pragma unroll
+            for (int t = 0; t < 4; ++t) acc[t][k] = fmaf(lane_of(d8, t), (float)(sc * (dot[t][k] - 32 * short_of(ss, t))), acc[t][k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) out[t][k] = rq_h2f((uint16_t)r[k].d16) * acc[t][k];
+}
+
+template <int R>
+__device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q8_0> (&r)[R], const uint8_t* __restrict__ rec, const int h, float (&out)[4][R]) {
+    const uint4* codes = (const uint4*)rec + 32 * h;
+    const float4* steps = (const float4*)(rec + 1024) + 4 * h;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int k = 0; k < R; ++k) out[t][k] = 0.f;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        int dot[4][R];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int k = 0; k < R; ++k) dot[t][k] = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const uint4 a = codes[8 * b + j];
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const uint4 q = r[k].q[2 * b + (j >> 2)];
+                const uint32_t w = (j & 3) == 0 ? q.x : ((j & 3) == 1 ? q.y : ((j & 3) == 2 ? q.z : q.w));
+#pragma unroll
+                for (int t = 0; t < 4; ++t) dot[t][k] = dp4a_ss(w, lane_of(a, t), dot[t][k]);
+            }
+        }
+        const float4 d8 = steps[b];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const float d = rq_h2f((uint16_t)((b < 2 ? r[k].dd.x : r[k].dd.y) >> (16 * (b & 1))));
+#pragma unroll
+            for (int t = 0; t < 4; ++t) out[t][k] = fmaf(__fmul_rn(lane_of(d8, t), d), (float)dot[t][k], out[t][k]);
+        }
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q4_0> (&r)[R], const uint8_t* __restrict__ rec, const int h, float (&out)[4][R]) {
+    const uint4* codes = (const uint4*)rec + 32 * h;
+    const float4* steps = (const float4*)(rec + 1024) + 4 * h;
+    const uint2* sum32 = (const uint2*)(rec + 1280) + 4 * h;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int k = 0; k < R; ++k) out[t][k] = 0.f;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        int lo[4][R], hi[4][R];
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int k = 0; k < R; ++k) lo[t][k] = hi[t][k] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint4 al = codes[8 * b + j], ah = codes[8 * b + 4 + j];
+#pragma unroll
+            for (int k = 0; k < R; ++k) {
+                const uint4 q = r[k].q[b];
+                const uint32_t w = j == 0 ? q.x : (j == 1 ? q.y : (j == 2 ? q.z : q.w));
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    lo[t][k] = dp4a_us(w & 0x0F0F0F0Fu, lane_of(al, t), lo[t][k]);
+                    hi[t][k] = dp4a_us(w & 0xF0F0F0F0u, lane_of(ah, t), hi[t][k]);
+                }
+            }
+        }
+        const float4 d8 = steps[b];
+        const uint2 gs = sum32[b];
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            const float d = rq_h2f((uint16_t)((b < 2 ? r[k].dd.x : r[k].dd.y) >> (16 * (b & 1))));
+#pragma unroll
+            for (int t = 0; t < 4; ++t) out[t][k] = fmaf(__fmul_rn(lane_of(d8, t), d), (float)(lo[t][k] + (hi[t][k] >> 4) - 8 * short_of(gs, t)), out[t][k]);
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -963,7 +1003,7 @@ __device__ __forceinline__ float rq_silu_portable(float x) { return __fmul_rn(x,
 // R = rows a thread takes per stage in the warp scheme (its weight registers): 2 only where the launch uses two. GATED: the two are
 // the gate row and the up row of one virtual row
 template <int TYPE, int MODE, int T, int NW, int R, bool GATED>
-__global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW <= 7 ? 2 : 1)) rq_gemv_stream_kernel(const __grid_constant__ StreamParams p) {
+__global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW <= 7 ? 2 : 1)) rq_gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr int kConsumers = NW * 32;
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full_bar[2 * kMaxStages];  // [slot][piece]
@@ -986,7 +1026,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
     __shared__ int4 stage_info[kMaxStages];
     // warp scheme with rows split over the warps: per stage in flight, each warp's sum of each row, and how many warps have
     // delivered. A warp is never more than the ring's depth ahead of the slowest, so kMaxStages + 1 buffers never collide.
-    constexpr int TR = T == 2 ? 2 : 1;  // tokens a thread keeps in registers (the warp schemes)
+    constexpr int TR = MODE == RQ_ACT_INT8 ? T : 1;  // tokens a thread sums at a time in the warp schemes
     __shared__ float cross_sum[kMaxStages + 1][TR][8][NW];
     __shared__ int cross_count[kMaxStages + 1];
 
@@ -1183,7 +1223,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
         // (all of the above is arithmetic on the launch's parameters: done before the wait, it costs the chain nothing)
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (!direct) stage_table();
-        ActHalf areg[TR];
+        ActHalf areg[T == 2 ? 2 : 1];  // (four tokens stay in shared memory)
         if (MODE == RQ_ACT_INT8 && p.act_regs) {
             // single token: this thread's 128 codes, steps and sums, kept in registers for the whole
             // kernel. They come from the records an earlier launch left in the scratch, or (fused
@@ -1199,7 +1239,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                 }
             } else if (act_owner) {
 #pragma unroll
-                for (int j = 0; j < TR; ++j) {
+                for (int j = 0; j < (T == 2 ? 2 : 1); ++j) {
                     const int tok = tok0 + j < p.tokens ? tok0 + j : tok0;  // a pair past the last token dots the first again and stores nothing
                     areg[j].load(p.act + ((size_t)tok * p.units + my_u) * kRecord, my_h);
                 }
@@ -1238,7 +1278,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
             }
             consumer_sync<kConsumers>();
         } else if (MODE == RQ_ACT_INT8 && T == 4) {
-            // four tokens' records, interleaved unit by unit (the layout item_dot_tok4 reads); a token past
+            // four tokens' records, interleaved unit by unit (the layout dot_regs_tok4 reads); a token past
             // the end of the batch is staged as zeros
             const int per_vec = p.units * (kRecord / 16), total = 4 * per_vec;
             for (int base_i = tid; base_i < total; base_i += 4 * kConsumers) {  // four 16-byte loads in flight per thread
@@ -1362,7 +1402,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
             }
         };
         constexpr int kSweep = kConsumers / 8;  // row tasks per sweep of the consumer threads
-        if (T <= 2 && p.warp_rows) {
+        if ((T <= 2 || MODE == RQ_ACT_INT8) && p.warp_rows) {
             // ---- the warp scheme: no partial sums in shared memory, no CTA-wide barrier. A row's items are
             // `group` adjacent lanes; a thread takes up to two rows of a stage (one per pass), holds their
             // weights in registers, releases the stage, and the lanes of a row join their sums by an xor tree.
@@ -1417,7 +1457,13 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                 // v[j][k]: token tok0 + j (the tokens a thread holds in registers) against row k of the stage; every token's
                 // dot and sums are the single-token ones, so a position gets the bits its own call gives
                 float v[TR][R];
-                if (MODE == RQ_ACT_INT8) {
+                if constexpr (MODE == RQ_ACT_INT8 && T == 4) {
+                    dot_regs_tok4<R>(wr, act_smem + (size_t)my_u * kRecord4, my_h, v);
+#pragma unroll
+                    for (int j = 0; j < TR; ++j)
+#pragma unroll
+                        for (int k = 0; k < R; ++k) v[j][k] = have[k] ? v[j][k] : 0.f;
+                } else if constexpr (MODE == RQ_ACT_INT8) {
 #pragma unroll
                     for (int j = 0; j < TR; ++j)
 #pragma unroll
@@ -1472,7 +1518,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                     if (arrived == NW - 1) {
                         __threadfence_block();
                         const int rows_here = info.x;
-                        // lanes 0..7 take the rows for the first token, lanes 8..15 for the second
+                        // lanes 0..7 take the rows for the first token, lanes 8..15 for the second, ..
                         const int row = lane & 7, j = lane >> 3;
                         if (row < rows_here && j < TR && tok0 + j < p.tokens) {
                             float out = 0.f;
@@ -1571,10 +1617,12 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T == 2 ? 2 : 3) : (NW
                         sc = (const uint16_t*)(stage + (size_t)p.subs * p.sub_main_bytes + (size_t)my_s * p.sub_scale_bytes + (first & 15)) + (size_t)my_su * p.scales_per_unit;
                     }
                     if constexpr (MODE == RQ_ACT_INT8 && T == 4) {
-                        float v4[4];
-                        item_dot_tok4<TYPE>(w, sc, act_smem + (size_t)my_u * kRecord4, my_h, my_u, v4);
+                        ItemRegs<TYPE> wr[1];
+                        float v4[4][1];
+                        wr[0].load(w, sc, my_h, my_u);
+                        dot_regs_tok4<1>(wr, act_smem + (size_t)my_u * kRecord4, my_h, v4);
 #pragma unroll
-                        for (int t = 0; t < 4; ++t) part[t * stage_items + tid] = v4[t];
+                        for (int t = 0; t < 4; ++t) part[t * stage_items + tid] = v4[t][0];
                     } else {
                         const uint8_t* a0 = act_smem + (size_t)sg.act[my_s] * p.act_bytes + (size_t)my_u * kRecord;
                         if constexpr (MODE == RQ_ACT_INT8) {
@@ -1660,9 +1708,11 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     // launches whose staged activations leave two CTAs no room for a ring (fp32 records of 14336 inputs are 62 KB).
     // token_pairs (int8 windows over rows of five consumer warps): two tokens' records in every thread's registers, 170
     // registers a thread, so two CTAs per SM instead of three
-    const int kCtasPerSm = one_per_sm ? 1 : (NW == 5 && !token_pairs ? 3 : 2);
+    const int kCtasPerSm = one_per_sm ? 1 : (NW == 5 && !token_pairs && p.tokens == 1 ? 3 : 2);
     // dynamic; with the static tables (about 10 KB) and the 1 KB the system keeps per CTA, two (three) CTAs fit an SM's 228 KB
-    const size_t kSmemBudget = one_per_sm ? 200 * 1024 : (NW == 5 && !token_pairs ? 64 * 1024 : 102 * 1024);
+    // (four int8 tokens: the warps' shares of a row take 9 KB more of static shared memory)
+    const bool quads = MODE == RQ_ACT_INT8 && p.tokens >= 2 && !token_pairs && vectors_per_launch == 0;
+    const size_t kSmemBudget = one_per_sm ? 200 * 1024 : (NW == 5 && !token_pairs && !quads ? 64 * 1024 : (quads ? 92 : 102) * 1024);
     constexpr int kRecord = MODE == RQ_ACT_INT8 ? RQ_ACT_RECORD_INT8 : RQ_ACT_RECORD_FLOAT;
     // NW = consumer warps: seven, so that with the producer warp a CTA is eight warps and two CTAs per SM leave each
     // thread 128 registers; eight (one CTA per SM then) only for rows too long for seven warps' worth of items.
@@ -1702,8 +1752,8 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     // the two rows in one thread.
     const bool gated_shape = p.subs == 2 && p.epilogue == RQ_EPI_GLU && vectors_per_launch <= 1 && p.table == nullptr;
     const bool warp_shape = gated_shape || (vectors_per_launch == 0 && p.table == nullptr && p.plan == nullptr && p.subs == 1 && p.epilogue == RQ_EPI_PLAIN);
-    // launches that run a warp scheme: int8 with register activations, fp32 with the token's record in shared memory
-    const bool warp_launch = warp_shape && (p.act_regs || (MODE == RQ_ACT_FLOAT && t == 1));
+    // launches that run a warp scheme: int8 with register activations or four tokens staged, fp32 with the token's record in shared memory
+    const bool warp_launch = warp_shape && (p.act_regs || (MODE == RQ_ACT_FLOAT && t == 1) || (MODE == RQ_ACT_INT8 && t == 4 && !gated_shape));
     int layout_group = 0, layout_chunks = 1;
     row_layout(2 * p.units, &layout_group, &layout_chunks);
     const bool split_shape = layout_chunks > 1 && layout_chunks == NW;
@@ -1761,6 +1811,9 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     if constexpr (NW == 5 && MODE == RQ_ACT_INT8) {
         if (token_pairs) return launch_stream<TYPE, MODE, 2, NW, 1>(p, grid_x, smem, s);
     }
+    if constexpr (MODE == RQ_ACT_INT8) {
+        if (t == 4 && p.warp_rows && p.rows_per_thread == 2) return launch_stream<TYPE, MODE, 4, NW, 2>(p, grid_x, smem, s);
+    }
     if (t == 4) return launch_stream<TYPE, MODE, 4, NW, 1>(p, grid_x, smem, s);
     if constexpr (NW != 5) {
         if (p.warp_rows && gated_shape) return launch_stream<TYPE, MODE, 1, NW, 2, true>(p, grid_x, smem, s);
@@ -1779,9 +1832,11 @@ int dispatch_stream(StreamParams& p, int sm_count, int vectors_per_launch, cudaS
         row_layout(ipr, &group, &chunks);
         if (chunks == 5 && vectors_per_launch == 0 && p.table == nullptr && p.plan == nullptr && p.subs == 1 && p.epilogue == RQ_EPI_PLAIN) {
             if (p.tokens == 1) return dispatch_stream_nw<TYPE, MODE, 5>(p, sm_count, vectors_per_launch, s);
-            // a window of positions: token pairs in registers (the weights are read once per pair, at the single-token rate)
-            // where the staged four-token pass is bound by its shared-memory loads
-            if (!p.fuse_step) {
+            // two positions: both in registers; more: four at a time from shared memory, two rows a thread
+            if (!p.fuse_step && p.tokens > 2) {
+                const int rc = dispatch_stream_nw<TYPE, MODE, 5>(p, sm_count, vectors_per_launch, s);
+                if (rc != RQ_ERR_UNSUPPORTED) return rc;
+            } else if (!p.fuse_step) {
                 const int rc = dispatch_stream_nw<TYPE, MODE, 5>(p, sm_count, vectors_per_launch, s, false, true);
                 if (rc != RQ_ERR_UNSUPPORTED) return rc;
             }
