@@ -182,17 +182,16 @@ int rq_add(rq_ctx* ctx, const float* a, const float* b, int64_t n, float* y, voi
 int rq_softcap(rq_ctx* ctx, const float* x, int64_t n, double cap, float* y, void* stream);
 
 /* The batched product (prefill, multi-sequence decode): the same contraction as rq_matvec for many
- * tokens, on the tensor cores (tcgen05.mma, fp32 accumulation in tensor memory) where a kernel serves
- * the case. Q4_K / Q6_K weights: exact-integer weight operands, activations as fp16 hi + lo pairs,
- * for RQ_ACT_FLOAT and for RQ_ACT_INT8 windows of twelve and more positions (the int8 answer is the
- * product over the records' code * step). Q8_0 / Q4_0 with RQ_ACT_FLOAT: weights dequantised a tile at
- * a time, both operands as hi + lo pairs. Everything else (shorter int8 windows, int8 over the 32-value
- * formats, the decode-only formats) runs the matvec kernels. Replaces contraction_forward_body's
+ * tokens, on the tensor cores (tcgen05.mma, fp32 accumulation in tensor memory) for Q4_K / Q6_K / Q8_0 /
+ * Q4_0 weights: exact-integer weight operands, activations as fp16 hi + lo pairs, for RQ_ACT_FLOAT and for
+ * RQ_ACT_INT8 windows of twelve and more positions (K-quants: the product over the records' code * step;
+ * Q8_0 / Q4_0: exact integer dots of the codes, scaled per 32 inputs). Everything else (shorter int8 windows,
+ * the decode-only formats) runs the matvec kernels. Replaces contraction_forward_body's
  * position loop and contraction_forward_gemm_body (amd-nv-cpu.ll:1231-2241, :3509-3649). Same
  * arguments as rq_matvec.
- * Range on the tensor-core routes: operands pass through fp16, so an activation of magnitude above
- * 65504 overflows (the result row is inf / NaN) and one below 6e-8 counts as zero; on the Q8_0 / Q4_0
- * route a dequantised weight of magnitude 256 or more overflows as well. rq_matvec has no such limit. */
+ * Range on the tensor-core routes, int8 over Q8_0 / Q4_0 excepted: activations pass through fp16, so one of
+ * magnitude above 65504 overflows (the result row is inf / NaN) and one below 6e-8 counts as zero.
+ * rq_matvec has no such limit. */
 int rq_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t x_k_stride, int64_t x_t_stride, int tokens,
               float* y, int64_t y_n_stride, int64_t y_t_stride, int act_mode, int step, void* stream);
 

@@ -9,17 +9,23 @@
 // fp16 holds every integer up to 2048 exactly, so the tensor core is fed the integers themselves (Q6_K: the fp16 rounding of
 // the integer plus its exact residual, -1 / 0 / 1) and the scale is applied outside it, when a sum leaves tensor memory.
 // Activations are fp32 and go in as fp16 pairs hi + lo (22 mantissa bits), prepared once per call (rq_tc_prep_kernel) in the
-// tensor core's 128-byte-swizzled K-major image; INT8 calls feed code * step through the same path.
+// tensor core's 128-byte-swizzled K-major image; INT8 calls over the K-quants feed code * step through the same path. INT8 calls
+// over Q8_0 and Q4_0 (CODES) feed the codes themselves: their scale changes every 32 inputs anyway, as the activations' step does,
+// so a sum of 32 products is an exact integer that both scale on its way out -- half the products, half the activation bytes,
+// the matvec kernel's arithmetic, and no fp16 range to stay in.
 //
 // One CTA per SM, persistent. Work is counted in UNITS, 256 inputs of one row tile (128 * MH rows) x one token tile: every CTA
 // takes the same number of whole tiles and then an equal share of the units that are left, whatever tile they fall in; a tile
-// that is shared by several CTAs is added up by rq_tc_sum_kernel in unit order (the same bits on every run). Roles in a CTA:
+// that is shared by several CTAs is added up, in unit order, by whichever of them is the last to leave its sums (the same bits on
+// every run; a kernel of its own would be one more launch in the chain). Roles in a CTA:
 //   * raw copies: one TMA tile of 128 rows x one unit of stored bytes at a time (Q8_0: half a unit) into a ring;
 //   * activation copies: one bulk copy per 64-wide slice, B_hi | B_lo of the token tile, into a ring;
 //   * staging groups of four warps (thread = row): stored bytes -> 64 fp16 integers -> operand slot in TENSOR MEMORY
 //     (tcgen05.st; the A operand of tcgen05.mma may live there, so the unpacked weights never touch shared memory). The groups
 //     take operand tiles in turn, so that their chains of latencies (barrier, load, unpack, store, fence) overlap;
-//   * one issuing thread: per slice and row half, the products into one of a ring of accumulators, one tcgen05.commit;
+//   * two issuing threads, alternate slices (MH = 2: a row half each): the products of a step into one of a ring of accumulators,
+//     one tcgen05.commit. Issuing a product holds its thread for about 70 cycles (as long as it runs), a look at a barrier or a
+//     commit for 100 to 300, so one thread's looks go behind the other's products;
 //   * eight drain warps: accumulator -> scale * sum -> fp32 registers, round-to-nearest, then Y or the partial sums.
 //
 // The tensor core adds into its fp32 accumulator by TRUNCATION, a bias that grows with the length of the chain (measured: 7e-7
@@ -46,12 +52,15 @@ namespace {
 
 constexpr int kDrainWarps = 8;
 constexpr int kDone = 32;                    // ring of "step finished" barriers, indexed by the step (see the kernel)
-constexpr int kMaxRaw = 8, kMaxB = 8, kMaxA = 8, kMaxAcc = 8;
+constexpr int kMaxRaw = 8, kMaxB = 12, kMaxA = 8, kMaxAcc = 8;
 constexpr float kMinScale = 256.0f, kMinUnscale = 1.0f / 256.0f;  // the minimum term's weights are scaled so that their fp16 residuals are no subnormals
 
+// groups: staging groups; cols: tokens per tile at most, the sums a drain thread holds; registers of the drain, staging and other
+// warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 768 x 80, 640 x 96)
 template <int MH> struct Shape;
-template <> struct Shape<1> { static constexpr int groups = 3, cols = 32; };   // staging groups; accumulator columns (tokens) a drain thread holds
-template <> struct Shape<2> { static constexpr int groups = 2, cols = 48; };
+template <> struct Shape<1> { static constexpr int groups = 3, cols = 64, drain_regs = 120, stage_regs = 64, other_regs = 48, launch_regs = 80; };
+template <> struct Shape<2> { static constexpr int groups = 2, cols = 96, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
+constexpr int kIssuers = 2;                  // with the two copying warps: one warpgroup
 template <int MH> __host__ __device__ constexpr int tc_threads() { return (kDrainWarps + 4 * Shape<MH>::groups + 4) * 32; }
 
 template <int TYPE> struct Format {
@@ -72,12 +81,14 @@ struct TcParams {
     int blocks32;          // 32-value blocks per row
     int units;             // 256-value units per row (a last one may be partial for the 32-value formats)
     int permuted;          // Q8_0 / Q4_0: the plane's chunks are permuted (rows of whole units)
-    const uint8_t* xs;     // activation images: [token tile][image tile][hi | lo][bn rows x 128 bytes, swizzled]
+    const uint8_t* xs;     // activation images: [token tile][image tile][hi | lo][bn rows x 128 bytes, swizzled] (CODES: one fp16 tile of codes)
+    const float* steps;    // CODES: [token tile][slice][half][bn]
     int image_tiles;       // 4 * units, then one per window of eight superblocks (Q4_K)
     int bn, tokens;
     float* y; int64_t yn, yt;
     int tiles_m, whole, rest_tiles;  // row tiles; whole tiles per CTA; tiles shared out by units
     float* partial;        // [2 * CTAs][bn][128 * MH]
+    int* arrived;          // per shared tile, how many of its CTAs have left their sums (zeroed by the preparation kernel)
     int raw_slots, b_slots, a_slots, accs;
     int* error_flag;
     unsigned long long wait_ns;
@@ -88,7 +99,7 @@ struct Walk {
     const int whole, units;
     int i, at, end;  // whole tiles taken; position among the shared units (fewer than CTAs x units of them: 32 bits)
     __device__ __forceinline__ Walk(int whole_, int rest, int units_) : whole(whole_), units(units_), i(0) {
-        const int64_t total = (int64_t)rest * units_;
+        const uint32_t total = (uint32_t)(rest * units_);
         at = (int)(blockIdx.x * total / gridDim.x);
         end = (int)((blockIdx.x + 1) * total / gridDim.x);
     }
@@ -127,16 +138,20 @@ __device__ __forceinline__ void unpack32(const uint8_t* tile, int r, int u, int 
         const uint8_t* blk = tile + r * 144;
         const uint4 hdr = *(const uint4*)blk;
         const uint4 q0 = *(const uint4*)(blk + 16 + 32 * sl), q1 = *(const uint4*)(blk + 32 + 32 * sl);
-        int sc, mn;
-        rq_q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * sl + half, sc, mn);
-        const __half2 sc2 = __half2half2(__int2half_rn(sc)), k1032 = __half2half2(__float2half_rn(1032.0f));
+        // the six-bit scale of sub-block 2 sl + half, without a branch: bytes 0 .. 3 of the first four, split ones after
+        const int at = 8 * ((2 * sl + half) & 3);
+        const uint32_t packed = sl < 2 ? hdr.y & 0x3f3f3f3fu : (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
+        const int sc = (packed >> at) & 0xff;
+        // a nibble in bits 4 .. 7 under an exponent of 0x6400 is 1024 + 16 q: times sc / 16, less 72 sc, is sc * (q - 8) -- sc / 16, 72 sc
+        // (a multiple of eight below 4608) and the result (at most 504) are fp16 numbers, so the fused operation is exact
+        const __half2 mul = __half2half2(__hmul(__int2half_rn(sc), __float2half_rn(0.0625f))), off = __half2half2(__int2half_rn(-72 * sc));
         const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const uint32_t a = ((w[j] >> (4 * half)) & 0x000F000Fu) | 0x64006400u;      // inputs 4j, 4j + 2
-            const uint32_t b = ((w[j] >> (4 * half + 8)) & 0x000F000Fu) | 0x64006400u;  // inputs 4j + 1, 4j + 3
-            o[2 * j] = as_u32(__hmul2(__hsub2(as_half2(a), k1032), sc2));
-            o[2 * j + 1] = as_u32(__hmul2(__hsub2(as_half2(b), k1032), sc2));
+            const uint32_t a = ((half ? w[j] : w[j] << 4) & 0x00F000F0u) | 0x64006400u;       // inputs 4j, 4j + 2
+            const uint32_t b = ((half ? w[j] >> 8 : w[j] >> 4) & 0x00F000F0u) | 0x64006400u;  // inputs 4j + 1, 4j + 3
+            o[2 * j] = as_u32(__hfma2(as_half2(a), mul, off));
+            o[2 * j + 1] = as_u32(__hfma2(as_half2(b), mul, off));
         }
     } else if (TYPE == RQ_Q6_K) {
         const int ch = sl >> 1, sel = sl & 1, g = 2 * sel + half;
@@ -211,26 +226,28 @@ __device__ __forceinline__ void minimum_terms(const uint4& hdr, bool low, uint32
 // code = clamp(rint(x * inverse)); the image holds code * d. STEP 0: fp32 activations. Rows past the last token and inputs past
 // the last column are zeros.
 // ------------------------------------------------------------------------------------------
-template <int STEP>
-__global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict__ x, int64_t sk, int64_t st, int cols, int units, int tokens, int bn, int padded_rows, int image_tiles,
-                                                          int windows, uint8_t* __restrict__ xs) {
+template <int STEP, bool CODES>
+__global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict__ x, int64_t sk, int64_t st, int cols, int units, int tokens, int bn, int image_tiles,
+                                                          int windows, uint8_t* __restrict__ xs, float* __restrict__ steps,
+                                                          int* __restrict__ arrived, int shared_tiles) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, unit = blockIdx.x;
-    const int row = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (row >= padded_rows) return;
+    const int row = blockIdx.y * 8 + (threadIdx.x >> 5);  // the padded rows are a multiple of sixteen: every warp has one
     const int nt = row / bn, r = row - nt * bn, k0 = unit * 256 + 8 * lane;
     const bool vec = sk == 1 && (st & 3) == 0 && ((uintptr_t)x & 15) == 0;
-    uint8_t* hi = xs + ((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * 2 * (size_t)bn * 128 + swizzled(r, lane & 7);
+    uint8_t* hi = xs + ((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * (CODES ? 1 : 2) * (size_t)bn * 128 + swizzled(r, lane & 7);
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (blockIdx.x == 0 && blockIdx.y == 0)
+        for (int i = threadIdx.x; i < shared_tiles; i += 256) arrived[i] = 0;
     float v[8];
     if (row < tokens && k0 < cols) {  // a width is a whole number of 32-value blocks: a lane's eight inputs are all inside or all outside
         const float* src = x + (int64_t)row * st + (int64_t)k0 * sk;
         if (vec) {
-            *(float4*)v = __ldg((const float4*)src);
-            *(float4*)(v + 4) = __ldg((const float4*)src + 1);
+            *(float4*)v = __ldcg((const float4*)src);
+            *(float4*)(v + 4) = __ldcg((const float4*)src + 1);
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __ldg(src + j * sk);
+            for (int j = 0; j < 8; ++j) v[j] = __ldcg(src + j * sk);
         }
     } else {
 #pragma unroll
@@ -254,8 +271,9 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict
         for (int j = 0; j < 8; ++j) {
             int code = __float2int_rn(__fmul_rn(v[j], inverse));
             code = code < -128 ? -128 : (code > 127 ? 127 : code);
-            v[j] = __fmul_rn((float)code, d);
+            v[j] = CODES ? (float)code : __fmul_rn((float)code, d);
         }
+        if (CODES && (lane & 3) == 0) steps[(((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * 2 + ((lane >> 2) & 1)) * bn + r] = d;
     }
     uint32_t hw[4], lw[4];
     split2(v[0], v[2], hw[0], lw[0]);  // the order the weights' nibble pairs come in
@@ -263,7 +281,7 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict
     split2(v[4], v[6], hw[2], lw[2]);
     split2(v[5], v[7], hw[3], lw[3]);
     *(uint4*)hi = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-    *(uint4*)(hi + (size_t)bn * 128) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+    if (!CODES) *(uint4*)(hi + (size_t)bn * 128) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
     if (windows) {
         // the unit's eight group sums: one 16-byte chunk of the window's image tile
         float s = 0.f;
@@ -287,42 +305,52 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict
     }
 }
 
-// eight columns at two places of this warp's 32 lanes
-__device__ __forceinline__ void tmem_ld8_pair(uint32_t a, uint32_t b, uint32_t (&u)[8], uint32_t (&v)[8]) {
+// sixteen columns at two places of this warp's 32 lanes; thirty-two at one
+__device__ __forceinline__ void tmem_ld16_pair(uint32_t a, uint32_t b, uint32_t (&u)[16], uint32_t (&v)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
         "tcgen05.wait::ld.sync.aligned;\n"
-        : "=&r"(u[0]), "=&r"(u[1]), "=&r"(u[2]), "=&r"(u[3]), "=&r"(u[4]), "=&r"(u[5]), "=&r"(u[6]), "=&r"(u[7]), "=&r"(v[0]), "=&r"(v[1]), "=&r"(v[2]), "=&r"(v[3]),
-          "=&r"(v[4]), "=&r"(v[5]), "=&r"(v[6]), "=&r"(v[7])
-        : "r"(a), "r"(b));
+        : "=&r"(u[0]), "=&r"(u[1]), "=&r"(u[2]), "=&r"(u[3]), "=&r"(u[4]), "=&r"(u[5]), "=&r"(u[6]), "=&r"(u[7]), "=&r"(u[8]), "=&r"(u[9]), "=&r"(u[10]), "=&r"(u[11]),
+          "=&r"(u[12]), "=&r"(u[13]), "=&r"(u[14]), "=&r"(u[15]), "=&r"(v[0]), "=&r"(v[1]), "=&r"(v[2]), "=&r"(v[3]), "=&r"(v[4]), "=&r"(v[5]), "=&r"(v[6]), "=&r"(v[7]),
+          "=&r"(v[8]), "=&r"(v[9]), "=&r"(v[10]), "=&r"(v[11]), "=&r"(v[12]), "=&r"(v[13]), "=&r"(v[14]), "=&r"(v[15])
+        : "r"(a), "r"(b)
+        : "memory");
 }
 
-// A ring position: slot index and the parity of its current use.
+// A ring position: slot index and the parity of its current use. (Kept by counting: a division by a ring's length, known at run time
+// only, is some thirty instructions.)
 struct Ring {
     int slot, n;
     uint32_t phase;
-    __device__ __forceinline__ explicit Ring(int n_) : slot(0), n(n_), phase(0) {}
+    __device__ __forceinline__ explicit Ring(int n_, int first = 0) : slot(0), n(n_), phase(0) { skip(first); }
     __device__ __forceinline__ void next() { if (++slot == n) { slot = 0; phase ^= 1; } }
+    __device__ __forceinline__ void skip(int by) { for (slot += by; slot >= n;) { slot -= n; phase ^= 1; } }
 };
 
-template <int TYPE, int MH>
+template <int TYPE, int MH, bool CODES>
 __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid_constant__ TcParams p) {
     using F = Format<TYPE>;
     constexpr int kGroups = Shape<MH>::groups, kStageFirst = kDrainWarps, kMiscFirst = kDrainWarps + 4 * kGroups, kCols = Shape<MH>::cols;
+    static_assert(256 * Shape<MH>::drain_regs + 128 * kGroups * Shape<MH>::stage_regs + 128 * Shape<MH>::other_regs <= tc_threads<MH>() * Shape<MH>::launch_regs, "more registers than the launch has: the increase would wait forever");
     constexpr int kHalves = F::halves, kMinSlices = TYPE == RQ_Q4_K ? 2 : 0;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzled tiles want 1024-byte alignment
     // A STEP is one sum that leaves tensor memory: (slice, row half, half slice), numbered in issue order. Its one commit arrives on
     // done[step % kDone]: the drain warps wait for it (the sum is complete), the staging warps for the last step that read their
     // operand slot, the activation copies for the last step that read theirs. Indexing by step keeps every parity wait within one
-    // phase: the issuing thread is never kDone steps ahead of anyone (slots x steps per slot < kDone).
+    // phase: no issuing thread is ever kDone steps ahead of anyone (slots x steps per slot < kDone).
     __shared__ __align__(8) uint64_t done[kDone], raw_full[kMaxRaw], raw_empty[kMaxRaw], b_full[kMaxB], a_full[kMaxA], acc_empty[kMaxAcc];
     __shared__ uint32_t tmem_base_slot;
+    __shared__ int last_piece;
+    // CODES: the activations' steps of a few slices, a ring of its own (the drain warps read it, well after the products are done)
+    constexpr int kStepSlots = CODES ? 8 : 1;
+    __shared__ __align__(16) float step_ring[kStepSlots][2][kCols];
+    __shared__ __align__(8) uint64_t steps_full[kStepSlots], steps_empty[kStepSlots];
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // visibly the same for the whole warp: the compiler budgets registers by role only then
-    const int bn = p.bn, b_bytes = bn * 256, a_slots = p.a_slots, accs = p.accs;
-    const int acc_cols = MH == 1 ? 2 * bn : bn;
+    const int bn = p.bn, b_bytes = bn * (CODES ? 128 : 256), a_slots = p.a_slots, accs = p.accs;
+    const int acc_cols = MH == 1 && !CODES ? 2 * bn : bn;
     uint8_t* raw = smem + (size_t)p.b_slots * b_bytes;
 
     if (tid == 0) {
@@ -330,7 +358,8 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
         for (int s = 0; s < kMaxRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4 * F::raw_slices); }
         for (int s = 0; s < kMaxB; ++s) mbar_init(&b_full[s], 1);
         for (int s = 0; s < kMaxA; ++s) mbar_init(&a_full[s], 4);
-        for (int s = 0; s < kMaxAcc; ++s) mbar_init(&acc_empty[s], kDrainWarps);
+        for (int s = 0; s < kMaxAcc; ++s) mbar_init(&acc_empty[s], 4);
+        for (int s = 0; s < kStepSlots; ++s) { mbar_init(&steps_full[s], 1); mbar_init(&steps_empty[s], MH == 1 ? 4 : kDrainWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMiscFirst) {
@@ -347,157 +376,235 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
 
     if (warp < kDrainWarps) {
         // ------------------------------------------------------------ drain warps
-        // launched with 96 registers a thread (MH = 2: 640 x 96 = 61440 in all): drain 256 x 152 + staging 256 x 64 + the rest 128 x 48
-        // = 61440 as well
-        if (MH == 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
-        // warp w may read accumulator rows 32 (w % 4) ..; warps 0-3 take the first half of the tile's tokens, warps 4-7 the second
-        const int quarter = warp & 3, tokens_here = bn >> 1, col0 = (warp >> 2) * tokens_here;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape<MH>::drain_regs));
+        // Warp w may read accumulator rows 32 (w % 4) .., so four warps drain a sum, and the two sets of four take turns: a sum's wait,
+        // loads and release are a chain of some thousand cycles however few its columns. MH = 1: even and odd slices, joined at the
+        // end of the tile; MH = 2: a row half each.
+        const int quarter = warp & 3, set = warp >> 2;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-        int step = 0;
-        Ring acc_at(accs);
+        float* const joined = (float*)(raw + (size_t)p.raw_slots * F::raw_bytes);  // MH = 1: [bn][128]
+        int slice_base = 0;  // slices of the segments before this one
+        Ring acc_at(accs, set * kHalves);  // the first accumulator of this set's next slice
         bool dead = false;
         while (walk.next(tile, u0, u1)) {
             const int mt = tile % p.tiles_m, nt = tile / p.tiles_m;
-            float sum[MH][kCols];
-            // this lane's row of half m, kept inside the weight for the scale loads (at most 2^31 rows)
-            auto row_of = [&](int m) -> int64_t { return min((uint32_t)(mt * MH + m) * 128u + (uint32_t)(quarter * 32 + lane), (uint32_t)(p.rows - 1)); };
+            const int64_t my_row0 = (int64_t)(mt * MH + (MH == 2 ? set : 0)) * 128;
+            float sum[kCols];
 #pragma unroll
-            for (int m = 0; m < MH; ++m) {
-#pragma unroll
-                for (int i = 0; i < kCols; ++i) sum[m][i] = 0.f;
-            }
-            auto drain = [&](int m, float d) {
-                if (!dead && !mbar_wait_warp(&done[step % kDone], (step / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 14); dead = true; }
+            for (int i = 0; i < kCols; ++i) sum[i] = 0.f;
+            // this lane's row, kept inside the weight for the scale loads
+            auto row_at = [&]() -> int64_t { return min(my_row0 + quarter * 32 + lane, p.rows - 1); };
+            // Slice ks of the segment: d0 (and d1: the second half's) scale its sums
+            auto drain = [&](int ks, float d0, float d1) {
+                const int all = slice_base + ks, last = (all * MH + (MH == 2 ? set : 0)) * kHalves + kHalves - 1;  // the slice's last step
+                if (!dead && !mbar_wait_warp(&done[last % kDone], (last / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 14); dead = true; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t at = tmem_base + lane_base + (uint32_t)(acc_at.slot * acc_cols + col0);
-                if (MH == 1) {
-#pragma unroll
-                    for (int c = 0; c < kCols; c += 8) {
-                        if (c < tokens_here) {
-                            uint32_t h[8], l[8];
-                            tmem_ld8_pair(at + c, at + bn + c, h, l);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) sum[m][c + j] = fmaf(d, __uint_as_float(h[j]) + __uint_as_float(l[j]), sum[m][c + j]);
-                        }
-                    }
-                } else {
+                const uint32_t acc0 = tmem_base + lane_base + (uint32_t)(acc_at.slot * acc_cols), acc1 = acc0 + (uint32_t)((kHalves - 1) * acc_cols);  // (an even number of accumulators: a slice's two are neighbours)
+                if constexpr (CODES) {
+                    const int slot = all % kStepSlots;
+                    if (!dead && !mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
+                    const float *d8 = &step_ring[slot][0][0], *e8 = d8 + bn;
 #pragma unroll
                     for (int c = 0; c < kCols; c += 16) {
-                        if (c < tokens_here) {
-                            uint32_t t[16];
-                            tmem_ld16(at + c, t);
+                        if (c < bn) {
+                            uint32_t t[16], u[16];
+                            tmem_ld16_pair(acc0 + c, acc1 + c, t, u);
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) sum[m][c + j] = fmaf(d, __uint_as_float(t[j]), sum[m][c + j]);
+                            for (int j = 0; j < 16; j += 4) {
+                                const float4 s4 = *(const float4*)(d8 + c + j), r4 = *(const float4*)(e8 + c + j);
+                                const float sv[4] = {s4.x, s4.y, s4.z, s4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+                                for (int q = 0; q < 4; ++q)
+                                    sum[c + j + q] += fmaf(__fmul_rn(rv[q], d1), __uint_as_float(u[j + q]), __fmul_rn(__fmul_rn(sv[q], d0), __uint_as_float(t[j + q])));
+                            }
+                        }
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&steps_empty[slot]);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < kHalves; ++h) {
+                        const uint32_t at = h ? acc1 : acc0;
+                        const float d = h ? d1 : d0;
+#pragma unroll
+                        for (int c = 0; c < kCols; c += MH == 1 ? 16 : 32) {
+                            if (c < bn) {
+                                uint32_t t[16], u[16];
+                                tmem_ld16_pair(at + c, at + (MH == 1 ? bn + c : c + 16), t, u);  // MH = 1: hi and lo of a token; else the next sixteen tokens
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) {
+                                    if (MH == 1) {
+                                        sum[c + j] = fmaf(d, __uint_as_float(t[j]) + __uint_as_float(u[j]), sum[c + j]);
+                                    } else {
+                                        sum[c + j] = fmaf(d, __uint_as_float(t[j]), sum[c + j]);
+                                        sum[c + 16 + j] = fmaf(d, __uint_as_float(u[j]), sum[c + 16 + j]);
+                                    }
+                                }
+                            }
                         }
                     }
                 }
-                // this warp has read the accumulator: the tensor core may overwrite it
+                // this warp has read the accumulators: the tensor core may overwrite them
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[acc_at.slot]);
-                ++step;
-                acc_at.next();
+                if (lane == 0) {
+                    mbar_arrive(&acc_empty[acc_at.slot]);
+                    if (kHalves == 2) mbar_arrive(&acc_empty[acc_at.slot + 1]);
+                }
+                acc_at.skip(2 * kHalves);
             };
+            constexpr int kStride = MH == 1 ? 2 : 1;
+            const int s0 = MH == 1 ? set : 0;  // (a segment has an even number of slices: parity by segment is parity overall)
+            const int main_slices = 4 * (u1 - u0), extra = kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0;
             if constexpr (F::kquant) {
-                auto d_of = [&](int m, int u) -> float {
-                    if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (row_of(m) * p.units + u) * 144)));
-                    return rq_h2f(__ldg(p.scale + row_of(m) * p.units + u));
+                auto d_of = [&](int u) -> float {
+                    if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (row_at() * p.units + u) * 144)));
+                    return rq_h2f(__ldg(p.scale + row_at() * p.units + u));
                 };
-                float d[MH], d_next[MH];
-#pragma unroll
-                for (int m = 0; m < MH; ++m) d_next[m] = d_of(m, u0);
+                float d_next = d_of(u0);
                 for (int u = u0; u < u1; ++u) {
-#pragma unroll
-                    for (int m = 0; m < MH; ++m) { d[m] = d_next[m]; if (u + 1 < u1) d_next[m] = d_of(m, u + 1); }  // the next unit's scale is on its way
+                    const float d = d_next;
+                    if (u + 1 < u1) d_next = d_of(u + 1);  // the next unit's scale is on its way
 #pragma unroll 1
-                    for (int sl = 0; sl < 4; ++sl)
-#pragma unroll
-                        for (int m = 0; m < MH; ++m) drain(m, d[m]);
+                    for (int sl = s0; sl < 4; sl += kStride) drain(4 * (u - u0) + sl, d, d);
                 }
                 if (kMinSlices) {
-                    const int extra = kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1);
 #pragma unroll 1
-                    for (int e = 0; e < extra; ++e)
-#pragma unroll
-                        for (int m = 0; m < MH; ++m) drain(m, -kMinUnscale);
+                    for (int e = s0; e < extra; e += kStride) drain(main_slices + e, -kMinUnscale, -kMinUnscale);
                 }
             } else {
-                // eight fp16 scales per unit; one word (two blocks: a slice) at a time, the next on its way
-                auto d_of = [&](int m, int b) -> uint32_t {  // b: an even block; rows of an odd number of blocks are only 2-byte aligned
-                    const uint16_t* at = p.scale + row_of(m) * p.blocks32;
-                    const uint32_t lo = b < p.blocks32 ? __ldg(at + b) : 0u, hi = b + 1 < p.blocks32 ? __ldg(at + b + 1) : 0u;
-                    return lo | (hi << 16);
+                // two fp16 scales a slice, the next slice's on their way; rows of an odd number of blocks are only 2-byte aligned
+                auto d_of = [&](int s) -> uint32_t {
+                    const int b = 2 * (4 * u0 + s);
+                    const uint16_t* at = p.scale + row_at() * p.blocks32 + b;
+                    return (b < p.blocks32 ? (uint32_t)__ldg(at) : 0u) | (b + 1 < p.blocks32 ? (uint32_t)__ldg(at + 1) << 16 : 0u);
                 };
-                uint32_t d[MH], d_next[MH];
-#pragma unroll
-                for (int m = 0; m < MH; ++m) d_next[m] = d_of(m, 8 * u0);
+                uint32_t d_next = d_of(s0);
 #pragma unroll 1
-                for (int s = 4 * u0; s < 4 * u1; ++s) {
-#pragma unroll
-                    for (int m = 0; m < MH; ++m) { d[m] = d_next[m]; if (s + 1 < 4 * u1) d_next[m] = d_of(m, 2 * s + 2); }
-#pragma unroll
-                    for (int m = 0; m < MH; ++m)
-#pragma unroll
-                        for (int h = 0; h < kHalves; ++h) drain(m, rq_h2f((uint16_t)(h ? d[m] >> 16 : d[m] & 0xffff)));
+                for (int s = s0; s < main_slices; s += kStride) {
+                    const uint32_t d = d_next;
+                    if (s + kStride < main_slices) d_next = d_of(s + kStride);
+                    drain(s, rq_h2f((uint16_t)(d & 0xffff)), rq_h2f((uint16_t)(d >> 16)));
                 }
             }
-            const bool whole = u0 == 0 && u1 == p.units;
-            float* part = p.partial + (size_t)(2 * blockIdx.x + (u0 == 0 ? 1 : 0)) * bn * 128 * MH;
+            slice_base += main_slices + extra;
+            const int r0 = quarter * 32 + lane;
+            if (MH == 1) {
+                // odd slices' sums join the even ones'
+                if (set == 1) {
 #pragma unroll
-            for (int m = 0; m < MH; ++m) {
-                const int r = m * 128 + quarter * 32 + lane;
-                const int64_t out_row = (int64_t)mt * MH * 128 + r;
+                    for (int j = 0; j < kCols; ++j)
+                        if (j < bn) joined[j * 128 + r0] = sum[j];
+                }
+                asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
+                if (set == 0) {
+#pragma unroll
+                    for (int j = 0; j < kCols; ++j)
+                        if (j < bn) sum[j] += joined[j * 128 + r0];
+                }
+                asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
+                if (set == 1) continue;
+            }
+            constexpr int kLeave = MH == 1 ? 128 : 256;  // threads that carry the tile out
+            const bool whole = u0 == 0 && u1 == p.units;
+            const int live_tokens = dead || my_row0 + r0 >= p.rows ? 0 : min(bn, p.tokens - nt * bn);
+            auto to_y = [&]() {
+                float* at = p.y + (my_row0 + r0) * p.yn + (int64_t)(nt * bn) * p.yt;
 #pragma unroll
                 for (int j = 0; j < kCols; ++j) {
-                    const int token = nt * bn + col0 + j;
-                    if (j < tokens_here && token < p.tokens && out_row < p.rows && !dead) {
-                        if (whole) p.y[out_row * p.yn + (int64_t)token * p.yt] = sum[m][j];
-                        else part[(size_t)(col0 + j) * 128 * MH + r] = sum[m][j];
+                    if (j < live_tokens) *at = sum[j];
+                    at += p.yt;
+                }
+            };
+            if (whole) {
+                to_y();
+            } else {
+                const size_t tile_floats = (size_t)bn * 128 * MH, mine = (MH == 2 ? set * 128 : 0) + r0;
+                float* part = p.partial + (size_t)(2 * blockIdx.x + (u0 == 0 ? 1 : 0)) * tile_floats + mine;
+#pragma unroll
+                for (int j = 0; j < kCols; ++j)
+                    if (j < live_tokens) part[j * 128 * MH] = sum[j];
+                // the CTAs that share this tile, in unit order: c0, c0 + 1, .. while their ranges reach into it
+                const int t = tile - p.whole * (int)gridDim.x;
+                // (fewer than 148 tiles of at most 65536 units among 148 CTAs: the products fit 32 bits)
+                const uint32_t total = (uint32_t)(p.rest_tiles * p.units), begin = (uint32_t)(t * p.units), end = begin + p.units;
+                auto range_begin = [&](int c) -> uint32_t { return (uint32_t)c * total / gridDim.x; };
+                int c0 = (int)(begin * gridDim.x / total);
+                while (c0 > 0 && range_begin(c0) > begin) --c0;
+                while (range_begin(c0 + 1) <= begin) ++c0;
+                int c1 = blockIdx.x;
+                while (c1 + 1 < (int)gridDim.x && range_begin(c1 + 1) < end) ++c1;
+                __threadfence();
+                asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
+                if (tid == 0) {
+                    asm volatile("griddepcontrol.wait;" ::: "memory");  // the counters were zeroed by the kernel before this one
+                    last_piece = atomicAdd(p.arrived + t, 1) == c1 - c0;
+                }
+                asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
+                if (last_piece) {
+                    __threadfence();
+#pragma unroll
+                    for (int j = 0; j < kCols; ++j) sum[j] = 0.f;
+                    for (int c = c0; c <= c1; ++c) {
+                        const float* piece = p.partial + (size_t)(2 * c + (range_begin(c) > begin ? 0 : 1)) * tile_floats + mine;
+                        // sixteen loads in flight (a branch for each would make each wait for the one before); the padding
+                        // tokens' places exist and hold nothing that is used
+#pragma unroll
+                        for (int j = 0; j < kCols; j += 16) {
+                            if (j < bn) {
+                                float v[16];
+#pragma unroll
+                                for (int q = 0; q < 16; ++q) v[q] = __ldcg(piece + (j + q) * 128 * MH);
+#pragma unroll
+                                for (int q = 0; q < 16; ++q) sum[j + q] += v[q];
+                            }
+                        }
                     }
+                    to_y();
                 }
             }
         }
     } else if (warp < kMiscFirst) {
         // ------------------------------------------------------------ staging groups: stored bytes -> integer operands in tensor memory
-        if (MH == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH>::stage_regs));
         const int group = (warp - kStageFirst) >> 2, r = (warp & 3) * 32 + lane;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        int a_base = 0, raw_base = 0;  // operand tiles and raw tiles of the segments before this one
+        Ring a_at(a_slots, group), raw_at(p.raw_slots);
+        int a = group, a_base = 0;         // this group's next operand tile; operand tiles of the segments before this one
+        int raw_here = 0, raw_base = 0;    // the tile of stored bytes raw_at stands at; tiles of the segments before this one
         bool dead = false;
         while (walk.next(tile, u0, u1)) {
             const int mt = tile % p.tiles_m;
             const int main_slices = 4 * (u1 - u0), extra = kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0;
             const int tiles = (main_slices + extra) * MH;
-            int first = group - a_base % kGroups;
-            if (first < 0) first += kGroups;
 #pragma unroll 1
-            for (int i = first; i < tiles; i += kGroups) {
-                const int ks = i / MH, m = i % MH, a = a_base + i;
-                const uint32_t at = a_ring + lane_base + (uint32_t)((a % a_slots) * F::a_cols);
-                const int freed = (a - a_slots) * kHalves + kHalves - 1;  // the last step that read the slot
-                bool free_slot = a < a_slots;
+            for (; a < a_base + tiles; a += kGroups, a_at.skip(kGroups)) {
+                const int ks = (a - a_base) / MH, m = (a - a_base) % MH;
+                const uint32_t at = a_ring + lane_base + (uint32_t)(a_at.slot * F::a_cols);
                 auto wait_slot = [&]() {
-                    if (!free_slot) {
+                    const int freed = (a - a_slots) * kHalves + kHalves - 1;  // the last step that read the slot
+                    if (freed >= 0) {
                         if (!dead && !mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 11); dead = true; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        free_slot = true;
                     }
                 };
                 if (ks < main_slices) {
-                    const int rt = raw_base + (ks / F::raw_slices) * MH + m, rslot = rt % p.raw_slots;
-                    if (!dead && !mbar_wait_warp(&raw_full[rslot], (rt / p.raw_slots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 18); dead = true; }
-                    const uint8_t* src = raw + (size_t)rslot * F::raw_bytes;
+                    const int rt = raw_base + (ks / F::raw_slices) * MH + m;
+                    raw_at.skip(rt - raw_here);
+                    raw_here = rt;
+                    if (!dead && !mbar_wait_warp(&raw_full[raw_at.slot], raw_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 18); dead = true; }
+                    const uint8_t* src = raw + (size_t)raw_at.slot * F::raw_bytes;
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
                         uint32_t o[16], res[16];
                         unpack32<TYPE>(src, r, u0 + (ks >> 2), ks & 3, half, p.permuted != 0, o, res);
-                        wait_slot();
+                        if (half == 0) wait_slot();
                         tmem_st16(at + 16 * half, o);
                         if (F::residual) tmem_st16(at + 32 + 16 * half, res);
                     }
                     // this warp has read its rows of the slice
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&raw_empty[rslot]);
+                    if (lane == 0) mbar_arrive(&raw_empty[raw_at.slot]);
                 } else if (TYPE == RQ_Q4_K) {
                     // the minimum terms of one window's superblocks, hi or lo: chunk j of the operand is superblock 8 w + j (zeros outside u0 .. u1)
                     const int e = ks - main_slices, window = (u0 >> 3) + (e >> 1);
@@ -520,87 +627,103 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                 tmem_st_wait();
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[a % a_slots]);  // one arrival per warp (an arrival is an atomic on the barrier)
+                if (lane == 0) mbar_arrive(&a_full[a_at.slot]);  // one arrival per warp (an arrival is an atomic on the barrier)
             }
             a_base += tiles;
             raw_base += main_slices / F::raw_slices * MH;
         }
     } else {
-        if (MH == 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
-        if (warp == kMiscFirst && elect_one()) {
-            // ------------------------------------------------------------ the issuing thread
-            const uint32_t idesc = instr_desc(bn), idesc2 = instr_desc(MH == 1 ? 2 * bn : bn);
-            Ring a_at(a_slots), b_at(p.b_slots), acc_at(accs);
-            int step = 0;
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH>::other_regs));
+        if (warp < kMiscFirst + kIssuers && elect_one()) {
+            // ------------------------------------------------------------ the issuing threads
+            const int me = warp - kMiscFirst;
+            const uint32_t idesc = instr_desc(bn), idesc2 = instr_desc(acc_cols);
+            constexpr int kSkip = MH == 1 ? kIssuers : 1, kTiles = MH == 1 ? kIssuers : 2;  // slices and operand tiles from one of this thread's to the next
+            Ring a_at(a_slots, me), b_at(p.b_slots, MH == 1 ? me : 0), acc_at(accs, me * kHalves);
+            int ks_all = 0;
             bool dead = false;
             while (walk.next(tile, u0, u1)) {
-                const int slices = 4 * (u1 - u0) + (kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0);
+                const int slices = 4 * (u1 - u0) + (kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0), end = ks_all + slices;
 #pragma unroll 1
-                for (int ks = 0; ks < slices; ++ks) {
-                    if (!dead && !mbar_wait(&b_full[b_at.slot], b_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
-                    const uint32_t bbase = smem_u32(smem + (size_t)b_at.slot * b_bytes);
+                for (int ks = ks_all + (MH == 1 ? me : 0); ks < end; ks += kSkip, a_at.skip(kTiles), b_at.skip(kSkip)) {  // (a segment has an even number of slices)
+                    const int a = MH == 1 ? ks : 2 * ks + me;  // operand tile
+                    const int bslot = b_at.slot, aslot = a_at.slot;
+                    if (!dead && !mbar_wait(&b_full[bslot], b_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
+                    const uint32_t bbase = smem_u32(smem + (size_t)bslot * b_bytes);
                     const uint64_t b_hi = smem_desc(bbase), b_lo = smem_desc(bbase + bn * 128);
-#pragma unroll 1
-                    for (int m = 0; m < MH; ++m) {
-                        if (!dead && !mbar_wait(&a_full[a_at.slot], a_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 13); dead = true; }
-                        const uint32_t a_hi = a_ring + (uint32_t)(a_at.slot * F::a_cols), a_res = a_hi + 32;
+                    if (!dead && !mbar_wait(&a_full[aslot], a_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 13); dead = true; }
+                    const uint32_t a_hi = a_ring + (uint32_t)(aslot * F::a_cols), a_res = a_hi + 32;
 #pragma unroll
-                        for (int h = 0; h < kHalves; ++h) {
-                            if (step >= accs && !dead && !mbar_wait(&acc_empty[acc_at.slot], acc_at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 15); dead = true; }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            if (!dead) {
-                                const uint32_t acc = tmem_base + (uint32_t)(acc_at.slot * acc_cols);
-                                constexpr int kk_n = 4 / kHalves;
-                                // kk: 16-wide steps, 32 bytes along K (in 16-byte units of the descriptor's start address), eight columns of A
-                                if (MH == 1) {
-                                    // columns [0, bn): A x B_hi; [bn, 2 bn): A x B_lo and, small as well, the residual x B_hi
+                    for (int h = 0; h < kHalves; ++h) {
+                        const int step = a * kHalves + h, slot = acc_at.slot;
+                        if (step >= accs && !dead && !mbar_wait(&acc_empty[slot], acc_at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 15); dead = true; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (!dead) {
+                            const uint32_t acc = tmem_base + (uint32_t)(slot * acc_cols);
+                            constexpr int kk_n = 4 / kHalves;
+                            // kk: 16-wide steps, 32 bytes along K (in 16-byte units of the descriptor's start address), eight columns of A
+                            if (CODES) {
 #pragma unroll
-                                    for (int k = 0; k < kk_n; ++k) { const int kk = h * kk_n + k; mma_f16_ts(acc, a_hi + 8 * kk, b_hi + 2 * kk, idesc2, k ? 1u : 0u); }
-                                    if (F::residual)
+                                for (int k = 0; k < kk_n; ++k) { const int kk = h * kk_n + k; mma_f16_ts(acc, a_hi + 8 * kk, b_hi + 2 * kk, idesc, k ? 1u : 0u); }
+                            } else if (MH == 1) {
+                                // columns [0, bn): A x B_hi; [bn, 2 bn): A x B_lo and, small as well, the residual x B_hi
 #pragma unroll
-                                        for (int kk = 0; kk < kk_n; ++kk) mma_f16_ts(acc + bn, a_res + 8 * kk, b_hi + 2 * kk, idesc, 1u);
-                                } else {
-                                    // the cross terms (2^-11 of the sum) first, while the accumulator is small
+                                for (int k = 0; k < kk_n; ++k) { const int kk = h * kk_n + k; mma_f16_ts(acc, a_hi + 8 * kk, b_hi + 2 * kk, idesc2, k ? 1u : 0u); }
+                                if (F::residual)
 #pragma unroll
-                                    for (int k = 0; k < kk_n; ++k) {
-                                        const int kk = h * kk_n + k;
-                                        mma_f16_ts(acc, a_hi + 8 * kk, b_lo + 2 * kk, idesc, k ? 1u : 0u);
-                                        if (F::residual) mma_f16_ts(acc, a_res + 8 * kk, b_hi + 2 * kk, idesc, 1u);
-                                    }
+                                    for (int kk = 0; kk < kk_n; ++kk) mma_f16_ts(acc + bn, a_res + 8 * kk, b_hi + 2 * kk, idesc, 1u);
+                            } else {
+                                // the cross terms (2^-11 of the sum) first, while the accumulator is small
 #pragma unroll
-                                    for (int k = 0; k < kk_n; ++k) { const int kk = h * kk_n + k; mma_f16_ts(acc, a_hi + 8 * kk, b_hi + 2 * kk, idesc, 1u); }
+                                for (int k = 0; k < kk_n; ++k) {
+                                    const int kk = h * kk_n + k;
+                                    mma_f16_ts(acc, a_hi + 8 * kk, b_lo + 2 * kk, idesc, k ? 1u : 0u);
+                                    if (F::residual) mma_f16_ts(acc, a_res + 8 * kk, b_hi + 2 * kk, idesc, 1u);
                                 }
-                                // one commit: the sum is complete and, after the last step that reads them, the operand and activation slots are free
-                                mma_commit(&done[step % kDone]);
+#pragma unroll
+                                for (int k = 0; k < kk_n; ++k) { const int kk = h * kk_n + k; mma_f16_ts(acc, a_hi + 8 * kk, b_hi + 2 * kk, idesc, 1u); }
                             }
-                            ++step;
-                            acc_at.next();
+                            // one commit: the sum is complete and, after the last step that reads them, the operand and activation slots are free
+                            mma_commit(&done[step % kDone]);
                         }
-                        a_at.next();
+                        acc_at.skip(h + 1 < kHalves ? 1 : 1 + (kTiles - 1) * kHalves);
                     }
-                    b_at.next();
                 }
+                ks_all = end;
             }
             // nothing may be in flight when tensor memory is freed: the drain warps have waited for every step by then
-        } else if (warp == kMiscFirst + 1 && elect_one()) {
+        } else if (warp == kMiscFirst + kIssuers && elect_one()) {
             // ------------------------------------------------------------ activation copies (the images were written by the kernel before this one)
             asm volatile("griddepcontrol.wait;" ::: "memory");
-            Ring b_at(p.b_slots);
+            Ring b_at(p.b_slots), steps_at(kStepSlots);
             int ks_all = 0;
             bool dead = false;
             while (!dead && walk.next(tile, u0, u1)) {
                 const uint8_t* src = p.xs + (size_t)(tile / p.tiles_m) * p.image_tiles * b_bytes;
                 const int main_slices = 4 * (u1 - u0), extra = kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0;
                 for (int ks = 0; ks < main_slices + extra; ++ks, ++ks_all) {
-                    const int freed = (ks_all - p.b_slots + 1) * MH * kHalves - 1;  // the last step that read the slot
-                    if (ks_all >= p.b_slots && !mbar_wait(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; break; }
+                    if (ks_all >= p.b_slots) {
+                        // the last steps that read the slot, one of each row half (they come from different threads)
+#pragma unroll
+                        for (int m = 0; m < MH && !dead; ++m) {
+                            const int freed = ((ks_all - p.b_slots) * MH + m) * kHalves + kHalves - 1;
+                            if (!mbar_wait(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; }
+                        }
+                        if (dead) break;
+                    }
                     const int image = ks < main_slices ? 4 * u0 + ks : 4 * p.units + (u0 >> 3) + ((ks - main_slices) >> 1);
                     mbar_expect_tx(&b_full[b_at.slot], (uint32_t)b_bytes);
                     bulk_g2s(smem + (size_t)b_at.slot * b_bytes, src + (size_t)image * b_bytes, (uint32_t)b_bytes, &b_full[b_at.slot]);
                     b_at.next();
+                    if (CODES) {
+                        if (ks_all >= kStepSlots && !mbar_wait(&steps_empty[steps_at.slot], steps_at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; break; }
+                        mbar_expect_tx(&steps_full[steps_at.slot], (uint32_t)(8 * bn));
+                        bulk_g2s(&step_ring[steps_at.slot][0][0], p.steps + ((size_t)(tile / p.tiles_m) * p.image_tiles + image) * 2 * bn, (uint32_t)(8 * bn), &steps_full[steps_at.slot]);
+                        steps_at.next();
+                    }
                 }
             }
-        } else if (warp == kMiscFirst + 2 && elect_one()) {
+        } else if (warp == kMiscFirst + kIssuers + 1 && elect_one()) {
             // ------------------------------------------------------------ stored bytes: constants of the model, nothing to wait for before the first fetches
             Ring at(p.raw_slots);
             int n = 0;
@@ -625,42 +748,14 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
     if (warp == kMiscFirst) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
 }
 
-// Adds up the tiles that several CTAs share, in unit order. grid (token lanes, shared tiles): a thread takes one row of a tile and
-// every gridDim.x-th token of it.
-template <int MH>
-__global__ void __launch_bounds__(128 * MH) rq_tc_sum_kernel(const float* __restrict__ partial, int ctas, int first_tile, int rest_tiles, int units, int tiles_m, int bn, int tokens, int64_t rows,
-                                                              float* __restrict__ y, int64_t yn, int64_t yt) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int t = blockIdx.y, tile = first_tile + t, mt = tile % tiles_m, nt = tile / tiles_m;
-    const int64_t total = (int64_t)rest_tiles * units, begin = (int64_t)t * units, end = begin + units;
-    int c0 = (int)(begin * ctas / total);
-    while (c0 > 0 && c0 * total / ctas > begin) --c0;
-    while ((c0 + 1) * total / ctas <= begin) ++c0;
-    if ((c0 + 1) * total / ctas >= end && c0 * total / ctas <= begin) return;  // one CTA had the whole tile and wrote it
-    const int64_t out_row = (int64_t)mt * 128 * MH + threadIdx.x;
-    if (out_row >= rows) return;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int j = blockIdx.x; j < bn && nt * bn + j < tokens; j += gridDim.x) {
-        float s = 0.f;
-        for (int c = c0; c < ctas; ++c) {
-            const int64_t lo = c * total / ctas, hi = (c + 1) * total / ctas;
-            if (lo >= end) break;
-            if (hi <= begin || hi == lo) continue;
-            const int slot = 2 * c + (lo > begin ? 0 : 1);
-            s += __ldcg(partial + ((size_t)slot * bn + j) * 128 * MH + threadIdx.x);
-        }
-        y[out_row * yn + (int64_t)(nt * bn + j) * yt] = s;
-    }
-}
-
-template <int TYPE, int MH>
+template <int TYPE, int MH, bool CODES>
 int launch_tc(const TcParams& p, int ctas, size_t smem, cudaStream_t s) {
-    auto kernel = rq_tc_kernel<TYPE, MH>;
+    auto kernel = rq_tc_kernel<TYPE, MH, CODES>;
     static bool configured[64] = {};
     int dev = 0;
     RQ_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        RQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024));
+        RQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (CODES ? 218 : 225) * 1024));  // 227 KB less the static part
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -677,15 +772,18 @@ int launch_tc(const TcParams& p, int ctas, size_t smem, cudaStream_t s) {
     return RQ_OK;
 }
 template <int TYPE>
-int launch_tc(const TcParams& p, int mh, int ctas, size_t smem, cudaStream_t s) {
-    return mh == 1 ? launch_tc<TYPE, 1>(p, ctas, smem, s) : launch_tc<TYPE, 2>(p, ctas, smem, s);
+int launch_tc(const TcParams& p, int mh, bool codes, int ctas, size_t smem, cudaStream_t s) {
+    if constexpr (!Format<TYPE>::kquant) {
+        if (codes) return mh == 1 ? launch_tc<TYPE, 1, true>(p, ctas, smem, s) : launch_tc<TYPE, 2, true>(p, ctas, smem, s);
+    }
+    return mh == 1 ? launch_tc<TYPE, 1, false>(p, ctas, smem, s) : launch_tc<TYPE, 2, false>(p, ctas, smem, s);
 }
 
 // How a call is cut: row halves and tokens per tile, CTAs, ring depths, shared memory and scratch.
 struct TcCut {
     int mh, bn, n_tiles, tiles_m, units, image_tiles, windows, ctas, whole, rest_tiles;
     int raw_slots, b_slots, a_slots, accs;
-    size_t smem, xs_bytes, partial_bytes;
+    size_t smem, xs_bytes, steps_bytes, partial_bytes;
 };
 struct FormatSizes { int raw_bytes, a_cols, raw_per_unit; };
 FormatSizes format_sizes(int type) {
@@ -696,11 +794,13 @@ FormatSizes format_sizes(int type) {
         default: return {Format<RQ_Q4_0>::raw_bytes, Format<RQ_Q4_0>::a_cols, 1};
     }
 }
-TcCut tc_cut(int type, int sm_count, int64_t rows, int64_t cols, int tokens) {
+TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t cols, int tokens) {
     TcCut c;
     const FormatSizes f = format_sizes(type);
-    c.mh = tokens <= 64 ? 1 : 2;
-    const int widest = 2 * (c.mh == 1 ? Shape<1>::cols : Shape<2>::cols), grain = c.mh == 1 ? 16 : 32;
+    // (fp32 activations over the 32-value formats: two accumulators a slice, of hi and lo columns each, twice; 48 tokens fit)
+    const int widest_1 = !codes && (type == RQ_Q8_0 || type == RQ_Q4_0) ? 48 : Shape<1>::cols;
+    c.mh = tokens <= widest_1 ? 1 : 2;
+    const int widest = c.mh == 1 ? widest_1 : Shape<2>::cols, grain = c.mh == 1 ? 16 : 32;
     c.n_tiles = (tokens + widest - 1) / widest;
     c.bn = ((tokens + c.n_tiles - 1) / c.n_tiles + grain - 1) / grain * grain;
     c.tiles_m = (int)((rows + 128 * c.mh - 1) / (128 * c.mh));
@@ -709,22 +809,35 @@ TcCut tc_cut(int type, int sm_count, int64_t rows, int64_t cols, int tokens) {
     c.image_tiles = 4 * c.units + c.windows;
     const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles, work = tiles * c.units;
     c.ctas = work < sm_count ? (int)work : sm_count;
+    // Few tiles: more CTAs to a tile shorten its products (some two microseconds a unit) and lengthen the last one's sum (most of a
+    // microsecond a piece, a trip to L2 each), so at most about the square root of twice its units share one.
+    int pieces = 1;
+    while ((pieces + 1) * (pieces + 1) <= 2 * c.units) ++pieces;
+    if (tiles * pieces < c.ctas) c.ctas = (int)(tiles * pieces);
     c.whole = (int)(tiles / c.ctas);
     c.rest_tiles = (int)(tiles - (int64_t)c.whole * c.ctas);
-    // tensor memory, 512 columns: operand slots, the rest accumulators
-    c.a_slots = type == RQ_Q6_K ? (c.mh == 1 ? 4 : 2) : 4;
-    const int acc_cols = c.mh == 1 ? 2 * c.bn : c.bn;
-    c.accs = (512 - c.a_slots * f.a_cols) / acc_cols;
+    // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: every ring is as long as
+    // keeps a slot with the same waiters. Accumulators, operand and (MH = 1) activation slots alternate between the two issuing
+    // threads: even numbers of slices. Stored bytes: with MH = 2 a staging group takes every second tile; with MH = 1 the three groups
+    // all read a tile of four slices, but one of two (Q8_0) misses one group in three.
+    // tensor memory, 512 columns: at least four operand slots (Q6_K with MH = 2: two), accumulators, more operand slots
+    const int halves = type == RQ_Q4_K || type == RQ_Q6_K ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn;
+    const int a_least = type == RQ_Q6_K && c.mh == 2 ? 2 : 4;
+    c.accs = (512 - a_least * f.a_cols) / acc_cols / (2 * halves) * (2 * halves);
     if (c.accs > kMaxAcc) c.accs = kMaxAcc;
-    // shared memory: activation slots, then as many slots of stored bytes as fit
-    const int budget = 220 * 1024, b_bytes = c.bn * 256;
-    c.b_slots = c.mh == 1 ? 4 : 3;
+    c.a_slots = (512 - c.accs * acc_cols) / f.a_cols & ~1;
+    if (c.a_slots > kMaxA) c.a_slots = kMaxA;
+    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums)
+    const int joined = c.mh == 1 ? c.bn * 128 * 4 : 0, budget = (codes ? 212 : 220) * 1024 - joined, b_bytes = c.bn * (codes ? 128 : 256);
+    c.b_slots = c.mh == 1 || codes ? 4 : 3;
     c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
-    const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw;
-    if (c.raw_slots > raw_max) c.raw_slots = raw_max;
-    while (c.b_slots < 6 && (c.b_slots + 1) * b_bytes + c.raw_slots * f.raw_bytes <= budget) ++c.b_slots;
-    c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + 1024;
+    const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 ? 2 : (f.raw_per_unit == 2 ? 3 : 1);
+    c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
+    const int b_max = c.mh == 1 ? kMaxB : 6, b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
+    while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
+    c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + joined + 1024;
     c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
+    c.steps_bytes = codes ? (size_t)c.n_tiles * c.image_tiles * 2 * c.bn * 4 : 0;
     c.partial_bytes = c.rest_tiles ? (size_t)2 * c.ctas * c.bn * 128 * c.mh * 4 : 0;
     return c;
 }
@@ -738,30 +851,37 @@ size_t rq_matmul_scratch_bytes(const rq_ctx* ctx, int64_t rows, int64_t cols, in
     const size_t image = (size_t)(tokens + 32 * tiles_n + 32) * 256 * (size_t)(4 * units + (units + 7) / 8);
     const int64_t work = ((rows + 127) / 128) * units * (tiles_n < 1 ? 1 : tiles_n);
     const size_t ctas = (size_t)(work < ctx->sm_count ? work : ctx->sm_count);
-    return image + 256 + 2 * ctas * (tokens > 64 ? 96 * 256 : 64 * 128) * 4;
+    return image + 256 + 4 * ctas + 2 * ctas * (tokens > 64 ? 96 * 256 : 64 * 128) * 4;
 }
 
 // RQ_ERR_UNSUPPORTED (no error text) = not one of the four formats. act_mode FLOAT or INT8 (step 32 / 256).
 int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int act_mode, int step, cudaStream_t s) {
     if (!w->has_tile_map || !rq_type_has_fast_path(w->type)) return RQ_ERR_UNSUPPORTED;
-    const TcCut cut = tc_cut(w->type, ctx->sm_count, w->rows, w->cols, tokens);
-    int rc = rq_ensure_act_scratch(ctx, cut.xs_bytes + cut.partial_bytes, s);
+    const bool codes = act_mode != RQ_ACT_FLOAT && (w->type == RQ_Q8_0 || w->type == RQ_Q4_0);
+    // fp32 activations over an odd number of 32-value blocks stay with the matvec kernel, as they were: it has no fp16 range to keep to
+    if (!codes && w->cols % BK) return RQ_ERR_UNSUPPORTED;
+    const TcCut cut = tc_cut(w->type, codes, ctx->sm_count, w->rows, w->cols, tokens);
+    int rc = rq_ensure_act_scratch(ctx, cut.xs_bytes + cut.steps_bytes + cut.partial_bytes + (size_t)cut.rest_tiles * 4, s);
     if (rc) return rc;
     ctx->act_cols = 0;  // whatever int8 records the scratch held for INT8_CACHED calls are gone
     uint8_t* xs = ctx->act_scratch;
+    float* partial = (float*)(xs + cut.xs_bytes + cut.steps_bytes);
+    int* arrived = (int*)((uint8_t*)partial + cut.partial_bytes);
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     {
         const int padded = cut.n_tiles * cut.bn;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)cut.units, (unsigned)((padded + 7) / 8));
+        cfg.gridDim = dim3((unsigned)cut.units, (unsigned)(padded / 8));
         cfg.blockDim = dim3(256);
         cfg.stream = s;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        auto prep = act_mode == RQ_ACT_FLOAT ? rq_tc_prep_kernel<0> : (step == 256 ? rq_tc_prep_kernel<256> : rq_tc_prep_kernel<32>);
-        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, cut.bn, padded, cut.image_tiles, cut.windows, xs));
+        auto prep = act_mode == RQ_ACT_FLOAT ? rq_tc_prep_kernel<0, false>
+                                             : (codes ? (step == 256 ? rq_tc_prep_kernel<256, true> : rq_tc_prep_kernel<32, true>)
+                                                      : (step == 256 ? rq_tc_prep_kernel<256, false> : rq_tc_prep_kernel<32, false>));
+        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, cut.bn, cut.image_tiles, cut.windows, xs, (float*)(xs + cut.xs_bytes), arrived, cut.rest_tiles));
     }
     TcParams p;
     p.tile_map = w->tile_map;
@@ -769,24 +889,15 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
     p.blocks32 = (int)(w->cols / 32); p.units = cut.units; p.permuted = rq_plane_permuted(w->type, w->cols) ? 1 : 0;
     p.xs = xs; p.image_tiles = cut.image_tiles; p.bn = cut.bn; p.tokens = tokens; p.y = y; p.yn = yn; p.yt = yt;
     p.tiles_m = cut.tiles_m; p.whole = cut.whole; p.rest_tiles = cut.rest_tiles;
-    p.partial = (float*)(xs + cut.xs_bytes);
+    p.steps = (const float*)(xs + cut.xs_bytes);
+    p.partial = partial; p.arrived = arrived;
     p.raw_slots = cut.raw_slots; p.b_slots = cut.b_slots; p.a_slots = cut.a_slots; p.accs = cut.accs;
     p.error_flag = ctx->error_flag; p.wait_ns = ctx->wait_limit_ns;
     switch (w->type) {
-        case RQ_Q4_K: rc = launch_tc<RQ_Q4_K>(p, cut.mh, cut.ctas, cut.smem, s); break;
-        case RQ_Q6_K: rc = launch_tc<RQ_Q6_K>(p, cut.mh, cut.ctas, cut.smem, s); break;
-        case RQ_Q8_0: rc = launch_tc<RQ_Q8_0>(p, cut.mh, cut.ctas, cut.smem, s); break;
-        default: rc = launch_tc<RQ_Q4_0>(p, cut.mh, cut.ctas, cut.smem, s); break;
+        case RQ_Q4_K: rc = launch_tc<RQ_Q4_K>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;
+        case RQ_Q6_K: rc = launch_tc<RQ_Q6_K>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;
+        case RQ_Q8_0: rc = launch_tc<RQ_Q8_0>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;
+        default: rc = launch_tc<RQ_Q4_0>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;
     }
-    if (rc || !cut.rest_tiles) return rc;
-    cudaLaunchConfig_t cfg = {};
-    const int lanes = cut.bn < 32 ? cut.bn : 32;
-    cfg.gridDim = dim3((unsigned)lanes, (unsigned)cut.rest_tiles);
-    cfg.blockDim = dim3((unsigned)(128 * cut.mh));
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    RQ_CUDA(cudaLaunchKernelEx(&cfg, cut.mh == 1 ? rq_tc_sum_kernel<1> : rq_tc_sum_kernel<2>, (const float*)p.partial, cut.ctas, cut.whole * cut.ctas, cut.rest_tiles, cut.units, cut.tiles_m,
-                               cut.bn, tokens, w->rows, y, yn, yt));
-    return RQ_OK;
+    return rc;
 }

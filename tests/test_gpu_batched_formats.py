@@ -9,7 +9,7 @@ from tests.test_gpu_parity import rel_err, torch_cuda
 pytestmark = pytest.mark.gpu
 
 SHAPES = [  # rows, cols, tokens
-    (1, 256, 12), (129, 512, 64), (257, 512, 65), (255, 1024, 96), (300, 768, 97), (520, 2304, 193), (40, 14336, 16), (4000, 256, 13), (9500, 512, 200),
+    (1, 256, 12), (129, 512, 64), (257, 512, 65), (255, 1024, 96), (300, 768, 97), (520, 2304, 193), (40, 14336, 16), (4000, 256, 13), (9500, 512, 200), (3879, 4352, 63), (2900, 2816, 33), (5000, 1792, 90),
 ]
 RAGGED = [(130, 32, 12), (200, 96, 70), (65, 1120, 31), (300, 2592, 100)]  # 32-value formats only
 
