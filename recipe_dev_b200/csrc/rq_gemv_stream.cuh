@@ -1722,7 +1722,7 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     if (vectors_per_launch > 0) {
         p.act_vectors = vectors_per_launch;  // expert banks: one token, a vector per slot
     } else {
-        t = token_pairs ? 2 : ((p.tokens >= 2 && 4 * p.act_bytes <= 40 * 1024) ? 4 : 1);
+        t = token_pairs ? 2 : ((p.tokens >= 2 && 4 * p.act_bytes <= (one_per_sm ? 80 : 40) * 1024) ? 4 : 1);
         p.act_vectors = t;
         // four int8 tokens are staged interleaved, kRecord4 bytes per unit: a quarter of that per vector
         if (MODE == RQ_ACT_INT8 && t == 4) p.act_bytes = ((size_t)p.units * (kRecord4 / 4) + 127) & ~(size_t)127;
@@ -1840,6 +1840,15 @@ int dispatch_stream(StreamParams& p, int sm_count, int vectors_per_launch, cudaS
                 const int rc = dispatch_stream_nw<TYPE, MODE, 5>(p, sm_count, vectors_per_launch, s, false, true);
                 if (rc != RQ_ERR_UNSUPPORTED) return rc;
             }
+        }
+    }
+    if constexpr (MODE == RQ_ACT_INT8) {
+        // a window of positions over long rows (14336 inputs): four tokens' records are 76 KB, which leaves room for a ring only with
+        // one CTA on the SM; still one pass over the weights where the tokens would take one each
+        const int64_t records = 4 * (int64_t)p.units * RQ_ACT_RECORD_INT8;
+        if (p.tokens > 2 && vectors_per_launch == 0 && p.subs == 1 && !p.fuse_step && records > 40 * 1024 && records <= 80 * 1024) {
+            const int rc = dispatch_stream_nw<TYPE, MODE, 7>(p, sm_count, vectors_per_launch, s, true);
+            if (rc != RQ_ERR_UNSUPPORTED) return rc;
         }
     }
     int rc = dispatch_stream_nw<TYPE, MODE, 7>(p, sm_count, vectors_per_launch, s);
