@@ -165,7 +165,8 @@ def _stream(stream) -> int:
     if stream is None:
         import torch
 
-        return torch.cuda.current_stream().cuda_stream
+        # the current stream's handle without a Stream object around it (a microsecond, as long as a short launch takes to enqueue)
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     return stream if isinstance(stream, int) else stream.cuda_stream
 
 
@@ -348,16 +349,18 @@ class Context:
     # ---- matvec ----
     def matvec(self, w: Weight, x, y=None, act_mode: int = ACT_FLOAT, step: int = 32, stream=None):
         """x: CUDA fp32, [cols] or [tokens, cols] (token-major) -> y [rows] or [tokens, rows]."""
-        import torch
-
         single = x.dim() == 1
         x2 = x.unsqueeze(0) if single else x
-        tokens, cols = x2.shape
+        tokens, _ = x2.shape
         if y is None:
+            import torch
+
             y = torch.empty((tokens, w.rows), dtype=torch.float32, device=x.device)
         y2 = y.unsqueeze(0) if y.dim() == 1 else y
-        _check(self.lib.rq_matvec(self.handle, w.handle, _ptr(x2), x2.stride(1), x2.stride(0), tokens,
-                                  _ptr(y2), y2.stride(1), y2.stride(0), act_mode, step, _stream(stream)))
+        (xt, xk), (yt, yn) = x2.stride(), y2.stride()
+        status = self.lib.rq_matvec(self.handle, w.handle, x2.data_ptr(), xk, xt, tokens, y2.data_ptr(), yn, yt, act_mode, step, _stream(stream))
+        if status:
+            _check(status)
         return y2[0] if single else y2
 
     def matvec_glu(self, gate: Weight, up: Weight, x, y=None, act_mode: int = ACT_FLOAT, step: int = 32, stream=None):
