@@ -318,6 +318,15 @@ __device__ __forceinline__ void tmem_ld16_pair(uint32_t a, uint32_t b, uint32_t 
         : "memory");
 }
 
+// Two fp32 numbers an instruction (the same roundings): the drain warps' arithmetic is half the instructions.
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair pair_of(uint32_t a, uint32_t b) { Pair v; asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(a), "r"(b)); return v; }
+__device__ __forceinline__ Pair pair_of(float a, float b) { return pair_of(__float_as_uint(a), __float_as_uint(b)); }
+__device__ __forceinline__ Pair pair_fma(Pair a, Pair b, Pair c) { Pair v; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c)); return v; }
+__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) { Pair v; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b)); return v; }
+__device__ __forceinline__ Pair pair_add(Pair a, Pair b) { Pair v; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b)); return v; }
+__device__ __forceinline__ float pair_at(Pair v, int i) { uint32_t a, b; asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v)); return __uint_as_float(i ? b : a); }
+
 // A ring position: slot index and the parity of its current use. (Kept by counting: a division by a ring's length, known at run time
 // only, is some thirty instructions.)
 struct Ring {
@@ -389,9 +398,9 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
         while (walk.next(tile, u0, u1)) {
             const int mt = tile % p.tiles_m, nt = tile / p.tiles_m;
             const int64_t my_row0 = (int64_t)(mt * MH + (MH == 2 ? set : 0)) * 128;
-            float sum[kCols];
+            Pair sum[kCols / 2];
 #pragma unroll
-            for (int i = 0; i < kCols; ++i) sum[i] = 0.f;
+            for (int i = 0; i < kCols / 2; ++i) sum[i] = 0;
             // this lane's row, kept inside the weight for the scale loads
             auto row_at = [&]() -> int64_t { return min(my_row0 + quarter * 32 + lane, p.rows - 1); };
             // Slice ks of the segment: d0 (and d1: the second half's) scale its sums
@@ -400,6 +409,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                 if (!dead && !mbar_wait_warp(&done[last % kDone], (last / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 14); dead = true; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc0 = tmem_base + lane_base + (uint32_t)(acc_at.slot * acc_cols), acc1 = acc0 + (uint32_t)((kHalves - 1) * acc_cols);  // (an even number of accumulators: a slice's two are neighbours)
+                const Pair scale0 = pair_of(d0, d0), scale1 = pair_of(d1, d1);
                 if constexpr (CODES) {
                     const int slot = all % kStepSlots;
                     if (!dead && !mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
@@ -412,10 +422,13 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
 #pragma unroll
                             for (int j = 0; j < 16; j += 4) {
                                 const float4 s4 = *(const float4*)(d8 + c + j), r4 = *(const float4*)(e8 + c + j);
-                                const float sv[4] = {s4.x, s4.y, s4.z, s4.w}, rv[4] = {r4.x, r4.y, r4.z, r4.w};
+                                const Pair sv[2] = {pair_of(s4.x, s4.y), pair_of(s4.z, s4.w)}, rv[2] = {pair_of(r4.x, r4.y), pair_of(r4.z, r4.w)};
 #pragma unroll
-                                for (int q = 0; q < 4; ++q)
-                                    sum[c + j + q] += fmaf(__fmul_rn(rv[q], d1), __uint_as_float(u[j + q]), __fmul_rn(__fmul_rn(sv[q], d0), __uint_as_float(t[j + q])));
+                                for (int q = 0; q < 2; ++q) {
+                                    const Pair even = pair_mul(pair_mul(sv[q], scale0), pair_of(t[j + 2 * q], t[j + 2 * q + 1]));
+                                    Pair& to = sum[(c + j) / 2 + q];
+                                    to = pair_add(to, pair_fma(pair_mul(rv[q], scale1), pair_of(u[j + 2 * q], u[j + 2 * q + 1]), even));
+                                }
                             }
                         }
                     }
@@ -425,19 +438,20 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
 #pragma unroll
                     for (int h = 0; h < kHalves; ++h) {
                         const uint32_t at = h ? acc1 : acc0;
-                        const float d = h ? d1 : d0;
+                        const Pair d = h ? scale1 : scale0;
 #pragma unroll
                         for (int c = 0; c < kCols; c += MH == 1 ? 16 : 32) {
                             if (c < bn) {
                                 uint32_t t[16], u[16];
                                 tmem_ld16_pair(at + c, at + (MH == 1 ? bn + c : c + 16), t, u);  // MH = 1: hi and lo of a token; else the next sixteen tokens
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) {
+                                for (int j = 0; j < 16; j += 2) {
+                                    const Pair a = pair_of(t[j], t[j + 1]), b = pair_of(u[j], u[j + 1]);
                                     if (MH == 1) {
-                                        sum[c + j] = fmaf(d, __uint_as_float(t[j]) + __uint_as_float(u[j]), sum[c + j]);
+                                        sum[(c + j) / 2] = pair_fma(d, pair_add(a, b), sum[(c + j) / 2]);
                                     } else {
-                                        sum[c + j] = fmaf(d, __uint_as_float(t[j]), sum[c + j]);
-                                        sum[c + 16 + j] = fmaf(d, __uint_as_float(u[j]), sum[c + 16 + j]);
+                                        sum[(c + j) / 2] = pair_fma(d, a, sum[(c + j) / 2]);
+                                        sum[(c + 16 + j) / 2] = pair_fma(d, b, sum[(c + 16 + j) / 2]);
                                     }
                                 }
                             }
@@ -494,13 +508,13 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                 if (set == 1) {
 #pragma unroll
                     for (int j = 0; j < kCols; ++j)
-                        if (j < bn) joined[j * 128 + r0] = sum[j];
+                        if (j < bn) joined[j * 128 + r0] = pair_at(sum[j / 2], j & 1);
                 }
                 asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
                 if (set == 0) {
 #pragma unroll
-                    for (int j = 0; j < kCols; ++j)
-                        if (j < bn) sum[j] += joined[j * 128 + r0];
+                    for (int j = 0; j < kCols; j += 2)
+                        if (j < bn) sum[j / 2] = pair_add(sum[j / 2], pair_of(joined[j * 128 + r0], joined[(j + 1) * 128 + r0]));
                 }
                 asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
                 if (set == 1) continue;
@@ -512,7 +526,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                 float* at = p.y + (my_row0 + r0) * p.yn + (int64_t)(nt * bn) * p.yt;
 #pragma unroll
                 for (int j = 0; j < kCols; ++j) {
-                    if (j < live_tokens) *at = sum[j];
+                    if (j < live_tokens) *at = pair_at(sum[j / 2], j & 1);
                     at += p.yt;
                 }
             };
@@ -523,7 +537,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                 float* part = p.partial + (size_t)(2 * blockIdx.x + (u0 == 0 ? 1 : 0)) * tile_floats + mine;
 #pragma unroll
                 for (int j = 0; j < kCols; ++j)
-                    if (j < live_tokens) part[j * 128 * MH] = sum[j];
+                    if (j < live_tokens) part[j * 128 * MH] = pair_at(sum[j / 2], j & 1);
                 // the CTAs that share this tile, in unit order: c0, c0 + 1, .. while their ranges reach into it
                 const int t = tile - p.whole * (int)gridDim.x;
                 // (fewer than 148 tiles of at most 65536 units among 148 CTAs: the products fit 32 bits)
@@ -544,7 +558,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                 if (last_piece) {
                     __threadfence();
 #pragma unroll
-                    for (int j = 0; j < kCols; ++j) sum[j] = 0.f;
+                    for (int j = 0; j < kCols / 2; ++j) sum[j] = 0;
                     for (int c = c0; c <= c1; ++c) {
                         const float* piece = p.partial + (size_t)(2 * c + (range_begin(c) > begin ? 0 : 1)) * tile_floats + mine;
                         // sixteen loads in flight (a branch for each would make each wait for the one before); the padding
@@ -556,7 +570,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
 #pragma unroll
                                 for (int q = 0; q < 16; ++q) v[q] = __ldcg(piece + (j + q) * 128 * MH);
 #pragma unroll
-                                for (int q = 0; q < 16; ++q) sum[j + q] += v[q];
+                                for (int q = 0; q < 16; q += 2) sum[(j + q) / 2] = pair_add(sum[(j + q) / 2], pair_of(v[q], v[q + 1]));
                             }
                         }
                     }
