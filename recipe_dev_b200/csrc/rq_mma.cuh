@@ -35,14 +35,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
     }
     return true;
 }
-// A whole warp waits, one lane looks: every look at a barrier is an operation on its shared-memory word, and thirty-two lanes
-// looking at once cost thirty-two of them (measured: some 300 cycles for a warp-wide look at a barrier that is already
-// complete). Lane 0 waits, the warp meets it at __syncwarp (which also orders memory between the lanes) and learns the outcome.
+// A whole warp waits: all lanes look together and agree (the vote also brings the warp back together for the warp-wide
+// instructions that follow). A look by lane 0 alone, with a __syncwarp and a shuffle to tell the others, made the batched kernel 10 to 17 %
+// slower: 512 tokens 218 against 193 us, 16 tokens 36.9 against 33.1 us.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned long long limit_ns) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, limit_ns) ? 1 : 0;
-    __syncwarp();
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns));
 }
 // True in one lane of a converged warp. The compiler knows that the code behind it runs in a single thread, so the operands of the
 // instructions that take uniform registers (tcgen05.mma, commits, copies) stay there.
