@@ -1361,6 +1361,30 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
         auto reduce_rows = [&](const float* part, const RqSegment& sg, int nr, int64_t lr0, int first, int sweep) {
             const int l8 = lane & 7;
             const int tasks = nr * T;
+            if (T == 1 && p.epilogue == RQ_EPI_WSUM && p.units <= 8) {
+                // Short sub-rows (an expert bank's down rows): a lane takes a whole sub-row, eight sub-rows at a time, where eight lanes
+                // on one sub-row after another are a chain of shuffles per sub-row. The additions are the same ones, in the same order.
+                for (int base = 0; base < tasks; base += sweep) {
+                    const int lr = base + first;
+                    const bool live = lr < tasks;
+                    float out = 0.f;
+                    for (int s0 = 0; s0 < subs; s0 += 8) {
+                        const float* lo = part + (s0 + l8) * su_cap + (live ? lr : 0) * p.units;
+                        const float* hi = lo + p.subs * su_cap;
+                        float w8[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) w8[j] = live && s0 + l8 < subs && j < p.units ? lo[j] + hi[j] : 0.f;
+                        const float sum = ((w8[0] + w8[4]) + (w8[2] + w8[6])) + ((w8[1] + w8[5]) + (w8[3] + w8[7]));
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            const float of_q = __shfl_sync(0xffffffffu, sum, (lane & 24) | q);
+                            if (s0 + q < subs) out = fmaf(of_q, sg.coef[s0 + q], out);
+                        }
+                    }
+                    if (live && l8 == 0) sg.y[(lr0 + lr) * p.yn + (int64_t)tok0 * p.yt] = out;
+                }
+                return;
+            }
             for (int base = 0; base < tasks; base += sweep) {  // uniform trip count: every lane takes part in the shuffles
                 const int task = base + first;
                 const bool live = task < tasks && tok0 + (task % T) < p.tokens;
