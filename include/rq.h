@@ -184,8 +184,8 @@ int rq_softcap(rq_ctx* ctx, const float* x, int64_t n, double cap, float* y, voi
 /* The batched product (prefill, multi-sequence decode): the same contraction as rq_matvec for many
  * tokens, on the tensor cores (tcgen05.mma, fp32 accumulation in tensor memory) for Q4_K / Q6_K / Q8_0 /
  * Q4_0 weights: exact-integer weight operands, activations as fp16 hi + lo pairs, for RQ_ACT_FLOAT and for
- * RQ_ACT_INT8 windows of twelve and more positions (K-quants: the product over the records' code * step;
- * Q8_0 / Q4_0: exact integer dots of the codes, scaled per 32 inputs). Everything else (shorter int8 windows,
+ * longer RQ_ACT_INT8 windows (K-quants, from twelve positions: the product over the records' code * step;
+ * Q8_0 / Q4_0, from nine, or five above 7680 inputs: exact integer dots of the codes, scaled per 32 inputs). Everything else (shorter int8 windows,
  * the decode-only formats) runs the matvec kernels. Replaces contraction_forward_body's
  * position loop and contraction_forward_gemm_body (amd-nv-cpu.ll:1231-2241, :3509-3649). Same
  * arguments as rq_matvec.

@@ -436,9 +436,13 @@ extern "C" int rq_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_
     if (rc) return rc;
     if (sk <= 0 || yn <= 0 || (tokens > 1 && (st <= 0 || yt <= 0))) return rq_fail(RQ_ERR_INVALID, "rq_matmul: strides must be positive");
     DeviceGuard guard(ctx->device);
-    // the tensor-core kernel, for fp32 activations and for int8 windows of twelve and more positions (below that the matvec kernel's
-    // exact integer dots, four tokens a pass, are faster)
-    if (act_mode == RQ_ACT_FLOAT || (act_mode == RQ_ACT_INT8 && tokens >= 12)) {
+    // The tensor-core kernel, for fp32 activations and for int8 windows from some length on: below it the matvec kernel's integer dots,
+    // four tokens a pass, are faster. Q8_0 / Q4_0: nine positions, a third pass (Q8_0 14336 x 4096, ten: 50.8 us there, 39.1 here; eight:
+    // 35.8 there); five where a pass takes an SM per CTA (more than 7680 inputs). The K-quants stay at twelve (Q4_K 14336 x
+    // 4096, ten: 46.4 there, 33.9 here): below that their products keep clear of fp16's range, as they always have.
+    const bool codes = w->type == RQ_Q8_0 || w->type == RQ_Q4_0;
+    const int from = !codes ? 12 : (w->cols > 7680 ? 5 : 9);
+    if (act_mode == RQ_ACT_FLOAT || (act_mode == RQ_ACT_INT8 && tokens >= from)) {
         rc = rq_launch_matmul(ctx, w, x, sk, st, tokens, y, yn, yt, act_mode, step, (cudaStream_t)stream);
         if (rc != RQ_ERR_UNSUPPORTED) return rc;
     }
