@@ -1785,7 +1785,8 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     int layout_group = 0, layout_chunks = 1;
     row_layout(2 * p.units, &layout_group, &layout_chunks);
     const bool split_shape = layout_chunks > 1 && layout_chunks == NW;
-    if (warp_shape && layout_group) { p.sum_group = layout_group; p.sum_chunks = layout_chunks; }
+    // (gated pairs over rows of five warps, which these seven do not split, run partial sums whatever the window: eight lanes a row there)
+    if (warp_shape && layout_group && (!gated_shape || layout_chunks == 1 || split_shape)) { p.sum_group = layout_group; p.sum_chunks = layout_chunks; }
     if (warp_launch && layout_group && layout_chunks == 1) {
         const int group = layout_group;
         p.warp_rows = 32 / group;
