@@ -1,0 +1,146 @@
+// How a batched product is cut: row halves and tokens per tile, CTAs, ring depths, shared memory and scratch, and the deal of the tiles
+// that several CTAs share. Arithmetic only and no CUDA in it, so that a host test can walk the work of a call over many shapes.
+#pragma once
+#include <stddef.h>
+#include <stdint.h>
+
+#include "rq.h"
+
+#ifdef __CUDACC__
+#define RQ_HOST_DEVICE __host__ __device__ __forceinline__
+#else
+#define RQ_HOST_DEVICE inline
+#endif
+
+namespace rqcut {
+
+constexpr int kMaxRaw = 8, kMaxB = 12, kMaxA = 8, kMaxAcc = 8;
+
+// groups: staging groups; cols: tokens per tile at most, the sums a drain thread holds; registers of the drain, staging and other
+// warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 768 x 80, 640 x 96)
+template <int MH> struct Shape;
+template <> struct Shape<1> { static constexpr int groups = 3, cols = 64, drain_regs = 120, stage_regs = 64, other_regs = 48, launch_regs = 80; };
+template <> struct Shape<2> { static constexpr int groups = 2, cols = 96, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
+
+template <int TYPE> struct Format {
+    static constexpr bool kquant = TYPE == RQ_Q4_K || TYPE == RQ_Q6_K;
+    static constexpr bool residual = TYPE == RQ_Q6_K;            // a second operand tile
+    static constexpr int halves = kquant ? 1 : 2;                // sums that leave tensor memory per 64-wide slice
+    static constexpr int box_bytes = TYPE == RQ_Q4_K ? 144 : (TYPE == RQ_Q6_K ? 208 : 128);  // stored bytes of a row in one TMA tile
+    static constexpr int raw_slices = TYPE == RQ_Q8_0 ? 2 : 4;   // slices in one TMA tile
+    static constexpr int raw_bytes = 128 * box_bytes;
+    static constexpr int a_cols = residual ? 64 : 32;            // tensor-memory columns of an operand slot
+};
+
+// The deal of the shared tiles: their units, numbered tile after tile, are cut into `share` ranges of equal length (to one unit), CTA c
+// of the launch takes range c and the CTAs from `share` on take none. No range is empty (share <= the units) and none is longer
+// than a tile, so the pieces of a tile are exactly the ranges first(t) .. last(t), and a CTA has at most two pieces: the end of one
+// tile and the start of the next. (Fewer than 148 tiles of at most 65536 units among 148 CTAs: the products fit 32 bits.)
+struct Deal {
+    uint32_t total;
+    int share, units;
+    RQ_HOST_DEVICE Deal(int share_, int rest_tiles, int units_) : total((uint32_t)rest_tiles * (uint32_t)units_), share(share_), units(units_) {}
+    RQ_HOST_DEVICE uint32_t begin(int c) const { return (uint32_t)c * total / (uint32_t)share; }
+    RQ_HOST_DEVICE int first(int t) const {
+        const uint32_t at = (uint32_t)t * (uint32_t)units;
+        int c = (int)(at * (uint32_t)share / total);
+        while (c > 0 && begin(c) > at) --c;
+        while (begin(c + 1) <= at) ++c;
+        return c;
+    }
+    RQ_HOST_DEVICE int last(int t, int c) const {  // c: a CTA that has a piece of the tile
+        const uint32_t end = (uint32_t)(t + 1) * (uint32_t)units;
+        while (c + 1 < share && begin(c + 1) < end) ++c;
+        return c;
+    }
+    // where CTA c leaves its sums of tile t: its first or its second place
+    RQ_HOST_DEVICE int place(int t, int c) const { return 2 * c + (begin(c) > (uint32_t)t * (uint32_t)units ? 0 : 1); }
+};
+
+// The tiles and unit ranges of one CTA, in the order every role walks them.
+struct Walk {
+    const int whole, units, ctas, cta;
+    int i, at, end;  // whole tiles taken; position among the shared units
+    RQ_HOST_DEVICE Walk(int whole_, int rest_tiles, int units_, int share, int ctas_, int cta_) : whole(whole_), units(units_), ctas(ctas_), cta(cta_), i(0), at(0), end(0) {
+        if (cta < share) {
+            const Deal deal(share, rest_tiles, units);
+            at = (int)deal.begin(cta);
+            end = (int)deal.begin(cta + 1);
+        }
+    }
+    RQ_HOST_DEVICE bool next(int& tile, int& u0, int& u1) {
+        if (i < whole) { tile = i * ctas + cta; u0 = 0; u1 = units; ++i; return true; }
+        if (at >= end) return false;
+        const int t = at / units;
+        tile = whole * ctas + t;
+        u0 = at - t * units;
+        u1 = units < u0 + end - at ? units : u0 + end - at;
+        at += u1 - u0;
+        return true;
+    }
+};
+
+struct TcCut {
+    int mh, bn, n_tiles, tiles_m, units, image_tiles, windows, ctas, whole, rest_tiles, share;
+    int raw_slots, b_slots, a_slots, accs;
+    size_t smem, xs_bytes, steps_bytes, partial_bytes;
+};
+struct FormatSizes { int raw_bytes, a_cols, raw_per_unit; };
+inline FormatSizes format_sizes(int type) {
+    switch (type) {
+        case RQ_Q4_K: return {Format<RQ_Q4_K>::raw_bytes, Format<RQ_Q4_K>::a_cols, 1};
+        case RQ_Q6_K: return {Format<RQ_Q6_K>::raw_bytes, Format<RQ_Q6_K>::a_cols, 1};
+        case RQ_Q8_0: return {Format<RQ_Q8_0>::raw_bytes, Format<RQ_Q8_0>::a_cols, 2};
+        default: return {Format<RQ_Q4_0>::raw_bytes, Format<RQ_Q4_0>::a_cols, 1};
+    }
+}
+inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t cols, int tokens) {
+    TcCut c;
+    const FormatSizes f = format_sizes(type);
+    // (fp32 activations over the 32-value formats: two accumulators a slice, of hi and lo columns each, twice; 48 tokens fit)
+    const int widest_1 = !codes && (type == RQ_Q8_0 || type == RQ_Q4_0) ? 48 : Shape<1>::cols;
+    c.mh = tokens <= widest_1 ? 1 : 2;
+    const int widest = c.mh == 1 ? widest_1 : Shape<2>::cols, grain = c.mh == 1 ? 16 : 32;
+    c.n_tiles = (tokens + widest - 1) / widest;
+    c.bn = ((tokens + c.n_tiles - 1) / c.n_tiles + grain - 1) / grain * grain;
+    c.tiles_m = (int)((rows + 128 * c.mh - 1) / (128 * c.mh));
+    c.units = (int)((cols + 255) / 256);
+    c.windows = type == RQ_Q4_K ? (c.units + 7) / 8 : 0;
+    c.image_tiles = 4 * c.units + c.windows;
+    const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles, work = tiles * c.units;
+    c.ctas = work < sm_count ? (int)work : sm_count;
+    // Few tiles to share: more CTAs to a tile shorten its products (some two microseconds a unit) and lengthen the last one's sum (most of
+    // a microsecond a piece, a trip to L2 each), so about the square root of twice its units share one, at most (never more than it has).
+    int pieces = 1;
+    while ((pieces + 1) * (pieces + 1) <= 2 * c.units) ++pieces;
+    if (tiles * pieces < c.ctas) c.ctas = (int)(tiles * pieces);
+    c.whole = (int)(tiles / c.ctas);
+    c.rest_tiles = (int)(tiles - (int64_t)c.whole * c.ctas);
+    c.share = (int64_t)c.rest_tiles * pieces < c.ctas ? c.rest_tiles * pieces : c.ctas;
+    // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: every ring is as long as
+    // keeps a slot with the same waiters. Accumulators, operand and (MH = 1) activation slots alternate between the two issuing
+    // threads: even numbers of slices. Stored bytes: with MH = 2 a staging group takes every second tile; with MH = 1 the three groups
+    // all read a tile of four slices, but one of two (Q8_0) misses one group in three.
+    // tensor memory, 512 columns: at least four operand slots (Q6_K with MH = 2: two), accumulators, more operand slots
+    const int halves = type == RQ_Q4_K || type == RQ_Q6_K ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn;
+    const int a_least = type == RQ_Q6_K && c.mh == 2 ? 2 : 4;
+    c.accs = (512 - a_least * f.a_cols) / acc_cols / (2 * halves) * (2 * halves);
+    if (c.accs > kMaxAcc) c.accs = kMaxAcc;
+    c.a_slots = (512 - c.accs * acc_cols) / f.a_cols & ~1;
+    if (c.a_slots > kMaxA) c.a_slots = kMaxA;
+    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums)
+    const int joined = c.mh == 1 ? c.bn * 128 * 4 : 0, budget = (codes ? 212 : 220) * 1024 - joined, b_bytes = c.bn * (codes ? 128 : 256);
+    c.b_slots = c.mh == 1 || codes ? 4 : 3;
+    c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
+    const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 ? 2 : (f.raw_per_unit == 2 ? 3 : 1);
+    c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
+    const int b_max = c.mh == 1 ? kMaxB : 6, b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
+    while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
+    c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + joined + 1024;
+    c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
+    c.steps_bytes = codes ? (size_t)c.n_tiles * c.image_tiles * 2 * c.bn * 4 : 0;
+    c.partial_bytes = (size_t)2 * c.share * c.bn * 128 * c.mh * 4;
+    return c;
+}
+
+}  // namespace rqcut

@@ -15,8 +15,8 @@
 // the matvec kernel's arithmetic, and no fp16 range to stay in.
 //
 // One CTA per SM, persistent. Work is counted in UNITS, 256 inputs of one row tile (128 * MH rows) x one token tile: every CTA
-// takes the same number of whole tiles and then an equal share of the units that are left, whatever tile they fall in; a tile
-// that is shared by several CTAs is added up, in unit order, by whichever of them is the last to leave its sums (the same bits on
+// takes the same number of whole tiles and then an equal share of the units that are left, whatever tile they fall in (where few are
+// left, only so many CTAs as a tile is worth cutting for: rq_matmul_cut.cuh); a tile that is shared by several CTAs is added up, in unit order, by whichever of them is the last to leave its sums (the same bits on
 // every run; a kernel of its own would be one more launch in the chain). Roles in a CTA:
 //   * raw copies: one TMA tile of 128 rows x one unit of stored bytes at a time (Q8_0: half a unit) into a ring;
 //   * activation copies: one bulk copy per 64-wide slice, B_hi | B_lo of the token tile, into a ring;
@@ -51,34 +51,20 @@
 // Every wait is bounded; a wait that runs out records a code in the context's error word, the thread stops waiting and the CTA
 // still frees its tensor memory before it exits.
 #include "rq_internal.cuh"
+#include "rq_matmul_cut.cuh"
 #include "rq_mma.cuh"
 
 using namespace rqmma;
+using namespace rqcut;
 
 namespace {
 
 constexpr int kDrainWarps = 8;
 constexpr int kDone = 32;                    // ring of "step finished" barriers, indexed by the step (see the kernel)
-constexpr int kMaxRaw = 8, kMaxB = 12, kMaxA = 8, kMaxAcc = 8;
 constexpr float kMinScale = 256.0f, kMinUnscale = 1.0f / 256.0f;  // the minimum term's weights are scaled so that their fp16 residuals are no subnormals
 
-// groups: staging groups; cols: tokens per tile at most, the sums a drain thread holds; registers of the drain, staging and other
-// warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 768 x 80, 640 x 96)
-template <int MH> struct Shape;
-template <> struct Shape<1> { static constexpr int groups = 3, cols = 64, drain_regs = 120, stage_regs = 64, other_regs = 48, launch_regs = 80; };
-template <> struct Shape<2> { static constexpr int groups = 2, cols = 96, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
 constexpr int kIssuers = 2;                  // with the two copying warps: one warpgroup
 template <int MH> __host__ __device__ constexpr int tc_threads() { return (kDrainWarps + 4 * Shape<MH>::groups + 4) * 32; }
-
-template <int TYPE> struct Format {
-    static constexpr bool kquant = TYPE == RQ_Q4_K || TYPE == RQ_Q6_K;
-    static constexpr bool residual = TYPE == RQ_Q6_K;            // a second operand tile
-    static constexpr int halves = kquant ? 1 : 2;                // sums that leave tensor memory per 64-wide slice
-    static constexpr int box_bytes = TYPE == RQ_Q4_K ? 144 : (TYPE == RQ_Q6_K ? 208 : 128);  // stored bytes of a row in one TMA tile
-    static constexpr int raw_slices = TYPE == RQ_Q8_0 ? 2 : 4;   // slices in one TMA tile
-    static constexpr int raw_bytes = 128 * box_bytes;
-    static constexpr int a_cols = residual ? 64 : 32;            // tensor-memory columns of an operand slot
-};
 
 struct TcParams {
     CUtensorMap tile_map;  // the weight's main plane as a [rows][row bytes] byte matrix (TMA descriptor; first: 64-byte aligned)
@@ -93,33 +79,12 @@ struct TcParams {
     int image_tiles;       // 4 * units, then one per window of eight superblocks (Q4_K)
     int bn, tokens;
     float* y; int64_t yn, yt;
-    int tiles_m, whole, rest_tiles;  // row tiles; whole tiles per CTA; tiles shared out by units
-    float* partial;        // [2 * CTAs][bn][128 * MH]
+    int tiles_m, whole, rest_tiles, share;  // row tiles; whole tiles per CTA; tiles shared out by units, and among how many CTAs
+    float* partial;        // [2 * share][bn][128 * MH]
     int* arrived;          // per shared tile, how many of its CTAs have left their sums (zeroed by the preparation kernel)
     int raw_slots, b_slots, a_slots, accs;
     int* error_flag;
     unsigned long long wait_ns;
-};
-
-// The tiles and unit ranges of one CTA, in the order every role walks them.
-struct Walk {
-    const int whole, units;
-    int i, at, end;  // whole tiles taken; position among the shared units (fewer than CTAs x units of them: 32 bits)
-    __device__ __forceinline__ Walk(int whole_, int rest, int units_) : whole(whole_), units(units_), i(0) {
-        const uint32_t total = (uint32_t)(rest * units_);
-        at = (int)(blockIdx.x * total / gridDim.x);
-        end = (int)((blockIdx.x + 1) * total / gridDim.x);
-    }
-    __device__ __forceinline__ bool next(int& tile, int& u0, int& u1) {
-        if (i < whole) { tile = i * gridDim.x + blockIdx.x; u0 = 0; u1 = units; ++i; return true; }
-        if (at >= end) return false;
-        const int t = at / units;
-        tile = whole * gridDim.x + t;
-        u0 = at - t * units;
-        u1 = min(units, u0 + end - at);
-        at += u1 - u0;
-        return true;
-    }
 };
 
 __device__ __forceinline__ __half2 as_half2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
@@ -387,7 +352,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = tmem_base_slot, a_ring = tmem_base + 512u - (uint32_t)(a_slots * F::a_cols);
-    Walk walk(p.whole, p.rest_tiles, p.units);
+    Walk walk(p.whole, p.rest_tiles, p.units, p.share, (int)gridDim.x, (int)blockIdx.x);
     int tile, u0, u1;
 
     if (warp < kDrainWarps) {
@@ -541,20 +506,14 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                 to_y();
             } else {
                 const size_t tile_floats = (size_t)bn * 128 * MH, mine = (MH == 2 ? set * 128 : 0) + r0;
-                float* part = p.partial + (size_t)(2 * blockIdx.x + (u0 == 0 ? 1 : 0)) * tile_floats + mine;
+                const Deal deal(p.share, p.rest_tiles, p.units);
+                const int t = tile - p.whole * (int)gridDim.x;
+                float* part = p.partial + (size_t)deal.place(t, (int)blockIdx.x) * tile_floats + mine;
 #pragma unroll
                 for (int j = 0; j < kCols; ++j)
                     if (j < live_tokens) part[j * 128 * MH] = pair_at(sum[j / 2], j & 1);
-                // the CTAs that share this tile, in unit order: c0, c0 + 1, .. while their ranges reach into it
-                const int t = tile - p.whole * (int)gridDim.x;
-                // (fewer than 148 tiles of at most 65536 units among 148 CTAs: the products fit 32 bits)
-                const uint32_t total = (uint32_t)(p.rest_tiles * p.units), begin = (uint32_t)(t * p.units), end = begin + p.units;
-                auto range_begin = [&](int c) -> uint32_t { return (uint32_t)c * total / gridDim.x; };
-                int c0 = (int)(begin * gridDim.x / total);
-                while (c0 > 0 && range_begin(c0) > begin) --c0;
-                while (range_begin(c0 + 1) <= begin) ++c0;
-                int c1 = blockIdx.x;
-                while (c1 + 1 < (int)gridDim.x && range_begin(c1 + 1) < end) ++c1;
+                // the CTAs that share this tile, in unit order
+                const int c0 = deal.first(t), c1 = deal.last(t, (int)blockIdx.x);
                 __threadfence();
                 asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
                 if (tid == 0) {
@@ -567,7 +526,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
 #pragma unroll
                     for (int j = 0; j < kCols / 2; ++j) sum[j] = 0;
                     for (int c = c0; c <= c1; ++c) {
-                        const float* piece = p.partial + (size_t)(2 * c + (range_begin(c) > begin ? 0 : 1)) * tile_floats + mine;
+                        const float* piece = p.partial + (size_t)deal.place(t, c) * tile_floats + mine;
                         // sixteen loads in flight (a branch for each would make each wait for the one before); the padding
                         // tokens' places exist and hold nothing that is used
 #pragma unroll
@@ -800,69 +759,6 @@ int launch_tc(const TcParams& p, int mh, bool codes, int ctas, size_t smem, cuda
     return mh == 1 ? launch_tc<TYPE, 1, false>(p, ctas, smem, s) : launch_tc<TYPE, 2, false>(p, ctas, smem, s);
 }
 
-// How a call is cut: row halves and tokens per tile, CTAs, ring depths, shared memory and scratch.
-struct TcCut {
-    int mh, bn, n_tiles, tiles_m, units, image_tiles, windows, ctas, whole, rest_tiles;
-    int raw_slots, b_slots, a_slots, accs;
-    size_t smem, xs_bytes, steps_bytes, partial_bytes;
-};
-struct FormatSizes { int raw_bytes, a_cols, raw_per_unit; };
-FormatSizes format_sizes(int type) {
-    switch (type) {
-        case RQ_Q4_K: return {Format<RQ_Q4_K>::raw_bytes, Format<RQ_Q4_K>::a_cols, 1};
-        case RQ_Q6_K: return {Format<RQ_Q6_K>::raw_bytes, Format<RQ_Q6_K>::a_cols, 1};
-        case RQ_Q8_0: return {Format<RQ_Q8_0>::raw_bytes, Format<RQ_Q8_0>::a_cols, 2};
-        default: return {Format<RQ_Q4_0>::raw_bytes, Format<RQ_Q4_0>::a_cols, 1};
-    }
-}
-TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t cols, int tokens) {
-    TcCut c;
-    const FormatSizes f = format_sizes(type);
-    // (fp32 activations over the 32-value formats: two accumulators a slice, of hi and lo columns each, twice; 48 tokens fit)
-    const int widest_1 = !codes && (type == RQ_Q8_0 || type == RQ_Q4_0) ? 48 : Shape<1>::cols;
-    c.mh = tokens <= widest_1 ? 1 : 2;
-    const int widest = c.mh == 1 ? widest_1 : Shape<2>::cols, grain = c.mh == 1 ? 16 : 32;
-    c.n_tiles = (tokens + widest - 1) / widest;
-    c.bn = ((tokens + c.n_tiles - 1) / c.n_tiles + grain - 1) / grain * grain;
-    c.tiles_m = (int)((rows + 128 * c.mh - 1) / (128 * c.mh));
-    c.units = (int)((cols + 255) / 256);
-    c.windows = type == RQ_Q4_K ? (c.units + 7) / 8 : 0;
-    c.image_tiles = 4 * c.units + c.windows;
-    const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles, work = tiles * c.units;
-    c.ctas = work < sm_count ? (int)work : sm_count;
-    // Few tiles: more CTAs to a tile shorten its products (some two microseconds a unit) and lengthen the last one's sum (most of a
-    // microsecond a piece, a trip to L2 each), so at most about the square root of twice its units share one.
-    int pieces = 1;
-    while ((pieces + 1) * (pieces + 1) <= 2 * c.units) ++pieces;
-    if (tiles * pieces < c.ctas) c.ctas = (int)(tiles * pieces);
-    c.whole = (int)(tiles / c.ctas);
-    c.rest_tiles = (int)(tiles - (int64_t)c.whole * c.ctas);
-    // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: every ring is as long as
-    // keeps a slot with the same waiters. Accumulators, operand and (MH = 1) activation slots alternate between the two issuing
-    // threads: even numbers of slices. Stored bytes: with MH = 2 a staging group takes every second tile; with MH = 1 the three groups
-    // all read a tile of four slices, but one of two (Q8_0) misses one group in three.
-    // tensor memory, 512 columns: at least four operand slots (Q6_K with MH = 2: two), accumulators, more operand slots
-    const int halves = type == RQ_Q4_K || type == RQ_Q6_K ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn;
-    const int a_least = type == RQ_Q6_K && c.mh == 2 ? 2 : 4;
-    c.accs = (512 - a_least * f.a_cols) / acc_cols / (2 * halves) * (2 * halves);
-    if (c.accs > kMaxAcc) c.accs = kMaxAcc;
-    c.a_slots = (512 - c.accs * acc_cols) / f.a_cols & ~1;
-    if (c.a_slots > kMaxA) c.a_slots = kMaxA;
-    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums)
-    const int joined = c.mh == 1 ? c.bn * 128 * 4 : 0, budget = (codes ? 212 : 220) * 1024 - joined, b_bytes = c.bn * (codes ? 128 : 256);
-    c.b_slots = c.mh == 1 || codes ? 4 : 3;
-    c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
-    const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 ? 2 : (f.raw_per_unit == 2 ? 3 : 1);
-    c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
-    const int b_max = c.mh == 1 ? kMaxB : 6, b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
-    while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
-    c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + joined + 1024;
-    c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
-    c.steps_bytes = codes ? (size_t)c.n_tiles * c.image_tiles * 2 * c.bn * 4 : 0;
-    c.partial_bytes = c.rest_tiles ? (size_t)2 * c.ctas * c.bn * 128 * c.mh * 4 : 0;
-    return c;
-}
-
 }  // namespace
 
 // Enough for every call of up to this many rows, inputs and tokens, of any format: token tiles are padded by less than 32 rows
@@ -909,7 +805,7 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
     p.main = w->main; p.scale = w->scale; p.rows = w->rows;
     p.blocks32 = (int)(w->cols / 32); p.units = cut.units; p.permuted = rq_plane_permuted(w->type, w->cols) ? 1 : 0;
     p.xs = xs; p.image_tiles = cut.image_tiles; p.bn = cut.bn; p.tokens = tokens; p.y = y; p.yn = yn; p.yt = yt;
-    p.tiles_m = cut.tiles_m; p.whole = cut.whole; p.rest_tiles = cut.rest_tiles;
+    p.tiles_m = cut.tiles_m; p.whole = cut.whole; p.rest_tiles = cut.rest_tiles; p.share = cut.share;
     p.steps = (const float*)(xs + cut.xs_bytes);
     p.partial = partial; p.arrived = arrived;
     p.raw_slots = cut.raw_slots; p.b_slots = cut.b_slots; p.a_slots = cut.a_slots; p.accs = cut.accs;

@@ -1,0 +1,69 @@
+// The cut of a batched product (recipe_dev_b200/csrc/rq_matmul_cut.cuh) walked on the host: every unit of every output tile is taken
+// exactly once, and every shared tile is added up by exactly one of its CTAs. Built and run by tests/test_matmul_cut.py. Prints "ok".
+#include <cstdio>
+#include <vector>
+
+#include "rq_matmul_cut.cuh"
+
+using namespace rqcut;
+
+static int fail(const char* what, int type, bool codes, int sms, long long rows, long long cols, int tokens) {
+    std::printf("%s: type %d codes %d, %d SMs, %lld x %lld, %d tokens\n", what, type, (int)codes, sms, rows, cols, tokens);
+    return 1;
+}
+
+static int walk_call(int type, bool codes, int sms, int64_t rows, int64_t cols, int tokens) {
+    const TcCut c = tc_cut(type, codes, sms, rows, cols, tokens);
+    const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles;
+    if (c.tiles_m * 128LL * c.mh < rows || (int64_t)c.n_tiles * c.bn < tokens) return fail("outputs outside every tile", type, codes, sms, rows, cols, tokens);
+    std::vector<int> next_unit(tiles, 0), arrivals(c.rest_tiles, 0), summed(c.rest_tiles, 0);
+    std::vector<char> place_used((size_t)2 * c.share, 0);
+    for (int cta = 0; cta < c.ctas; ++cta) {  // in CTA order, a tile's pieces come in unit order
+        Walk walk(c.whole, c.rest_tiles, c.units, c.share, c.ctas, cta);
+        int tile, u0, u1, segments = 0;
+        while (walk.next(tile, u0, u1)) {
+            ++segments;
+            if (tile < 0 || tile >= tiles || u0 < 0 || u0 >= u1 || u1 > c.units) return fail("a segment outside the work", type, codes, sms, rows, cols, tokens);
+            if (next_unit[tile] != u0) return fail("a unit missed or taken twice", type, codes, sms, rows, cols, tokens);
+            next_unit[tile] = u1;
+            if (u0 == 0 && u1 == c.units) continue;  // written by the CTA itself
+            const int t = (int)(tile - (int64_t)c.whole * c.ctas);
+            if (t < 0 || t >= c.rest_tiles) return fail("a whole tile cut in pieces", type, codes, sms, rows, cols, tokens);
+            const Deal deal(c.share, c.rest_tiles, c.units);
+            const int first = deal.first(t), last = deal.last(t, cta), place = deal.place(t, cta);
+            if (cta < first || cta > last || place < 0 || place >= 2 * c.share || place_used[place]) return fail("a piece's place", type, codes, sms, rows, cols, tokens);
+            place_used[place] = 1;
+            if (arrivals[t]++ == last - first) {  // the last one to arrive adds the pieces first .. last
+                ++summed[t];
+                for (int p = first; p <= last; ++p)
+                    if (!place_used[deal.place(t, p)]) return fail("a sum over a piece nobody left", type, codes, sms, rows, cols, tokens);
+            }
+        }
+        if (segments > c.whole + 2) return fail("more than two pieces", type, codes, sms, rows, cols, tokens);
+    }
+    for (int64_t t = 0; t < tiles; ++t)
+        if (next_unit[t] != c.units) return fail("a tile not finished", type, codes, sms, rows, cols, tokens);
+    for (int t = 0; t < c.rest_tiles; ++t)
+        if (arrivals[t] ? summed[t] != 1 : 0) return fail("a shared tile nobody adds up", type, codes, sms, rows, cols, tokens);
+    return 0;
+}
+
+int main() {
+    const int types[4] = {RQ_Q4_K, RQ_Q6_K, RQ_Q8_0, RQ_Q4_0};
+    const int64_t named[][3] = {{14336, 4096, 673}, {14336, 4096, 700}, {14336, 4096, 768}, {28672, 8192, 300}, {151936, 4096, 1}, {151936, 2560, 16}, {152064, 3584, 16}, {11008, 4096, 600},
+                                {8192, 2048, 400}, {25600, 5120, 200}, {19072, 512, 16}, {19200, 4096, 16}, {19072, 4096, 100}, {1, 256, 12}, {300, 16777216, 9}};
+    for (int type : types)
+        for (int codes = 0; codes < (type == RQ_Q8_0 || type == RQ_Q4_0 ? 2 : 1); ++codes) {
+            for (const auto& n : named)
+                if (walk_call(type, codes, 148, n[0], n[1], (int)n[2])) return 1;
+            uint64_t state = 88172645463325252ull + type;
+            auto pick = [&](int64_t lo, int64_t hi) { state ^= state << 13; state ^= state >> 7; state ^= state << 17; return lo + (int64_t)(state % (uint64_t)(hi - lo + 1)); };
+            for (int i = 0; i < 20000; ++i) {
+                const int sms = i % 4 ? 148 : (int)pick(1, 160);
+                const int64_t rows = pick(1, i % 2 ? 30000 : 160000), units = pick(1, i % 3 ? 20 : 64), tokens = pick(1, i % 5 ? 200 : 1200);
+                if (walk_call(type, codes, sms, rows, units * 256, (int)tokens)) return 1;
+            }
+        }
+    std::printf("ok\n");
+    return 0;
+}

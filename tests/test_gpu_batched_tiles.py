@@ -1,0 +1,40 @@
+"""The batched product where few tiles are left over once every SM has its whole ones: outputs filled with NaN beforehand and every one
+of them compared, all formats and both activation modes. GPU only (-m gpu)."""
+import pytest
+
+from tests import oracle_lib as ol
+
+pytestmark = pytest.mark.gpu
+
+
+def _rounded(x, step):
+    """int8 codes times their steps, fp32 arithmetic as the format defines it, in 64 bits."""
+    import torch
+
+    g = x.reshape(x.shape[0], -1, step)
+    best = g.gather(2, g.abs().argmax(2, keepdim=True))
+    inverse = torch.full_like(best, -127.0) / best
+    return (torch.round(g * inverse).clamp(-128, 127).double() * (torch.ones_like(inverse) / inverse).double()).reshape(x.shape)
+
+
+@pytest.mark.parametrize("t", [ol.Q4_K, ol.Q6_K, ol.Q8_0, ol.Q4_0])
+@pytest.mark.parametrize("tiles,rows,cols,tokens", [(1, 0, 512, 16), (2, -5, 4096, 16), (3, 0, 256, 33), (0, 19200, 2560, 100), (0, 14336, 4096, 700), (0, 8192, 2048, 400)])
+def test_every_output_is_written(rq_ctx, t, tiles, rows, cols, tokens):
+    import torch
+
+    # `tiles` row tiles more than the GPU has SMs, the last of them `-rows` rows short, or `rows` as given
+    rows = 128 * (torch.cuda.get_device_properties(0).multi_processor_count + tiles) + rows if tiles else rows
+    gen = torch.Generator(device="cuda").manual_seed(rows + t)
+    w = rq_ctx.weight_from_device(t, rq_ctx.quantize(t, 0.02 * torch.randn(rows * cols, generator=gen, device="cuda")), rows, cols)
+    x = torch.randn((tokens, cols), generator=gen, device="cuda")
+    dense = rq_ctx.dequant(w).reshape(rows, cols)
+    for mode in (0, 1):
+        y = torch.full((tokens, rows), float("nan"), device="cuda")
+        rq_ctx.matmul(w, x, y=y, act_mode=mode)
+        torch.cuda.synchronize()
+        xd, worst = x.double() if mode == 0 else _rounded(x, 32), 0.0
+        for r in range(0, rows, 4096):
+            worst = max(worst, (y[:, r : r + 4096].double() - xd @ dense[r : r + 4096].double().T).abs().max().item())
+        # 3e-6 of an output's usual size: 22 mantissa bits an input, sums of 64 products truncated once each, fp32 additions after that
+        assert not torch.isnan(y).any() and worst <= 3e-6 * 5.0 * 0.02 * cols**0.5
+    rq_ctx.check()
