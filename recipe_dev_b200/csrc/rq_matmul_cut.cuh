@@ -142,5 +142,18 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     c.partial_bytes = (size_t)2 * c.share * c.bn * 128 * c.mh * 4;
     return c;
 }
+// Work area of a call: the image, its steps, the shared tiles' sums and a counter for each of them.
+inline size_t scratch_bytes(const TcCut& c) { return c.xs_bytes + c.steps_bytes + c.partial_bytes + (size_t)c.rest_tiles * 4; }
+
+// Enough for every call of up to this many rows, inputs and tokens, of any format and activation mode. Tokens are padded by less than
+// 32 to a token tile; the shared tiles' sums are two tiles a CTA: 64 x 128 numbers of one row half, of two row halves (from 49
+// tokens on for fp32 activations over the 32-value formats) 64 x 256, from 65 tokens on 96 x 256.
+inline size_t scratch_bound(int sm_count, int64_t rows, int64_t cols, int tokens) {
+    const int64_t units = (cols + 255) / 256, tiles_n = (tokens + 95) / 96;
+    const size_t image = (size_t)(tokens + 32 * tiles_n + 32) * 256 * (size_t)(4 * units + (units + 7) / 8);
+    const int64_t work = ((rows + 127) / 128) * units * tiles_n;
+    const size_t ctas = (size_t)(work < sm_count ? work : sm_count);
+    return image + 4 * ctas + 2 * ctas * (size_t)(tokens > 64 ? 96 * 256 : (tokens > 48 ? 64 * 256 : 64 * 128)) * 4;
+}
 
 }  // namespace rqcut

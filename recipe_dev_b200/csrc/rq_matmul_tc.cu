@@ -761,15 +761,7 @@ int launch_tc(const TcParams& p, int mh, bool codes, int ctas, size_t smem, cuda
 
 }  // namespace
 
-// Enough for every call of up to this many rows, inputs and tokens, of any format: token tiles are padded by less than 32 rows
-// each, and the shared tiles' sums are two tiles a CTA.
-size_t rq_matmul_scratch_bytes(const rq_ctx* ctx, int64_t rows, int64_t cols, int tokens) {
-    const int64_t units = (cols + 255) / 256, tiles_n = (tokens + 95) / 96;
-    const size_t image = (size_t)(tokens + 32 * tiles_n + 32) * 256 * (size_t)(4 * units + (units + 7) / 8);
-    const int64_t work = ((rows + 127) / 128) * units * (tiles_n < 1 ? 1 : tiles_n);
-    const size_t ctas = (size_t)(work < ctx->sm_count ? work : ctx->sm_count);
-    return image + 256 + 4 * ctas + 2 * ctas * (tokens > 64 ? 96 * 256 : 64 * 128) * 4;
-}
+size_t rq_matmul_scratch_bytes(const rq_ctx* ctx, int64_t rows, int64_t cols, int tokens) { return scratch_bound(ctx->sm_count, rows, cols, tokens); }
 
 // RQ_ERR_UNSUPPORTED (no error text) = not one of the four formats. act_mode FLOAT or INT8 (step 32 / 256).
 int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int act_mode, int step, cudaStream_t s) {
@@ -778,7 +770,7 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
     // fp32 activations over an odd number of 32-value blocks stay with the matvec kernel, as they were: it has no fp16 range to keep to
     if (!codes && w->cols % BK) return RQ_ERR_UNSUPPORTED;
     const TcCut cut = tc_cut(w->type, codes, ctx->sm_count, w->rows, w->cols, tokens);
-    int rc = rq_ensure_act_scratch(ctx, cut.xs_bytes + cut.steps_bytes + cut.partial_bytes + (size_t)cut.rest_tiles * 4, s);
+    int rc = rq_ensure_act_scratch(ctx, scratch_bytes(cut), s);
     if (rc) return rc;
     ctx->act_cols = 0;  // whatever int8 records the scratch held for INT8_CACHED calls are gone
     uint8_t* xs = ctx->act_scratch;

@@ -1,5 +1,5 @@
 // The cut of a batched product (recipe_dev_b200/csrc/rq_matmul_cut.cuh) walked on the host: every unit of every output tile is taken
-// exactly once, and every shared tile is added up by exactly one of its CTAs. Built and run by tests/test_matmul_cut.py. Prints "ok".
+// exactly once, every shared tile is added up by exactly one of its CTAs, and a work area sized ahead of time holds the call's. Built and run by tests/test_matmul_cut.py. Prints "ok".
 #include <cstdio>
 #include <vector>
 
@@ -62,6 +62,10 @@ int main() {
                 const int sms = i % 4 ? 148 : (int)pick(1, 160);
                 const int64_t rows = pick(1, i % 2 ? 30000 : 160000), units = pick(1, i % 3 ? 20 : 64), tokens = pick(1, i % 5 ? 200 : 1200);
                 if (walk_call(type, codes, sms, rows, units * 256, (int)tokens)) return 1;
+                // reserved for this shape and for a larger one
+                const size_t need = scratch_bytes(tc_cut(type, codes, sms, rows, units * 256, (int)tokens));
+                if (scratch_bound(sms, rows, units * 256, (int)tokens) < need) return fail("reserved too little", type, codes, sms, rows, units * 256, (int)tokens);
+                if (scratch_bound(sms, rows + pick(0, 5000), 256 * (units + pick(0, 8)), (int)(tokens + pick(0, 100))) < need) return fail("a larger shape reserved too little", type, codes, sms, rows, units * 256, (int)tokens);
             }
         }
     std::printf("ok\n");

@@ -1,5 +1,5 @@
 """The batched product where few tiles are left over once every SM has its whole ones: outputs filled with NaN beforehand and every one
-of them compared, all formats and both activation modes. GPU only (-m gpu)."""
+of them compared, all formats and both activation modes; and the work area such calls were reserved. GPU only (-m gpu)."""
 import pytest
 
 from tests import oracle_lib as ol
@@ -38,3 +38,28 @@ def test_every_output_is_written(rq_ctx, t, tiles, rows, cols, tokens):
         # 3e-6 of an output's usual size: 22 mantissa bits an input, sums of 64 products truncated once each, fp32 additions after that
         assert not torch.isnan(y).any() and worst <= 3e-6 * 5.0 * 0.02 * cols**0.5
     rq_ctx.check()
+
+
+@pytest.mark.parametrize("tokens", [48, 49, 56, 64])
+def test_a_reserved_context_holds_the_widest_window(tokens):
+    """Rows enough for every SM, windows where fp32 calls over the 32-value formats go to two row halves."""
+    import recipe_dev_b200 as rq
+    import torch
+
+    rows, cols = 14336, 1024
+    ctx = rq.Context(0)
+    ctx.reserve(rows, cols, tokens)
+    x = torch.randn((tokens, cols), device="cuda")
+    ws = [ctx.weight_from_device(t, ctx.quantize(t, 0.02 * torch.randn(rows * cols, device="cuda")), rows, cols) for t in (ol.Q4_K, ol.Q6_K, ol.Q8_0, ol.Q4_0)]
+    calls = [(w, n, mode, torch.empty((n, rows), device="cuda")) for w in ws for n in {tokens, 48} for mode in (0, 1)]
+    torch.cuda.synchronize()
+    stream = ctx.sequence_begin()  # a recorded call that would have to allocate is refused
+    for w, n, mode, y in calls:
+        ctx.matmul(w, x[:n], y=y, act_mode=mode, stream=stream)
+    seq = ctx.sequence_end()
+    seq.run()
+    torch.cuda.synchronize()
+    ctx.check()
+    for w, n, mode, y in calls:
+        assert torch.equal(y, ctx.matmul(w, x[:n], act_mode=mode))
+    seq.free()
