@@ -58,7 +58,8 @@ enum { RQ_ACT_FLOAT = 0, RQ_ACT_INT8 = 1,
        /* INT8 where the caller states that x is the same column, token count and step as the previous
         * RQ_ACT_INT8 call on this context (q/k/v, or gate/up, read one activation): the library may
         * reuse the records it derived then instead of deriving them again. The results are the same
-        * bits either way. Fails if the previous INT8 call was of another width, token count or step. */
+        * bits either way. Fails if the previous INT8 call was of another width, token count or step,
+        * or a K-quant rq_matmul of twelve and more tokens (its product takes no records and leaves none). */
        RQ_ACT_INT8_CACHED = 2 };
 
 /* Routing (Scoring, recipe.rs:13955). */

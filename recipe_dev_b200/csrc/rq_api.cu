@@ -442,7 +442,7 @@ extern "C" int rq_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_
     // 4096, ten: 46.4 there, 33.9 here): below that their products keep clear of fp16's range, as they always have.
     const bool codes = w->type == RQ_Q8_0 || w->type == RQ_Q4_0;
     const int from = !codes ? 12 : (w->cols > 7680 ? 5 : 9);
-    if (act_mode == RQ_ACT_FLOAT || (act_mode == RQ_ACT_INT8 && tokens >= from)) {
+    if (act_mode == RQ_ACT_FLOAT || ((act_mode == RQ_ACT_INT8 || codes) && tokens >= from)) {  // (cached records: of Q8_0 / Q4_0 calls)
         rc = rq_launch_matmul(ctx, w, x, sk, st, tokens, y, yn, yt, act_mode, step, (cudaStream_t)stream);
         if (rc != RQ_ERR_UNSUPPORTED) return rc;
     }

@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "rq.h"
+#include "rq_act_layout.cuh"
 
 // ---------------------------------------------------------------------------------
 // Data layout in HBM.
@@ -71,19 +72,8 @@ struct DeviceGuard {
     ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
 
-// Device-side activation scratch, per token (INT8 path).
-// Inputs that are whole 256-value units use one padded record per unit, the layout the streaming
-// kernel keeps in shared memory:
-//   codes[256] int8 | d[8] fp32 @256 | sum16[16] int16 @288 | sum32[8] int16 @320   (336 bytes)
-// Other widths use three planes: codes [cols] int8 | d [cols/32] fp32 | sum16 [cols/16] int16.
-// d = the step of a 32-value group, sum16 = the sum of the 16 codes of a slice.
-#define RQ_ACT_RECORD_INT8 336
+// fp32 activations of 256 inputs in the streaming kernel's shared memory (rq_gemv_stream.cuh)
 #define RQ_ACT_RECORD_FLOAT 976
-__host__ __device__ inline bool rq_act_unit_layout(int64_t cols) { return cols % 256 == 0; }
-__host__ __device__ inline size_t rq_act_token_bytes(int64_t cols) {
-    return rq_act_unit_layout(cols) ? (size_t)(cols / 256) * RQ_ACT_RECORD_INT8
-                                    : (size_t)cols + (size_t)(cols / 32) * 4 + (size_t)(cols / 16) * 2;
-}
 
 // Whether an INT8 call quantises inside the matvec launch. Every CTA of such a launch reads all of x: beyond 8192 inputs that
 // traffic (some 300 CTAs x 4 bytes x inputs) costs more than the quantiser launch it saves.
@@ -114,7 +104,8 @@ int rq_launch_gemv_multi(rq_ctx* ctx, int n, const rq_weight* const* ws, const f
                          float* const* ys, int64_t yn, int64_t yt, int act_mode, int step, cudaStream_t s);
 int rq_launch_gemv_tiled_int8(rq_ctx* ctx, const rq_weight* w, int tokens, float* y, int64_t yn, int64_t yt, const uint8_t* act, cudaStream_t s);
 // The batched product with integer weight operands (rq_matmul_tc.cu): FLOAT or INT8 activations.
-// RQ_ERR_UNSUPPORTED (no error text) = not one of the four formats it serves.
+// INT8 over Q8_0 / Q4_0 leaves the records of the matvec kernels as well, and INT8_CACHED (those two only) reads them.
+// RQ_ERR_UNSUPPORTED (no error text) = not one of the four formats it serves, or no cached records it could use.
 int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int act_mode,
                      int step, cudaStream_t s);
 // scratch bytes that are enough for rq_launch_matmul over any weight of up to this shape and up to this many tokens (its activation image and shared tiles' sums)

@@ -5,12 +5,7 @@
 #include <stdint.h>
 
 #include "rq.h"
-
-#ifdef __CUDACC__
-#define RQ_HOST_DEVICE __host__ __device__ __forceinline__
-#else
-#define RQ_HOST_DEVICE inline
-#endif
+#include "rq_act_layout.cuh"
 
 namespace rqcut {
 
@@ -83,7 +78,7 @@ struct Walk {
 struct TcCut {
     int mh, bn, n_tiles, tiles_m, units, image_tiles, windows, ctas, whole, rest_tiles, share;
     int raw_slots, b_slots, a_slots, accs;
-    size_t smem, xs_bytes, steps_bytes, partial_bytes;
+    size_t smem, records_bytes, xs_bytes, steps_bytes, partial_bytes;
 };
 struct FormatSizes { int raw_bytes, a_cols, raw_per_unit; };
 inline FormatSizes format_sizes(int type) {
@@ -137,23 +132,25 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     const int b_max = c.mh == 1 ? kMaxB : 6, b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
     while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
     c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + joined + 1024;
+    c.records_bytes = codes ? (rq_act_token_bytes(cols) * (size_t)tokens + 255) & ~(size_t)255 : 0;
     c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
     c.steps_bytes = codes ? (size_t)c.n_tiles * c.image_tiles * 2 * c.bn * 4 : 0;
     c.partial_bytes = (size_t)2 * c.share * c.bn * 128 * c.mh * 4;
     return c;
 }
-// Work area of a call: the image, its steps, the shared tiles' sums and a counter for each of them.
-inline size_t scratch_bytes(const TcCut& c) { return c.xs_bytes + c.steps_bytes + c.partial_bytes + (size_t)c.rest_tiles * 4; }
+// Work area of a call: the records (where INT8_CACHED calls look for them), the image, its steps, the shared tiles' sums and a counter
+// for each of them.
+inline size_t scratch_bytes(const TcCut& c) { return c.records_bytes + c.xs_bytes + c.steps_bytes + c.partial_bytes + (size_t)c.rest_tiles * 4; }
 
 // Enough for every call of up to this many rows, inputs and tokens, of any format and activation mode. Tokens are padded by less than
-// 32 to a token tile; the shared tiles' sums are two tiles a CTA: 64 x 128 numbers of one row half, of two row halves (from 49
+// 32 to a token tile (four bytes an input: the codes' image, steps and records are less); the shared tiles' sums are two tiles a CTA: 64 x 128 numbers of one row half, of two row halves (from 49
 // tokens on for fp32 activations over the 32-value formats) 64 x 256, from 65 tokens on 96 x 256.
 inline size_t scratch_bound(int sm_count, int64_t rows, int64_t cols, int tokens) {
     const int64_t units = (cols + 255) / 256, tiles_n = (tokens + 95) / 96;
     const size_t image = (size_t)(tokens + 32 * tiles_n + 32) * 256 * (size_t)(4 * units + (units + 7) / 8);
     const int64_t work = ((rows + 127) / 128) * units * tiles_n;
     const size_t ctas = (size_t)(work < sm_count ? work : sm_count);
-    return image + 4 * ctas + 2 * ctas * (size_t)(tokens > 64 ? 96 * 256 : (tokens > 48 ? 64 * 256 : 64 * 128)) * 4;
+    return image + 256 + 4 * ctas + 2 * ctas * (size_t)(tokens > 64 ? 96 * 256 : (tokens > 48 ? 64 * 256 : 64 * 128)) * 4;
 }
 
 }  // namespace rqcut

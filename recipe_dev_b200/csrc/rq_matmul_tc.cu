@@ -195,12 +195,13 @@ __device__ __forceinline__ void minimum_terms(const uint4& hdr, bool low, uint32
 // X -> the tensor core's operand images. A warp takes one unit of one token row: lane l the eight inputs 8 l .. 8 l + 7, so reads
 // and writes are whole lines. INT8 quantises on the way with the reference's arithmetic: the extreme of a group of STEP inputs
 // is the FIRST input of strictly largest magnitude, signed; inverse = -127 / extreme and d = 1 / inverse are IEEE divides,
-// code = clamp(rint(x * inverse)); the image holds code * d. STEP 0: fp32 activations. Rows past the last token and inputs past
-// the last column are zeros.
+// code = clamp(rint(x * inverse)); the image holds code * d. STEP 0: fp32 activations. CODES: the image holds the codes, and the
+// matvec kernels' records of the same inputs are left beside it for INT8_CACHED calls; STEP -1 reads those records instead of x. Rows
+// past the last token and inputs past the last column are zeros.
 // ------------------------------------------------------------------------------------------
 template <int STEP, bool CODES>
 __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict__ x, int64_t sk, int64_t st, int cols, int units, int tokens, int bn, int image_tiles,
-                                                          int windows, uint8_t* __restrict__ xs, float* __restrict__ steps,
+                                                          int windows, uint8_t* records, uint8_t* __restrict__ xs, float* __restrict__ steps,
                                                           int* __restrict__ arrived, int shared_tiles) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, unit = blockIdx.x;
@@ -211,8 +212,29 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (blockIdx.x == 0 && blockIdx.y == 0)
         for (int i = threadIdx.x; i < shared_tiles; i += 256) arrived[i] = 0;
-    float v[8];
-    if (row < tokens && k0 < cols) {  // a width is a whole number of 32-value blocks: a lane's eight inputs are all inside or all outside
+    float v[8], d = 0.f;
+    // CODES: where this lane's eight codes, their group's step and the sums lie in the token's records
+    const bool inside = row < tokens && k0 < cols;
+    uint8_t *rec_codes = nullptr, *rec_step = nullptr, *rec_sum16 = nullptr;
+    if (CODES && inside) {
+        uint8_t* tok = records + (size_t)row * rq_act_token_bytes(cols);
+        if (rq_act_unit_layout(cols)) {
+            uint8_t* rec = tok + (size_t)unit * RQ_ACT_RECORD_INT8;
+            rec_codes = rec + 8 * lane; rec_step = rec + 256 + 4 * (lane >> 2); rec_sum16 = rec + 288 + 2 * (lane >> 1);
+        } else {
+            rec_codes = tok + k0; rec_step = tok + cols + 4 * (k0 >> 5); rec_sum16 = tok + cols + 4 * (cols >> 5) + 2 * (k0 >> 4);
+        }
+    }
+    if (STEP < 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = 0.f;
+        if (inside) {
+            const uint2 c = __ldcg((const uint2*)rec_codes);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = (float)(int8_t)((j < 4 ? c.x : c.y) >> (8 * (j & 3)));
+            d = __ldcg((const float*)rec_step);
+        }
+    } else if (inside) {  // a width is a whole number of 32-value blocks: a lane's eight inputs are all inside or all outside
         const float* src = x + (int64_t)row * st + (int64_t)k0 * sk;
         if (vec) {
             *(float4*)v = __ldcg((const float4*)src);
@@ -225,7 +247,7 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = 0.f;
     }
-    if (STEP != 0) {
+    if (STEP > 0) {
         float best = 0.f;  // a NaN is never larger, so it never becomes the extreme
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -238,14 +260,31 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict
         }
         const bool nonzero = fabsf(best) > 0.f;
         const float inverse = nonzero ? __fdiv_rn(-127.0f, best) : 0.f;
-        const float d = nonzero ? __fdiv_rn(1.0f, inverse) : 0.f;
+        d = nonzero ? __fdiv_rn(1.0f, inverse) : 0.f;
+        uint32_t packed[2] = {0, 0};
+        int sum = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             int code = __float2int_rn(__fmul_rn(v[j], inverse));
             code = code < -128 ? -128 : (code > 127 ? 127 : code);
             v[j] = CODES ? (float)code : __fmul_rn((float)code, d);
+            sum += code;
+            packed[j >> 2] |= (uint32_t)(code & 0xff) << (8 * (j & 3));
         }
-        if (CODES && (lane & 3) == 0) steps[(((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * 2 + ((lane >> 2) & 1)) * bn + r] = d;
+        if (CODES) {
+            const int sum16 = sum + __shfl_xor_sync(0xffffffffu, sum, 1), sum32 = sum16 + __shfl_xor_sync(0xffffffffu, sum16, 2);
+            if (inside) {
+                *(uint2*)rec_codes = make_uint2(packed[0], packed[1]);
+                if ((lane & 1) == 0) *(int16_t*)rec_sum16 = (int16_t)sum16;
+                if ((lane & 3) == 0) {
+                    *(float*)rec_step = d;
+                    if (rq_act_unit_layout(cols)) *(int16_t*)(rec_codes - 8 * lane + 320 + 2 * (lane >> 2)) = (int16_t)sum32;
+                }
+            }
+        }
+    }
+    if (CODES) {
+        if ((lane & 3) == 0) steps[(((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * 2 + ((lane >> 2) & 1)) * bn + r] = d;
     }
     uint32_t hw[4], lw[4];
     split2(v[0], v[2], hw[0], lw[0]);  // the order the weights' nibble pairs come in
@@ -763,17 +802,20 @@ int launch_tc(const TcParams& p, int mh, bool codes, int ctas, size_t smem, cuda
 
 size_t rq_matmul_scratch_bytes(const rq_ctx* ctx, int64_t rows, int64_t cols, int tokens) { return scratch_bound(ctx->sm_count, rows, cols, tokens); }
 
-// RQ_ERR_UNSUPPORTED (no error text) = not one of the four formats. act_mode FLOAT or INT8 (step 32 / 256).
+// RQ_ERR_UNSUPPORTED (no error text) = not one of the four formats; INT8_CACHED: no records of this call's column, or no room for the
+// image beside them (a cached call allocates nothing). act_mode FLOAT, INT8 (step 32 / 256), over Q8_0 / Q4_0 also INT8_CACHED.
 int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int act_mode, int step, cudaStream_t s) {
     if (!w->has_tile_map || !rq_type_has_fast_path(w->type)) return RQ_ERR_UNSUPPORTED;
     const bool codes = act_mode != RQ_ACT_FLOAT && (w->type == RQ_Q8_0 || w->type == RQ_Q4_0);
     // fp32 activations over an odd number of 32-value blocks stay with the matvec kernel, as they were: it has no fp16 range to keep to
     if (!codes && w->cols % BK) return RQ_ERR_UNSUPPORTED;
     const TcCut cut = tc_cut(w->type, codes, ctx->sm_count, w->rows, w->cols, tokens);
+    const bool cached = act_mode == RQ_ACT_INT8_CACHED;
+    if (cached && (!codes || ctx->act_cols != w->cols || ctx->act_tokens != tokens || ctx->act_step != step || scratch_bytes(cut) > ctx->act_scratch_bytes)) return RQ_ERR_UNSUPPORTED;
     int rc = rq_ensure_act_scratch(ctx, scratch_bytes(cut), s);
     if (rc) return rc;
-    ctx->act_cols = 0;  // whatever int8 records the scratch held for INT8_CACHED calls are gone
-    uint8_t* xs = ctx->act_scratch;
+    uint8_t* xs = ctx->act_scratch + cut.records_bytes;
+    if (!cached) ctx->act_cols = 0;  // whatever int8 records the scratch held for INT8_CACHED calls are gone
     float* partial = (float*)(xs + cut.xs_bytes + cut.steps_bytes);
     int* arrived = (int*)((uint8_t*)partial + cut.partial_bytes);
     cudaLaunchAttribute attr[1];
@@ -788,9 +830,10 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         auto prep = act_mode == RQ_ACT_FLOAT ? rq_tc_prep_kernel<0, false>
+               : cached                    ? rq_tc_prep_kernel<-1, true>
                                              : (codes ? (step == 256 ? rq_tc_prep_kernel<256, true> : rq_tc_prep_kernel<32, true>)
                                                       : (step == 256 ? rq_tc_prep_kernel<256, false> : rq_tc_prep_kernel<32, false>));
-        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, cut.bn, cut.image_tiles, cut.windows, xs, (float*)(xs + cut.xs_bytes), arrived, cut.rest_tiles));
+        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, cut.bn, cut.image_tiles, cut.windows, ctx->act_scratch, xs, (float*)(xs + cut.xs_bytes), arrived, cut.rest_tiles));
     }
     TcParams p;
     p.tile_map = w->tile_map;
@@ -808,5 +851,6 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
         case RQ_Q8_0: rc = launch_tc<RQ_Q8_0>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;
         default: rc = launch_tc<RQ_Q4_0>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;
     }
+    if (rc == RQ_OK && codes) { ctx->act_cols = w->cols; ctx->act_tokens = tokens; ctx->act_step = step; }
     return rc;
 }
