@@ -8,9 +8,11 @@
 #pragma once
 #include "rq_internal.cuh"
 
+// x may be what the kernel before this one wrote, read after griddepcontrol.wait: its pointer carries no __restrict__ and
+// its loads are plain ones, not __ldg, or the compiler may take them for loads of constants and move them ahead of the wait.
 // `tok` = where this token's records go (unit-record layout when `unit_layout`, else planes);
 // `records36` = optional [recs][36] copy in the reference's own record format, or null.
-__device__ __forceinline__ void rq_quantise_group(const float* __restrict__ xt, int64_t sk, int64_t cols, int step, int64_t g, int lane,
+__device__ __forceinline__ void rq_quantise_group(const float* xt, int64_t sk, int64_t cols, int step, int64_t g, int lane,
                                                   uint8_t* __restrict__ tok, bool unit_layout, uint8_t* __restrict__ records36) {
     const int span = step >> 5;  // 32-value records per group
     const int64_t recs = cols >> 5;
@@ -23,7 +25,7 @@ __device__ __forceinline__ void rq_quantise_group(const float* __restrict__ xt, 
     for (int j = 0; j < 8; ++j) {
         v[j] = 0.f;
         if (j < n) {
-            v[j] = __ldg(xt + ((rec0 + j) * 32 + lane) * sk);
+            v[j] = xt[((rec0 + j) * 32 + lane) * sk];
             if (fabsf(v[j]) > fabsf(best)) { best = v[j]; best_at = j * 32 + lane; }
         }
     }

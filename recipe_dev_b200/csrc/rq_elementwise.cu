@@ -16,8 +16,8 @@ namespace {
 // per thread are loaded at once and kept for the second pass, the tree has one barrier (every warp adds the 256 partial sums up
 // for itself: the pairs t, t + 128, then t, t + 64, .. of a tree in shared memory, the last five steps by shuffles, the same
 // bits). HELD = 0: rows beyond 8192 values are read twice.
-// x is what the kernel before this one wrote, and this one may start before that one has ended: its loads are spelled __ldcg and the
-// pointers carry no __restrict__, or the compiler may take them for loads of constants and move them ahead of the wait.
+// x is what the kernel before this one wrote, and this one may start before that one has ended: the pointers carry no __restrict__ and
+// the loads are not __ldg, or the compiler may take them for loads of constants and move them ahead of the wait.
 template <int HELD>
 __global__ void __launch_bounds__(256) rq_rmsnorm_kernel(const float* x, int64_t sk, int64_t st, int64_t n, const float* gain,
                                                           float epsilon, float* y, int64_t yk, int64_t yt) {
@@ -70,7 +70,8 @@ __global__ void __launch_bounds__(256) rq_rmsnorm_kernel(const float* x, int64_t
     }
 }
 
-__global__ void __launch_bounds__(256) rq_add_kernel(const float* __restrict__ a, const float* __restrict__ b, int64_t n, float* __restrict__ y) {
+// (no __restrict__ here either: see the norm)
+__global__ void __launch_bounds__(256) rq_add_kernel(const float* a, const float* b, int64_t n, float* y) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) y[i] = __fadd_rn(a[i], b[i]);
@@ -115,7 +116,7 @@ __device__ float tanh_portable(float xf) {
     return (float)(u / (u + 2.0));
 }
 
-__global__ void __launch_bounds__(256) rq_softcap_kernel(const float* __restrict__ x, int64_t n, float down, float up, float* __restrict__ y) {
+__global__ void __launch_bounds__(256) rq_softcap_kernel(const float* x, int64_t n, float down, float up, float* y) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)

@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kThreads) rq_gemv_kernel(GemvParams p) {
 // The extreme is the FIRST input of strictly largest magnitude, signed; inverse = -127/extreme
 // and d = 1/inverse are IEEE fp32 divides; code = clamp(rint(x * inverse)).
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) rq_act_quant_kernel(const float* __restrict__ x, int64_t sk, int64_t st, int64_t cols, int tokens,
+__global__ void __launch_bounds__(kThreads) rq_act_quant_kernel(const float* x, int64_t sk, int64_t st, int64_t cols, int tokens,
                                                                int step, uint8_t* __restrict__ scratch, uint8_t* __restrict__ records36) {
     // Programmatic dependent launch: the matvec behind this kernel may start streaming its weights
     // now; x may come from the kernel before this one, so wait for that one before reading it.
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kThreads) rq_act_quant_kernel(const float* __r
 // format -- as a short straight line of code: the kernel sits in the chain of a decode layer's launches (between gate/up and
 // down), runs once per layer on an instruction cache that other kernels have filled, and what it costs there is the length of
 // its instruction stream and its one trip to L2, not its arithmetic. Same operations in the same order as rq_quantise_group.
-__global__ void __launch_bounds__(kThreads) rq_act_quant32_kernel(const float* __restrict__ x, int64_t st, int units, uint8_t* __restrict__ scratch) {
+__global__ void __launch_bounds__(kThreads) rq_act_quant32_kernel(const float* x, int64_t st, int units, uint8_t* __restrict__ scratch) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const int rec = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);  // 32-value record = group
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kThreads) rq_act_quant32_kernel(const float* _
     const float* src = x + (int64_t)blockIdx.y * st + rec * 32 + lane;
     uint8_t* unit = scratch + ((size_t)blockIdx.y * units + (rec >> 3)) * RQ_ACT_RECORD_INT8;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const float v = __ldg(src);
+    const float v = *src;
     const unsigned key = __float_as_uint(fabsf(v)) <= 0x7f800000u ? __float_as_uint(fabsf(v)) : 0u;  // a NaN is never the extreme
     const unsigned top = __reduce_max_sync(0xffffffffu, key);
     const unsigned first = __reduce_min_sync(0xffffffffu, key == top && top != 0u ? (unsigned)lane : 0xffffffffu);

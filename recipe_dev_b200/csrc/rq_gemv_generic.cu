@@ -231,7 +231,7 @@ template <> struct GroupBytes<RQ_Q3_K> {
 // weights: two or three to isolate the codes, eight to make them floats, four products). Measured, Q5_K 14336 x 4096, one token: 28.2 us;
 // decoding value by value, every header field once per value, took 175.6.
 template <int TYPE, int ROWS>
-__global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* __restrict__ x,
+__global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* x,
                                                                         int64_t sk, int64_t st, float* __restrict__ y, int64_t yn, int64_t yt) {
     extern __shared__ __align__(16) float xs[];
     constexpr bool kOffset = TYPE == RQ_Q4_1 || TYPE == RQ_Q5_1 || TYPE == RQ_Q5_K || TYPE == RQ_Q2_K;
@@ -303,13 +303,13 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint
 // `.int(4)`: int8 activation records against Q4_1 blocks (block32 slice kind 3, build.rs:777-796). Per 16-value slice
 // r = q8_d * (d * f32(dot) + m * f32(sum of the slice's activation codes)); slice 0 takes the low nibbles, slice 1 the high
 // ones. A warp owns a row, lane l the blocks l, l + 32, ..; dots by dp4a over the nibbles in place; fixed xor tree.
-__global__ void __launch_bounds__(kWarps * 32) rq_gemv_q41_int8_kernel(const uint8_t* __restrict__ blocks, int64_t rows, int64_t cols, const uint8_t* __restrict__ records,
+__global__ void __launch_bounds__(kWarps * 32) rq_gemv_q41_int8_kernel(const uint8_t* __restrict__ blocks, int64_t rows, int64_t cols, const uint8_t* records,
                                                                          size_t token_bytes, float* __restrict__ y, int64_t yn, int64_t yt) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, token = blockIdx.y;
     const uint8_t* tok = records + (size_t)token * token_bytes;
     const bool unit = rq_act_unit_layout(cols);
     const int64_t nb = cols >> 5;
-    // Programmatic dependent launch: the records come from the quantiser launched before this kernel; the weights are
+    // Programmatic dependent launch: the records (read by plain loads, through a pointer the compiler may not take for one to constants) come from the quantiser launched before this kernel; the weights are
     // constants of the model, so the first round's weight loads go out before the wait for that kernel.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     bool records_ready = false;
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_q41_int8_kernel(const uin
                 float q8_d; uint32_t sums;
                 if (unit) {
                     const uint8_t* rec = tok + (size_t)(b >> 3) * RQ_ACT_RECORD_INT8;  // records are 16-byte aligned
-                    const uint4 lo = __ldg((const uint4*)(rec + 32 * (b & 7))), hi = __ldg((const uint4*)(rec + 32 * (b & 7)) + 1);
+                    const uint4 lo = *(const uint4*)(rec + 32 * (b & 7)), hi = *((const uint4*)(rec + 32 * (b & 7)) + 1);
                     cl[0] = (int)lo.x; cl[1] = (int)lo.y; cl[2] = (int)lo.z; cl[3] = (int)lo.w;
                     ch[0] = (int)hi.x; ch[1] = (int)hi.y; ch[2] = (int)hi.z; ch[3] = (int)hi.w;
                     q8_d = ((const float*)(rec + 256))[b & 7];
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_q41_int8_kernel(const uin
                 } else {
                     const int* codes = (const int*)(tok + b * 32);  // a token's planes start on a multiple of 8 bytes
 #pragma unroll
-                    for (int w = 0; w < 4; ++w) { cl[w] = __ldg(codes + w); ch[w] = __ldg(codes + 4 + w); }
+                    for (int w = 0; w < 4; ++w) { cl[w] = codes[w]; ch[w] = codes[4 + w]; }
                     q8_d = ((const float*)(tok + cols))[b];
                     sums = ((const uint32_t*)(tok + cols + nb * 4))[b];
                 }

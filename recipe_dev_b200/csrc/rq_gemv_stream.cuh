@@ -889,7 +889,9 @@ __device__ __forceinline__ void digits_to_smem(const float (&f)[16], uint8_t* __
 // strictly largest magnitude, inverse = -127 / extreme, d = 1 / inverse (IEEE divides),
 // code = clamp(rint(x * inverse)).
 template <int THREADS>
-__device__ __forceinline__ void quantise_to_smem(const float* __restrict__ x, int64_t sk, int cols, int step, uint8_t* __restrict__ rec_base, int tid) {
+// (x: plain loads through a pointer without __restrict__, so that none is taken for a load of a constant and moved ahead of the launch's
+// wait; a thread's four loads lie in one line, which L1 keeps: with __ldcg a layer of ten launches took 51.5 us for 48.8.)
+__device__ __forceinline__ void quantise_to_smem(const float* x, int64_t sk, int cols, int step, uint8_t* __restrict__ rec_base, int tid) {
     constexpr int kRecord = RQ_ACT_RECORD_INT8;
     const int slices = cols >> 4;
     const bool vec = sk == 1 && ((uintptr_t)x & 15) == 0;
@@ -897,10 +899,10 @@ __device__ __forceinline__ void quantise_to_smem(const float* __restrict__ x, in
         if (sl < slices) {
             if (vec) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) *(float4*)&v[4 * j] = __ldg((const float4*)(x + 16 * (int64_t)sl) + j);
+                for (int j = 0; j < 4; ++j) *(float4*)&v[4 * j] = ((const float4*)(x + 16 * (int64_t)sl))[j];
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __ldg(x + (16 * (int64_t)sl + j) * sk);
+                for (int j = 0; j < 16; ++j) v[j] = x[(16 * (int64_t)sl + j) * sk];
             }
         } else {
 #pragma unroll
@@ -1291,7 +1293,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     got[j] = make_uint4(0, 0, 0, 0);
                     if (i < total) {
                         const int v = i / per_vec, e = i - v * per_vec;
-                        if (tok0 + v < p.tokens) got[j] = __ldg((const uint4*)(p.act + (size_t)(tok0 + v) * per_vec * 16) + e);
+                        if (tok0 + v < p.tokens) got[j] = ((const uint4*)(p.act + (size_t)(tok0 + v) * per_vec * 16))[e];
                     }
                 }
 #pragma unroll
@@ -1331,7 +1333,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                         const int v = i / per_vec, e = i - v * per_vec;
                         const int vec = tok0 + v;
                         const bool live = p.act_vectors > T || vec < p.tokens;
-                        if (live) got[j] = __ldg((const uint4*)(p.act + (size_t)vec * src_bytes) + e);
+                        if (live) got[j] = ((const uint4*)(p.act + (size_t)vec * src_bytes))[e];
                     }
                 }
 #pragma unroll

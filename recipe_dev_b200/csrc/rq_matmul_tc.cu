@@ -200,9 +200,9 @@ __device__ __forceinline__ void minimum_terms(const uint4& hdr, bool low, uint32
 // past the last token and inputs past the last column are zeros.
 // ------------------------------------------------------------------------------------------
 template <int STEP, bool CODES>
-__global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* __restrict__ x, int64_t sk, int64_t st, int cols, int units, int tokens, int bn, int image_tiles,
-                                                          int windows, uint8_t* records, uint8_t* __restrict__ xs, float* __restrict__ steps,
-                                                          int* __restrict__ arrived, int shared_tiles) {
+__global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t sk, int64_t st, int cols, int units, int tokens, int bn, int image_tiles,
+                                                          int windows, uint8_t* records, uint8_t* xs, float* steps,
+                                                          int* arrived, int shared_tiles) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, unit = blockIdx.x;
     const int row = blockIdx.y * 8 + (threadIdx.x >> 5);  // the padded rows are a multiple of sixteen: every warp has one

@@ -65,3 +65,47 @@ def test_every_call_sees_the_one_before(rq_ctx, oracle, mode, hidden, ffn):
             assert torch.equal(a, want)
     ctx.check()
     seq.free()
+
+
+@pytest.mark.parametrize("cols", [768, 4096, 14336])
+def test_windows_and_elementwise_steps_see_the_one_before(cols):
+    """Four int8 positions whose codes are made from what the launch before wrote, steps in between, a Q4_1 window."""
+    import recipe_dev_b200 as rq
+    import torch
+
+    ctx = rq.Context(0)
+    ctx.reserve(cols, cols, 4)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    k8 = ctx.weight_from_device(rq.Q8_0, ctx.quantize(rq.Q8_0, 0.02 * torch.randn(640 * cols, generator=gen, device="cuda")), 640, cols)
+    k4 = ctx.weight_from_host(ol.Q4_1, ol.random_blocks(ol.Q4_1, 96 * cols // 32, np.random.default_rng(5)), 96, cols)
+    x = torch.empty((4, cols), device="cuda")
+    a, c, y8, y1, y4 = torch.empty_like(x), torch.empty_like(x), torch.empty((4, 640), device="cuda"), torch.empty(640, device="cuda"), torch.empty((4, 96), device="cuda")
+
+    def calls(stream, after):
+        for f in (lambda: ctx.add(x, x, y=a, stream=stream), lambda: ctx.softcap(a, 30.0, y=c, stream=stream), lambda: ctx.matvec(k8, c, y=y8, act_mode=1, stream=stream),
+                  lambda: ctx.add(c, a, y=c, stream=stream), lambda: ctx.matvec(k8, c[0], y=y1, act_mode=1, stream=stream), lambda: ctx.softcap(c, 20.0, y=a, stream=stream),
+                  lambda: ctx.matvec(k4, a, y=y4, act_mode=1, stream=stream)):
+            f()
+            after()
+
+    torch.cuda.synchronize()
+    stream = ctx.sequence_begin()
+    calls(stream, lambda: None)
+    seq = ctx.sequence_end()
+    planes = [a, c, y8, y1, y4]
+    for trial in range(6):
+        x.copy_(20.0 * torch.randn(x.shape, generator=gen, device="cuda"))
+        for p in planes:
+            p.fill_(float(trial))
+        torch.cuda.synchronize()
+        seq.run()
+        torch.cuda.synchronize()
+        got = [p.clone() for p in planes]
+        for p in planes:
+            p.fill_(-1.0)
+        torch.cuda.synchronize()
+        calls(None, torch.cuda.synchronize)
+        for g, want in zip(got, planes):
+            assert torch.equal(g, want)
+    ctx.check()
+    seq.free()
