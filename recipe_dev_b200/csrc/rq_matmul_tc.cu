@@ -200,17 +200,18 @@ __device__ __forceinline__ void minimum_terms(const uint4& hdr, bool low, uint32
 // past the last token and inputs past the last column are zeros.
 // ------------------------------------------------------------------------------------------
 template <int STEP, bool CODES>
-__global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t sk, int64_t st, int cols, int units, int tokens, int bn, int image_tiles,
+__global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t sk, int64_t st, int cols, int units, int tokens, int padded, int bn, int image_tiles,
                                                           int windows, uint8_t* records, uint8_t* xs, float* steps,
                                                           int* arrived, int shared_tiles) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, unit = blockIdx.x;
-    const int row = blockIdx.y * 8 + (threadIdx.x >> 5);  // the padded rows are a multiple of sixteen: every warp has one
+    const int row = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + (threadIdx.x >> 5);  // the padded rows are a multiple of sixteen
+    if (row >= padded) return;  // a last layer of the grid that is not full (more rows than one layer takes)
     const int nt = row / bn, r = row - nt * bn, k0 = unit * 256 + 8 * lane;
     const bool vec = sk == 1 && (st & 3) == 0 && ((uintptr_t)x & 15) == 0;
     uint8_t* hi = xs + ((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * (CODES ? 1 : 2) * (size_t)bn * 128 + swizzled(r, lane & 7);
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (blockIdx.x == 0 && blockIdx.y == 0)
+    if (blockIdx.x == 0 && row < 8)
         for (int i = threadIdx.x; i < shared_tiles; i += 256) arrived[i] = 0;
     float v[8], d = 0.f;
     // CODES: where this lane's eight codes, their group's step and the sums lie in the token's records
@@ -824,7 +825,8 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
     {
         const int padded = cut.n_tiles * cut.bn;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)cut.units, (unsigned)(padded / 8));
+        const unsigned groups = (unsigned)(padded / 8), deep = (groups + 65534) / 65535;
+        cfg.gridDim = dim3((unsigned)cut.units, (groups + deep - 1) / deep, deep);
         cfg.blockDim = dim3(256);
         cfg.stream = s;
         cfg.attrs = attr;
@@ -833,7 +835,7 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
                : cached                    ? rq_tc_prep_kernel<-1, true>
                                              : (codes ? (step == 256 ? rq_tc_prep_kernel<256, true> : rq_tc_prep_kernel<32, true>)
                                                       : (step == 256 ? rq_tc_prep_kernel<256, false> : rq_tc_prep_kernel<32, false>));
-        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, cut.bn, cut.image_tiles, cut.windows, ctx->act_scratch, xs, (float*)(xs + cut.xs_bytes), arrived, cut.rest_tiles));
+        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, padded, cut.bn, cut.image_tiles, cut.windows, ctx->act_scratch, xs, (float*)(xs + cut.xs_bytes), arrived, cut.rest_tiles));
     }
     TcParams p;
     p.tile_map = w->tile_map;

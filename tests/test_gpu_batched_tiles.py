@@ -63,3 +63,22 @@ def test_a_reserved_context_holds_the_widest_window(tokens):
     for w, n, mode, y in calls:
         assert torch.equal(y, ctx.matmul(w, x[:n], act_mode=mode))
     seq.free()
+
+
+@pytest.mark.parametrize("t,mode", [(ol.Q4_K, 0), (ol.Q6_K, 1), (ol.Q8_0, 0)])
+def test_more_tokens_than_one_grid_layer_takes(rq_ctx, t, mode):
+    import torch
+
+    rows, cols, tokens = 9, 256, 8 * 65535 + 100
+    gen = torch.Generator(device="cuda").manual_seed(t)
+    w = rq_ctx.weight_from_device(t, rq_ctx.quantize(t, 0.02 * torch.randn(rows * cols, generator=gen, device="cuda")), rows, cols)
+    x = torch.randn((tokens, cols), generator=gen, device="cuda")
+    y = torch.full((tokens, rows), float("nan"), device="cuda")
+    rq_ctx.matmul(w, x, y=y, act_mode=mode)
+    dense = rq_ctx.dequant(w).reshape(rows, cols).double().T
+    worst = 0.0
+    for i in range(0, tokens, 1 << 17):
+        xd = x[i : i + (1 << 17)]
+        worst = max(worst, (y[i : i + (1 << 17)].double() - (xd.double() if mode == 0 else _rounded(xd, 32)) @ dense).abs().max().item())
+    assert not torch.isnan(y).any() and worst <= 3e-6 * 5.0 * 0.02 * cols**0.5
+    rq_ctx.check()
