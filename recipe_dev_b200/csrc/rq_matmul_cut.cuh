@@ -12,10 +12,13 @@ namespace rqcut {
 constexpr int kMaxRaw = 8, kMaxB = 12, kMaxA = 8, kMaxAcc = 8;
 
 // groups: staging groups; cols: tokens per tile at most, the sums a drain thread holds; registers of the drain, staging and other
-// warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 768 x 80, 640 x 96)
-template <int MH> struct Shape;
-template <> struct Shape<1> { static constexpr int groups = 3, cols = 64, drain_regs = 120, stage_regs = 64, other_regs = 48, launch_regs = 80; };
-template <> struct Shape<2> { static constexpr int groups = 2, cols = 96, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
+// warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 768 x 80, 640 x 96).
+// CODES: int8 activations over the 32-value formats.
+template <int MH, bool CODES> struct Shape;
+template <> struct Shape<1, false> { static constexpr int groups = 3, cols = 64, drain_regs = 120, stage_regs = 64, other_regs = 48, launch_regs = 80; };
+template <> struct Shape<2, false> { static constexpr int groups = 2, cols = 96, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
+template <> struct Shape<1, true> { static constexpr int groups = 3, cols = 64, drain_regs = 128, stage_regs = 56, other_regs = 48, launch_regs = 80; };
+template <> struct Shape<2, true> { static constexpr int groups = 2, cols = 64, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
 
 template <int TYPE> struct Format {
     static constexpr bool kquant = TYPE == RQ_Q4_K || TYPE == RQ_Q6_K;
@@ -93,9 +96,9 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     TcCut c;
     const FormatSizes f = format_sizes(type);
     // (fp32 activations over the 32-value formats: two accumulators a slice, of hi and lo columns each, twice; 48 tokens fit)
-    const int widest_1 = !codes && (type == RQ_Q8_0 || type == RQ_Q4_0) ? 48 : Shape<1>::cols;
+    const int widest_1 = !codes && (type == RQ_Q8_0 || type == RQ_Q4_0) ? 48 : Shape<1, false>::cols;
     c.mh = tokens <= widest_1 ? 1 : 2;
-    const int widest = c.mh == 1 ? widest_1 : Shape<2>::cols, grain = c.mh == 1 ? 16 : 32;
+    const int widest = c.mh == 1 ? widest_1 : (codes ? Shape<2, true>::cols : Shape<2, false>::cols), grain = c.mh == 1 ? 16 : 32;
     c.n_tiles = (tokens + widest - 1) / widest;
     c.bn = ((tokens + c.n_tiles - 1) / c.n_tiles + grain - 1) / grain * grain;
     c.tiles_m = (int)((rows + 128 * c.mh - 1) / (128 * c.mh));
@@ -116,12 +119,14 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     // keeps a slot with the same waiters. Accumulators, operand and (MH = 1) activation slots alternate between the two issuing
     // threads: even numbers of slices. Stored bytes: with MH = 2 a staging group takes every second tile; with MH = 1 the three groups
     // all read a tile of four slices, but one of two (Q8_0) misses one group in three.
-    // tensor memory, 512 columns: at least four operand slots (Q6_K with MH = 2: two), accumulators, more operand slots
+    // tensor memory, 512 columns: at least four operand slots (Q6_K with MH = 2: two), accumulators, (codes) two sets of totals, more
+    // operand slots
     const int halves = type == RQ_Q4_K || type == RQ_Q6_K ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn;
     const int a_least = type == RQ_Q6_K && c.mh == 2 ? 2 : 4;
-    c.accs = (512 - a_least * f.a_cols) / acc_cols / (2 * halves) * (2 * halves);
+    const int totals = codes ? 2 * c.bn : 0;
+    c.accs = (512 - a_least * f.a_cols - totals) / acc_cols / (2 * halves) * (2 * halves);
     if (c.accs > kMaxAcc) c.accs = kMaxAcc;
-    c.a_slots = (512 - c.accs * acc_cols) / f.a_cols & ~1;
+    c.a_slots = (512 - c.accs * acc_cols - totals) / f.a_cols & ~1;
     if (c.a_slots > kMaxA) c.a_slots = kMaxA;
     // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums)
     const int joined = c.mh == 1 ? c.bn * 128 * 4 : 0, budget = (codes ? 212 : 220) * 1024 - joined, b_bytes = c.bn * (codes ? 128 : 256);
@@ -129,7 +134,10 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
     const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 ? 2 : (f.raw_per_unit == 2 ? 3 : 1);
     c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
-    const int b_max = c.mh == 1 ? kMaxB : 6, b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
+    // codes, two row halves: four slots of each are enough, and what they leave is L1, where the drain warps' scale loads want to stay
+    // (4096 x 14336, 509 tokens: 312 us so, 343 with rings as deep as fit)
+    if (codes && c.mh == 2) c.raw_slots = 4;
+    const int b_max = c.mh == 1 ? kMaxB : (codes ? 4 : 6), b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
     while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
     c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + joined + 1024;
     c.records_bytes = codes ? (rq_act_token_bytes(cols) * (size_t)tokens + 255) & ~(size_t)255 : 0;

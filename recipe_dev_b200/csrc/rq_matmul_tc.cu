@@ -64,7 +64,7 @@ constexpr int kDone = 32;                    // ring of "step finished" barriers
 constexpr float kMinScale = 256.0f, kMinUnscale = 1.0f / 256.0f;  // the minimum term's weights are scaled so that their fp16 residuals are no subnormals
 
 constexpr int kIssuers = 2;                  // with the two copying warps: one warpgroup
-template <int MH> __host__ __device__ constexpr int tc_threads() { return (kDrainWarps + 4 * Shape<MH>::groups + 4) * 32; }
+template <int MH, bool CODES> __host__ __device__ constexpr int tc_threads() { return (kDrainWarps + 4 * Shape<MH, CODES>::groups + 4) * 32; }
 
 struct TcParams {
     CUtensorMap tile_map;  // the weight's main plane as a [rows][row bytes] byte matrix (TMA descriptor; first: 64-byte aligned)
@@ -350,10 +350,10 @@ struct Ring {
 };
 
 template <int TYPE, int MH, bool CODES>
-__global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid_constant__ TcParams p) {
+__global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const __grid_constant__ TcParams p) {
     using F = Format<TYPE>;
-    constexpr int kGroups = Shape<MH>::groups, kStageFirst = kDrainWarps, kMiscFirst = kDrainWarps + 4 * kGroups, kCols = Shape<MH>::cols;
-    static_assert(256 * Shape<MH>::drain_regs + 128 * kGroups * Shape<MH>::stage_regs + 128 * Shape<MH>::other_regs <= tc_threads<MH>() * Shape<MH>::launch_regs, "more registers than the launch has: the increase would wait forever");
+    constexpr int kGroups = Shape<MH, CODES>::groups, kStageFirst = kDrainWarps, kMiscFirst = kDrainWarps + 4 * kGroups, kCols = Shape<MH, CODES>::cols;
+    static_assert(256 * Shape<MH, CODES>::drain_regs + 128 * kGroups * Shape<MH, CODES>::stage_regs + 128 * Shape<MH, CODES>::other_regs <= tc_threads<MH, CODES>() * Shape<MH, CODES>::launch_regs, "more registers than the launch has: the increase would wait forever");
     constexpr int kHalves = F::halves, kMinSlices = TYPE == RQ_Q4_K ? 2 : 0;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzled tiles want 1024-byte alignment
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
 
     if (warp < kDrainWarps) {
         // ------------------------------------------------------------ drain warps
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape<MH>::drain_regs));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape<MH, CODES>::drain_regs));
         // Warp w may read accumulator rows 32 (w % 4) .., so four warps drain a sum, and the two sets of four take turns: a sum's wait,
         // loads and release are a chain of some thousand cycles however few its columns. MH = 1: even and odd slices, joined at the
         // end of the tile; MH = 2: a row half each.
@@ -413,6 +413,66 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
             Pair sum[kCols / 2];
 #pragma unroll
             for (int i = 0; i < kCols / 2; ++i) sum[i] = 0;
+            // CODES: the products are exact, so what a sum loses it loses where its terms (32 inputs each) are added up, and up to 448 of them one
+            // after another in one fp32 register lose more than the matvec kernel's tree does. Every few slices the sums go into totals in
+            // tensor memory, and what that addition rounds off stays in the register as the start of the next run. Error against 64 bits,
+            // 14336 inputs and 509 tokens: 2.0e-7 without, 0.7e-7 so; the matvec kernel 0.9e-7. (Other places for the totals: shared memory, twice
+            // the cost, and the L1 it takes is missed by the scale loads; registers spill; a compensated sum at every slice 406 us for 340.)
+            const int own = (MH == 1 ? 2 : 4) * (u1 - u0), run_length = own <= 16 ? 2 : (own <= 64 ? 4 : 8);  // (a set's slices of this segment)
+            int run = 0;
+            bool flushed = false;
+            const uint32_t totals = tmem_base + lane_base + (uint32_t)(accs * acc_cols + set * bn);
+            const Pair minus = pair_of(-1.0f, -1.0f);
+            auto flush = [&]() {
+                run = 0;
+                Pair lost = 0;
+#pragma unroll
+                for (int c = 0; c < kCols; c += 16) {
+                    if (c < bn) {
+                        uint32_t v[16];
+                        if (flushed) {
+                            tmem_ld16(totals + c, v);
+#pragma unroll
+                            for (int j = 0; j < 16; j += 2) {
+                                Pair& s = sum[(c + j) / 2];
+                                const Pair a = pair_of(v[j], v[j + 1]), t = pair_add(a, s);
+                                s = pair_fma(minus, pair_fma(minus, a, t), s);
+                                lost = pair_add(lost, s);
+                                v[j] = __float_as_uint(pair_at(t, 0));
+                                v[j + 1] = __float_as_uint(pair_at(t, 1));
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(pair_at(sum[(c + j) / 2], j & 1));
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) sum[c / 2 + j] = 0;
+                        }
+                        tmem_st16(totals + c, v);
+                    }
+                }
+                tmem_st_wait();
+                flushed = true;
+                // an infinite total has no rounding error to carry on
+                if (!(fabsf(pair_at(lost, 0) + pair_at(lost, 1)) <= 3.402823466e38f)) {
+#pragma unroll
+                    for (int i = 0; i < kCols / 2; ++i) {
+                        const float e0 = pair_at(sum[i], 0), e1 = pair_at(sum[i], 1);
+                        sum[i] = pair_of(fabsf(e0) <= 3.402823466e38f ? e0 : 0.f, fabsf(e1) <= 3.402823466e38f ? e1 : 0.f);
+                    }
+                }
+            };
+            // sum[c ..] = the totals at `at` + sum[c ..]
+            auto add_totals = [&](uint32_t at) {
+#pragma unroll
+                for (int c = 0; c < kCols; c += 16) {
+                    if (c < bn) {
+                        uint32_t v[16];
+                        tmem_ld16(at + c, v);
+#pragma unroll
+                        for (int j = 0; j < 16; j += 2) sum[(c + j) / 2] = pair_add(pair_of(v[j], v[j + 1]), sum[(c + j) / 2]);
+                    }
+                }
+            };
             // this lane's row, kept inside the weight for the scale loads
             auto row_at = [&]() -> int64_t { return min(my_row0 + quarter * 32 + lane, p.rows - 1); };
             // Slice ks of the segment: d0 (and d1: the second half's) scale its sums
@@ -478,6 +538,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                     if (kHalves == 2) mbar_arrive(&acc_empty[acc_at.slot + 1]);
                 }
                 acc_at.skip(2 * kHalves);
+                if (CODES && ++run == run_length) flush();
             };
             constexpr int kStride = MH == 1 ? 2 : 1;
             const int s0 = MH == 1 ? set : 0;  // (a segment has an even number of slices: parity by segment is parity overall)
@@ -515,6 +576,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
             }
             slice_base += main_slices + extra;
             const int r0 = quarter * 32 + lane;
+            if (CODES && flushed) add_totals(totals);
             if (MH == 1) {
                 // odd slices' sums join the even ones'
                 if (set == 1) {
@@ -565,18 +627,21 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
                     __threadfence();
 #pragma unroll
                     for (int j = 0; j < kCols / 2; ++j) sum[j] = 0;
-                    for (int c = c0; c <= c1; ++c) {
+                    for (int c = c0; c <= c1; c += 2) {
+                        const bool two = c < c1;
                         const float* piece = p.partial + (size_t)deal.place(t, c) * tile_floats + mine;
-                        // sixteen loads in flight (a branch for each would make each wait for the one before); the padding
+                        const float* other = two ? p.partial + (size_t)deal.place(t, c + 1) * tile_floats + mine : piece;
+                        // thirty-two loads in flight (a branch for each would make each wait for the one before); the padding
                         // tokens' places exist and hold nothing that is used
 #pragma unroll
                         for (int j = 0; j < kCols; j += 16) {
                             if (j < bn) {
-                                float v[16];
+                                float v[16], w[16];
 #pragma unroll
-                                for (int q = 0; q < 16; ++q) v[q] = __ldcg(piece + (j + q) * 128 * MH);
+                                for (int q = 0; q < 16; ++q) { v[q] = __ldcg(piece + (j + q) * 128 * MH); w[q] = __ldcg(other + (j + q) * 128 * MH); }
 #pragma unroll
-                                for (int q = 0; q < 16; q += 2) sum[(j + q) / 2] = pair_add(sum[(j + q) / 2], pair_of(v[q], v[q + 1]));
+                                for (int q = 0; q < 16; q += 2)
+                                    sum[(j + q) / 2] = pair_add(sum[(j + q) / 2], two ? pair_add(pair_of(v[q], v[q + 1]), pair_of(w[q], w[q + 1])) : pair_of(v[q], v[q + 1]));
                             }
                         }
                     }
@@ -586,7 +651,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
         }
     } else if (warp < kMiscFirst) {
         // ------------------------------------------------------------ staging groups: stored bytes -> integer operands in tensor memory
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH>::stage_regs));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH, CODES>::stage_regs));
         const int group = (warp - kStageFirst) >> 2, r = (warp & 3) * 32 + lane;
         const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
         Ring a_at(a_slots, group), raw_at(p.raw_slots);
@@ -653,7 +718,7 @@ __global__ void __launch_bounds__(tc_threads<MH>(), 1) rq_tc_kernel(const __grid
             raw_base += main_slices / F::raw_slices * MH;
         }
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH>::other_regs));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH, CODES>::other_regs));
         if (warp < kMiscFirst + kIssuers && elect_one()) {
             // ------------------------------------------------------------ the issuing threads
             const int me = warp - kMiscFirst;
@@ -780,7 +845,7 @@ int launch_tc(const TcParams& p, int ctas, size_t smem, cudaStream_t s) {
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(tc_threads<MH>());
+    cfg.blockDim = dim3(tc_threads<MH, CODES>());
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
