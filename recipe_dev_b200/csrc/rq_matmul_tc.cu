@@ -36,14 +36,14 @@
 // eight) instructions (each costs the same 70 cycles for 16 columns as for 128) and the low products have accumulators of their own;
 // the time goes to unpacking and to the weights' bytes, so three staging groups. MH = 2 (token tiles of up to 96): two row halves share each activation tile, which halves
 // the activation bytes a CTA pulls from L2 (they, at 4 bytes per input and token, are what the large shapes would be bound
-// by); products of hi and lo share an accumulator, four drain warps to a row half with 96 fp32 sums a thread (setmaxnreg). Measured
+// by); products of hi and lo share an accumulator, four drain warps to a row half with 96 fp32 sums a thread (setmaxnreg; CODES: tiles of up to 64). Measured
 // between them (Q4_K 14336 x 4096): the one form for every token count 274 us at 512 tokens where both made 234.
 //
 // What bounds it is the chains of latencies of the staging and drain warps, not the tensor cores (29 % active at 512 tokens) and, but for
 // a few tokens, not the weights' bytes. Measured on one B200, graphs over distinct copies, against the two kernels it replaced (a
 // single accumulator pair, operands staged slice by slice by all warps): Q4_K 14336 x 4096 16 / 64 / 512 tokens 58 / 61 / 294 us ->
 // 33.5 / 48.6 / 191 us; Q6_K 4096 x 14336 int8 55 / 64 / 296 -> 34.9 / 52.4 / 199; Q8_0 4096 x 14336 int8, 509 tokens 5230 us as passes
-// of the matvec kernel -> 340.
+// of the matvec kernel -> 331.
 //
 // The Q4_K minimum term, sum_g (8 * d * sc_g - dmin * m_g) * (sum of x over group g), is a second, 32 times smaller product: per
 // window of eight superblocks two more slices (the terms' fp16 hi and lo) whose "activations" are the group sums.
@@ -415,9 +415,10 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             for (int i = 0; i < kCols / 2; ++i) sum[i] = 0;
             // CODES: the products are exact, so what a sum loses it loses where its terms (32 inputs each) are added up, and up to 448 of them one
             // after another in one fp32 register lose more than the matvec kernel's tree does. Every few slices the sums go into totals in
-            // tensor memory, and what that addition rounds off stays in the register as the start of the next run. Error against 64 bits,
-            // 14336 inputs and 509 tokens: 2.0e-7 without, 0.7e-7 so; the matvec kernel 0.9e-7. (Other places for the totals: shared memory, twice
-            // the cost, and the L1 it takes is missed by the scale loads; registers spill; a compensated sum at every slice 406 us for 340.)
+            // tensor memory, and what that addition rounds off stays in the register as the start of the next run (runs of two to eight slices:
+            // the shorter the segment, the more the additions inside a run weigh). Error against 64 bits, 4096 x 14336 and 509 tokens: 2.0e-7
+            // without, 0.79e-7 so, the matvec kernel 0.90e-7; time 312 -> 331 us, and 14336 x 4096 with 32 tokens 44.7 -> 48.5. (Totals in shared
+            // memory 352 us: the L1 it takes is missed by the scale loads; in registers they spill, 372; a compensated sum at every slice 406.)
             const int own = (MH == 1 ? 2 : 4) * (u1 - u0), run_length = own <= 16 ? 2 : (own <= 64 ? 4 : 8);  // (a set's slices of this segment)
             int run = 0;
             bool flushed = false;
