@@ -2,11 +2,12 @@
 // IQ4_NL, Q8_1, Q2_K, Q3_K, Q8_K, IQ4_XS): fp32 activations against the decoded weights, the reference's run decoders
 // (recipe.rs:7826-7917: one fused-multiply-add chain per unit of 32 values; the units of a row add up, ll:3451-3492; here
 // the additions are regrouped, within the 1e-3 band). A LANE owns a group of 32 values: it fetches the group's bytes in
-// words, turns them into eight words of byte codes whatever the format, dots the codes with 32 inputs it holds in registers
-// and applies the scale and offset of each sixteen once. `.int(8)` never reaches these formats: the reference re-encodes
+// words, turns them into eight words of byte codes whatever the format, and makes them weights with the scale and offset of each
+// sixteen, for 32 inputs it holds in registers. `.int(8)` never reaches these formats: the reference re-encodes
 // them to Q8_0 at load (rq_weight_requantize), and that weight takes the streaming kernel. `.int(4)` stores Q4_1 and dots it
 // with int8 activation records: rq_gemv_q41_int8_kernel below.
 #include "rq_decode.cuh"
+#include "rq_pairs.cuh"
 
 namespace {
 
@@ -227,9 +228,12 @@ template <> struct GroupBytes<RQ_Q3_K> {
 };
 
 // A warp owns ROWS rows, its lanes the groups g, g + 32, ..: a lane reads its group's 32 inputs from shared memory once and uses them
-// for all of its rows, whose bytes are all in flight before the first is decoded. What bounds it is instruction issue (per four
-// weights: two or three to isolate the codes, eight to make them floats, four products). Measured, Q5_K 14336 x 4096, one token: 28.2 us;
-// decoding value by value, every header field once per value, took 175.6.
+// for all of its rows, whose bytes are all in flight before the first is decoded. A weight is put together whole (scale * code + offset,
+// rounded once, as the decoders do) before it meets its input: scaled and offset sums kept apart cost two multiplies less per four weights,
+// but cancel against each other (2.3e-7 against 64 bits where decoding value by value has 1.0e-7, Q5_K over 512 inputs), and a code
+// times a large input can leave the range that the weight's own product stays in. What bounds it is instruction issue (per four
+// weights: two or three to isolate the codes, four to place them, six packed ones). Measured, Q5_K 14336 x 4096, one token: 26.8 us (28.2 with the sums kept apart); decoding value by
+// value, every header field once per value, took 175.6.
 template <int TYPE, int ROWS>
 __global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* x,
                                                                         int64_t sk, int64_t st, float* __restrict__ y, int64_t yn, int64_t yt) {
@@ -257,38 +261,33 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint
             GroupBytes<TYPE> raw[ROWS];
 #pragma unroll
             for (int r = 0; r < ROWS; ++r) raw[r].load(base[r], g);
-            float v[32], half_sum[2] = {0.f, 0.f};
+            Pair v[16];  // the group's inputs
 #pragma unroll
-            for (int j = 0; j < 8; ++j) *(float4*)(v + 4 * j) = *(const float4*)(xs + i * kGroupFloats + 4 * j);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) half_sum[j >> 4] += v[j];
+            for (int j = 0; j < 8; ++j) {
+                const ulonglong2 four = *(const ulonglong2*)(xs + i * kGroupFloats + 4 * j);
+                v[2 * j] = four.x;
+                v[2 * j + 1] = four.y;
+            }
 #pragma unroll
             for (int r = 0; r < ROWS; ++r) {
                 uint32_t c[8];
                 float scale[2], offset[2];
                 raw[r].decode(g, c, scale, offset);
+                Pair even = 0, odd = 0;  // inputs 0, 1 and 2, 3 of every four
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float a = 0.f, b = 0.f;
-#pragma unroll
-                    for (int j = 4 * h; j < 4 * h + 4; ++j) {
-                        // 0x4B0000cc is 2^23 + code: the subtraction leaves the code less its bias, exactly
-                        constexpr float kOff = 8388608.0f + (float)GroupBytes<TYPE>::bias;
-                        a = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7650)) - kOff, v[4 * j], a);
-                        b = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7651)) - kOff, v[4 * j + 1], b);
-                        a = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7652)) - kOff, v[4 * j + 2], a);
-                        b = fmaf(__uint_as_float(__byte_perm(c[j], 0x4B000000u, 0x7653)) - kOff, v[4 * j + 3], b);
-                    }
-                    if (!kOffset || fabsf(half_sum[h]) <= 3.402823466e38f) {
-                        sum[r] = fmaf(scale[h], a + b, sum[r]);
-                        if (kOffset) sum[r] = fmaf(offset[h], half_sum[h], sum[r]);
-                    } else {
-                        // an infinite input (or a NaN): scale and offset taken apart would meet as inf - inf
-                        const int64_t first = ((row0 + r < rows ? row0 + r : rows - 1) * groups + g) * 32 + 16 * h;
-#pragma unroll 1
-                        for (int j = 0; j < 16; ++j) sum[r] = fmaf(rq_decode_value<TYPE>(main_plane, nullptr, first + j, 0), xs[i * kGroupFloats + 16 * h + j], sum[r]);
-                    }
+                for (int j = 0; j < 8; ++j) {
+                    const Pair by = pair_of(scale[j >> 2], scale[j >> 2]), plus = pair_of(offset[j >> 2], offset[j >> 2]);
+                    // 0x4B0000cc is 2^23 + code: the subtraction leaves the code less its bias, exactly
+                    constexpr float kOff = -8388608.0f - (float)GroupBytes<TYPE>::bias;
+                    Pair lo = pair_add(pair_of(__byte_perm(c[j], 0x4B000000u, 0x7650), __byte_perm(c[j], 0x4B000000u, 0x7651)), pair_of(kOff, kOff));
+                    Pair hi = pair_add(pair_of(__byte_perm(c[j], 0x4B000000u, 0x7652), __byte_perm(c[j], 0x4B000000u, 0x7653)), pair_of(kOff, kOff));
+                    lo = kOffset ? pair_fma(lo, by, plus) : pair_mul(lo, by);
+                    hi = kOffset ? pair_fma(hi, by, plus) : pair_mul(hi, by);
+                    even = j ? pair_fma(lo, v[2 * j], even) : pair_mul(lo, v[2 * j]);
+                    odd = j ? pair_fma(hi, v[2 * j + 1], odd) : pair_mul(hi, v[2 * j + 1]);
                 }
+                const Pair both = pair_add(even, odd);
+                sum[r] += pair_at(both, 0) + pair_at(both, 1);
             }
         }
     }

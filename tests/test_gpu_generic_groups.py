@@ -46,3 +46,38 @@ def test_infinite_inputs_meet_the_weight_itself(rq_ctx, oracle, t):
             want = dense[:, at] * np.float32(bad)
         assert np.array_equal(np.isnan(y), np.isnan(want))
         assert np.array_equal(y[~np.isnan(want)], want[~np.isnan(want)])
+
+
+def _value_by_value(dense, x):
+    """Every weight decoded to fp32 and met with its input by one fused operation: 32 chains over the units of a row, then a tree."""
+    units = dense.reshape(dense.shape[0], -1, 32).astype(np.float64)
+    acc = np.zeros((dense.shape[0], 32), np.float32)
+    for u in range(units.shape[1]):
+        acc = (acc.astype(np.float64) + units[:, u] * x[32 * u : 32 * u + 32].astype(np.float64)).astype(np.float32)
+    while acc.shape[1] > 1:
+        acc = acc[:, : acc.shape[1] // 2] + acc[:, acc.shape[1] // 2 :]
+    return acc[:, 0]
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("cols", [512, 4096])
+def test_as_close_to_64_bits_as_decoding_value_by_value(rq_ctx, oracle, t, cols):
+    rows = 600
+    blocks = ol.random_blocks(t, rows * cols // ol.GEOMETRY[t][0], np.random.default_rng(t + cols))
+    w = rq_ctx.weight_from_host(t, blocks, rows, cols)
+    dense = oracle.dequantize(t, blocks).reshape(rows, cols)
+    x = oracle.normal(93, t, cols, 1.0)
+    exact = dense.astype(np.float64) @ x.astype(np.float64)
+    error = np.linalg.norm(rq_ctx.matvec(w, torch_cuda(x)).cpu().numpy() - exact)
+    assert error <= np.linalg.norm(_value_by_value(dense, x) - exact)
+
+
+@pytest.mark.parametrize("t", TYPES)
+def test_inputs_whose_products_with_the_codes_leave_the_range(rq_ctx, oracle, t):
+    rows, cols = 90, 512
+    blocks = ol.random_blocks(t, rows * cols // ol.GEOMETRY[t][0], np.random.default_rng(t + 7))
+    w = rq_ctx.weight_from_host(t, blocks, rows, cols)
+    dense = oracle.dequantize(t, blocks).reshape(rows, cols).astype(np.float64)
+    x = (5e37 * np.clip(oracle.normal(94, t, cols, 1.0), -4, 4)).astype(np.float32)
+    y = rq_ctx.matvec(w, torch_cuda(x)).cpu().numpy().astype(np.float64)
+    assert np.all(np.abs(y - dense @ x.astype(np.float64)) <= 2.0**-20 * (np.abs(dense) @ np.abs(x.astype(np.float64))))
