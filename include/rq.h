@@ -52,7 +52,10 @@ enum { RQ_Q4_0 = 2, RQ_Q8_0 = 8, RQ_Q4_K = 12, RQ_Q6_K = 14,
        RQ_Q8_1 = 9, RQ_Q2_K = 10, RQ_Q3_K = 11, RQ_Q8_K = 15, RQ_IQ4_XS = 23 };
 
 /* Activation handling, what `.fp(32)` / `.int(8)` select (recipe.rs:14027-14054, :22326-22369):
- * FLOAT keeps the activations as they are (run decoders, recipe.rs:7826-7917);
+ * FLOAT keeps the activations as they are (run decoders, recipe.rs:7826-7917). In sums over the four formats with whole 256-value
+ * units a row, each group of 32 inputs is held as 24-bit integers in steps of its largest magnitude / 8355000: an input is off by
+ * at most 2^-24 of that. A group whose inputs (other than zeros) are on average some 2^7 or more below its largest, or whose largest is
+ * below 2^-100, is not: the few inputs that stand out, or all of them, meet the weights as fp32 numbers by themselves;
  * INT8 rounds them to int8 records with one fp32 step per `step` inputs (amd-nv-cpu.ll:1381-1517). */
 enum { RQ_ACT_FLOAT = 0, RQ_ACT_INT8 = 1,
        /* INT8 where the caller states that x is the same column, token count and step as the previous
@@ -192,7 +195,7 @@ int rq_softcap(rq_ctx* ctx, const float* x, int64_t n, double cap, float* y, voi
  * arguments as rq_matvec.
  * Range on the tensor-core routes, int8 over Q8_0 / Q4_0 excepted: activations pass through fp16, so one of
  * magnitude above 65504 overflows (the result row is inf / NaN) and one below 6e-8 counts as zero.
- * rq_matvec has no such limit. */
+ * rq_matvec has no such limit (how it holds fp32 inputs: RQ_ACT_FLOAT above). */
 int rq_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t x_k_stride, int64_t x_t_stride, int tokens,
               float* y, int64_t y_n_stride, int64_t y_t_stride, int act_mode, int step, void* stream);
 

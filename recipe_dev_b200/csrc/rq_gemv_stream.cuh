@@ -129,11 +129,19 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 template <int THREADS>
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
+// the same, and whether any of them came with `mine`
+template <int THREADS>
+__device__ __forceinline__ bool consumer_sync_any(bool mine) {
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.u32 %0, 1, 0, q;\n}" : "=r"(any) : "r"((uint32_t)mine), "n"(THREADS) : "memory");
+    return any != 0;
+}
 __device__ __forceinline__ int dp4a_us(uint32_t a_unsigned, uint32_t b_signed, int c) {
     int d;
     asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a_unsigned), "r"(b_signed), "r"(c));
     return d;
 }
+__device__ __forceinline__ int dp4a_uu(uint32_t a, uint32_t b, int c) { return (int)__dp4a(a, b, (uint32_t)c); }
 __device__ __forceinline__ int dp4a_ss(uint32_t a, uint32_t b, int c) { return __dp4a((int)a, (int)b, c); }
 
 // Four unsigned bytes of `w` as floats, exactly: 0x4B0000bb is 2^23 + bb.
@@ -151,14 +159,16 @@ __device__ __forceinline__ float diff_of_products(float a, float b, float c, flo
 //   INT8  (336 bytes): codes[256] int8 | d[8] fp32 @256 | sum16[16] int16 @288 | sum32[8] int16 @320
 //          d = the step of each 32-value group, sum16 / sum32 = the sum of the codes of each
 //          16-value slice / 32-value group
-//   FLOAT (976 bytes): fp32 inputs as 24-bit integers in units of their 32-input group's step (the group's largest magnitude
-//          over 8355000; the largest group's error is 2^-24 of that magnitude, what an fp32 sum loses anyway), in three planes
-//          of signed base-256 digits: high[256] | middle[256] | low[256] | step[8] fp32 @768 | sum32[8] fp32 @800 (the sum of
-//          the group's inputs) | sum16[16] @832: per 16-input slice two int32, the sum of its 256 * middle + low digits and
-//          the sum of its high digits. A byte of weight codes then meets the activations in dp4a, four products an
+//   FLOAT (1008 bytes): fp32 inputs as 24-bit integers in units of their 32-input group's step (the group's largest magnitude
+//          over 8355000), in three planes of signed base-256 digits: high[256] | middle[256] | low[256] | step[8] fp32 @768 |
+//          sum32[8] fp32 @800 (the sum of the group's inputs) | sum16[16] @832: per 16-input slice two int32, the sum of its
+//          256 * middle + low digits and the sum of its high digits | which[8] @960, odd[8] @992: a word a group, which of its
+//          inputs stay out of all this, and a byte, whether any do (the word is valid then; odd_groups_to_smem). An input is off by at most 2^-24 of the largest, what a sum that the largest is part of
+//          loses anyway; where it is not part of it (its weight is zero) inputs far below it would lose more, and such
+//          groups are what those are for. A byte of weight codes then meets the activations in dp4a, four products an
 //          instruction and exact, where fp32 products cost a conversion and a multiply-add each: three dp4a and a mask per
 //          four weights against thirteen instructions.
-// 336 = 84 words and 976 = 244 words are odd counts of sixteen bytes, so the 128-bit loads of eight threads
+// 336 = 84 words and 1008 = 252 words are odd counts of sixteen bytes, so the 128-bit loads of eight threads
 // on adjacent units fall in eight different bank groups.
 
 // The int8 activations one item needs: the 128 codes of its half record, their four steps, and
@@ -835,20 +845,78 @@ __device__ __forceinline__ void dot_regs_float(const ItemRegs<RQ_Q4_0> (&r)[R], 
     for (int k = 0; k < R; ++k) out[k] = have[k] ? acc[k] : 0.f;
 }
 
+// ------------------------------------------------------------------------------------------
+// Inputs that the digits of their group would not hold: each meets its weights by itself, one fused fp32 operation a row. A group's
+// byte in `odd` says whether it has any, its word in `which` which they are (odd_groups_to_smem). Rare, and the loops are kept rolled: the weights are picked out of the registers.
+// ------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i < 2 ? (i == 0 ? v.x : v.y) : (i == 2 ? v.z : v.w); }
+// weight k of group g of the item
+__device__ __forceinline__ float weight_of(const ItemRegs<RQ_Q4_K>& r, int h, int g, int k) {
+    const uint4 line = g < 2 ? (k < 16 ? r.q[0] : r.q[1]) : (k < 16 ? r.q[2] : r.q[3]);
+    const int code = (word_of(line, (k >> 2) & 3) >> (8 * (k & 3) + 4 * (g & 1))) & 15;
+    const uint32_t scw = h == 0 ? (r.hdr.y & 0x3f3f3f3fu) : ((r.hdr.w & 0x0f0f0f0fu) | ((r.hdr.y >> 2) & 0x30303030u));
+    const uint32_t mnw = h == 0 ? (r.hdr.z & 0x3f3f3f3fu) : (((r.hdr.w >> 4) & 0x0f0f0f0fu) | ((r.hdr.z >> 2) & 0x30303030u));
+    // both products are exact, their difference is rounded once
+    return diff_of_products(rq_h2f((uint16_t)(r.hdr.x & 0xffff)), (float)(((scw >> (8 * g)) & 0xff) * code), rq_h2f((uint16_t)(r.hdr.x >> 16)), (float)((mnw >> (8 * g)) & 0xff));
+}
+__device__ __forceinline__ float weight_of(const ItemRegs<RQ_Q6_K>& r, int, int g, int k) {
+    const uint4 low = (g & 1) == 0 ? (k < 16 ? r.ql[0] : r.ql[1]) : (k < 16 ? r.ql[2] : r.ql[3]), high = k < 16 ? r.qh[0] : r.qh[1];
+    const int w = (k >> 2) & 3, byte = 8 * (k & 3), at = 2 * g + (k >> 4);
+    const int code = ((word_of(low, w) >> (byte + (g < 2 ? 0 : 4))) & 15) | (((word_of(high, w) >> (byte + 2 * g)) & 3) << 4);
+    const int sc = (int)(int8_t)((at < 4 ? r.sc.x : r.sc.y) >> (8 * (at & 3)));
+    return __fmul_rn(rq_h2f((uint16_t)r.d16), (float)(sc * (code - 32)));
+}
+__device__ __forceinline__ float weight_of(const ItemRegs<RQ_Q8_0>& r, int, int g, int k) {
+    const uint4 a = g < 2 ? (g == 0 ? r.q[0] : r.q[2]) : (g == 2 ? r.q[4] : r.q[6]), b = g < 2 ? (g == 0 ? r.q[1] : r.q[3]) : (g == 2 ? r.q[5] : r.q[7]);
+    const int code = (int)(int8_t)(word_of(k < 16 ? a : b, (k >> 2) & 3) >> (8 * (k & 3)));
+    return __fmul_rn(rq_h2f((uint16_t)((g < 2 ? r.dd.x : r.dd.y) >> (16 * (g & 1)))), (float)code);
+}
+__device__ __forceinline__ float weight_of(const ItemRegs<RQ_Q4_0>& r, int, int g, int k) {
+    const uint4 line = g < 2 ? (g == 0 ? r.q[0] : r.q[1]) : (g == 2 ? r.q[2] : r.q[3]);
+    const int code = (int)((word_of(line, (k >> 2) & 3) >> (8 * (k & 3) + 4 * (k >> 4))) & 15) - 8;
+    return __fmul_rn(rq_h2f((uint16_t)((g < 2 ? r.dd.x : r.dd.y) >> (16 * (g & 1)))), (float)code);
+}
+// adds to out[] what the item's odd inputs are worth; x: the item's 128 inputs, sk apart
+template <int TYPE, int R>
+__device__ __forceinline__ void add_odd_inputs(const ItemRegs<TYPE> (&r)[R], const bool (&have)[R], uint32_t odd, const uint32_t* which, const float* x, int64_t sk, int h, float (&out)[R]) {
+#pragma unroll 1
+    for (int g = 0; g < 4; ++g, odd >>= 8) {
+#pragma unroll 1
+        for (uint32_t left = odd & 0xff ? which[g] : 0u; left; left &= left - 1) {
+            const int i = __ffs(left) - 1;
+            const float v = x[(int64_t)(32 * g + i) * sk];
+#pragma unroll
+            for (int k = 0; k < R; ++k)
+                if (have[k]) out[k] = fmaf(weight_of(r[k], h, g, i), v, out[k]);
+        }
+    }
+}
+
 // Sixteen fp32 inputs (slice `slot` of their unit) as 24-bit integers in three digit planes of the unit record `rec`; the lane's
 // xor-1 neighbour holds the other slice of the 32-input group. An input that is no number or infinite makes the group's step a
 // NaN, and with it every sum the group enters, as fp32 products with offsets taken off afterwards do.
-__device__ __forceinline__ void digits_to_smem(const float (&f)[16], uint8_t* __restrict__ rec, int slot, bool store) {
-    uint32_t top = 0;
+// True when the digits do not do for the group: its inputs are on average more than seven powers of two below the largest (a zero counts
+// as far below here), or the largest is below 2^-100 and the step would leave the normal range. The group's odd byte is then
+// one, and odd_groups_to_smem does it over. Rare by the numbers: of groups of normal values none, of silu(g) * u less than one in ten thousand.
+// Measured, looking alone: a decode layer with fp32 activations 64.5 -> 66.8 us, an expert bank 28.9 -> 29.1 us with one token, 86.1 -> 88.1
+// with sixteen (with a second copy of the row loop for launches without such groups 67.2: the kernel runs on a cold instruction cache).
+// (`used` false: a bank's slot without an expert, whose inputs are whatever lies there.)
+__device__ __forceinline__ bool digits_to_smem(const float (&f)[16], uint8_t* __restrict__ rec, int slot, bool store, bool used) {
+    uint32_t top = 0, a[16], exponents[4];  // half the exponents of four inputs, a byte each
 #pragma unroll
-    for (int j = 0; j < 16; ++j) top = max(top, __float_as_uint(f[j]) & 0x7fffffffu);  // magnitudes of floats order as their bits
+    for (int j = 0; j < 16; ++j) a[j] = __float_as_uint(f[j]) & 0x7fffffffu;  // magnitudes of floats order as their bits
+#pragma unroll
+    for (int j = 0; j < 16; ++j) top = max(top, a[j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) exponents[j] = __byte_perm(__byte_perm(a[4 * j], a[4 * j + 1], 0x0073), __byte_perm(a[4 * j + 2], a[4 * j + 3], 0x0073), 0x5410);
+    int magnitude = dp4a_uu(exponents[1], 0x01010101u, dp4a_uu(exponents[0], 0x01010101u, 0)) + dp4a_uu(exponents[3], 0x01010101u, dp4a_uu(exponents[2], 0x01010101u, 0));
     top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    magnitude += __shfl_xor_sync(0xffffffffu, magnitude, 1);
     const bool finite = top < 0x7f800000u;
-    // below 2^-100 the step itself would leave the normal range: the inputs are scaled up first (exactly)
-    const float lift = top < 0x0d800000u ? 1.2676506e30f : 1.0f, drop = top < 0x0d800000u ? 7.8886091e-31f : 1.0f;
-    const float largest = finite ? __fmul_rn(__uint_as_float(top), lift) : 0.f;
+    const bool odd = used && finite && top != 0 && (top < 0x0d800000u || 16 * ((int)(top >> 23) - 7) - 8 > magnitude);  // (a half rounds down by a quarter on average)
+    const float largest = finite ? __uint_as_float(top) : 0.f;
     const float inverse = largest > 0.f ? __fdiv_rn(8355000.0f, largest) : 0.f;
-    const float step = !finite ? __uint_as_float(0x7fffffffu) : (largest > 0.f ? __fmul_rn(__fdiv_rn(largest, 8355000.0f), drop) : 0.f);
+    const float step = !finite ? __uint_as_float(0x7fffffffu) : (largest > 0.f ? __fdiv_rn(largest, 8355000.0f) : 0.f);
     uint4 plane[3];
     uint32_t* pw[3] = {(uint32_t*)&plane[0], (uint32_t*)&plane[1], (uint32_t*)&plane[2]};
     int sum = 0, sum_high = 0;
@@ -857,7 +925,7 @@ __device__ __forceinline__ void digits_to_smem(const float (&f)[16], uint8_t* __
         uint32_t m[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int n = finite ? __float2int_rn(__fmul_rn(__fmul_rn(f[4 * j + b], lift), inverse)) : 0;  // |n| <= 8355001 < 2^23 - 2^15
+            const int n = finite ? __float2int_rn(__fmul_rn(f[4 * j + b], inverse)) : 0;  // |n| <= 8355001 < 2^23 - 2^15
             sum += n;
             m[b] = (uint32_t)(n + 0x00808080);  // three biased digits
         }
@@ -877,6 +945,59 @@ __device__ __forceinline__ void digits_to_smem(const float (&f)[16], uint8_t* __
         if ((slot & 1) == 0) {
             ((float*)(rec + 768))[slot >> 1] = step;
             ((float*)(rec + 800))[slot >> 1] = __fmul_rn(step, (float)pair);
+            rec[992 + (slot >> 1)] = odd ? 1 : 0;
+        }
+    }
+    return odd && store;
+}
+
+// The groups whose odd byte digits_to_smem has set, a warp to a group and a lane to an input. The largest inputs leave the digits, one
+// magnitude after another, until the others (zeros not counted) are on average no more than six powers of two below the largest of
+// them; past eight magnitudes, or where the largest is below 2^-100, all do. The group's word says which have left.
+template <int NW>
+__device__ __forceinline__ void odd_groups_to_smem(uint8_t* act, size_t act_bytes, int vectors, int units, const float* x, int64_t sk, int64_t st, int tid) {
+    constexpr int kRecord = RQ_ACT_RECORD_FLOAT;
+    const int lane = tid & 31, per_vec = 8 * units, total = vectors * per_vec;
+#pragma unroll 1
+    for (int base = 32 * (tid >> 5); base < total; base += 32 * NW) {
+        const int mine = base + lane, v_mine = mine / per_vec, g_mine = mine - v_mine * per_vec;
+        unsigned left = __ballot_sync(0xffffffffu, mine < total && act[v_mine * act_bytes + (size_t)(g_mine >> 3) * kRecord + 992 + (g_mine & 7)] != 0);
+#pragma unroll 1
+        for (; left; left &= left - 1) {
+            const int at = base + __ffs(left) - 1, v = at / per_vec, g = at - v * per_vec;
+            uint8_t* rec = act + v * act_bytes + (size_t)(g >> 3) * kRecord;
+            const float f = x[(int64_t)v * st + (int64_t)(32 * g + lane) * sk];
+            const uint32_t a = __float_as_uint(f) & 0x7fffffffu;
+            uint32_t limit = 0;  // the largest of the inputs that stay in the digits; 0: none do
+            bool in = a != 0;
+#pragma unroll 1
+            for (int gone = 0; gone <= 8; ++gone) {
+                const uint32_t top = __reduce_max_sync(0xffffffffu, in ? a : 0u);
+                if (top < 0x0d800000u) break;
+                if (__reduce_add_sync(0xffffffffu, in ? (int)(top >> 23) - (int)(a >> 23) - 6 : 0) <= 0) { limit = top; break; }
+                in = in && a != top;
+            }
+            in = in && limit != 0;
+            const float largest = __uint_as_float(limit);
+            const int n = in ? __float2int_rn(__fmul_rn(f, __fdiv_rn(8355000.0f, largest))) : 0;
+            const float step = limit ? __fdiv_rn(largest, 8355000.0f) : 0.f;
+            const uint32_t m = (uint32_t)(n + 0x00808080);
+            const int high = (int)((m >> 16) & 0xff) - 128;
+            const unsigned half = lane < 16 ? 0x0000ffffu : 0xffff0000u;
+            const int sum = __reduce_add_sync(half, n), sum_high = __reduce_add_sync(half, high);
+            const unsigned odd = __ballot_sync(0xffffffffu, !in && a != 0);
+            uint8_t* to = rec + 32 * (g & 7) + lane;
+            to[0] = (uint8_t)high;
+            to[256] = (uint8_t)((m >> 8) ^ 0x80);
+            to[512] = (uint8_t)(m ^ 0x80);
+            if ((lane & 15) == 0) ((int2*)(rec + 832))[2 * (g & 7) + (lane >> 4)] = make_int2(sum - 65536 * sum_high, sum_high);
+            const int pair = sum + __shfl_xor_sync(0xffffffffu, sum, 16);
+            if (lane == 0) {
+                ((float*)(rec + 768))[g & 7] = step;
+                ((float*)(rec + 800))[g & 7] = __fmul_rn(step, (float)pair);
+                ((uint32_t*)(rec + 960))[g & 7] = odd;
+                rec[992 + (g & 7)] = odd ? 1 : 0;
+            }
         }
     }
 }
@@ -1269,18 +1390,23 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             };
             int v = tid / per_vec, s2 = tid - v * per_vec;
             float cur[16], nxt[16];
+            bool odd = false;
+            const int used = p.plan && p.act_vectors > 1 ? plan->subs : p.act_vectors;
             fetch(tid, v, s2, cur);
 #pragma unroll 1
             for (int base_i = 0; base_i < total; base_i += kConsumers) {  // uniform: the two threads of a group exchange by shuffles
                 int nv = v + adv_v, ns = s2 + adv_s;
                 if (ns >= per_vec) { ns -= per_vec; ++nv; }
                 fetch(base_i + kConsumers + tid, nv, ns, nxt);
-                digits_to_smem(cur, act_smem + v * p.act_bytes + (size_t)(s2 >> 4) * kRecord, s2 & 15, base_i + tid < total);
+                odd |= digits_to_smem(cur, act_smem + v * p.act_bytes + (size_t)(s2 >> 4) * kRecord, s2 & 15, base_i + tid < total, v < used);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) cur[j] = nxt[j];
                 v = nv; s2 = ns;
             }
-            consumer_sync<kConsumers>();
+            if (__builtin_expect(consumer_sync_any<kConsumers>(odd), 0)) {
+                odd_groups_to_smem<NW>(act_smem, p.act_bytes, p.act_vectors, p.units, xbase + (int64_t)tok0 * p.st, p.sk, p.st, tid);
+                consumer_sync<kConsumers>();
+            }
         } else if (MODE == RQ_ACT_INT8 && T == 4) {
             // four tokens' records, interleaved unit by unit (the layout dot_regs_tok4 reads); a token past
             // the end of the batch is staged as zeros
@@ -1442,6 +1568,8 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             const size_t my_off = (size_t)row_in_pass * row_bytes + (size_t)my_u * p.unit_bytes;
             const size_t pass_bytes = (size_t)rows_per_pass * row_bytes;
             const bool writer = (lane & (group - 1)) == 0;
+            // whether this thread's half record has inputs that are not in the digits
+            const uint32_t odd = MODE == RQ_ACT_FLOAT ? *(const uint32_t*)(act_smem + (size_t)my_u * kRecord + 992 + 4 * my_h) : 0u;
             // Gated launches: the sums of a virtual row's gate and up rows wait in the warp's lanes, one virtual row a lane, until the
             // lanes are full or the rows are over: silu goes through double precision, a long chain that one lane would otherwise walk
             // for every row by itself.
@@ -1499,7 +1627,13 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
 #pragma unroll
                         for (int k = 0; k < R; ++k) v[j][k] = have[k] ? dot_regs(wr[k], areg[j], my_h) : 0.f;
                 } else {
+                    float extra[R];
+#pragma unroll
+                    for (int k = 0; k < R; ++k) extra[k] = 0.f;
+                    if (__builtin_expect(odd != 0, 0)) add_odd_inputs<TYPE, R>(wr, have, odd, (const uint32_t*)(act_smem + (size_t)my_u * kRecord + 960 + 16 * my_h), xbase + (int64_t)tok0 * p.st + (int64_t)(256 * my_u + 128 * my_h) * p.sk, p.sk, my_h, extra);
                     dot_regs_float<R>(wr, have, act_smem + (size_t)my_u * kRecord, my_h, v[0]);
+#pragma unroll
+                    for (int k = 0; k < R; ++k) v[0][k] = __fadd_rn(v[0][k], extra[k]);  // (not contracted with what made v: the same bits in every scheme)
                 }
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) {
@@ -1668,8 +1802,12 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                             wr[0].load(w, sc, my_h, my_u);
 #pragma unroll
                             for (int t = 0; t < T; ++t) {
-                                dot_regs_float<1>(wr, have, a0 + t * p.act_bytes, my_h, v);
-                                part[t * stage_items + tid] = v[0];
+                                const uint8_t* rec = a0 + t * p.act_bytes;
+                                const uint32_t odd = *(const uint32_t*)(rec + 992 + 4 * my_h);
+                                float extra[1] = {0.f};
+                                if (__builtin_expect(odd != 0, 0)) add_odd_inputs<TYPE, 1>(wr, have, odd, (const uint32_t*)(rec + 960 + 16 * my_h), xbase + (int64_t)(tok0 + sg.act[my_s] + t) * p.st + (int64_t)(256 * my_u + 128 * my_h) * p.sk, p.sk, my_h, extra);
+                                dot_regs_float<1>(wr, have, rec, my_h, v);
+                                part[t * stage_items + tid] = __fadd_rn(v[0], extra[0]);
                             }
                         }
                     }

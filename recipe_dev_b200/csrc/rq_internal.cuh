@@ -73,7 +73,7 @@ struct DeviceGuard {
 };
 
 // fp32 activations of 256 inputs in the streaming kernel's shared memory (rq_gemv_stream.cuh)
-#define RQ_ACT_RECORD_FLOAT 976
+#define RQ_ACT_RECORD_FLOAT 1008
 
 // Whether an INT8 call quantises inside the matvec launch. Every CTA of such a launch reads all of x: beyond 8192 inputs that
 // traffic (some 300 CTAs x 4 bytes x inputs) costs more than the quantiser launch it saves.
