@@ -227,15 +227,24 @@ template <> struct GroupBytes<RQ_Q3_K> {
     }
 };
 
+// CTAs the registers are cut for: what is in flight per SM counts more than what a warp has in flight by itself, until the formats of many
+// words a group begin to spill with four rows. (4096 x 4096, a row a warp, four CTAs: Q4_1 6.8 us, Q5_0 7.5, Q2_K 7.3; left to the
+// compiler 8.6, 9.7, 9.8. Q5_K 14336 x 4096, four rows: two CTAs 22.9, three 35.6.)
+template <int TYPE, int ROWS>
+constexpr int ctas_per_sm() {
+    constexpr bool many = TYPE == RQ_Q5_K || TYPE == RQ_Q3_K || TYPE == RQ_Q8_1 || TYPE == RQ_Q8_K || TYPE == RQ_IQ4_XS;
+    return ROWS == 1 ? 4 : (ROWS == 4 && many ? 2 : 3);
+}
+
 // A warp owns ROWS rows, its lanes the groups g, g + 32, ..: a lane reads its group's 32 inputs from shared memory once and uses them
 // for all of its rows, whose bytes are all in flight before the first is decoded. A weight is put together whole (scale * code + offset,
 // rounded once, as the decoders do) before it meets its input: scaled and offset sums kept apart cost two multiplies less per four weights,
 // but cancel against each other (2.3e-7 against 64 bits where decoding value by value has 1.0e-7, Q5_K over 512 inputs), and a code
 // times a large input can leave the range that the weight's own product stays in. What bounds it is instruction issue (per four
-// weights: two or three to isolate the codes, four to place them, six packed ones). Measured, Q5_K 14336 x 4096, one token: 26.8 us (28.2 with the sums kept apart); decoding value by
+// weights: two or three to isolate the codes, four to place them, six packed ones). Measured, Q5_K 14336 x 4096, one token: 26.5 us (28.2 with the sums kept apart); decoding value by
 // value, every header field once per value, took 175.6.
 template <int TYPE, int ROWS>
-__global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* x,
+__global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* x,
                                                                         int64_t sk, int64_t st, float* __restrict__ y, int64_t yn, int64_t yt) {
     extern __shared__ __align__(16) float xs[];
     constexpr bool kOffset = TYPE == RQ_Q4_1 || TYPE == RQ_Q5_1 || TYPE == RQ_Q5_K || TYPE == RQ_Q2_K;
@@ -273,7 +282,7 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint
                 uint32_t c[8];
                 float scale[2], offset[2];
                 raw[r].decode(g, c, scale, offset);
-                Pair even = 0, odd = 0;  // inputs 0, 1 and 2, 3 of every four
+                Pair acc[2][2];  // per sixteen: inputs 0, 1 and 2, 3 of every four
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const Pair by = pair_of(scale[j >> 2], scale[j >> 2]), plus = pair_of(offset[j >> 2], offset[j >> 2]);
@@ -283,10 +292,10 @@ __global__ void __launch_bounds__(kWarps * 32) rq_gemv_generic_kernel(const uint
                     Pair hi = pair_add(pair_of(__byte_perm(c[j], 0x4B000000u, 0x7652), __byte_perm(c[j], 0x4B000000u, 0x7653)), pair_of(kOff, kOff));
                     lo = kOffset ? pair_fma(lo, by, plus) : pair_mul(lo, by);
                     hi = kOffset ? pair_fma(hi, by, plus) : pair_mul(hi, by);
-                    even = j ? pair_fma(lo, v[2 * j], even) : pair_mul(lo, v[2 * j]);
-                    odd = j ? pair_fma(hi, v[2 * j + 1], odd) : pair_mul(hi, v[2 * j + 1]);
+                    acc[j >> 2][0] = j & 3 ? pair_fma(lo, v[2 * j], acc[j >> 2][0]) : pair_mul(lo, v[2 * j]);
+                    acc[j >> 2][1] = j & 3 ? pair_fma(hi, v[2 * j + 1], acc[j >> 2][1]) : pair_mul(hi, v[2 * j + 1]);
                 }
-                const Pair both = pair_add(even, odd);
+                const Pair both = pair_add(pair_add(acc[0][0], acc[0][1]), pair_add(acc[1][0], acc[1][1]));
                 sum[r] += pair_at(both, 0) + pair_at(both, 1);
             }
         }
