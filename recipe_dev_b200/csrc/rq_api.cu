@@ -155,13 +155,15 @@ static const char* wait_code_text(int code) {
         case 2: return "matvec producer: a copy it issued never landed";
         case 3: return "matvec consumer: a stage never arrived";
         case 4: return "matvec producer: an earlier copy of its window never landed";
-        case 11: return "batched product, staging warps: a stage never came free";
-        case 12: return "batched product, drain warps: the last product never finished";
-        case 13: return "batched product, issuing warp: a stage was never filled";
-        case 14: return "batched product, drain warps: an accumulator never filled";
-        case 15: return "batched product, issuing warp: an accumulator never came free";
-        case 16: return "batched product, copy warp: a stage never came free";
-        case 17: return "batched product: the activation sums never arrived";
+        case 11: return "batched product, staging warps: an operand slot never came free";
+        case 13: return "batched product, issuing thread: an operand was never staged";
+        case 14: return "batched product, drain warps: a sum was never finished";
+        case 15: return "batched product, issuing thread: an accumulator never came free";
+        case 16: return "batched product, activation copies: a slot never came free";
+        case 17: return "batched product, issuing thread: a slice of the activations never arrived";
+        case 18: return "batched product, staging warps: the stored bytes never arrived";
+        case 19: return "batched product, copies of stored bytes: a slot never came free";
+        case 20: return "batched product, drain warps: the activations' steps never arrived";
         case 21: return "wait self-test: the barrier nothing arrives on";
         case 31: return "exchange: a peer's arrival flag never came";
         default: return "unknown wait";
@@ -437,7 +439,7 @@ extern "C" int rq_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_
     if (sk <= 0 || yn <= 0 || (tokens > 1 && (st <= 0 || yt <= 0))) return rq_fail(RQ_ERR_INVALID, "rq_matmul: strides must be positive");
     DeviceGuard guard(ctx->device);
     // The tensor-core kernel, for fp32 activations and for int8 windows from some length on: below it the matvec kernel's integer dots,
-    // four tokens a pass, are faster. Q8_0 / Q4_0: nine positions, a third pass (Q8_0 14336 x 4096, ten: 50.8 us there, 39.1 here; eight:
+    // four tokens a pass, are faster. Q8_0 / Q4_0: nine positions, a third pass (Q8_0 14336 x 4096, ten: 50.8 us there, 40.8 here; eight:
     // 35.8 there); five where a pass takes an SM per CTA (more than 7680 inputs). The K-quants stay at twelve (Q4_K 14336 x
     // 4096, ten: 46.4 there, 33.9 here): below that their products keep clear of fp16's range, as they always have.
     const bool codes = w->type == RQ_Q8_0 || w->type == RQ_Q4_0;

@@ -477,7 +477,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 const Pair scale0 = pair_of(d0, d0), scale1 = pair_of(d1, d1);
                 if constexpr (CODES) {
                     const int slot = all % kStepSlots;
-                    if (!dead && !mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
+                    if (!dead && !mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 20); dead = true; }
                     const float *d8 = &step_ring[slot][0][0], *e8 = d8 + bn;
 #pragma unroll
                     for (int c = 0; c < kCols; c += 16) {
