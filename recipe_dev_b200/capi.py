@@ -406,7 +406,7 @@ class Context:
         return y
 
     def matmul(self, w: Weight, x, y=None, act_mode: int = ACT_FLOAT, step: int = 32, stream=None):
-        """x: CUDA fp32 [tokens, cols] -> y [tokens, rows]; the tensor-core path for RQ_ACT_FLOAT."""
+        """x: CUDA fp32 [tokens, cols] -> y [tokens, rows]: the tensor cores for fp32 activations and longer int8 windows, else the matvec kernels."""
         import torch
 
         tokens, cols = x.shape

@@ -12,7 +12,7 @@
 // per row adds the row's partials in item order: no floating-point atomics, the same bits on
 // every run.
 // The activation column sits in shared memory as one padded record per 256 inputs (int8 codes
-// with their steps and slice sums, or fp32 inputs as three planes of digits), padded so that threads on
+// with their steps and slice sums, or fp32 inputs as three planes of digits and a list of those that stay out), padded so that threads on
 // adjacent units read different banks; it is staged while the first weight stages are in flight.
 //
 // Every wait on an mbarrier is bounded in time: when the limit runs out a thread records an
@@ -677,8 +677,8 @@ __device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q4_0> (&r)[R], c
 // fp32 activations: the weights of the thread's R rows sit in registers, the digits of the item's 128 inputs come from the unit
 // record in shared memory and each word serves all R rows. A sum over a slice or group is three exact integers, put together
 // in fp32 once and scaled (by the step first: a step times a weight's scale could leave the normal range). Every caller, whatever its R, has the same operations in the same order, so a row has the same
-// bits whichever path computes it. Measured, one token: Q4_K 14336 x 4096 12.6 us, Q6_K 4096 x 14336 20.2 us; with fp32 products 19.1 and
-// 32.7 us.
+// bits whichever path computes it. Measured, one token, before digits_to_smem looked for odd groups (see there): Q4_K 14336 x 4096 12.6 us,
+// Q6_K 4096 x 14336 20.2 us; with fp32 products 19.1 and 32.7 us.
 // ------------------------------------------------------------------------------------------
 struct DigitWords { uint4 d[3]; };  // sixteen inputs: high, middle, low
 __device__ __forceinline__ void load_digits(const uint8_t* __restrict__ at, DigitWords& v) {
@@ -898,7 +898,7 @@ __device__ __forceinline__ void add_odd_inputs(const ItemRegs<TYPE> (&r)[R], con
 // True when the digits do not do for the group: its inputs are on average more than seven powers of two below the largest (a zero counts
 // as far below here), or the largest is below 2^-100 and the step would leave the normal range. The group's odd byte is then
 // one, and odd_groups_to_smem does it over. Rare by the numbers: of groups of normal values none, of silu(g) * u less than one in ten thousand.
-// Measured, looking alone: a decode layer with fp32 activations 64.5 -> 66.8 us, an expert bank 28.9 -> 29.1 us with one token, 86.1 -> 88.1
+// Measured, looking alone: a decode layer with fp32 activations 64.6 -> 66.0 us, an expert bank 28.8 -> 29.8 us with one token, 86.0 -> 88.1
 // with sixteen (with a second copy of the row loop for launches without such groups 67.2: the kernel runs on a cold instruction cache).
 // (`used` false: a bank's slot without an expert, whose inputs are whatever lies there.)
 __device__ __forceinline__ bool digits_to_smem(const float (&f)[16], uint8_t* __restrict__ rec, int slot, bool store, bool used) {
@@ -1873,7 +1873,7 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     // interleave, and when a CTA of one launch exits, a CTA of the next launch (programmatic
     // dependent launch) takes its place and prefetches weights while the other is still working.
     // five consumer warps: three CTAs of six warps per SM. one_per_sm: a single CTA with the whole SM's shared memory, for
-    // launches whose staged activations leave two CTAs no room for a ring (fp32 records of 14336 inputs are 62 KB).
+    // launches whose staged activations leave two CTAs no room for a ring (fp32 records of 32768 inputs are 126 KB).
     // token_pairs (int8 windows over rows of five consumer warps): two tokens' records in every thread's registers, 170
     // registers a thread, so two CTAs per SM instead of three
     const int kCtasPerSm = one_per_sm ? 1 : (NW == 5 && !token_pairs && p.tokens == 1 ? 3 : 2);
