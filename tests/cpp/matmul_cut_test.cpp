@@ -1,5 +1,5 @@
 // The cut of a batched product (recipe_dev_b200/csrc/rq_matmul_cut.cuh) walked on the host: every unit of every output tile is taken
-// exactly once, every shared tile is added up by exactly one of its CTAs, and a work area sized ahead of time holds the call's. Built and run by tests/test_matmul_cut.py. Prints "ok".
+// exactly once, the rings fit, every shared tile is added up by exactly one of its CTAs, and a work area sized ahead of time holds the call's. Built and run by tests/test_matmul_cut.py. Prints "ok".
 #include <cstdio>
 #include <vector>
 
@@ -16,6 +16,12 @@ static int walk_call(int type, bool codes, int sms, int64_t rows, int64_t cols, 
     const TcCut c = tc_cut(type, codes, sms, rows, cols, tokens);
     const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles;
     if (c.tiles_m * 128LL * c.mh < rows || (int64_t)c.n_tiles * c.bn < tokens) return fail("outputs outside every tile", type, codes, sms, rows, cols, tokens);
+    // tensor memory: accumulators, totals of the codes' sums, operand slots; rings that alternate between two issuing threads; shared memory
+    const bool k = type == RQ_Q4_K || type == RQ_Q6_K;
+    const int acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn;
+    if (c.accs * acc_cols + (codes ? 2 * c.bn : 0) + c.a_slots * format_sizes(type).a_cols > 512 || c.accs < (k ? 2 : 4) || c.accs > kMaxAcc || c.accs % (k ? 2 : 4) || c.a_slots < 2 || c.a_slots > kMaxA ||
+        c.a_slots % 2 || c.b_slots < 2 || c.b_slots > kMaxB || c.raw_slots < 2 || c.raw_slots > kMaxRaw || c.smem > (size_t)(codes ? 218 : 225) * 1024 || c.b_slots * c.mh * (k ? 1 : 2) >= 32)
+        return fail("rings", type, codes, sms, rows, cols, tokens);
     std::vector<int> next_unit(tiles, 0), arrivals(c.rest_tiles, 0), summed(c.rest_tiles, 0);
     std::vector<char> place_used((size_t)2 * c.share, 0);
     for (int cta = 0; cta < c.ctas; ++cta) {  // in CTA order, a tile's pieces come in unit order
