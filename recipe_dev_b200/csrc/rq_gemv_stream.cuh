@@ -677,8 +677,8 @@ __device__ __forceinline__ void dot_regs_tok4(const ItemRegs<RQ_Q4_0> (&r)[R], c
 // fp32 activations: the weights of the thread's R rows sit in registers, the digits of the item's 128 inputs come from the unit
 // record in shared memory and each word serves all R rows. A sum over a slice or group is three exact integers, put together
 // in fp32 once and scaled (by the step first: a step times a weight's scale could leave the normal range). Every caller, whatever its R, has the same operations in the same order, so a row has the same
-// bits whichever path computes it. Measured, one token, before digits_to_smem looked for odd groups (see there): Q4_K 14336 x 4096 12.6 us,
-// Q6_K 4096 x 14336 20.2 us; with fp32 products 19.1 and 32.7 us.
+// bits whichever path computes it. Measured, one token: Q4_K 14336 x 4096 13.3 us, Q6_K 4096 x 14336 20.4 us (12.6 and
+// 20.2 before digits_to_smem looked for odd groups); with fp32 products 19.1 and 32.7 us.
 // ------------------------------------------------------------------------------------------
 struct DigitWords { uint4 d[3]; };  // sixteen inputs: high, middle, low
 __device__ __forceinline__ void load_digits(const uint8_t* __restrict__ at, DigitWords& v) {
