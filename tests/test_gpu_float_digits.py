@@ -179,3 +179,22 @@ def test_gated_pairs_and_expert_banks_with_large_inputs(rq_ctx, oracle, t, hidde
     want = g / (1.0 + np.exp(-g)) * u
     assert np.linalg.norm(both - want) <= 2e-6 * np.linalg.norm(want)
     rq_ctx.check()
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("cols", [2560, 4096, 14336])
+@pytest.mark.parametrize("zeros", [0.5, 0.8])
+def test_large_inputs_among_small_ones_and_zeros(rq_ctx, oracle, t, cols, zeros):
+    """Zeros take no part in what the inputs of a group are on average."""
+    rows, at = 33, _outlier_columns(cols, 1)
+    blocks, exact = _with_zero_columns(oracle, t, rows, cols, at, t + cols + 1)
+    w = rq_ctx.weight_from_host(t, blocks, rows, cols)
+    rng = np.random.default_rng(cols)
+    small = np.where(rng.random(cols) < zeros, 0.0, oracle.normal(90, cols, cols, 1.0)).astype(np.float32)
+    small[at] = 0.0
+    x = small.copy()
+    x[at] = 1e6
+    for z in (x, small):
+        y = rq_ctx.matvec(w, torch_cuda(z)).cpu().numpy()
+        assert np.linalg.norm(y - exact @ small.astype(np.float64)) <= 4e-7 * np.linalg.norm(exact @ small.astype(np.float64))
+    rq_ctx.check()
