@@ -10,15 +10,16 @@
 namespace rqcut {
 
 constexpr int kMaxRaw = 8, kMaxB = 12, kMaxA = 8, kMaxAcc = 8;
+constexpr int kStashBytes = 4 * 128 * 16;  // Q4_K, a row half: the headers of a window's superblocks
 
-// groups: staging groups; cols: tokens per tile at most, the sums a drain thread holds; registers of the drain, staging and other
-// warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 768 x 80, 640 x 96).
+// drain_warps; groups: staging groups of four warps; cols: tokens per tile at most; registers of the drain, staging and other
+// warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 896 x 72, 640 x 96).
 // CODES: int8 activations over the 32-value formats.
 template <int MH, bool CODES> struct Shape;
-template <> struct Shape<1, false> { static constexpr int groups = 3, cols = 64, drain_regs = 120, stage_regs = 64, other_regs = 48, launch_regs = 80; };
-template <> struct Shape<2, false> { static constexpr int groups = 2, cols = 96, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
-template <> struct Shape<1, true> { static constexpr int groups = 3, cols = 64, drain_regs = 128, stage_regs = 56, other_regs = 48, launch_regs = 80; };
-template <> struct Shape<2, true> { static constexpr int groups = 2, cols = 64, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
+template <> struct Shape<1, false> { static constexpr int drain_warps = 8, groups = 4, cols = 64, drain_regs = 120, stage_regs = 56, other_regs = 40, launch_regs = 72; };
+template <> struct Shape<2, false> { static constexpr int drain_warps = 8, groups = 2, cols = 128, drain_regs = 168, stage_regs = 56, other_regs = 32, launch_regs = 96; };
+template <> struct Shape<1, true> { static constexpr int drain_warps = 8, groups = 4, cols = 64, drain_regs = 128, stage_regs = 48, other_regs = 40, launch_regs = 72; };
+template <> struct Shape<2, true> { static constexpr int drain_warps = 8, groups = 2, cols = 64, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
 
 template <int TYPE> struct Format {
     static constexpr bool kquant = TYPE == RQ_Q4_K || TYPE == RQ_Q6_K;
@@ -28,6 +29,14 @@ template <int TYPE> struct Format {
     static constexpr int raw_slices = TYPE == RQ_Q8_0 ? 2 : 4;   // slices in one TMA tile
     static constexpr int raw_bytes = 128 * box_bytes;
     static constexpr int a_cols = residual ? 64 : 32;            // tensor-memory columns of an operand slot
+};
+
+// The slices of a segment (units u0 .. u1 - 1 of a tile) in the order every role takes them: four a unit and, over Q4_K, behind the last unit of every
+// aligned window of four (or the segment's last) one more for the window's minimum terms.
+template <int TYPE> struct Slices {
+    static constexpr bool minimum = TYPE == RQ_Q4_K;
+    static RQ_HOST_DEVICE int count(int u0, int u1) { return 4 * (u1 - u0) + (minimum ? ((u1 - 1) >> 2) - (u0 >> 2) + 1 : 0); }
+    static RQ_HOST_DEVICE bool closes(int u, int u1) { return minimum && ((u & 3) == 3 || u == u1 - 1); }
 };
 
 // The deal of the shared tiles: their units, numbered tile after tile, are cut into `share` ranges of equal length (to one unit), CTA c
@@ -80,7 +89,7 @@ struct Walk {
 
 struct TcCut {
     int mh, bn, n_tiles, tiles_m, units, image_tiles, windows, ctas, whole, rest_tiles, share;
-    int raw_slots, b_slots, a_slots, accs;
+    int raw_slots, b_slots, a_slots, accs, accs_more;  // (accs_more: a last step's accumulators, where an odd number of steps fits)
     size_t smem, records_bytes, xs_bytes, steps_bytes, partial_bytes;
 };
 struct FormatSizes { int raw_bytes, a_cols, raw_per_unit; };
@@ -95,15 +104,16 @@ inline FormatSizes format_sizes(int type) {
 inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t cols, int tokens) {
     TcCut c;
     const FormatSizes f = format_sizes(type);
-    // (fp32 activations over the 32-value formats: two accumulators a slice, of hi and lo columns each, twice; 48 tokens fit)
-    const int widest_1 = !codes && (type == RQ_Q8_0 || type == RQ_Q4_0) ? 48 : Shape<1, false>::cols;
+    const bool kquant = type == RQ_Q4_K || type == RQ_Q6_K;
+    // (fp32 activations over the 32-value formats: two accumulators a slice, of hi and lo columns each, twice; 48 tokens fit, 96 of two row halves)
+    const int widest_1 = !codes && !kquant ? 48 : Shape<1, false>::cols;
     c.mh = tokens <= widest_1 ? 1 : 2;
-    const int widest = c.mh == 1 ? widest_1 : (codes ? Shape<2, true>::cols : Shape<2, false>::cols), grain = c.mh == 1 ? 16 : 32;
+    const int widest = c.mh == 1 ? widest_1 : (codes ? Shape<2, true>::cols : (kquant ? Shape<2, false>::cols : 96)), grain = c.mh == 2 ? 32 : 16;
     c.n_tiles = (tokens + widest - 1) / widest;
     c.bn = ((tokens + c.n_tiles - 1) / c.n_tiles + grain - 1) / grain * grain;
     c.tiles_m = (int)((rows + 128 * c.mh - 1) / (128 * c.mh));
     c.units = (int)((cols + 255) / 256);
-    c.windows = type == RQ_Q4_K ? (c.units + 7) / 8 : 0;
+    c.windows = type == RQ_Q4_K ? (c.units + 3) / 4 : 0;
     c.image_tiles = 4 * c.units + c.windows;
     const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles, work = tiles * c.units;
     c.ctas = work < sm_count ? (int)work : sm_count;
@@ -115,31 +125,29 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     c.whole = (int)(tiles / c.ctas);
     c.rest_tiles = (int)(tiles - (int64_t)c.whole * c.ctas);
     c.share = (int64_t)c.rest_tiles * pieces < c.ctas ? c.rest_tiles * pieces : c.ctas;
-    // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: every ring is as long as
-    // keeps a slot with the same waiters. Accumulators, operand and (MH = 1) activation slots alternate between the two issuing
-    // threads: even numbers of slices. Stored bytes: with MH = 2 a staging group takes every second tile; with MH = 1 the three groups
-    // all read a tile of four slices, but one of two (Q8_0) misses one group in three.
-    // tensor memory, 512 columns: at least four operand slots (Q6_K with MH = 2: two), accumulators, (codes) two sets of totals, more
-    // operand slots
-    const int halves = type == RQ_Q4_K || type == RQ_Q6_K ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn;
-    const int a_least = type == RQ_Q6_K && c.mh == 2 ? 2 : 4;
-    const int totals = codes ? 2 * c.bn : 0;
-    c.accs = (512 - a_least * f.a_cols - totals) / acc_cols / (2 * halves) * (2 * halves);
-    if (c.accs > kMaxAcc) c.accs = kMaxAcc;
-    c.a_slots = (512 - c.accs * acc_cols - totals) / f.a_cols & ~1;
-    if (c.a_slots > kMaxA) c.a_slots = kMaxA;
-    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums)
-    const int joined = c.mh == 1 ? c.bn * 128 * 4 : 0, budget = (codes ? 212 : 220) * 1024 - joined, b_bytes = c.bn * (codes ? 128 : 256);
+    // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: MH = 1, the issuing warps
+    // take alternate activation slots, and Q8_0's staging groups every second tile of stored bytes; MH = 2, a staging group every second
+    // tile: even numbers of each. (The steps' own barriers are indexed by the step.)
+    // tensor memory, 512 columns: operand slots (a power of two; eight where two steps' accumulators still fit beside them), totals
+    // (codes), and accumulators of as many steps as are left room for: a step's are drained while the next ones are filled
+    const int halves = kquant ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn, step_cols = halves * acc_cols, totals = codes ? 2 * c.bn : 0;
+    c.a_slots = type == RQ_Q6_K ? (c.mh == 1 ? 4 : 2) : (c.mh == 1 && 512 - 8 * f.a_cols - totals >= 2 * step_cols ? 8 : 4);
+    int steps = (512 - c.a_slots * f.a_cols - totals) / step_cols;
+    if (steps > kMaxAcc / halves) steps = kMaxAcc / halves;
+    c.accs = (steps & ~1) * halves;
+    c.accs_more = (steps & 1) * halves;
+    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window)
+    const int kept = (c.mh == 1 ? c.bn * 128 * 4 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0), budget = (codes ? 212 : 220) * 1024 - kept, b_bytes = c.bn * (codes ? 128 : 256);
     c.b_slots = c.mh == 1 || codes ? 4 : 3;
     c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
-    const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 ? 2 : (f.raw_per_unit == 2 ? 3 : 1);
+    const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 || f.raw_per_unit == 2 ? 2 : 1;
     c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
     // codes, two row halves: four slots of each are enough, and what they leave is L1, where the drain warps' scale loads want to stay
     // (4096 x 14336, 509 tokens: 312 us so, 343 with rings as deep as fit)
     if (codes && c.mh == 2) c.raw_slots = 4;
     const int b_max = c.mh == 1 ? kMaxB : (codes ? 4 : 6), b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
     while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
-    c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + joined + 1024;
+    c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + kept + 1024;
     c.records_bytes = codes ? (rq_act_token_bytes(cols) * (size_t)tokens + 255) & ~(size_t)255 : 0;
     c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
     c.steps_bytes = codes ? (size_t)c.n_tiles * c.image_tiles * 2 * c.bn * 4 : 0;
@@ -152,13 +160,13 @@ inline size_t scratch_bytes(const TcCut& c) { return c.records_bytes + c.xs_byte
 
 // Enough for every call of up to this many rows, inputs and tokens, of any format and activation mode. Tokens are padded by less than
 // 32 to a token tile (four bytes an input: the codes' image, steps and records are less); the shared tiles' sums are two tiles a CTA: 64 x 128 numbers of one row half, of two row halves (from 49
-// tokens on for fp32 activations over the 32-value formats) 64 x 256, from 65 tokens on 96 x 256.
+// tokens on for fp32 activations over the 32-value formats) 64 x 256, from 65 tokens on 128 x 256.
 inline size_t scratch_bound(int sm_count, int64_t rows, int64_t cols, int tokens) {
     const int64_t units = (cols + 255) / 256, tiles_n = (tokens + 95) / 96;
-    const size_t image = (size_t)(tokens + 32 * tiles_n + 32) * 256 * (size_t)(4 * units + (units + 7) / 8);
+    const size_t image = (size_t)(tokens + 32 * tiles_n + 32) * 256 * (size_t)(4 * units + (units + 3) / 4);
     const int64_t work = ((rows + 127) / 128) * units * tiles_n;
     const size_t ctas = (size_t)(work < sm_count ? work : sm_count);
-    return image + 256 + 4 * ctas + 2 * ctas * (size_t)(tokens > 64 ? 96 * 256 : (tokens > 48 ? 64 * 256 : 64 * 128)) * 4;
+    return image + 256 + 4 * ctas + 2 * ctas * (size_t)(tokens > 64 ? 128 * 256 : (tokens > 48 ? 64 * 256 : 64 * 128)) * 4;
 }
 
 }  // namespace rqcut

@@ -21,11 +21,10 @@
 //   * raw copies: one TMA tile of 128 rows x one unit of stored bytes at a time (Q8_0: half a unit) into a ring;
 //   * activation copies: one bulk copy per 64-wide slice, B_hi | B_lo of the token tile, into a ring;
 //   * staging groups of four warps (thread = row): stored bytes -> 64 fp16 integers -> operand slot in TENSOR MEMORY
-//     (tcgen05.st; the A operand of tcgen05.mma may live there, so the unpacked weights never touch shared memory). The groups
-//     take operand tiles in turn, so that their chains of latencies (barrier, load, unpack, store, fence) overlap;
-//   * two issuing threads, alternate slices (MH = 2: a row half each): the products of a step into one of a ring of accumulators,
-//     one tcgen05.commit. Issuing a product holds its thread for about 70 cycles (as long as it runs), a look at a barrier or a
-//     commit for 100 to 300, so one thread's looks go behind the other's products;
+//     (tcgen05.st; the A operand of tcgen05.mma may live there, so the unpacked weights never touch shared memory). A group has
+//     one slice of every unit (MH = 1, four groups) or one row half (MH = 2, two);
+//   * two issuing warps, alternate slices (MH = 2: a row half each): the products of a step into one of a ring of accumulators,
+//     one tcgen05.commit. One thread issues a product of 16 .. 32 columns every 33 cycles, of 64 / 96 / 128 every 41 / 56 / 71;
 //   * eight drain warps: accumulator -> scale * sum -> fp32 registers, round-to-nearest, then Y or the partial sums.
 //
 // The tensor core adds into its fp32 accumulator by TRUNCATION, a bias that grows with the length of the chain (measured: 7e-7
@@ -33,20 +32,21 @@
 // formats whose scale changes there) and the small cross terms go first or into columns of their own.
 //
 // Two forms. MH = 1 (token tiles of up to 64): B_hi and B_lo are one operand of 2 * bn columns, so a slice is four (Q6_K:
-// eight) instructions (each costs the same 70 cycles for 16 columns as for 128) and the low products have accumulators of their own;
-// the time goes to unpacking and to the weights' bytes, so three staging groups. MH = 2 (token tiles of up to 96): two row halves share each activation tile, which halves
-// the activation bytes a CTA pulls from L2 (they, at 4 bytes per input and token, are what the large shapes would be bound
-// by); products of hi and lo share an accumulator, four drain warps to a row half with 96 fp32 sums a thread (setmaxnreg; CODES: tiles of up to 64). Measured
-// between them (Q4_K 14336 x 4096): the one form for every token count 274 us at 512 tokens where both made 234.
+// eight) instructions and the low products have accumulators of their own. MH = 2 (token tiles of up to 128, of 96 over the 32-value
+// formats, whose two sums a slice take the columns): two row halves share each activation tile, which halves the activation bytes a
+// CTA pulls from L2 (they, at 4 bytes per input and token, are what the large shapes would be bound by); products of hi and lo
+// share an accumulator, a row half has four drain warps with up to 128 fp32 sums a thread (setmaxnreg; CODES: tiles of up to 64).
 //
-// What bounds it is the chains of latencies of the staging and drain warps, not the tensor cores (29 % active at 512 tokens) and, but for
-// a few tokens, not the weights' bytes. Measured on one B200, graphs over distinct copies, against the two kernels it replaced (a
-// single accumulator pair, operands staged slice by slice by all warps): Q4_K 14336 x 4096 16 / 64 / 512 tokens 58 / 61 / 294 us ->
-// 33.5 / 48.6 / 191 us; Q6_K 4096 x 14336 int8 55 / 64 / 296 -> 34.9 / 52.4 / 199; Q8_0 4096 x 14336 int8, 509 tokens 5230 us as passes
-// of the matvec kernel -> 331.
+// What bounds it, from cycles counted around every wait: 512 tokens, the tensor cores are busy for half of the time and the rest is
+// accumulators being drained (three of 128 columns are what tensor memory holds); a few tokens, a third is the wait for the
+// activation image, the rest the chain staging -> products -> drain of a slice. Measured on one B200, calls back to back, before (staging
+// groups took slices in turn; a lone lane looked at barriers; columns were tested for in sixteens; tiles of 96; the minimum terms
+// read their headers again) and now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 30.0 / 42.5 / 45.9 / 125;
+// Q6_K 4096 x 14336 int8 64 tokens 50.8 -> 47.1; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 38.9, 4096 x 8192 fp32 200 tokens 84.3 -> 67.4.
 //
 // The Q4_K minimum term, sum_g (8 * d * sc_g - dmin * m_g) * (sum of x over group g), is a second, 32 times smaller product: per
-// window of eight superblocks two more slices (the terms' fp16 hi and lo) whose "activations" are the group sums.
+// window of four superblocks one more slice (the terms' fp16 values and, behind them, their residuals) whose "activations" are the group
+// sums, twice.
 //
 // Every wait is bounded; a wait that runs out records a code in the context's error word, the thread stops waiting and the CTA
 // still frees its tensor memory before it exits.
@@ -60,12 +60,11 @@ using namespace rqcut;
 
 namespace {
 
-constexpr int kDrainWarps = 8;
 constexpr int kDone = 32;                    // ring of "step finished" barriers, indexed by the step (see the kernel)
 constexpr float kMinScale = 256.0f, kMinUnscale = 1.0f / 256.0f;  // the minimum term's weights are scaled so that their fp16 residuals are no subnormals
 
 constexpr int kIssuers = 2;                  // with the two copying warps: one warpgroup
-template <int MH, bool CODES> __host__ __device__ constexpr int tc_threads() { return (kDrainWarps + 4 * Shape<MH, CODES>::groups + 4) * 32; }
+template <int MH, bool CODES> __host__ __device__ constexpr int tc_threads() { return (Shape<MH, CODES>::drain_warps + 4 * Shape<MH, CODES>::groups + 4) * 32; }
 
 struct TcParams {
     CUtensorMap tile_map;  // the weight's main plane as a [rows][row bytes] byte matrix (TMA descriptor; first: 64-byte aligned)
@@ -77,7 +76,7 @@ struct TcParams {
     int permuted;          // Q8_0 / Q4_0: the plane's chunks are permuted (rows of whole units)
     const uint8_t* xs;     // activation images: [token tile][image tile][hi | lo][bn rows x 128 bytes, swizzled] (CODES: one fp16 tile of codes)
     const float* steps;    // CODES: [token tile][slice][half][bn]
-    int image_tiles;       // 4 * units, then one per window of eight superblocks (Q4_K)
+    int image_tiles;       // 4 * units, then one per window of four superblocks (Q4_K)
     int bn, tokens;
     float* y; int64_t yn, yt;
     int tiles_m, whole, rest_tiles, share;  // row tiles; whole tiles per CTA; tiles shared out by units, and among how many CTAs
@@ -101,94 +100,120 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
 __device__ __forceinline__ uint4 swizzled_chunk(const uint8_t* tile, int row, int chunk) { return *(const uint4*)(tile + swizzled(row, chunk)); }
 
 // ------------------------------------------------------------------------------------------
-// 32 consecutive inputs of one row (`half` of the 64-wide slice `sl` of unit `u`) from the stored bytes in shared memory, as 32
-// fp16 integers (sixteen words), inputs in the order 0 2 1 3 within every four: the order the nibbles of a word come out in.
-// 0x6400 | n is the fp16 number 1024 + n; the subtraction that follows and the product with a scale are exact.
+// 64 inputs of one row (slice `sl` of unit `u`): the stored bytes, and 32 of them at a time (`half`) as fp16 integers (sixteen words),
+// inputs in the order 0 2 1 3 within every four: the order the nibbles of a word come out in. 0x6400 | n is the fp16 number
+// 1024 + n; the subtraction that follows and the product with a scale are exact. The loads come before the arithmetic: a store to
+// tensor memory between them would hold the second half's loads back.
 // ------------------------------------------------------------------------------------------
-template <int TYPE>
-__device__ __forceinline__ void unpack32(const uint8_t* tile, int r, int u, int sl, int half, bool permuted, uint32_t (&o)[16], uint32_t (&res)[16]) {
-    if (TYPE == RQ_Q4_K) {
-        const uint8_t* blk = tile + r * 144;
-        const uint4 hdr = *(const uint4*)blk;
-        const uint4 q0 = *(const uint4*)(blk + 16 + 32 * sl), q1 = *(const uint4*)(blk + 32 + 32 * sl);
-        // the six-bit scale of sub-block 2 sl + half, without a branch: bytes 0 .. 3 of the first four, split ones after
-        const int at = 8 * ((2 * sl + half) & 3);
-        const uint32_t packed = sl < 2 ? hdr.y & 0x3f3f3f3fu : (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
-        const int sc = (packed >> at) & 0xff;
-        // a nibble in bits 4 .. 7 under an exponent of 0x6400 is 1024 + 16 q: times sc / 16, less 72 sc, is sc * (q - 8) -- sc / 16, 72 sc
-        // (a multiple of eight below 4608) and the result (at most 504) are fp16 numbers, so the fused operation is exact
-        const __half2 mul = __half2half2(__hmul(__int2half_rn(sc), __float2half_rn(0.0625f))), off = __half2half2(__int2half_rn(-72 * sc));
-        const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+template <int TYPE> struct Stored {
+    uint4 v[TYPE == RQ_Q6_K || TYPE == RQ_Q8_0 ? 4 : (TYPE == RQ_Q4_K ? 3 : 2)];
+    uint32_t scales;
+    __device__ __forceinline__ void load(const uint8_t* tile, int r, int u, int sl, bool permuted) {
+        if (TYPE == RQ_Q4_K) {
+            const uint8_t* blk = tile + r * 144;
+            v[0] = *(const uint4*)blk;
+            v[1] = *(const uint4*)(blk + 16 + 32 * sl);
+            v[2] = *(const uint4*)(blk + 32 + 32 * sl);
+        } else if (TYPE == RQ_Q6_K) {
+            const int ch = sl >> 1, sel = sl & 1;
+            const uint8_t* body = tile + r * 208;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t a = ((half ? w[j] : w[j] << 4) & 0x00F000F0u) | 0x64006400u;       // inputs 4j, 4j + 2
-            const uint32_t b = ((half ? w[j] >> 8 : w[j] >> 4) & 0x00F000F0u) | 0x64006400u;  // inputs 4j + 1, 4j + 3
-            o[2 * j] = as_u32(__hfma2(as_half2(a), mul, off));
-            o[2 * j + 1] = as_u32(__hfma2(as_half2(b), mul, off));
-        }
-    } else if (TYPE == RQ_Q6_K) {
-        const int ch = sl >> 1, sel = sl & 1, g = 2 * sel + half;
-        const uint8_t* body = tile + r * 208;
-        const uint4 l0 = *(const uint4*)(body + 64 * ch + 32 * half), l1 = *(const uint4*)(body + 64 * ch + 32 * half + 16);
-        const uint4 h0 = *(const uint4*)(body + 128 + 32 * ch), h1 = *(const uint4*)(body + 128 + 32 * ch + 16);
-        const uint32_t scales = *(const uint16_t*)(body + 192 + 8 * ch + 2 * g);  // two int8 scales: inputs 0..15 and 16..31 of the group
-        const uint32_t lw[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w}, hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-        const __half2 s_first = __half2half2(__int2half_rn((int)(int8_t)(scales & 0xff)));
-        const __half2 s_second = __half2half2(__int2half_rn((int)(int8_t)(scales >> 8)));
-        const __half2 k1056 = __half2half2(__float2half_rn(1056.0f));
+            for (int i = 0; i < 2; ++i) { v[i] = *(const uint4*)(body + 64 * ch + 16 * i); v[2 + i] = *(const uint4*)(body + 128 + 32 * ch + 16 * i); }
+            scales = *(const uint32_t*)(body + 192 + 8 * ch + 4 * sel);  // int8 scales of the inputs 0..15, 16..31, 32..47, 48..63
+        } else if (TYPE == RQ_Q8_0) {
+            const int x = permuted ? u & 7 : 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const __half2 s2 = j < 4 ? s_first : s_second;
-            const uint32_t q4 = ((lw[j] >> (4 * sel)) & 0x0F0F0F0Fu) | (((hw[j] >> (2 * g)) & 0x03030303u) << 4);  // four six-bit codes
-            const uint32_t a = (q4 & 0x00FF00FFu) | 0x64006400u, b = ((q4 >> 8) & 0x00FF00FFu) | 0x64006400u;
-            const __half2 ca = __hsub2(as_half2(a), k1056), cb = __hsub2(as_half2(b), k1056);  // q - 32
-            const __half2 ha = __hmul2(ca, s2), hb = __hmul2(cb, s2);
-            o[2 * j] = as_u32(ha);
-            o[2 * j + 1] = as_u32(hb);
-            res[2 * j] = as_u32(__hfma2(ca, s2, __hneg2(ha)));  // the product less its rounding: -1, 0 or 1
-            res[2 * j + 1] = as_u32(__hfma2(cb, s2, __hneg2(hb)));
-        }
-    } else if (TYPE == RQ_Q8_0) {
-        const int x = permuted ? u & 7 : 0, c = 4 * (sl & 1) + 2 * half;  // the tile holds half a unit: chunks 0..7
-        const uint4 q0 = swizzled_chunk(tile, r, c ^ x), q1 = swizzled_chunk(tile, r, (c + 1) ^ x);
-        const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const __half2 k1152 = __half2half2(__float2half_rn(1152.0f));
+            for (int i = 0; i < 4; ++i) v[i] = swizzled_chunk(tile, r, (4 * (sl & 1) + i) ^ x);  // the tile holds half a unit: chunks 0..7
+        } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t v = w[j] ^ 0x80808080u;  // code + 128
-            o[2 * j] = as_u32(__hsub2(as_half2((v & 0x00FF00FFu) | 0x64006400u), k1152));
-            o[2 * j + 1] = as_u32(__hsub2(as_half2(((v >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
-        }
-    } else {
-        const uint4 q = swizzled_chunk(tile, r, (2 * sl + half) ^ (permuted ? u & 7 : 0));  // a block: low nibbles are its first sixteen values
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-        const __half2 k1032 = __half2half2(__float2half_rn(1032.0f));
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            o[2 * j] = as_u32(__hsub2(as_half2((w[j] & 0x000F000Fu) | 0x64006400u), k1032));
-            o[2 * j + 1] = as_u32(__hsub2(as_half2(((w[j] >> 8) & 0x000F000Fu) | 0x64006400u), k1032));
-            o[8 + 2 * j] = as_u32(__hsub2(as_half2(((w[j] >> 4) & 0x000F000Fu) | 0x64006400u), k1032));
-            o[8 + 2 * j + 1] = as_u32(__hsub2(as_half2(((w[j] >> 12) & 0x000F000Fu) | 0x64006400u), k1032));
+            for (int i = 0; i < 2; ++i) v[i] = swizzled_chunk(tile, r, (2 * sl + i) ^ (permuted ? u & 7 : 0));  // a block: low nibbles are its first sixteen values
         }
     }
-}
+    // Q6_K: the second half's low bits, once the first half's are spent (the operands and their residuals take the registers)
+    __device__ __forceinline__ void load_second(const uint8_t* tile, int r, int sl) {
+        if (TYPE == RQ_Q6_K) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) v[i] = *(const uint4*)(tile + r * 208 + 64 * (sl >> 1) + 32 + 16 * i);
+        }
+    }
+    __device__ __forceinline__ void expand(int sl, int half, uint32_t (&o)[16], uint32_t (&res)[16]) const {
+        if (TYPE == RQ_Q4_K) {
+            const uint4& hdr = v[0];
+            // the six-bit scale of sub-block 2 sl + half, without a branch: bytes 0 .. 3 of the first four, split ones after
+            const int at = 8 * ((2 * sl + half) & 3);
+            const uint32_t packed = sl < 2 ? hdr.y & 0x3f3f3f3fu : (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u);
+            const int sc = (packed >> at) & 0xff;
+            // a nibble in bits 4 .. 7 under an exponent of 0x6400 is 1024 + 16 q: times sc / 16, less 72 sc, is sc * (q - 8) -- sc / 16, 72 sc
+            // (a multiple of eight below 4608) and the result (at most 504) are fp16 numbers, so the fused operation is exact
+            const __half2 mul = __half2half2(__hmul(__int2half_rn(sc), __float2half_rn(0.0625f))), off = __half2half2(__int2half_rn(-72 * sc));
+            const uint32_t w[8] = {v[1].x, v[1].y, v[1].z, v[1].w, v[2].x, v[2].y, v[2].z, v[2].w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t a = ((half ? w[j] : w[j] << 4) & 0x00F000F0u) | 0x64006400u;       // inputs 4j, 4j + 2
+                const uint32_t b = ((half ? w[j] >> 8 : w[j] >> 4) & 0x00F000F0u) | 0x64006400u;  // inputs 4j + 1, 4j + 3
+                o[2 * j] = as_u32(__hfma2(as_half2(a), mul, off));
+                o[2 * j + 1] = as_u32(__hfma2(as_half2(b), mul, off));
+            }
+        } else if (TYPE == RQ_Q6_K) {
+            const int sel = sl & 1, g = 2 * sel + half;
+            const uint32_t lw[8] = {v[0].x, v[0].y, v[0].z, v[0].w, v[1].x, v[1].y, v[1].z, v[1].w}, hw[8] = {v[2].x, v[2].y, v[2].z, v[2].w, v[3].x, v[3].y, v[3].z, v[3].w};
+            const __half2 s_first = __half2half2(__int2half_rn((int)(int8_t)(scales >> (16 * half))));
+            const __half2 s_second = __half2half2(__int2half_rn((int)(int8_t)(scales >> (16 * half + 8))));
+            const __half2 k1056 = __half2half2(__float2half_rn(1056.0f));
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const __half2 s2 = j < 4 ? s_first : s_second;
+                const uint32_t q4 = ((lw[j] >> (4 * sel)) & 0x0F0F0F0Fu) | (((hw[j] >> (2 * g)) & 0x03030303u) << 4);  // four six-bit codes
+                const uint32_t a = (q4 & 0x00FF00FFu) | 0x64006400u, b = ((q4 >> 8) & 0x00FF00FFu) | 0x64006400u;
+                const __half2 ca = __hsub2(as_half2(a), k1056), cb = __hsub2(as_half2(b), k1056);  // q - 32
+                const __half2 ha = __hmul2(ca, s2), hb = __hmul2(cb, s2);
+                o[2 * j] = as_u32(ha);
+                o[2 * j + 1] = as_u32(hb);
+                res[2 * j] = as_u32(__hfma2(ca, s2, __hneg2(ha)));  // the product less its rounding: -1, 0 or 1
+                res[2 * j + 1] = as_u32(__hfma2(cb, s2, __hneg2(hb)));
+            }
+        } else if (TYPE == RQ_Q8_0) {
+            const uint4 &q0 = v[2 * half], &q1 = v[2 * half + 1];
+            const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+            const __half2 k1152 = __half2half2(__float2half_rn(1152.0f));
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t c = w[j] ^ 0x80808080u;  // code + 128
+                o[2 * j] = as_u32(__hsub2(as_half2((c & 0x00FF00FFu) | 0x64006400u), k1152));
+                o[2 * j + 1] = as_u32(__hsub2(as_half2(((c >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
+            }
+        } else {
+            const uint4& q = v[half];
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+            const __half2 k1032 = __half2half2(__float2half_rn(1032.0f));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                o[2 * j] = as_u32(__hsub2(as_half2((w[j] & 0x000F000Fu) | 0x64006400u), k1032));
+                o[2 * j + 1] = as_u32(__hsub2(as_half2(((w[j] >> 8) & 0x000F000Fu) | 0x64006400u), k1032));
+                o[8 + 2 * j] = as_u32(__hsub2(as_half2(((w[j] >> 4) & 0x000F000Fu) | 0x64006400u), k1032));
+                o[8 + 2 * j + 1] = as_u32(__hsub2(as_half2(((w[j] >> 12) & 0x000F000Fu) | 0x64006400u), k1032));
+            }
+        }
+    }
+};
 
 // Q4_K: 2^8 * (dmin * m_g - 8 * d * sc_g) of a superblock's eight sub-blocks (what is left of the minimum once the codes are
 // centred: for weights spread about zero an order of magnitude smaller than dmin * m_g, and so are the truncations of its sums)
-// as fp16; `low`: the residual of that rounding.
-__device__ __forceinline__ void minimum_terms(const uint4& hdr, bool low, uint32_t* out) {
-    const float dmin = rq_h2f((uint16_t)(hdr.x >> 16)), d8 = __fmul_rn(8.0f, rq_h2f((uint16_t)(hdr.x & 0xffff)));
+// as fp16, and the residuals of that rounding.
+__device__ __forceinline__ void minimum_terms(const uint4& hdr, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+    // both products are exact in fp32 (an fp16 times an integer below 64); their difference is rounded once
+    const float dmin = __fmul_rn(kMinScale, rq_h2f((uint16_t)(hdr.x >> 16))), d8 = __fmul_rn(-8.0f * kMinScale, rq_h2f((uint16_t)(hdr.x & 0xffff)));
+    const uint32_t sc[2] = {hdr.y & 0x3f3f3f3fu, (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u)};
+    const uint32_t mn[2] = {hdr.z & 0x3f3f3f3fu, ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u)};
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        int s0, m0, s1, m1;
-        rq_q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * j, s0, m0);
-        rq_q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * j + 1, s1, m1);
-        // both products are exact in fp32 (an fp16 times an integer below 64); their difference is rounded once
-        const float a = __fmul_rn(__fsub_rn(__fmul_rn(dmin, (float)m0), __fmul_rn(d8, (float)s0)), kMinScale);
-        const float b = __fmul_rn(__fsub_rn(__fmul_rn(dmin, (float)m1), __fmul_rn(d8, (float)s1)), kMinScale);
-        uint32_t h, l;
-        split2(a, b, h, l);
-        out[j] = low ? l : h;
+        float t[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int at = 16 * (j & 1) + 8 * i;
+            t[i] = __fmaf_rn(dmin, (float)((mn[j >> 1] >> at) & 0xff), __fmul_rn(d8, (float)((sc[j >> 1] >> at) & 0xff)));
+        }
+        split2(t[0], t[1], hi[j], lo[j]);
     }
 }
 
@@ -305,15 +330,19 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t
         const float next = __shfl_down_sync(0xffffffffu, s, 4);
         uint32_t h, l;
         split2(s, next, h, l);  // in lanes 0, 8, 16, 24: groups 0 1 | 2 3 | 4 5 | 6 7
-        uint8_t* sums = xs + ((size_t)nt * image_tiles + 4 * units + (unit >> 3)) * 2 * (size_t)bn * 128;
+        // (twice: the window's operand is the terms' fp16 values and, behind them, their residuals)
+        uint8_t* sums = xs + ((size_t)nt * image_tiles + 4 * units + (unit >> 2)) * 2 * (size_t)bn * 128;
         if ((lane & 7) == 0) {
-            const int at = swizzled(r, unit & 7) + 4 * (lane >> 3);
-            *(uint32_t*)(sums + at) = h;
-            *(uint32_t*)(sums + (size_t)bn * 128 + at) = l;
+#pragma unroll
+            for (int again = 0; again < 8; again += 4) {
+                const int at = swizzled(r, again + (unit & 3)) + 4 * (lane >> 3);
+                *(uint32_t*)(sums + at) = h;
+                *(uint32_t*)(sums + (size_t)bn * 128 + at) = l;
+            }
         }
         if (unit == units - 1) {  // groups past the last superblock of the window count as zeros
             const int chunk = lane & 7;
-            if (chunk > (unit & 7) && lane < 16) *(uint4*)(sums + (lane < 8 ? 0 : (size_t)bn * 128) + swizzled(r, chunk)) = make_uint4(0, 0, 0, 0);
+            if ((chunk & 3) > (unit & 3) && lane < 16) *(uint4*)(sums + (lane < 8 ? 0 : (size_t)bn * 128) + swizzled(r, chunk)) = make_uint4(0, 0, 0, 0);
         }
     }
 }
@@ -331,6 +360,23 @@ __device__ __forceinline__ void tmem_ld16_pair(uint32_t a, uint32_t b, uint32_t 
         : "memory");
 }
 
+// eight columns at four places
+__device__ __forceinline__ void tmem_ld8_quad(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&s)[8], uint32_t (&t)[8], uint32_t (&u)[8], uint32_t (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%32];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%33];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%34];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%35];\n"
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "=&r"(s[0]), "=&r"(s[1]), "=&r"(s[2]), "=&r"(s[3]), "=&r"(s[4]), "=&r"(s[5]), "=&r"(s[6]), "=&r"(s[7]), "=&r"(t[0]), "=&r"(t[1]), "=&r"(t[2]), "=&r"(t[3]),
+          "=&r"(t[4]), "=&r"(t[5]), "=&r"(t[6]), "=&r"(t[7]), "=&r"(u[0]), "=&r"(u[1]), "=&r"(u[2]), "=&r"(u[3]), "=&r"(u[4]), "=&r"(u[5]), "=&r"(u[6]), "=&r"(u[7]),
+          "=&r"(v[0]), "=&r"(v[1]), "=&r"(v[2]), "=&r"(v[3]), "=&r"(v[4]), "=&r"(v[5]), "=&r"(v[6]), "=&r"(v[7])
+        : "r"(a), "r"(b), "r"(c), "r"(d)
+        : "memory");
+}
+
+template <int N> struct Columns { static constexpr int value = N; };
+
 // A ring position: slot index and the parity of its current use. (Kept by counting: a division by a ring's length, known at run time
 // only, is some thirty instructions.)
 struct Ring {
@@ -344,34 +390,44 @@ struct Ring {
 template <int TYPE, int MH, bool CODES>
 __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const __grid_constant__ TcParams p) {
     using F = Format<TYPE>;
-    constexpr int kGroups = Shape<MH, CODES>::groups, kStageFirst = kDrainWarps, kMiscFirst = kDrainWarps + 4 * kGroups, kCols = Shape<MH, CODES>::cols;
-    static_assert(256 * Shape<MH, CODES>::drain_regs + 128 * kGroups * Shape<MH, CODES>::stage_regs + 128 * Shape<MH, CODES>::other_regs <= tc_threads<MH, CODES>() * Shape<MH, CODES>::launch_regs, "more registers than the launch has: the increase would wait forever");
-    constexpr int kHalves = F::halves, kMinSlices = TYPE == RQ_Q4_K ? 2 : 0;
+    using S = Shape<MH, CODES>;
+    using Order = Slices<TYPE>;
+    constexpr int kDrainWarps = S::drain_warps, kGroups = S::groups, kStageFirst = kDrainWarps, kMiscFirst = kDrainWarps + 4 * kGroups;
+    static_assert(32 * kDrainWarps * S::drain_regs + 128 * kGroups * S::stage_regs + 128 * S::other_regs <= tc_threads<MH, CODES>() * S::launch_regs, "more registers than the launch has: the increase would wait forever");
+    static_assert(kDrainWarps == 8 && kGroups == (MH == 1 ? 4 : 2), "a staging group has one slice of every unit (MH = 1) or one row half (MH = 2)");
+    constexpr int kHalves = F::halves;
+    // What a drain thread holds: MH = 1, a row of the even or of the odd slices; MH = 2, a row of its row half, or (CODES) two rows, one of each
+    // half, of half the tokens: a token's step, read from shared memory, then serves two sums (a step is as many bytes
+    // as a sum, at a quarter of tensor memory's rate).
+    constexpr bool kBoth = MH == 2 && CODES;
+    constexpr int kRows = kBoth ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzled tiles want 1024-byte alignment
-    // A STEP is one sum that leaves tensor memory: (slice, row half, half slice), numbered in issue order. Its one commit arrives on
-    // done[step % kDone]: the drain warps wait for it (the sum is complete), the staging warps for the last step that read their
-    // operand slot, the activation copies for the last step that read theirs. Indexing by step keeps every parity wait within one
-    // phase: no issuing thread is ever kDone steps ahead of anyone (slots x steps per slot < kDone).
-    __shared__ __align__(8) uint64_t done[kDone], raw_full[kMaxRaw], raw_empty[kMaxRaw], b_full[kMaxB], a_full[kMaxA], acc_empty[kMaxAcc];
+    // A STEP is one operand tile's products: (slice, row half), numbered in issue order. Its one commit arrives on done[step % kDone]: the
+    // drain warps wait for it (the sums are complete), the staging warps for the step that read their operand slot, the activation
+    // copies for the last step that read theirs. What the drain warps have read they say on drained[step % kDone], and a staged tile is
+    // announced on a_full[step % kDone]. Indexing by step keeps every parity wait within one phase whatever the rings' lengths: no
+    // thread is ever kDone steps ahead of anyone (activation slots x steps per slot < kDone).
+    __shared__ __align__(8) uint64_t done[kDone], drained[kDone], a_full[kDone], raw_full[kMaxRaw], raw_empty[kMaxRaw], b_full[kMaxB];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int last_piece;
     // CODES: the activations' steps of a few slices, a ring of its own (the drain warps read it, well after the products are done)
     constexpr int kStepSlots = CODES ? 8 : 1;
-    __shared__ __align__(16) float step_ring[kStepSlots][2][kCols];
+    __shared__ __align__(16) float step_ring[kStepSlots][2][S::cols];
     __shared__ __align__(8) uint64_t steps_full[kStepSlots], steps_empty[kStepSlots];
     const int tid = threadIdx.x, lane = tid & 31;
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // visibly the same for the whole warp: the compiler budgets registers by role only then
-    const int bn = p.bn, b_bytes = bn * (CODES ? 128 : 256), a_slots = p.a_slots, accs = p.accs;
+    const int bn = p.bn, b_bytes = bn * (CODES ? 128 : 256), a_mask = p.a_slots - 1, sums = p.accs / kHalves;  // sums: steps that have accumulators of their own
     const int acc_cols = MH == 1 && !CODES ? 2 * bn : bn;
     uint8_t* raw = smem + (size_t)p.b_slots * b_bytes;
+    // Q4_K: the headers of a window's four superblocks, each left by the thread that will turn them into the window's minimum terms (read
+    // again from global memory when those are due they cost a trip to memory in the middle of the chain).
+    uint4* const stash = (uint4*)(raw + (size_t)p.raw_slots * F::raw_bytes + (MH == 1 ? (size_t)bn * 512 : 0));
 
     if (tid == 0) {
-        for (int s = 0; s < kDone; ++s) mbar_init(&done[s], 1);
-        for (int s = 0; s < kMaxRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], 4 * F::raw_slices); }
+        for (int s = 0; s < kDone; ++s) { mbar_init(&done[s], 1); mbar_init(&drained[s], kBoth ? kDrainWarps : 4); mbar_init(&a_full[s], 4); }
+        for (int s = 0; s < kMaxRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], MH == 1 ? 4 * F::raw_slices : 4); }
         for (int s = 0; s < kMaxB; ++s) mbar_init(&b_full[s], 1);
-        for (int s = 0; s < kMaxA; ++s) mbar_init(&a_full[s], 4);
-        for (int s = 0; s < kMaxAcc; ++s) mbar_init(&acc_empty[s], 4);
         for (int s = 0; s < kStepSlots; ++s) { mbar_init(&steps_full[s], 1); mbar_init(&steps_empty[s], MH == 1 ? 4 : kDrainWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -383,361 +439,470 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = tmem_base_slot, a_ring = tmem_base + 512u - (uint32_t)(a_slots * F::a_cols);
+    const uint32_t tmem_base = tmem_base_slot, a_ring = tmem_base + 512u - (uint32_t)(p.a_slots * F::a_cols);
     Walk walk(p.whole, p.rest_tiles, p.units, p.share, (int)gridDim.x, (int)blockIdx.x);
     int tile, u0, u1;
 
     if (warp < kDrainWarps) {
         // ------------------------------------------------------------ drain warps
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape<MH, CODES>::drain_regs));
-        // Warp w may read accumulator rows 32 (w % 4) .., so four warps drain a sum, and the two sets of four take turns: a sum's wait,
-        // loads and release are a chain of some thousand cycles however few its columns. MH = 1: even and odd slices, joined at the
-        // end of the tile; MH = 2: a row half each.
-        const int quarter = warp & 3, set = warp >> 2;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::drain_regs));
+        // Warp w may read accumulator rows 32 (w % 4) .., so four warps, a SET, drain a sum's columns. MH = 1: the even and the odd slices, joined at
+        // the end of the tile; MH = 2: a row half each, or (kBoth) half the columns of both.
+        const int quarter = warp & 3, set = warp >> 2, half0 = MH == 2 && !kBoth ? set : 0;
+        const int col0 = kBoth ? set * (bn / 2) : 0;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         float* const joined = (float*)(raw + (size_t)p.raw_slots * F::raw_bytes);  // MH = 1: [bn][128]
         int slice_base = 0;  // slices of the segments before this one
-        Ring acc_at(accs, set * kHalves);  // the first accumulator of this set's next slice
+        Ring acc_at(sums, kBoth ? 0 : set);  // the accumulators of this set's next slice
         bool dead = false;
-        while (walk.next(tile, u0, u1)) {
-            const int mt = tile % p.tiles_m, nt = tile / p.tiles_m;
-            const int64_t my_row0 = (int64_t)(mt * MH + (MH == 2 ? set : 0)) * 128;
-            Pair sum[kCols / 2];
-#pragma unroll
-            for (int i = 0; i < kCols / 2; ++i) sum[i] = 0;
-            // CODES: the products are exact, so what a sum loses it loses where its terms (32 inputs each) are added up, and up to 448 of them one
-            // after another in one fp32 register lose more than the matvec kernel's tree does. Every few slices the sums go into totals in
-            // tensor memory, and what that addition rounds off stays in the register as the start of the next run (runs of two to eight slices:
-            // the shorter the segment, the more the additions inside a run weigh). Error against 64 bits, 4096 x 14336 and 509 tokens: 2.0e-7
-            // without, 0.79e-7 so, the matvec kernel 0.90e-7; time 312 -> 331 us, and 14336 x 4096 with 32 tokens 44.7 -> 48.5. (Totals in shared
-            // memory 352 us: the L1 it takes is missed by the scale loads; in registers they spill, 372; a compensated sum at every slice 406.)
-            const int own = (MH == 1 ? 2 : 4) * (u1 - u0), run_length = own <= 16 ? 2 : (own <= 64 ? 4 : 8);  // (a set's slices of this segment)
-            int run = 0;
-            bool flushed = false;
-            const uint32_t totals = tmem_base + lane_base + (uint32_t)(accs * acc_cols + set * bn);
-            const Pair minus = pair_of(-1.0f, -1.0f);
-            auto flush = [&]() {
-                run = 0;
-                Pair lost = 0;
-#pragma unroll
-                for (int c = 0; c < kCols; c += 16) {
-                    if (c < bn) {
-                        uint32_t v[16];
-                        if (flushed) {
-                            tmem_ld16(totals + c, v);
-#pragma unroll
-                            for (int j = 0; j < 16; j += 2) {
-                                Pair& s = sum[(c + j) / 2];
-                                const Pair a = pair_of(v[j], v[j + 1]), t = pair_add(a, s);
-                                s = pair_fma(minus, pair_fma(minus, a, t), s);
-                                lost = pair_add(lost, s);
-                                v[j] = __float_as_uint(pair_at(t, 0));
-                                v[j + 1] = __float_as_uint(pair_at(t, 1));
+        // The number of columns is known where the loops are unrolled: with a test for each sixteen of them the sums went through copies, and a
+        // drain of 128 columns took 1340 cycles instead of 550 (512 tokens: 135 us).
+        auto run_tiles = [&](auto columns) {
+            constexpr int kMine = decltype(columns)::value;
+            while (walk.next(tile, u0, u1)) {
+                const int mt = tile % p.tiles_m, nt = tile / p.tiles_m;
+                Pair sum[kRows][kMine / 2];
+    #pragma unroll
+                for (int m = 0; m < kRows; ++m)
+    #pragma unroll
+                    for (int i = 0; i < kMine / 2; ++i) sum[m][i] = 0;
+                // CODES: the products are exact, so what a sum loses it loses where its terms (32 inputs each) are added up, and up to 448 of them one
+                // after another in one fp32 register lose more than the matvec kernel's tree does. Every few slices the sums go into totals in
+                // tensor memory, and what that addition rounds off stays in the register as the start of the next run (runs of two to eight slices:
+                // the shorter the segment, the more the additions inside a run weigh). Error against 64 bits, 4096 x 14336 and 509 tokens: 2.0e-7
+                // without, 0.79e-7 so, the matvec kernel 0.90e-7. (Totals in shared memory take L1 that the scale loads miss; in registers they
+                // spill; a compensated sum at every slice is slower than either.)
+                const int own = (MH == 1 ? 2 : 4) * (u1 - u0), run_length = own <= 16 ? 2 : (own <= 64 ? 4 : 8);  // (a set's slices of this segment)
+                int run = 0;
+                bool flushed = false;
+                const uint32_t totals = tmem_base + lane_base + (uint32_t)(p.accs * acc_cols + (MH == 1 ? set * bn : col0));
+                const Pair minus = pair_of(-1.0f, -1.0f);
+                auto flush = [&]() {
+                    run = 0;
+                    Pair lost = 0;
+    #pragma unroll
+                    for (int m = 0; m < kRows; ++m) {
+    #pragma unroll
+                        for (int c = 0; c < kMine; c += 16) {
+                            {
+                                uint32_t v[16];
+                                if (flushed) {
+                                    tmem_ld16(totals + m * bn + c, v);
+    #pragma unroll
+                                    for (int j = 0; j < 16; j += 2) {
+                                        Pair& s = sum[m][(c + j) / 2];
+                                        const Pair a = pair_of(v[j], v[j + 1]), t = pair_add(a, s);
+                                        s = pair_fma(minus, pair_fma(minus, a, t), s);
+                                        lost = pair_add(lost, s);
+                                        v[j] = __float_as_uint(pair_at(t, 0));
+                                        v[j + 1] = __float_as_uint(pair_at(t, 1));
+                                    }
+                                } else {
+    #pragma unroll
+                                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(pair_at(sum[m][(c + j) / 2], j & 1));
+    #pragma unroll
+                                    for (int j = 0; j < 8; ++j) sum[m][c / 2 + j] = 0;
+                                }
+                                tmem_st16(totals + m * bn + c, v);
                             }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(pair_at(sum[(c + j) / 2], j & 1));
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) sum[c / 2 + j] = 0;
                         }
-                        tmem_st16(totals + c, v);
                     }
-                }
-                tmem_st_wait();
-                flushed = true;
-                // an infinite total has no rounding error to carry on
-                if (!(fabsf(pair_at(lost, 0) + pair_at(lost, 1)) <= 3.402823466e38f)) {
-#pragma unroll
-                    for (int i = 0; i < kCols / 2; ++i) {
-                        const float e0 = pair_at(sum[i], 0), e1 = pair_at(sum[i], 1);
-                        sum[i] = pair_of(fabsf(e0) <= 3.402823466e38f ? e0 : 0.f, fabsf(e1) <= 3.402823466e38f ? e1 : 0.f);
+                    tmem_st_wait();
+                    flushed = true;
+                    // an infinite total has no rounding error to carry on
+                    if (!(fabsf(pair_at(lost, 0) + pair_at(lost, 1)) <= 3.402823466e38f)) {
+    #pragma unroll
+                        for (int m = 0; m < kRows; ++m)
+    #pragma unroll
+                            for (int i = 0; i < kMine / 2; ++i) {
+                                const float e0 = pair_at(sum[m][i], 0), e1 = pair_at(sum[m][i], 1);
+                                sum[m][i] = pair_of(fabsf(e0) <= 3.402823466e38f ? e0 : 0.f, fabsf(e1) <= 3.402823466e38f ? e1 : 0.f);
+                            }
                     }
-                }
-            };
-            // sum[c ..] = the totals at `at` + sum[c ..]
-            auto add_totals = [&](uint32_t at) {
-#pragma unroll
-                for (int c = 0; c < kCols; c += 16) {
-                    if (c < bn) {
-                        uint32_t v[16];
-                        tmem_ld16(at + c, v);
-#pragma unroll
-                        for (int j = 0; j < 16; j += 2) sum[(c + j) / 2] = pair_add(pair_of(v[j], v[j + 1]), sum[(c + j) / 2]);
-                    }
-                }
-            };
-            // this lane's row, kept inside the weight for the scale loads
-            auto row_at = [&]() -> int64_t { return min(my_row0 + quarter * 32 + lane, p.rows - 1); };
-            // Slice ks of the segment: d0 (and d1: the second half's) scale its sums
-            auto drain = [&](int ks, float d0, float d1) {
-                const int all = slice_base + ks, last = (all * MH + (MH == 2 ? set : 0)) * kHalves + kHalves - 1;  // the slice's last step
-                if (!dead && !mbar_wait_warp(&done[last % kDone], (last / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 14); dead = true; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t acc0 = tmem_base + lane_base + (uint32_t)(acc_at.slot * acc_cols), acc1 = acc0 + (uint32_t)((kHalves - 1) * acc_cols);  // (an even number of accumulators: a slice's two are neighbours)
-                const Pair scale0 = pair_of(d0, d0), scale1 = pair_of(d1, d1);
-                if constexpr (CODES) {
-                    const int slot = all % kStepSlots;
-                    if (!dead && !mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 20); dead = true; }
-                    const float *d8 = &step_ring[slot][0][0], *e8 = d8 + bn;
-#pragma unroll
-                    for (int c = 0; c < kCols; c += 16) {
-                        if (c < bn) {
-                            uint32_t t[16], u[16];
-                            tmem_ld16_pair(acc0 + c, acc1 + c, t, u);
-#pragma unroll
-                            for (int j = 0; j < 16; j += 4) {
-                                const float4 s4 = *(const float4*)(d8 + c + j), r4 = *(const float4*)(e8 + c + j);
-                                const Pair sv[2] = {pair_of(s4.x, s4.y), pair_of(s4.z, s4.w)}, rv[2] = {pair_of(r4.x, r4.y), pair_of(r4.z, r4.w)};
-#pragma unroll
-                                for (int q = 0; q < 2; ++q) {
-                                    const Pair even = pair_mul(pair_mul(sv[q], scale0), pair_of(t[j + 2 * q], t[j + 2 * q + 1]));
-                                    Pair& to = sum[(c + j) / 2 + q];
-                                    to = pair_add(to, pair_fma(pair_mul(rv[q], scale1), pair_of(u[j + 2 * q], u[j + 2 * q + 1]), even));
+                };
+                // this lane's row (of row half half0 + m), kept inside the weight for the scale loads
+                auto row_at = [&](int m) -> int64_t { return min((int64_t)(mt * MH + half0 + m) * 128 + quarter * 32 + lane, p.rows - 1); };
+                // Slice `all` of the CTA's: d[m][0] (and d[m][1]: the second half slice's) scale its sums
+                auto drain = [&](int all, const float (&d)[kRows][2]) {
+                    const int step = MH == 1 ? all : 2 * all + half0;
+    #pragma unroll
+                    for (int m = 0; m < kRows; ++m)
+                        if (!dead && !mbar_wait_warp(&done[(step + m) % kDone], ((step + m) / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 14); dead = true; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t acc0 = tmem_base + lane_base + (uint32_t)(acc_at.slot * kHalves * acc_cols + col0), acc1 = acc0 + (uint32_t)((kHalves - 1) * acc_cols);
+                    if constexpr (CODES) {
+                        const int slot = all % kStepSlots;
+                        if (!dead && !mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 20); dead = true; }
+                        const float *d8 = &step_ring[slot][0][0] + col0, *e8 = d8 + bn;
+                        constexpr int kAt = 16 / kRows;  // columns at a time
+    #pragma unroll
+                        for (int c = 0; c < kMine; c += kAt) {
+                            {
+                                uint32_t t[kRows][2][kAt];
+                                if constexpr (kBoth) tmem_ld8_quad(acc0 + c, acc1 + c, acc0 + 2 * acc_cols + c, acc1 + 2 * acc_cols + c, t[0][0], t[0][1], t[1][0], t[1][1]);  // (an even number of steps' accumulators: a slice's are neighbours)
+                                else tmem_ld16_pair(acc0 + c, acc1 + c, t[0][0], t[0][1]);
+    #pragma unroll
+                                for (int j = 0; j < kAt; j += 4) {
+                                    const float4 s4 = *(const float4*)(d8 + c + j), r4 = *(const float4*)(e8 + c + j);
+                                    const Pair sv[2] = {pair_of(s4.x, s4.y), pair_of(s4.z, s4.w)}, rv[2] = {pair_of(r4.x, r4.y), pair_of(r4.z, r4.w)};
+    #pragma unroll
+                                    for (int m = 0; m < kRows; ++m) {
+                                        const Pair scale0 = pair_of(d[m][0], d[m][0]), scale1 = pair_of(d[m][1], d[m][1]);
+    #pragma unroll
+                                        for (int q = 0; q < 2; ++q) {
+                                            const Pair even = pair_mul(pair_mul(sv[q], scale0), pair_of(t[m][0][j + 2 * q], t[m][0][j + 2 * q + 1]));
+                                            Pair& to = sum[m][(c + j) / 2 + q];
+                                            to = pair_add(to, pair_fma(pair_mul(rv[q], scale1), pair_of(t[m][1][j + 2 * q], t[m][1][j + 2 * q + 1]), even));
+                                        }
+                                    }
                                 }
                             }
                         }
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&steps_empty[slot]);
-                } else {
-#pragma unroll
-                    for (int h = 0; h < kHalves; ++h) {
-                        const uint32_t at = h ? acc1 : acc0;
-                        const Pair d = h ? scale1 : scale0;
-#pragma unroll
-                        for (int c = 0; c < kCols; c += MH == 1 ? 16 : 32) {
-                            if (c < bn) {
-                                uint32_t t[16], u[16];
-                                tmem_ld16_pair(at + c, at + (MH == 1 ? bn + c : c + 16), t, u);  // MH = 1: hi and lo of a token; else the next sixteen tokens
-#pragma unroll
-                                for (int j = 0; j < 16; j += 2) {
-                                    const Pair a = pair_of(t[j], t[j + 1]), b = pair_of(u[j], u[j + 1]);
-                                    if (MH == 1) {
-                                        sum[(c + j) / 2] = pair_fma(d, pair_add(a, b), sum[(c + j) / 2]);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&steps_empty[slot]);
+                    } else {
+    #pragma unroll
+                        for (int h = 0; h < kHalves; ++h) {
+                            const uint32_t at = h ? acc1 : acc0;
+                            const Pair scale = pair_of(d[0][h], d[0][h]);
+    #pragma unroll
+                            for (int c = 0; c < kMine; c += 16) {
+                                {
+                                    uint32_t t[16];
+                                    if (MH == 1) {  // hi and lo of a token
+                                        uint32_t u[16];
+                                        tmem_ld16_pair(at + c, at + bn + c, t, u);
+    #pragma unroll
+                                        for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_fma(scale, pair_add(pair_of(t[j], t[j + 1]), pair_of(u[j], u[j + 1])), sum[0][(c + j) / 2]);
                                     } else {
-                                        sum[(c + j) / 2] = pair_fma(d, a, sum[(c + j) / 2]);
-                                        sum[(c + 16 + j) / 2] = pair_fma(d, b, sum[(c + 16 + j) / 2]);
+                                        tmem_ld16(at + c, t);
+    #pragma unroll
+                                        for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_fma(scale, pair_of(t[j], t[j + 1]), sum[0][(c + j) / 2]);
                                     }
                                 }
                             }
                         }
                     }
-                }
-                // this warp has read the accumulators: the tensor core may overwrite them
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&acc_empty[acc_at.slot]);
-                    if (kHalves == 2) mbar_arrive(&acc_empty[acc_at.slot + 1]);
-                }
-                acc_at.skip(2 * kHalves);
-                if (CODES && ++run == run_length) flush();
-            };
-            constexpr int kStride = MH == 1 ? 2 : 1;
-            const int s0 = MH == 1 ? set : 0;  // (a segment has an even number of slices: parity by segment is parity overall)
-            const int main_slices = 4 * (u1 - u0), extra = kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0;
-            if constexpr (F::kquant) {
-                auto d_of = [&](int u) -> float {
-                    if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (row_at() * p.units + u) * 144)));
-                    return rq_h2f(__ldg(p.scale + row_at() * p.units + u));
+                    // this warp has read the accumulators: the tensor core may overwrite them
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0)
+    #pragma unroll
+                        for (int m = 0; m < kRows; ++m) mbar_arrive(&drained[(step + m) % kDone]);
+                    acc_at.skip(2);
+                    if (CODES && ++run == run_length) flush();
                 };
-                float d_next = d_of(u0);
-                for (int u = u0; u < u1; ++u) {
-                    const float d = d_next;
-                    if (u + 1 < u1) d_next = d_of(u + 1);  // the next unit's scale is on its way
-#pragma unroll 1
-                    for (int sl = s0; sl < 4; sl += kStride) drain(4 * (u - u0) + sl, d, d);
+                if constexpr (F::kquant) {
+                    auto d_of = [&](int u) -> float {
+                        if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (row_at(0) * p.units + u) * 144)));
+                        return rq_h2f(__ldg(p.scale + row_at(0) * p.units + u));
+                    };
+                    float d_next = d_of(u0);
+                    int all = slice_base;
+                    for (int u = u0; u < u1; ++u) {
+                        const float d = d_next;
+                        if (u + 1 < u1) d_next = d_of(u + 1);  // the next unit's scale is on its way
+                        const int n = Order::closes(u, u1) ? 5 : 4;
+    #pragma unroll 1
+                        for (int sl = 0; sl < n; ++sl, ++all)
+                            // MH = 1: this set's slices are the even or the odd ones of the CTA's
+                            if (MH == 2 || (all & 1) == set) {
+                                const float scale[1][2] = {{sl < 4 ? d : -kMinUnscale, 0.f}};
+                                drain(all, scale);
+                            }
+                    }
+                } else {
+                    // a unit's eight fp16 scales, the next unit's on their way: one load where rows are whole units (a load of two bytes goes to
+                    // 32 lines, as one of sixteen does)
+                    const bool wide = (p.blocks32 & 7) == 0 && ((uintptr_t)p.scale & 15) == 0;
+                    auto d_of = [&](int m, int u) -> uint4 {
+                        const uint16_t* at = p.scale + row_at(m) * p.blocks32 + 8 * u;
+                        if (wide) return __ldg((const uint4*)at);
+                        uint32_t w[4];
+    #pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int b = 8 * u + 2 * i;
+                            w[i] = (b < p.blocks32 ? (uint32_t)__ldg(at + 2 * i) : 0u) | (b + 1 < p.blocks32 ? (uint32_t)__ldg(at + 2 * i + 1) << 16 : 0u);
+                        }
+                        return make_uint4(w[0], w[1], w[2], w[3]);
+                    };
+                    uint4 next[kRows];
+    #pragma unroll
+                    for (int m = 0; m < kRows; ++m) next[m] = d_of(m, u0);
+                    int all = slice_base;  // (a multiple of four)
+    #pragma unroll 1
+                    for (int u = u0; u < u1; ++u, all += 4) {
+                        uint4 d[kRows];
+    #pragma unroll
+                        for (int m = 0; m < kRows; ++m) {
+                            d[m] = next[m];
+                            if (u + 1 < u1) next[m] = d_of(m, u + 1);
+                        }
+    #pragma unroll 1
+                        for (int sl = MH == 1 ? set : 0; sl < 4; sl += MH == 1 ? 2 : 1) {
+                            float scale[kRows][2];
+    #pragma unroll
+                            for (int m = 0; m < kRows; ++m) {
+                                const uint32_t w = sl < 2 ? (sl == 0 ? d[m].x : d[m].y) : (sl == 2 ? d[m].z : d[m].w);
+                                scale[m][0] = rq_h2f((uint16_t)(w & 0xffff));
+                                scale[m][1] = rq_h2f((uint16_t)(w >> 16));
+                            }
+                            drain(all + sl, scale);
+                        }
+                    }
                 }
-                if (kMinSlices) {
-#pragma unroll 1
-                    for (int e = s0; e < extra; e += kStride) drain(main_slices + e, -kMinUnscale, -kMinUnscale);
+                slice_base += Order::count(u0, u1);
+                const int r0 = quarter * 32 + lane;
+                if (CODES && flushed) {  // the totals and what is in the registers
+    #pragma unroll
+                    for (int m = 0; m < kRows; ++m)
+    #pragma unroll
+                        for (int c = 0; c < kMine; c += 16) {
+                            {
+                                uint32_t v[16];
+                                tmem_ld16(totals + m * bn + c, v);
+    #pragma unroll
+                                for (int j = 0; j < 16; j += 2) sum[m][(c + j) / 2] = pair_add(pair_of(v[j], v[j + 1]), sum[m][(c + j) / 2]);
+                            }
+                        }
                 }
-            } else {
-                // two fp16 scales a slice, the next slice's on their way; rows of an odd number of blocks are only 2-byte aligned
-                auto d_of = [&](int s) -> uint32_t {
-                    const int b = 2 * (4 * u0 + s);
-                    const uint16_t* at = p.scale + row_at() * p.blocks32 + b;
-                    return (b < p.blocks32 ? (uint32_t)__ldg(at) : 0u) | (b + 1 < p.blocks32 ? (uint32_t)__ldg(at + 1) << 16 : 0u);
-                };
-                uint32_t d_next = d_of(s0);
-#pragma unroll 1
-                for (int s = s0; s < main_slices; s += kStride) {
-                    const uint32_t d = d_next;
-                    if (s + kStride < main_slices) d_next = d_of(s + kStride);
-                    drain(s, rq_h2f((uint16_t)(d & 0xffff)), rq_h2f((uint16_t)(d >> 16)));
+                if (MH == 1) {
+                    // odd slices' sums join the even ones'
+                    if (set == 1) {
+    #pragma unroll
+                        for (int j = 0; j < kMine; ++j)
+                            joined[j * 128 + r0] = pair_at(sum[0][j / 2], j & 1);
+                    }
+                    asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
+                    if (set == 0) {
+    #pragma unroll
+                        for (int j = 0; j < kMine; j += 2)
+                            sum[0][j / 2] = pair_add(sum[0][j / 2], pair_of(joined[j * 128 + r0], joined[(j + 1) * 128 + r0]));
+                    }
+                    asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
+                    if (set == 1) continue;
                 }
-            }
-            slice_base += main_slices + extra;
-            const int r0 = quarter * 32 + lane;
-            if (CODES && flushed) add_totals(totals);
-            if (MH == 1) {
-                // odd slices' sums join the even ones'
-                if (set == 1) {
-#pragma unroll
-                    for (int j = 0; j < kCols; ++j)
-                        if (j < bn) joined[j * 128 + r0] = pair_at(sum[j / 2], j & 1);
-                }
-                asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
-                if (set == 0) {
-#pragma unroll
-                    for (int j = 0; j < kCols; j += 2)
-                        if (j < bn) sum[j / 2] = pair_add(sum[j / 2], pair_of(joined[j * 128 + r0], joined[(j + 1) * 128 + r0]));
-                }
-                asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
-                if (set == 1) continue;
-            }
-            constexpr int kLeave = MH == 1 ? 128 : 256;  // threads that carry the tile out
-            const bool whole = u0 == 0 && u1 == p.units;
-            const int live_tokens = dead || my_row0 + r0 >= p.rows ? 0 : min(bn, p.tokens - nt * bn);
-            auto to_y = [&]() {
-                float* at = p.y + (my_row0 + r0) * p.yn + (int64_t)(nt * bn) * p.yt;
-#pragma unroll
-                for (int j = 0; j < kCols; ++j) {
-                    if (j < live_tokens) *at = pair_at(sum[j / 2], j & 1);
-                    at += p.yt;
-                }
-            };
-            if (whole) {
-                to_y();
-            } else {
-                const size_t tile_floats = (size_t)bn * 128 * MH, mine = (MH == 2 ? set * 128 : 0) + r0;
-                const Deal deal(p.share, p.rest_tiles, p.units);
-                const int t = tile - p.whole * (int)gridDim.x;
-                float* part = p.partial + (size_t)deal.place(t, (int)blockIdx.x) * tile_floats + mine;
-#pragma unroll
-                for (int j = 0; j < kCols; ++j)
-                    if (j < live_tokens) part[j * 128 * MH] = pair_at(sum[j / 2], j & 1);
-                // the CTAs that share this tile, in unit order
-                const int c0 = deal.first(t), c1 = deal.last(t, (int)blockIdx.x);
-                __threadfence();
-                asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
-                if (tid == 0) {
-                    asm volatile("griddepcontrol.wait;" ::: "memory");  // the counters were zeroed by the kernel before this one
-                    last_piece = atomicAdd(p.arrived + t, 1) == c1 - c0;
-                }
-                asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
-                if (last_piece) {
+                constexpr int kLeave = MH == 1 ? 128 : kDrainWarps * 32;  // threads that carry the tile out
+                const bool whole = u0 == 0 && u1 == p.units;
+                const int tokens_here = dead ? 0 : min(kMine, p.tokens - nt * bn - col0);
+                // row half m's row of this thread: how many tokens of it count, and where they go
+                auto live = [&](int m) { return (int64_t)(mt * MH + half0 + m) * 128 + r0 < p.rows ? tokens_here : 0; };
+                auto out = [&](int m) { return p.y + ((int64_t)(mt * MH + half0 + m) * 128 + r0) * p.yn + (int64_t)(nt * bn + col0) * p.yt; };
+                if (whole) {
+    #pragma unroll
+                    for (int m = 0; m < kRows; ++m) {
+                        const int n = live(m);
+                        float* at = out(m);
+    #pragma unroll
+                        for (int j = 0; j < kMine; ++j) {
+                            if (j < n) *at = pair_at(sum[m][j / 2], j & 1);
+                            at += p.yt;
+                        }
+                    }
+                } else {
+                    const size_t tile_floats = (size_t)bn * 128 * MH, place0 = (size_t)col0 * 128 * MH + half0 * 128 + r0;
+                    const Deal deal(p.share, p.rest_tiles, p.units);
+                    const int t = tile - p.whole * (int)gridDim.x;
+    #pragma unroll
+                    for (int m = 0; m < kRows; ++m) {
+                        const int n = live(m);
+                        float* at = p.partial + (size_t)deal.place(t, (int)blockIdx.x) * tile_floats + place0 + 128 * m;
+    #pragma unroll
+                        for (int j = 0; j < kMine; ++j)
+                            if (j < n) at[j * 128 * MH] = pair_at(sum[m][j / 2], j & 1);
+                    }
+                    // the CTAs that share this tile, in unit order
+                    const int c0 = deal.first(t), c1 = deal.last(t, (int)blockIdx.x);
                     __threadfence();
-#pragma unroll
-                    for (int j = 0; j < kCols / 2; ++j) sum[j] = 0;
-                    for (int c = c0; c <= c1; c += 2) {
-                        const bool two = c < c1;
-                        const float* piece = p.partial + (size_t)deal.place(t, c) * tile_floats + mine;
-                        const float* other = two ? p.partial + (size_t)deal.place(t, c + 1) * tile_floats + mine : piece;
-                        // thirty-two loads in flight (a branch for each would make each wait for the one before); the padding
-                        // tokens' places exist and hold nothing that is used
-#pragma unroll
-                        for (int j = 0; j < kCols; j += 16) {
-                            if (j < bn) {
-                                float v[16], w[16];
-#pragma unroll
-                                for (int q = 0; q < 16; ++q) { v[q] = __ldcg(piece + (j + q) * 128 * MH); w[q] = __ldcg(other + (j + q) * 128 * MH); }
-#pragma unroll
-                                for (int q = 0; q < 16; q += 2)
-                                    sum[(j + q) / 2] = pair_add(sum[(j + q) / 2], two ? pair_add(pair_of(v[q], v[q + 1]), pair_of(w[q], w[q + 1])) : pair_of(v[q], v[q + 1]));
+                    asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
+                    if (tid == 0) {
+                        asm volatile("griddepcontrol.wait;" ::: "memory");  // the counters were zeroed by the kernel before this one
+                        last_piece = atomicAdd(p.arrived + t, 1) == c1 - c0;
+                    }
+                    asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
+                    if (last_piece) {
+                        __threadfence();
+                        // A few tokens at a time, two pieces at a time: 64 loads in flight, in the registers that the sums have left (a branch for each
+                        // load would make each wait for the one before; the padding tokens' places exist and hold nothing that is used).
+                        constexpr int kAtOnce = kMine % 32 ? 16 : 32;
+    #pragma unroll 1
+                        for (int m = 0; m < kRows; ++m) {
+                            const int n = live(m);
+    #pragma unroll 1
+                            for (int j0 = 0; j0 < n; j0 += kAtOnce) {
+                                const float* const first = p.partial + place0 + 128 * m + (size_t)j0 * 128 * MH;
+                                Pair total[kAtOnce / 2];
+    #pragma unroll
+                                for (int q = 0; q < kAtOnce / 2; ++q) total[q] = 0;
+    #pragma unroll 1
+                                for (int c = c0; c <= c1; c += 2) {
+                                    const bool two = c < c1;
+                                    const float* piece = first + (size_t)deal.place(t, c) * tile_floats;
+                                    const float* other = two ? first + (size_t)deal.place(t, c + 1) * tile_floats : piece;
+                                    float v[kAtOnce], w[kAtOnce];
+    #pragma unroll
+                                    for (int q = 0; q < kAtOnce; ++q) {
+                                        v[q] = __ldcg(piece + q * 128 * MH);
+                                        w[q] = __ldcg(other + q * 128 * MH);
+                                    }
+    #pragma unroll
+                                    for (int q = 0; q < kAtOnce; q += 2)
+                                        total[q / 2] = pair_add(total[q / 2], two ? pair_add(pair_of(v[q], v[q + 1]), pair_of(w[q], w[q + 1])) : pair_of(v[q], v[q + 1]));
+                                }
+                                float* at = out(m) + (int64_t)j0 * p.yt;
+    #pragma unroll
+                                for (int q = 0; q < kAtOnce; ++q) {
+                                    if (j0 + q < n) *at = pair_at(total[q / 2], q & 1);
+                                    at += p.yt;
+                                }
                             }
                         }
                     }
-                    to_y();
                 }
+            }
+        };
+        if constexpr (kBoth) {
+            run_tiles(Columns<S::cols / 2>());  // (windows of more than 64 tokens are cut into tiles of 33 to 64)
+        } else if constexpr (MH == 2) {
+            if (bn == 96) run_tiles(Columns<96>());
+            else run_tiles(Columns<F::kquant ? S::cols : 64>());
+        } else {
+            switch (bn) {
+                case 16: run_tiles(Columns<16>()); break;
+                case 32: run_tiles(Columns<32>()); break;
+                case 48: run_tiles(Columns<48>()); break;
+                default: run_tiles(Columns<64>()); break;
             }
         }
     } else if (warp < kMiscFirst) {
         // ------------------------------------------------------------ staging groups: stored bytes -> integer operands in tensor memory
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH, CODES>::stage_regs));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::stage_regs));
         const int group = (warp - kStageFirst) >> 2, r = (warp & 3) * 32 + lane;
-        const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-        Ring a_at(a_slots, group), raw_at(p.raw_slots);
-        int a = group, a_base = 0;         // this group's next operand tile; operand tiles of the segments before this one
-        int raw_here = 0, raw_base = 0;    // the tile of stored bytes raw_at stands at; tiles of the segments before this one
+        const uint32_t a_lane = a_ring + ((uint32_t)((warp & 3) * 32) << 16);
+        uint4* const left = stash + (MH == 1 ? 0 : group * 128) + r;  // [4] of this thread's, 128 * MH apart
+        Ring raw_at(p.raw_slots);
         bool dead = false;
-        while (walk.next(tile, u0, u1)) {
-            const int mt = tile % p.tiles_m;
-            const int main_slices = 4 * (u1 - u0), extra = kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0;
-            const int tiles = (main_slices + extra) * MH;
-#pragma unroll 1
-            for (; a < a_base + tiles; a += kGroups, a_at.skip(kGroups)) {
-                const int ks = (a - a_base) / MH, m = (a - a_base) % MH;
-                const uint32_t at = a_ring + lane_base + (uint32_t)(a_at.slot * F::a_cols);
-                auto wait_slot = [&]() {
-                    const int freed = (a - a_slots) * kHalves + kHalves - 1;  // the last step that read the slot
-                    if (freed >= 0) {
-                        if (!dead && !mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 11); dead = true; }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    }
-                };
-                if (ks < main_slices) {
-                    const int rt = raw_base + (ks / F::raw_slices) * MH + m;
-                    raw_at.skip(rt - raw_here);
-                    raw_here = rt;
-                    if (!dead && !mbar_wait_warp(&raw_full[raw_at.slot], raw_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 18); dead = true; }
-                    const uint8_t* src = raw + (size_t)raw_at.slot * F::raw_bytes;
+        // the operand slot of a step, once the step that read it is done
+        auto wait_slot = [&](int step) {
+            const int freed = step - p.a_slots;
+            if (freed >= 0) {
+                if (!dead && !mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 11); dead = true; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+        };
+        auto staged = [&](int step) {
+            tmem_st_wait();
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&a_full[step % kDone]);  // one arrival per warp (an arrival is an atomic on the barrier)
+        };
+        auto wait_raw = [&]() {
+            if (!dead && !mbar_wait_warp(&raw_full[raw_at.slot], raw_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 18); dead = true; }
+        };
+        // This warp has read its rows of a slot: said behind the stores that needed them (said behind the loads, some lanes were given the
+        // slot's next bytes).
+        auto release_raw = [&]() {
+            if (lane == 0) mbar_arrive(&raw_empty[raw_at.slot]);
+        };
+        // the window's minimum terms: inputs 8 j .. of the operand are superblock j's (zeros outside u0 .. u1), 32 + 8 j .. their residuals
+        auto stage_minimum = [&](int u, int step) {
+            wait_slot(step);
+            const uint32_t at = a_lane + (uint32_t)((step & a_mask) * F::a_cols);
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        uint32_t o[16], res[16];
-                        unpack32<TYPE>(src, r, u0 + (ks >> 2), ks & 3, half, p.permuted != 0, o, res);
-                        if (half == 0) wait_slot();
-                        tmem_st16(at + 16 * half, o);
-                        if (F::residual) tmem_st16(at + 32 + 16 * half, res);
-                    }
-                    // this warp has read its rows of the slice
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&raw_empty[raw_at.slot]);
-                } else if (TYPE == RQ_Q4_K) {
-                    // the minimum terms of one window's superblocks, hi or lo: chunk j of the operand is superblock 8 w + j (zeros outside u0 .. u1)
-                    const int e = ks - main_slices, window = (u0 >> 3) + (e >> 1);
-                    const int64_t rr = ((int64_t)mt * MH + m) * 128 + r;
-                    const uint8_t* base = p.main + (rr < p.rows ? rr : p.rows - 1) * p.units * 144;
-                    wait_slot();
+            for (int j = 0; j < 4; ++j) {
+                const int of = (u & ~3) + j;
+                const uint4 hdr = of >= u0 && of < u1 ? left[j * (128 * MH)] : make_uint4(0, 0, 0, 0);
+                uint32_t hi[4], lo[4];
+                minimum_terms(hdr, hi, lo);
+                tmem_st4(at + 4 * j, hi);
+                tmem_st4(at + 16 + 4 * j, lo);
+            }
+            staged(step);
+        };
+        // slice sl of unit u, whose stored bytes are at src
+        auto stage = [&](int sl, int u, const uint8_t* src, int step) {
+            Stored<TYPE> w;
+            w.load(src, r, u, sl, p.permuted != 0);
+            if (TYPE == RQ_Q4_K && sl == 0) left[(u & 3) * (128 * MH)] = w.v[0];
+            const uint32_t at = a_lane + (uint32_t)((step & a_mask) * F::a_cols);
+            uint32_t o[16], res[16];
+            w.expand(sl, 0, o, res);
+            wait_slot(step);
+            tmem_st16(at, o);
+            if (F::residual) tmem_st16(at + 32, res);
+            w.load_second(src, r, sl);
+            w.expand(sl, 1, o, res);
+            tmem_st16(at + 16, o);
+            if (F::residual) tmem_st16(at + 48, res);
+            staged(step);
+        };
+        if constexpr (MH == 1) {
+            // a group has the same slice of every unit; group 0 the minimum terms too, of the headers that it sees
+            constexpr int kPer = 4 / F::raw_slices;
+            raw_at.skip(group / F::raw_slices);
+            int first = 0;  // the unit's first slice, of the CTA's
+            while (walk.next(tile, u0, u1)) {
 #pragma unroll 1
-                    for (int q = 0; q < 2; ++q) {
-                        uint32_t o[16];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int u = 8 * window + 4 * q + j;
-                            const bool in = u >= u0 && u < u1;
-                            const uint4 hdr = in ? __ldg((const uint4*)(base + (int64_t)u * 144)) : make_uint4(0, 0, 0, 0);
-                            minimum_terms(hdr, (e & 1) != 0, o + 4 * j);
-                        }
-                        tmem_st16(at + 16 * q, o);
+                for (int u = u0; u < u1; ++u, first += 4, raw_at.skip(kPer)) {
+                    wait_raw();
+                    stage(group, u, raw + (size_t)raw_at.slot * F::raw_bytes, first + group);
+                    release_raw();
+                    if (Order::closes(u, u1)) {
+                        if (group == 0) stage_minimum(u, first + 4);
+                        ++first;
                     }
                 }
-                tmem_st_wait();
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&a_full[a_at.slot]);  // one arrival per warp (an arrival is an atomic on the barrier)
             }
-            a_base += tiles;
-            raw_base += main_slices / F::raw_slices * MH;
+        } else {
+            // a group has a row half: every second operand tile, every second tile of stored bytes
+            raw_at.skip(group);
+            int step = group;
+            while (walk.next(tile, u0, u1)) {
+#pragma unroll 1
+                for (int u = u0; u < u1; ++u) {
+                    const uint8_t* src = raw;
+#pragma unroll 1
+                    for (int sl = 0; sl < 4; ++sl, step += 2) {
+                        if (sl % F::raw_slices == 0) {
+                            wait_raw();
+                            src = raw + (size_t)raw_at.slot * F::raw_bytes;
+                        }
+                        stage(sl, u, src, step);
+                        if (sl % F::raw_slices == F::raw_slices - 1) { release_raw(); raw_at.skip(2); }
+                    }
+                    if (Order::closes(u, u1)) { stage_minimum(u, step); step += 2; }
+                }
+            }
         }
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Shape<MH, CODES>::other_regs));
-        if (warp < kMiscFirst + kIssuers && elect_one()) {
-            // ------------------------------------------------------------ the issuing threads
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::other_regs));
+        // These warps wait as a whole and one lane acts: a look at a barrier by a lone lane is not suspended, it is repeated every 160 cycles, and
+        // sees an arrival 100 to 200 cycles later than a whole warp does (Q4_K 14336 x 4096, 512 tokens: 154 us so, 135 with whole warps).
+        const bool leader = elect_one();  // (the same lane every time)
+        if (warp < kMiscFirst + kIssuers) {
+            // ------------------------------------------------------------ the issuing warps
             const int me = warp - kMiscFirst;
             const uint32_t idesc = instr_desc(bn), idesc2 = instr_desc(acc_cols);
-            constexpr int kSkip = MH == 1 ? kIssuers : 1, kTiles = MH == 1 ? kIssuers : 2;  // slices and operand tiles from one of this thread's to the next
-            Ring a_at(a_slots, me), b_at(p.b_slots, MH == 1 ? me : 0), acc_at(accs, me * kHalves);
-            int ks_all = 0;
+            constexpr int kSkip = MH == 1 ? kIssuers : 1;  // slices from one of this warp's to the next (steps: two)
+            Ring b_at(p.b_slots, MH == 1 ? me : 0), acc_at(sums, me);
+            int ks = MH == 1 ? me : 0, end = 0;
             bool dead = false;
             while (walk.next(tile, u0, u1)) {
-                const int slices = 4 * (u1 - u0) + (kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0), end = ks_all + slices;
+                end += Order::count(u0, u1);
 #pragma unroll 1
-                for (int ks = ks_all + (MH == 1 ? me : 0); ks < end; ks += kSkip, a_at.skip(kTiles), b_at.skip(kSkip)) {  // (a segment has an even number of slices)
-                    const int a = MH == 1 ? ks : 2 * ks + me;  // operand tile
-                    const int bslot = b_at.slot, aslot = a_at.slot;
-                    if (!dead && !mbar_wait(&b_full[bslot], b_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
+                for (; ks < end; ks += kSkip, b_at.skip(kSkip), acc_at.skip(2)) {
+                    const int step = MH == 1 ? ks : 2 * ks + me, bslot = b_at.slot;
+                    if (!dead && !mbar_wait_warp(&b_full[bslot], b_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
                     const uint32_t bbase = smem_u32(smem + (size_t)bslot * b_bytes);
                     const uint64_t b_hi = smem_desc(bbase), b_lo = smem_desc(bbase + bn * 128);
-                    if (!dead && !mbar_wait(&a_full[aslot], a_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 13); dead = true; }
-                    const uint32_t a_hi = a_ring + (uint32_t)(aslot * F::a_cols), a_res = a_hi + 32;
+                    if (step >= sums && !dead && !mbar_wait_warp(&drained[(step - sums) % kDone], ((step - sums) / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 15); dead = true; }
+                    if (!dead && !mbar_wait_warp(&a_full[step % kDone], (step / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 13); dead = true; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a_hi = a_ring + (uint32_t)((step & a_mask) * F::a_cols), a_res = a_hi + 32;
+                    if (leader && !dead) {
 #pragma unroll
-                    for (int h = 0; h < kHalves; ++h) {
-                        const int step = a * kHalves + h, slot = acc_at.slot;
-                        if (step >= accs && !dead && !mbar_wait(&acc_empty[slot], acc_at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 15); dead = true; }
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        if (!dead) {
-                            const uint32_t acc = tmem_base + (uint32_t)(slot * acc_cols);
+                        for (int h = 0; h < kHalves; ++h) {
+                            const uint32_t acc = tmem_base + (uint32_t)((acc_at.slot * kHalves + h) * acc_cols);
                             constexpr int kk_n = 4 / kHalves;
                             // kk: 16-wide steps, 32 bytes along K (in 16-byte units of the descriptor's start address), eight columns of A
                             if (CODES) {
@@ -761,16 +926,15 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
 #pragma unroll
                                 for (int k = 0; k < kk_n; ++k) { const int kk = h * kk_n + k; mma_f16_ts(acc, a_hi + 8 * kk, b_hi + 2 * kk, idesc, 1u); }
                             }
-                            // one commit: the sum is complete and, after the last step that reads them, the operand and activation slots are free
-                            mma_commit(&done[step % kDone]);
                         }
-                        acc_at.skip(h + 1 < kHalves ? 1 : 1 + (kTiles - 1) * kHalves);
+                        // one commit: the sums are complete and, after the last step that reads them, the operand and activation slots are free
+                        mma_commit(&done[step % kDone]);
                     }
+                    __syncwarp();
                 }
-                ks_all = end;
             }
             // nothing may be in flight when tensor memory is freed: the drain warps have waited for every step by then
-        } else if (warp == kMiscFirst + kIssuers && elect_one()) {
+        } else if (warp == kMiscFirst + kIssuers) {
             // ------------------------------------------------------------ activation copies (the images were written by the kernel before this one)
             asm volatile("griddepcontrol.wait;" ::: "memory");
             Ring b_at(p.b_slots), steps_at(kStepSlots);
@@ -778,30 +942,35 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             bool dead = false;
             while (!dead && walk.next(tile, u0, u1)) {
                 const uint8_t* src = p.xs + (size_t)(tile / p.tiles_m) * p.image_tiles * b_bytes;
-                const int main_slices = 4 * (u1 - u0), extra = kMinSlices ? kMinSlices * (((u1 - 1) >> 3) - (u0 >> 3) + 1) : 0;
-                for (int ks = 0; ks < main_slices + extra; ++ks, ++ks_all) {
+                int u = u0, sl = 0;
+                for (int left = Order::count(u0, u1); left > 0; --left, ++ks_all) {
                     if (ks_all >= p.b_slots) {
-                        // the last steps that read the slot, one of each row half (they come from different threads)
+                        // the last steps that read the slot, one of each row half (they come from different warps)
 #pragma unroll
                         for (int m = 0; m < MH && !dead; ++m) {
-                            const int freed = ((ks_all - p.b_slots) * MH + m) * kHalves + kHalves - 1;
-                            if (!mbar_wait(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; }
+                            const int freed = (ks_all - p.b_slots) * MH + m;
+                            if (!mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; }
                         }
                         if (dead) break;
                     }
-                    const int image = ks < main_slices ? 4 * u0 + ks : 4 * p.units + (u0 >> 3) + ((ks - main_slices) >> 1);
-                    mbar_expect_tx(&b_full[b_at.slot], (uint32_t)b_bytes);
-                    bulk_g2s(smem + (size_t)b_at.slot * b_bytes, src + (size_t)image * b_bytes, (uint32_t)b_bytes, &b_full[b_at.slot]);
+                    const int image = sl < 4 ? 4 * u + sl : 4 * p.units + (u >> 2);
+                    if (++sl >= 4 && !(sl == 4 && Order::closes(u, u1))) { sl = 0; ++u; }
+                    if (leader) {
+                        mbar_expect_tx(&b_full[b_at.slot], (uint32_t)b_bytes);
+                        bulk_g2s(smem + (size_t)b_at.slot * b_bytes, src + (size_t)image * b_bytes, (uint32_t)b_bytes, &b_full[b_at.slot]);
+                    }
                     b_at.next();
                     if (CODES) {
-                        if (ks_all >= kStepSlots && !mbar_wait(&steps_empty[steps_at.slot], steps_at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; break; }
-                        mbar_expect_tx(&steps_full[steps_at.slot], (uint32_t)(8 * bn));
-                        bulk_g2s(&step_ring[steps_at.slot][0][0], p.steps + ((size_t)(tile / p.tiles_m) * p.image_tiles + image) * 2 * bn, (uint32_t)(8 * bn), &steps_full[steps_at.slot]);
+                        if (ks_all >= kStepSlots && !mbar_wait_warp(&steps_empty[steps_at.slot], steps_at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; break; }
+                        if (leader) {
+                            mbar_expect_tx(&steps_full[steps_at.slot], (uint32_t)(8 * bn));
+                            bulk_g2s(&step_ring[steps_at.slot][0][0], p.steps + ((size_t)(tile / p.tiles_m) * p.image_tiles + image) * 2 * bn, (uint32_t)(8 * bn), &steps_full[steps_at.slot]);
+                        }
                         steps_at.next();
                     }
                 }
             }
-        } else if (warp == kMiscFirst + kIssuers + 1 && elect_one()) {
+        } else {
             // ------------------------------------------------------------ stored bytes: constants of the model, nothing to wait for before the first fetches
             Ring at(p.raw_slots);
             int n = 0;
@@ -811,9 +980,11 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 constexpr int kPer = 4 / F::raw_slices;  // TMA tiles per unit and row half
                 for (int t = u0 * kPer; t < u1 * kPer && !dead; ++t)
                     for (int m = 0; m < MH; ++m, ++n) {
-                        if (n >= p.raw_slots && !mbar_wait(&raw_empty[at.slot], at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 19); dead = true; break; }
-                        mbar_expect_tx(&raw_full[at.slot], F::raw_bytes);
-                        tma_load_2d(raw + (size_t)at.slot * F::raw_bytes, &p.tile_map, t * F::box_bytes, (mt * MH + m) * 128, &raw_full[at.slot]);
+                        if (n >= p.raw_slots && !mbar_wait_warp(&raw_empty[at.slot], at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 19); dead = true; break; }
+                        if (leader) {
+                            mbar_expect_tx(&raw_full[at.slot], F::raw_bytes);
+                            tma_load_2d(raw + (size_t)at.slot * F::raw_bytes, &p.tile_map, t * F::box_bytes, (mt * MH + m) * 128, &raw_full[at.slot]);
+                        }
                         at.next();
                     }
             }
@@ -903,7 +1074,7 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
     p.tiles_m = cut.tiles_m; p.whole = cut.whole; p.rest_tiles = cut.rest_tiles; p.share = cut.share;
     p.steps = (const float*)(xs + cut.xs_bytes);
     p.partial = partial; p.arrived = arrived;
-    p.raw_slots = cut.raw_slots; p.b_slots = cut.b_slots; p.a_slots = cut.a_slots; p.accs = cut.accs;
+    p.raw_slots = cut.raw_slots; p.b_slots = cut.b_slots; p.a_slots = cut.a_slots; p.accs = cut.accs + cut.accs_more;
     p.error_flag = ctx->error_flag; p.wait_ns = ctx->wait_limit_ns;
     switch (w->type) {
         case RQ_Q4_K: rc = launch_tc<RQ_Q4_K>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;
