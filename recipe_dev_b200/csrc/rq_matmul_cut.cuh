@@ -129,21 +129,20 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     // take alternate activation slots, and Q8_0's staging groups every second tile of stored bytes; MH = 2, a staging group every second
     // tile: even numbers of each. (The steps' own barriers are indexed by the step.)
     // tensor memory, 512 columns: operand slots (a power of two; eight where two steps' accumulators still fit beside them), totals
-    // (codes), and accumulators of as many steps as are left room for: a step's are drained while the next ones are filled
-    const int halves = kquant ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn, step_cols = halves * acc_cols, totals = codes ? 2 * c.bn : 0;
+    // (codes, one row half), and accumulators of as many steps as are left room for: a step's are drained while the next ones are filled
+    const int halves = kquant ? 1 : 2, acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn, step_cols = halves * acc_cols, totals = codes && c.mh == 1 ? 2 * c.bn : 0;
     c.a_slots = type == RQ_Q6_K ? (c.mh == 1 ? 4 : 2) : (c.mh == 1 && 512 - 8 * f.a_cols - totals >= 2 * step_cols ? 8 : 4);
     int steps = (512 - c.a_slots * f.a_cols - totals) / step_cols;
     if (steps > kMaxAcc / halves) steps = kMaxAcc / halves;
     c.accs = (steps & ~1) * halves;
     c.accs_more = (steps & 1) * halves;
-    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window)
-    const int kept = (c.mh == 1 ? c.bn * 128 * 4 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0), budget = (codes ? 212 : 220) * 1024 - kept, b_bytes = c.bn * (codes ? 128 : 256);
+    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window; codes, MH = 2: and the totals)
+    const int kept = (c.mh == 1 ? c.bn * 128 * 4 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0) + (codes && c.mh == 2 ? c.bn * 256 * 4 : 0), budget = (codes ? 212 : 220) * 1024 - kept, b_bytes = c.bn * (codes ? 128 : 256);
     c.b_slots = c.mh == 1 || codes ? 4 : 3;
     c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
     const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 || f.raw_per_unit == 2 ? 2 : 1;
     c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
-    // codes, two row halves: four slots of each are enough, and what they leave is L1, where the drain warps' scale loads want to stay
-    // (4096 x 14336, 509 tokens: 312 us so, 343 with rings as deep as fit)
+    // codes, two row halves: four slots of each are enough beside the totals
     if (codes && c.mh == 2) c.raw_slots = 4;
     const int b_max = c.mh == 1 ? kMaxB : (codes ? 4 : 6), b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
     while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;

@@ -39,10 +39,13 @@
 //
 // What bounds it, from cycles counted around every wait: 512 tokens, the tensor cores are busy for half of the time and the rest is
 // accumulators being drained (three of 128 columns are what tensor memory holds); a few tokens, a third is the wait for the
-// activation image, the rest the chain staging -> products -> drain of a slice. Measured on one B200, calls back to back, before (staging
-// groups took slices in turn; a lone lane looked at barriers; columns were tested for in sixteens; tiles of 96; the minimum terms
-// read their headers again) and now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 30.0 / 42.5 / 45.9 / 125;
-// Q6_K 4096 x 14336 int8 64 tokens 50.8 -> 47.1; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 38.9, 4096 x 8192 fp32 200 tokens 84.3 -> 67.4.
+// activation image, the rest the chain staging -> products -> drain of a slice; CODES with two row halves, instructions (5700 a slice of
+// 256 rows x 64 tokens x 64 inputs, a quarter of them the scaling, issued in 57 % of the cycles). Measured on one B200, calls back to back,
+// before (staging groups took slices in turn; a lone lane looked at barriers; columns were tested for in sixteens; tiles of 96;
+// the minimum terms read their headers again; CODES drained a row half by four warps, from one slice's accumulators, and kept totals in tensor memory) and
+// now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 28.8 / 41.1 / 44.4 / 117; Q6_K 4096 x 14336 int8 64
+// tokens 50.8 -> 46.3; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 36.5, 4096 x 8192 fp32 200 tokens 84.3 -> 63.0, 4096 x 14336 int8 509 tokens
+// 332 -> 285.
 //
 // The Q4_K minimum term, sum_g (8 * d * sc_g - dmin * m_g) * (sum of x over group g), is a second, 32 times smaller product: per
 // window of four superblocks one more slice (the terms' fp16 values and, behind them, their residuals) whose "activations" are the group
@@ -360,21 +363,6 @@ __device__ __forceinline__ void tmem_ld16_pair(uint32_t a, uint32_t b, uint32_t 
         : "memory");
 }
 
-// eight columns at four places
-__device__ __forceinline__ void tmem_ld8_quad(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t (&s)[8], uint32_t (&t)[8], uint32_t (&u)[8], uint32_t (&v)[8]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%32];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%33];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%34];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%35];\n"
-        "tcgen05.wait::ld.sync.aligned;\n"
-        : "=&r"(s[0]), "=&r"(s[1]), "=&r"(s[2]), "=&r"(s[3]), "=&r"(s[4]), "=&r"(s[5]), "=&r"(s[6]), "=&r"(s[7]), "=&r"(t[0]), "=&r"(t[1]), "=&r"(t[2]), "=&r"(t[3]),
-          "=&r"(t[4]), "=&r"(t[5]), "=&r"(t[6]), "=&r"(t[7]), "=&r"(u[0]), "=&r"(u[1]), "=&r"(u[2]), "=&r"(u[3]), "=&r"(u[4]), "=&r"(u[5]), "=&r"(u[6]), "=&r"(u[7]),
-          "=&r"(v[0]), "=&r"(v[1]), "=&r"(v[2]), "=&r"(v[3]), "=&r"(v[4]), "=&r"(v[5]), "=&r"(v[6]), "=&r"(v[7])
-        : "r"(a), "r"(b), "r"(c), "r"(d)
-        : "memory");
-}
-
 template <int N> struct Columns { static constexpr int value = N; };
 
 // A ring position: slot index and the parity of its current use. (Kept by counting: a division by a ring's length, known at run time
@@ -396,18 +384,19 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
     static_assert(32 * kDrainWarps * S::drain_regs + 128 * kGroups * S::stage_regs + 128 * S::other_regs <= tc_threads<MH, CODES>() * S::launch_regs, "more registers than the launch has: the increase would wait forever");
     static_assert(kDrainWarps == 8 && kGroups == (MH == 1 ? 4 : 2), "a staging group has one slice of every unit (MH = 1) or one row half (MH = 2)");
     constexpr int kHalves = F::halves;
-    // What a drain thread holds: MH = 1, a row of the even or of the odd slices; MH = 2, a row of its row half, or (CODES) two rows, one of each
+    // What a drain thread holds: MH = 1, a row of the even or of the odd slices; MH = 2, a row of its row half, or (kBoth) two rows, one of each
     // half, of half the tokens: a token's step, read from shared memory, then serves two sums (a step is as many bytes
     // as a sum, at a quarter of tensor memory's rate).
     constexpr bool kBoth = MH == 2 && CODES;
     constexpr int kRows = kBoth ? 2 : 1;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzled tiles want 1024-byte alignment
-    // A STEP is one operand tile's products: (slice, row half), numbered in issue order. Its one commit arrives on done[step % kDone]: the
-    // drain warps wait for it (the sums are complete), the staging warps for the step that read their operand slot, the activation
-    // copies for the last step that read theirs. What the drain warps have read they say on drained[step % kDone], and a staged tile is
-    // announced on a_full[step % kDone]. Indexing by step keeps every parity wait within one phase whatever the rings' lengths: no
-    // thread is ever kDone steps ahead of anyone (activation slots x steps per slot < kDone).
+    // A STEP is one operand tile's products: (slice, row half), numbered in issue order; with kBoth a slice's, two commits. A step's commit
+    // arrives on done[step % kDone]: the drain warps wait for it (the sums are complete), the staging warps for the step that read
+    // their operand slot, the activation copies for the last step that read theirs. What the drain warps have read they say on
+    // drained[step % kDone] (kBoth: of every half slice), and a staged tile (slice, row half) is announced on a_full[tile % kDone].
+    // Indexing by step keeps every parity wait within one phase whatever the rings' lengths: no thread is ever kDone steps ahead
+    // of anyone (activation slots x steps per slot < kDone).
     __shared__ __align__(8) uint64_t done[kDone], drained[kDone], a_full[kDone], raw_full[kMaxRaw], raw_empty[kMaxRaw], b_full[kMaxB];
     __shared__ uint32_t tmem_base_slot;
     __shared__ int last_piece;
@@ -425,7 +414,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
     uint4* const stash = (uint4*)(raw + (size_t)p.raw_slots * F::raw_bytes + (MH == 1 ? (size_t)bn * 512 : 0));
 
     if (tid == 0) {
-        for (int s = 0; s < kDone; ++s) { mbar_init(&done[s], 1); mbar_init(&drained[s], kBoth ? kDrainWarps : 4); mbar_init(&a_full[s], 4); }
+        for (int s = 0; s < kDone; ++s) { mbar_init(&done[s], kBoth ? kIssuers : 1); mbar_init(&drained[s], kBoth ? kDrainWarps : 4); mbar_init(&a_full[s], 4); }
         for (int s = 0; s < kMaxRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], MH == 1 ? 4 * F::raw_slices : 4); }
         for (int s = 0; s < kMaxB; ++s) mbar_init(&b_full[s], 1);
         for (int s = 0; s < kStepSlots; ++s) { mbar_init(&steps_full[s], 1); mbar_init(&steps_empty[s], MH == 1 ? 4 : kDrainWarps); }
@@ -462,58 +451,70 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             while (walk.next(tile, u0, u1)) {
                 const int mt = tile % p.tiles_m, nt = tile / p.tiles_m;
                 Pair sum[kRows][kMine / 2];
-    #pragma unroll
+#pragma unroll
                 for (int m = 0; m < kRows; ++m)
-    #pragma unroll
+#pragma unroll
                     for (int i = 0; i < kMine / 2; ++i) sum[m][i] = 0;
                 // CODES: the products are exact, so what a sum loses it loses where its terms (32 inputs each) are added up, and up to 448 of them one
-                // after another in one fp32 register lose more than the matvec kernel's tree does. Every few slices the sums go into totals in
-                // tensor memory, and what that addition rounds off stays in the register as the start of the next run (runs of two to eight slices:
-                // the shorter the segment, the more the additions inside a run weigh). Error against 64 bits, 4096 x 14336 and 509 tokens: 2.0e-7
-                // without, 0.79e-7 so, the matvec kernel 0.90e-7. (Totals in shared memory take L1 that the scale loads miss; in registers they
-                // spill; a compensated sum at every slice is slower than either.)
-                const int own = (MH == 1 ? 2 : 4) * (u1 - u0), run_length = own <= 16 ? 2 : (own <= 64 ? 4 : 8);  // (a set's slices of this segment)
+                // after another in one fp32 register lose more than the matvec kernel's tree does. Every few slices the sums go into totals,
+                // and what that addition rounds off stays in the register as the start of the next run (the shorter the segment, the more the
+                // additions inside a run weigh). Error against 64 bits, 4096 x 14336 and 509 tokens: 2.0e-7 without, 0.75e-7 so, the matvec
+                // kernel 0.90e-7. The totals lie in tensor memory (MH = 1) or, where its columns are better spent on accumulators, in shared
+                // memory, a thread's own. (In registers they spill; a compensated sum at every slice is slower than either.)
+                const int own = (MH == 1 ? 2 : 4) * (u1 - u0);  // (a set's slices of this segment)
+                const int run_length = own <= 16 ? 2 : (own <= 64 ? (kBoth ? 3 : 4) : (kBoth ? 5 : 8));
                 int run = 0;
                 bool flushed = false;
-                const uint32_t totals = tmem_base + lane_base + (uint32_t)(p.accs * acc_cols + (MH == 1 ? set * bn : col0));
+                const uint32_t totals = tmem_base + lane_base + (uint32_t)(p.accs * acc_cols + set * bn);
+                [[maybe_unused]] Pair* const totals_both = (Pair*)(raw + (size_t)p.raw_slots * F::raw_bytes) + tid;  // [row half][columns / 2][256]
                 const Pair minus = pair_of(-1.0f, -1.0f);
                 auto flush = [&]() {
                     run = 0;
                     Pair lost = 0;
-    #pragma unroll
-                    for (int m = 0; m < kRows; ++m) {
-    #pragma unroll
-                        for (int c = 0; c < kMine; c += 16) {
-                            {
-                                uint32_t v[16];
-                                if (flushed) {
-                                    tmem_ld16(totals + m * bn + c, v);
-    #pragma unroll
-                                    for (int j = 0; j < 16; j += 2) {
-                                        Pair& s = sum[m][(c + j) / 2];
-                                        const Pair a = pair_of(v[j], v[j + 1]), t = pair_add(a, s);
-                                        s = pair_fma(minus, pair_fma(minus, a, t), s);
-                                        lost = pair_add(lost, s);
-                                        v[j] = __float_as_uint(pair_at(t, 0));
-                                        v[j + 1] = __float_as_uint(pair_at(t, 1));
-                                    }
-                                } else {
-    #pragma unroll
-                                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(pair_at(sum[m][(c + j) / 2], j & 1));
-    #pragma unroll
-                                    for (int j = 0; j < 8; ++j) sum[m][c / 2 + j] = 0;
-                                }
-                                tmem_st16(totals + m * bn + c, v);
-                            }
+                    auto into = [&](Pair total, Pair& s) -> Pair {  // total + s; s = what that rounds off
+                        const Pair t = pair_add(total, s);
+                        s = pair_fma(minus, pair_fma(minus, total, t), s);
+                        lost = pair_add(lost, s);
+                        return t;
+                    };
+                    if constexpr (kBoth) {
+#pragma unroll
+                        for (int m = 0; m < kRows; ++m) {
+                            Pair* const at = totals_both + m * (kMine / 2) * (32 * kDrainWarps);
+                            Pair total[kMine / 2];
+#pragma unroll
+                            for (int i = 0; i < kMine / 2; ++i) total[i] = flushed ? at[i * (32 * kDrainWarps)] : 0;
+#pragma unroll
+                            for (int i = 0; i < kMine / 2; ++i) at[i * (32 * kDrainWarps)] = into(total[i], sum[m][i]);
                         }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < kMine; c += 16) {
+                            uint32_t v[16];
+                            if (flushed) {
+                                tmem_ld16(totals + c, v);
+#pragma unroll
+                                for (int j = 0; j < 16; j += 2) {
+                                    const Pair t = into(pair_of(v[j], v[j + 1]), sum[0][(c + j) / 2]);
+                                    v[j] = __float_as_uint(pair_at(t, 0));
+                                    v[j + 1] = __float_as_uint(pair_at(t, 1));
+                                }
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(pair_at(sum[0][(c + j) / 2], j & 1));
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) sum[0][c / 2 + j] = 0;
+                            }
+                            tmem_st16(totals + c, v);
+                        }
+                        tmem_st_wait();
                     }
-                    tmem_st_wait();
                     flushed = true;
                     // an infinite total has no rounding error to carry on
                     if (!(fabsf(pair_at(lost, 0) + pair_at(lost, 1)) <= 3.402823466e38f)) {
-    #pragma unroll
+#pragma unroll
                         for (int m = 0; m < kRows; ++m)
-    #pragma unroll
+#pragma unroll
                             for (int i = 0; i < kMine / 2; ++i) {
                                 const float e0 = pair_at(sum[m][i], 0), e1 = pair_at(sum[m][i], 1);
                                 sum[m][i] = pair_of(fabsf(e0) <= 3.402823466e38f ? e0 : 0.f, fabsf(e1) <= 3.402823466e38f ? e1 : 0.f);
@@ -522,61 +523,91 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 };
                 // this lane's row (of row half half0 + m), kept inside the weight for the scale loads
                 auto row_at = [&](int m) -> int64_t { return min((int64_t)(mt * MH + half0 + m) * 128 + quarter * 32 + lane, p.rows - 1); };
-                // Slice `all` of the CTA's: d[m][0] (and d[m][1]: the second half slice's) scale its sums
-                auto drain = [&](int all, const float (&d)[kRows][2]) {
-                    const int step = MH == 1 ? all : 2 * all + half0;
-    #pragma unroll
-                    for (int m = 0; m < kRows; ++m)
-                        if (!dead && !mbar_wait_warp(&done[(step + m) % kDone], ((step + m) / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 14); dead = true; }
+                // kBoth: slice `all` of the CTA's, d[m] holds the two fp16 scales of row half m's row
+                auto drain_both = [&](int all, const uint32_t (&d)[2]) {
+                    if (!mbar_wait_warp(&done[all % kDone], (all / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 14);
+                    const int slot = all % kStepSlots;
+                    if (!mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 20);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t acc0 = tmem_base + lane_base + (uint32_t)(acc_at.slot * kHalves * acc_cols + col0), acc1 = acc0 + (uint32_t)((kHalves - 1) * acc_cols);
+                    const float* const d8 = &step_ring[slot][0][0] + col0;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t acc = tmem_base + lane_base + (uint32_t)(acc_at.slot * 2 * acc_cols + col0);
+                        const float d0 = rq_h2f((uint16_t)(d[0] >> (16 * h))), d1 = rq_h2f((uint16_t)(d[1] >> (16 * h)));
+                        const Pair scale[2] = {pair_of(d0, d0), pair_of(d1, d1)};
+#pragma unroll
+                        for (int c = 0; c < kMine; c += 16) {
+                            uint32_t t[2][16];
+                            tmem_ld16_pair(acc + c, acc + acc_cols + c, t[0], t[1]);
+#pragma unroll
+                            for (int j = 0; j < 16; j += 4) {
+                                const float4 s4 = *(const float4*)(d8 + h * S::cols + c + j);
+                                const Pair sv[2] = {pair_of(s4.x, s4.y), pair_of(s4.z, s4.w)};
+#pragma unroll
+                                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                                    for (int q = 0; q < 2; ++q) {
+                                        Pair& to = sum[m % kRows][(c + j) / 2 + q];
+                                        to = pair_fma(pair_mul(sv[q], scale[m]), pair_of(t[m][j + 2 * q], t[m][j + 2 * q + 1]), to);
+                                    }
+                            }
+                        }
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) {
+                            mbar_arrive(&drained[(2 * all + h) % kDone]);
+                            if (h) mbar_arrive(&steps_empty[slot]);
+                        }
+                        acc_at.next();
+                    }
+                    if (++run == run_length) flush();
+                };
+                // Slice `all` of the CTA's: d[0] (and d[1]: the second half slice's) scale its sums
+                auto drain = [&](int all, const float (&d)[2]) {
+                    const int step = MH == 1 ? all : 2 * all + half0;
+                    if (!mbar_wait_warp(&done[step % kDone], (step / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 14);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t acc0 = tmem_base + lane_base + (uint32_t)(acc_at.slot * kHalves * acc_cols), acc1 = acc0 + (uint32_t)((kHalves - 1) * acc_cols);
+                    const Pair scale0 = pair_of(d[0], d[0]), scale1 = pair_of(d[1], d[1]);
                     if constexpr (CODES) {
                         const int slot = all % kStepSlots;
-                        if (!dead && !mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns)) { atomicExch(p.error_flag, 20); dead = true; }
-                        const float *d8 = &step_ring[slot][0][0] + col0, *e8 = d8 + bn;
-                        constexpr int kAt = 16 / kRows;  // columns at a time
-    #pragma unroll
-                        for (int c = 0; c < kMine; c += kAt) {
-                            {
-                                uint32_t t[kRows][2][kAt];
-                                if constexpr (kBoth) tmem_ld8_quad(acc0 + c, acc1 + c, acc0 + 2 * acc_cols + c, acc1 + 2 * acc_cols + c, t[0][0], t[0][1], t[1][0], t[1][1]);  // (an even number of steps' accumulators: a slice's are neighbours)
-                                else tmem_ld16_pair(acc0 + c, acc1 + c, t[0][0], t[0][1]);
-    #pragma unroll
-                                for (int j = 0; j < kAt; j += 4) {
-                                    const float4 s4 = *(const float4*)(d8 + c + j), r4 = *(const float4*)(e8 + c + j);
-                                    const Pair sv[2] = {pair_of(s4.x, s4.y), pair_of(s4.z, s4.w)}, rv[2] = {pair_of(r4.x, r4.y), pair_of(r4.z, r4.w)};
-    #pragma unroll
-                                    for (int m = 0; m < kRows; ++m) {
-                                        const Pair scale0 = pair_of(d[m][0], d[m][0]), scale1 = pair_of(d[m][1], d[m][1]);
-    #pragma unroll
-                                        for (int q = 0; q < 2; ++q) {
-                                            const Pair even = pair_mul(pair_mul(sv[q], scale0), pair_of(t[m][0][j + 2 * q], t[m][0][j + 2 * q + 1]));
-                                            Pair& to = sum[m][(c + j) / 2 + q];
-                                            to = pair_add(to, pair_fma(pair_mul(rv[q], scale1), pair_of(t[m][1][j + 2 * q], t[m][1][j + 2 * q + 1]), even));
-                                        }
-                                    }
+                        if (!mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 20);
+                        const float *d8 = &step_ring[slot][0][0], *e8 = d8 + bn;
+#pragma unroll
+                        for (int c = 0; c < kMine; c += 16) {
+                            uint32_t t[16], u[16];
+                            tmem_ld16_pair(acc0 + c, acc1 + c, t, u);
+#pragma unroll
+                            for (int j = 0; j < 16; j += 4) {
+                                const float4 s4 = *(const float4*)(d8 + c + j), r4 = *(const float4*)(e8 + c + j);
+                                const Pair sv[2] = {pair_of(s4.x, s4.y), pair_of(s4.z, s4.w)}, rv[2] = {pair_of(r4.x, r4.y), pair_of(r4.z, r4.w)};
+#pragma unroll
+                                for (int q = 0; q < 2; ++q) {
+                                    const Pair even = pair_mul(pair_mul(sv[q], scale0), pair_of(t[j + 2 * q], t[j + 2 * q + 1]));
+                                    Pair& to = sum[0][(c + j) / 2 + q];
+                                    to = pair_add(to, pair_fma(pair_mul(rv[q], scale1), pair_of(u[j + 2 * q], u[j + 2 * q + 1]), even));
                                 }
                             }
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&steps_empty[slot]);
                     } else {
-    #pragma unroll
+#pragma unroll
                         for (int h = 0; h < kHalves; ++h) {
                             const uint32_t at = h ? acc1 : acc0;
-                            const Pair scale = pair_of(d[0][h], d[0][h]);
-    #pragma unroll
+                            const Pair scale = h ? scale1 : scale0;
+#pragma unroll
                             for (int c = 0; c < kMine; c += 16) {
                                 {
                                     uint32_t t[16];
                                     if (MH == 1) {  // hi and lo of a token
                                         uint32_t u[16];
                                         tmem_ld16_pair(at + c, at + bn + c, t, u);
-    #pragma unroll
+#pragma unroll
                                         for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_fma(scale, pair_add(pair_of(t[j], t[j + 1]), pair_of(u[j], u[j + 1])), sum[0][(c + j) / 2]);
                                     } else {
                                         tmem_ld16(at + c, t);
-    #pragma unroll
+#pragma unroll
                                         for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_fma(scale, pair_of(t[j], t[j + 1]), sum[0][(c + j) / 2]);
                                     }
                                 }
@@ -586,9 +617,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     // this warp has read the accumulators: the tensor core may overwrite them
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0)
-    #pragma unroll
-                        for (int m = 0; m < kRows; ++m) mbar_arrive(&drained[(step + m) % kDone]);
+                    if (lane == 0) mbar_arrive(&drained[step % kDone]);
                     acc_at.skip(2);
                     if (CODES && ++run == run_length) flush();
                 };
@@ -603,11 +632,11 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         const float d = d_next;
                         if (u + 1 < u1) d_next = d_of(u + 1);  // the next unit's scale is on its way
                         const int n = Order::closes(u, u1) ? 5 : 4;
-    #pragma unroll 1
+#pragma unroll 1
                         for (int sl = 0; sl < n; ++sl, ++all)
                             // MH = 1: this set's slices are the even or the odd ones of the CTA's
                             if (MH == 2 || (all & 1) == set) {
-                                const float scale[1][2] = {{sl < 4 ? d : -kMinUnscale, 0.f}};
+                                const float scale[2] = {sl < 4 ? d : -kMinUnscale, 0.f};
                                 drain(all, scale);
                             }
                     }
@@ -619,7 +648,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         const uint16_t* at = p.scale + row_at(m) * p.blocks32 + 8 * u;
                         if (wide) return __ldg((const uint4*)at);
                         uint32_t w[4];
-    #pragma unroll
+#pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const int b = 8 * u + 2 * i;
                             w[i] = (b < p.blocks32 ? (uint32_t)__ldg(at + 2 * i) : 0u) | (b + 1 < p.blocks32 ? (uint32_t)__ldg(at + 2 * i + 1) << 16 : 0u);
@@ -627,55 +656,62 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         return make_uint4(w[0], w[1], w[2], w[3]);
                     };
                     uint4 next[kRows];
-    #pragma unroll
+#pragma unroll
                     for (int m = 0; m < kRows; ++m) next[m] = d_of(m, u0);
                     int all = slice_base;  // (a multiple of four)
-    #pragma unroll 1
+#pragma unroll 1
                     for (int u = u0; u < u1; ++u, all += 4) {
                         uint4 d[kRows];
-    #pragma unroll
+#pragma unroll
                         for (int m = 0; m < kRows; ++m) {
                             d[m] = next[m];
                             if (u + 1 < u1) next[m] = d_of(m, u + 1);
                         }
-    #pragma unroll 1
-                        for (int sl = MH == 1 ? set : 0; sl < 4; sl += MH == 1 ? 2 : 1) {
-                            float scale[kRows][2];
-    #pragma unroll
-                            for (int m = 0; m < kRows; ++m) {
-                                const uint32_t w = sl < 2 ? (sl == 0 ? d[m].x : d[m].y) : (sl == 2 ? d[m].z : d[m].w);
-                                scale[m][0] = rq_h2f((uint16_t)(w & 0xffff));
-                                scale[m][1] = rq_h2f((uint16_t)(w >> 16));
+                        if constexpr (kBoth) {
+#pragma unroll 1
+                            for (int sl = 0; sl < 4; ++sl) {
+                                const uint32_t w[2] = {sl < 2 ? (sl == 0 ? d[0].x : d[0].y) : (sl == 2 ? d[0].z : d[0].w),
+                                                       sl < 2 ? (sl == 0 ? d[kRows - 1].x : d[kRows - 1].y) : (sl == 2 ? d[kRows - 1].z : d[kRows - 1].w)};
+                                drain_both(all + sl, w);
                             }
-                            drain(all + sl, scale);
+                        } else {
+#pragma unroll 1
+                            for (int sl = MH == 1 ? set : 0; sl < 4; sl += MH == 1 ? 2 : 1) {
+                                const uint32_t w = sl < 2 ? (sl == 0 ? d[0].x : d[0].y) : (sl == 2 ? d[0].z : d[0].w);
+                                const float scale[2] = {rq_h2f((uint16_t)(w & 0xffff)), rq_h2f((uint16_t)(w >> 16))};
+                                drain(all + sl, scale);
+                            }
                         }
                     }
                 }
                 slice_base += Order::count(u0, u1);
                 const int r0 = quarter * 32 + lane;
                 if (CODES && flushed) {  // the totals and what is in the registers
-    #pragma unroll
-                    for (int m = 0; m < kRows; ++m)
-    #pragma unroll
+                    if constexpr (kBoth) {
+#pragma unroll
+                        for (int m = 0; m < kRows; ++m)
+#pragma unroll
+                            for (int i = 0; i < kMine / 2; ++i) sum[m][i] = pair_add(totals_both[(m * (kMine / 2) + i) * (32 * kDrainWarps)], sum[m][i]);
+                    } else {
+#pragma unroll
                         for (int c = 0; c < kMine; c += 16) {
-                            {
-                                uint32_t v[16];
-                                tmem_ld16(totals + m * bn + c, v);
-    #pragma unroll
-                                for (int j = 0; j < 16; j += 2) sum[m][(c + j) / 2] = pair_add(pair_of(v[j], v[j + 1]), sum[m][(c + j) / 2]);
-                            }
+                            uint32_t v[16];
+                            tmem_ld16(totals + c, v);
+#pragma unroll
+                            for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_add(pair_of(v[j], v[j + 1]), sum[0][(c + j) / 2]);
                         }
+                    }
                 }
                 if (MH == 1) {
                     // odd slices' sums join the even ones'
                     if (set == 1) {
-    #pragma unroll
+#pragma unroll
                         for (int j = 0; j < kMine; ++j)
                             joined[j * 128 + r0] = pair_at(sum[0][j / 2], j & 1);
                     }
                     asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
                     if (set == 0) {
-    #pragma unroll
+#pragma unroll
                         for (int j = 0; j < kMine; j += 2)
                             sum[0][j / 2] = pair_add(sum[0][j / 2], pair_of(joined[j * 128 + r0], joined[(j + 1) * 128 + r0]));
                     }
@@ -689,11 +725,11 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 auto live = [&](int m) { return (int64_t)(mt * MH + half0 + m) * 128 + r0 < p.rows ? tokens_here : 0; };
                 auto out = [&](int m) { return p.y + ((int64_t)(mt * MH + half0 + m) * 128 + r0) * p.yn + (int64_t)(nt * bn + col0) * p.yt; };
                 if (whole) {
-    #pragma unroll
+#pragma unroll
                     for (int m = 0; m < kRows; ++m) {
                         const int n = live(m);
                         float* at = out(m);
-    #pragma unroll
+#pragma unroll
                         for (int j = 0; j < kMine; ++j) {
                             if (j < n) *at = pair_at(sum[m][j / 2], j & 1);
                             at += p.yt;
@@ -703,11 +739,11 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     const size_t tile_floats = (size_t)bn * 128 * MH, place0 = (size_t)col0 * 128 * MH + half0 * 128 + r0;
                     const Deal deal(p.share, p.rest_tiles, p.units);
                     const int t = tile - p.whole * (int)gridDim.x;
-    #pragma unroll
+#pragma unroll
                     for (int m = 0; m < kRows; ++m) {
                         const int n = live(m);
                         float* at = p.partial + (size_t)deal.place(t, (int)blockIdx.x) * tile_floats + place0 + 128 * m;
-    #pragma unroll
+#pragma unroll
                         for (int j = 0; j < kMine; ++j)
                             if (j < n) at[j * 128 * MH] = pair_at(sum[m][j / 2], j & 1);
                     }
@@ -725,32 +761,32 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         // A few tokens at a time, two pieces at a time: 64 loads in flight, in the registers that the sums have left (a branch for each
                         // load would make each wait for the one before; the padding tokens' places exist and hold nothing that is used).
                         constexpr int kAtOnce = kMine % 32 ? 16 : 32;
-    #pragma unroll 1
+#pragma unroll 1
                         for (int m = 0; m < kRows; ++m) {
                             const int n = live(m);
-    #pragma unroll 1
+#pragma unroll 1
                             for (int j0 = 0; j0 < n; j0 += kAtOnce) {
                                 const float* const first = p.partial + place0 + 128 * m + (size_t)j0 * 128 * MH;
                                 Pair total[kAtOnce / 2];
-    #pragma unroll
+#pragma unroll
                                 for (int q = 0; q < kAtOnce / 2; ++q) total[q] = 0;
-    #pragma unroll 1
+#pragma unroll 1
                                 for (int c = c0; c <= c1; c += 2) {
                                     const bool two = c < c1;
                                     const float* piece = first + (size_t)deal.place(t, c) * tile_floats;
                                     const float* other = two ? first + (size_t)deal.place(t, c + 1) * tile_floats : piece;
                                     float v[kAtOnce], w[kAtOnce];
-    #pragma unroll
+#pragma unroll
                                     for (int q = 0; q < kAtOnce; ++q) {
                                         v[q] = __ldcg(piece + q * 128 * MH);
                                         w[q] = __ldcg(other + q * 128 * MH);
                                     }
-    #pragma unroll
+#pragma unroll
                                     for (int q = 0; q < kAtOnce; q += 2)
                                         total[q / 2] = pair_add(total[q / 2], two ? pair_add(pair_of(v[q], v[q + 1]), pair_of(w[q], w[q + 1])) : pair_of(v[q], v[q + 1]));
                                 }
                                 float* at = out(m) + (int64_t)j0 * p.yt;
-    #pragma unroll
+#pragma unroll
                                 for (int q = 0; q < kAtOnce; ++q) {
                                     if (j0 + q < n) *at = pair_at(total[q / 2], q & 1);
                                     at += p.yt;
@@ -784,9 +820,10 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
         bool dead = false;
         // the operand slot of a step, once the step that read it is done
         auto wait_slot = [&](int step) {
-            const int freed = step - p.a_slots;
+            int freed = step - p.a_slots;
             if (freed >= 0) {
-                if (!dead && !mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 11); dead = true; }
+                if (kBoth) freed >>= 1;
+                if (!mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 11);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
         };
@@ -797,7 +834,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             if (lane == 0) mbar_arrive(&a_full[step % kDone]);  // one arrival per warp (an arrival is an atomic on the barrier)
         };
         auto wait_raw = [&]() {
-            if (!dead && !mbar_wait_warp(&raw_full[raw_at.slot], raw_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 18); dead = true; }
+            if (!mbar_wait_warp(&raw_full[raw_at.slot], raw_at.phase, p.wait_ns, dead)) atomicExch(p.error_flag, 18);
         };
         // This warp has read its rows of a slot: said behind the stores that needed them (said behind the loads, some lanes were given the
         // slot's next bytes).
@@ -884,22 +921,34 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             const int me = warp - kMiscFirst;
             const uint32_t idesc = instr_desc(bn), idesc2 = instr_desc(acc_cols);
             constexpr int kSkip = MH == 1 ? kIssuers : 1;  // slices from one of this warp's to the next (steps: two)
-            Ring b_at(p.b_slots, MH == 1 ? me : 0), acc_at(sums, me);
+            Ring b_at(p.b_slots, MH == 1 ? me : 0), acc_at(sums, kBoth ? 0 : me);
             int ks = MH == 1 ? me : 0, end = 0;
             bool dead = false;
             while (walk.next(tile, u0, u1)) {
                 end += Order::count(u0, u1);
 #pragma unroll 1
-                for (; ks < end; ks += kSkip, b_at.skip(kSkip), acc_at.skip(2)) {
+                for (; ks < end; ks += kSkip, b_at.skip(kSkip), acc_at.skip(kBoth ? 0 : 2)) {
                     const int step = MH == 1 ? ks : 2 * ks + me, bslot = b_at.slot;
-                    if (!dead && !mbar_wait_warp(&b_full[bslot], b_at.phase, p.wait_ns)) { atomicExch(p.error_flag, 17); dead = true; }
+                    if (!mbar_wait_warp(&b_full[bslot], b_at.phase, p.wait_ns, dead)) atomicExch(p.error_flag, 17);
                     const uint32_t bbase = smem_u32(smem + (size_t)bslot * b_bytes);
                     const uint64_t b_hi = smem_desc(bbase), b_lo = smem_desc(bbase + bn * 128);
-                    if (step >= sums && !dead && !mbar_wait_warp(&drained[(step - sums) % kDone], ((step - sums) / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 15); dead = true; }
-                    if (!dead && !mbar_wait_warp(&a_full[step % kDone], (step / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 13); dead = true; }
+                    if (!kBoth && step >= sums && !mbar_wait_warp(&drained[(step - sums) % kDone], ((step - sums) / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 15);
+                    if (!mbar_wait_warp(&a_full[step % kDone], (step / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 13);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t a_hi = a_ring + (uint32_t)((step & a_mask) * F::a_cols), a_res = a_hi + 32;
-                    if (leader && !dead) {
+                    if constexpr (kBoth) {
+#pragma unroll
+                        for (int h = 0; h < 2; ++h, acc_at.next()) {
+                            const int at = 2 * ks + h;
+                            if (at >= sums && !mbar_wait_warp(&drained[(at - sums) % kDone], ((at - sums) / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 15);
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            if (leader && !dead) {
+#pragma unroll
+                                for (int k = 0; k < 2; ++k) mma_f16_ts(tmem_base + (uint32_t)((2 * acc_at.slot + me) * acc_cols), a_hi + 8 * (2 * h + k), b_hi + 2 * (2 * h + k), idesc, k ? 1u : 0u);
+                                if (h) mma_commit(&done[ks % kDone]);
+                            }
+                        }
+                    } else if (leader && !dead) {
 #pragma unroll
                         for (int h = 0; h < kHalves; ++h) {
                             const uint32_t acc = tmem_base + (uint32_t)((acc_at.slot * kHalves + h) * acc_cols);
@@ -947,9 +996,9 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     if (ks_all >= p.b_slots) {
                         // the last steps that read the slot, one of each row half (they come from different warps)
 #pragma unroll
-                        for (int m = 0; m < MH && !dead; ++m) {
-                            const int freed = (ks_all - p.b_slots) * MH + m;
-                            if (!mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; }
+                        for (int m = 0; m < (kBoth ? 1 : MH) && !dead; ++m) {
+                            const int freed = kBoth ? ks_all - p.b_slots : (ks_all - p.b_slots) * MH + m;
+                            if (!mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 16); }
                         }
                         if (dead) break;
                     }
@@ -961,7 +1010,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     }
                     b_at.next();
                     if (CODES) {
-                        if (ks_all >= kStepSlots && !mbar_wait_warp(&steps_empty[steps_at.slot], steps_at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 16); dead = true; break; }
+                        if (ks_all >= kStepSlots && !mbar_wait_warp(&steps_empty[steps_at.slot], steps_at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 16); break; }
                         if (leader) {
                             mbar_expect_tx(&steps_full[steps_at.slot], (uint32_t)(8 * bn));
                             bulk_g2s(&step_ring[steps_at.slot][0][0], p.steps + ((size_t)(tile / p.tiles_m) * p.image_tiles + image) * 2 * bn, (uint32_t)(8 * bn), &steps_full[steps_at.slot]);
@@ -980,7 +1029,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 constexpr int kPer = 4 / F::raw_slices;  // TMA tiles per unit and row half
                 for (int t = u0 * kPer; t < u1 * kPer && !dead; ++t)
                     for (int m = 0; m < MH; ++m, ++n) {
-                        if (n >= p.raw_slots && !mbar_wait_warp(&raw_empty[at.slot], at.phase ^ 1, p.wait_ns)) { atomicExch(p.error_flag, 19); dead = true; break; }
+                        if (n >= p.raw_slots && !mbar_wait_warp(&raw_empty[at.slot], at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 19); break; }
                         if (leader) {
                             mbar_expect_tx(&raw_full[at.slot], F::raw_bytes);
                             tma_load_2d(raw + (size_t)at.slot * F::raw_bytes, &p.tile_map, t * F::box_bytes, (mt * MH + m) * 128, &raw_full[at.slot]);

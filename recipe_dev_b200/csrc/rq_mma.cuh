@@ -37,9 +37,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
 }
 // A whole warp waits: all lanes look together and agree (the vote also brings the warp back together for the warp-wide
 // instructions that follow). A look by lane 0 alone, with a __syncwarp and a shuffle to tell the others, made the batched kernel 10 to 17 %
-// slower: 512 tokens 218 against 193 us, 16 tokens 36.9 against 33.1 us.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned long long limit_ns) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns));
+// slower. The common case, a barrier that is complete at the first look, is a straight line; `dead` (the limit ran out once: the warp
+// waits no more) is only asked behind it. False: the limit ran out now.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned long long limit_ns, bool& dead) {
+    if (__builtin_expect(__all_sync(0xffffffffu, mbar_try_wait(bar, parity)), 1)) return true;
+    if (!dead) dead = !__all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns));
+    else return true;
+    return !dead;
 }
 // True in one lane of a converged warp. The compiler knows that the code behind it runs in a single thread, so the operands of the
 // instructions that take uniform registers (tcgen05.mma, commits, copies) stay there.
