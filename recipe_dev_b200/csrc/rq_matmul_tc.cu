@@ -43,9 +43,10 @@
 // 256 rows x 64 tokens x 64 inputs, a quarter of them the scaling, issued in 57 % of the cycles). Measured on one B200, calls back to back,
 // before (staging groups took slices in turn; a lone lane looked at barriers; columns were tested for in sixteens; tiles of 96;
 // the minimum terms read their headers again; CODES drained a row half by four warps, from one slice's accumulators, and kept totals in tensor memory) and
-// now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 28.8 / 41.1 / 44.4 / 117; Q6_K 4096 x 14336 int8 64
-// tokens 50.8 -> 46.3; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 36.5, 4096 x 8192 fp32 200 tokens 84.3 -> 63.0, 4096 x 14336 int8 509 tokens
-// 332 -> 285.
+// now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 27.7 / 41.2 / 45.9 / 118; Q6_K 4096 x 14336 int8 64
+// tokens 50.8 -> 45.1; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 36.2, 4096 x 8192 fp32 200 tokens 84.3 -> 62.1, 4096 x 14336 int8 509 tokens
+// 332 -> 282. The shared tiles' sums as the last thing a CTA does, by drain and staging warps together, were slower (64 tokens 48.8): a CTA is
+// then the last of both of its tiles more often.
 //
 // The Q4_K minimum term, sum_g (8 * d * sc_g - dmin * m_g) * (sum of x over group g), is a second, 32 times smaller product: per
 // window of four superblocks one more slice (the terms' fp16 values and, behind them, their residuals) whose "activations" are the group
@@ -450,6 +451,15 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             constexpr int kMine = decltype(columns)::value;
             while (walk.next(tile, u0, u1)) {
                 const int mt = tile % p.tiles_m, nt = tile / p.tiles_m;
+                // the CTAs that share this tile, in unit order (some divisions: before the sums are there, not behind them)
+                const bool whole = u0 == 0 && u1 == p.units;
+                const int t = tile - p.whole * (int)gridDim.x;
+                int c0 = 0, c1 = 0;
+                if (!whole) {
+                    const Deal deal(p.share, p.rest_tiles, p.units);
+                    c0 = deal.first(t);
+                    c1 = deal.last(t, (int)blockIdx.x);
+                }
                 Pair sum[kRows][kMine / 2];
 #pragma unroll
                 for (int m = 0; m < kRows; ++m)
@@ -465,7 +475,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 const int run_length = own <= 16 ? 2 : (own <= 64 ? (kBoth ? 3 : 4) : (kBoth ? 5 : 8));
                 int run = 0;
                 bool flushed = false;
-                const uint32_t totals = tmem_base + lane_base + (uint32_t)(p.accs * acc_cols + set * bn);
+                [[maybe_unused]] const uint32_t totals = tmem_base + lane_base + (uint32_t)(p.accs * acc_cols + set * bn);
                 [[maybe_unused]] Pair* const totals_both = (Pair*)(raw + (size_t)p.raw_slots * F::raw_bytes) + tid;  // [row half][columns / 2][256]
                 const Pair minus = pair_of(-1.0f, -1.0f);
                 auto flush = [&]() {
@@ -702,79 +712,77 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         }
                     }
                 }
+                // MH = 1: each set gives the other half of the columns and keeps the sums of the even and odd slices of its own half
+                constexpr int kLeave = MH == 1 ? kMine / 2 : kMine;  // tokens that a thread carries out, of each of its rows
+                Pair left[kRows][kLeave / 2];
                 if (MH == 1) {
-                    // odd slices' sums join the even ones'
-                    if (set == 1) {
+                    const int give = (1 - set) * kLeave, keep = set * kLeave;
 #pragma unroll
-                        for (int j = 0; j < kMine; ++j)
-                            joined[j * 128 + r0] = pair_at(sum[0][j / 2], j & 1);
-                    }
+                    for (int j = 0; j < kLeave; ++j) joined[(give + j) * 128 + r0] = pair_at(set ? sum[0][j / 2] : sum[0][(kLeave + j) / 2], j & 1);
                     asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
-                    if (set == 0) {
 #pragma unroll
-                        for (int j = 0; j < kMine; j += 2)
-                            sum[0][j / 2] = pair_add(sum[0][j / 2], pair_of(joined[j * 128 + r0], joined[(j + 1) * 128 + r0]));
-                    }
+                    for (int j = 0; j < kLeave; j += 2)
+                        left[0][j / 2] = pair_add(set ? sum[0][(kLeave + j) / 2] : sum[0][j / 2], pair_of(joined[(keep + j) * 128 + r0], joined[(keep + j + 1) * 128 + r0]));
                     asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
-                    if (set == 1) continue;
+                } else {
+#pragma unroll
+                    for (int m = 0; m < kRows; ++m)
+#pragma unroll
+                        for (int j = 0; j < kLeave / 2; ++j) left[m][j] = sum[m][j];
                 }
-                constexpr int kLeave = MH == 1 ? 128 : kDrainWarps * 32;  // threads that carry the tile out
-                const bool whole = u0 == 0 && u1 == p.units;
-                const int tokens_here = dead ? 0 : min(kMine, p.tokens - nt * bn - col0);
+                const int from = MH == 1 ? set * kLeave : col0;  // the first of them
+                const int tokens_here = dead ? 0 : min(kLeave, p.tokens - nt * bn - from);
                 // row half m's row of this thread: how many tokens of it count, and where they go
                 auto live = [&](int m) { return (int64_t)(mt * MH + half0 + m) * 128 + r0 < p.rows ? tokens_here : 0; };
-                auto out = [&](int m) { return p.y + ((int64_t)(mt * MH + half0 + m) * 128 + r0) * p.yn + (int64_t)(nt * bn + col0) * p.yt; };
+                auto out = [&](int m) { return p.y + ((int64_t)(mt * MH + half0 + m) * 128 + r0) * p.yn + (int64_t)(nt * bn + from) * p.yt; };
                 if (whole) {
 #pragma unroll
                     for (int m = 0; m < kRows; ++m) {
                         const int n = live(m);
                         float* at = out(m);
 #pragma unroll
-                        for (int j = 0; j < kMine; ++j) {
-                            if (j < n) *at = pair_at(sum[m][j / 2], j & 1);
+                        for (int j = 0; j < kLeave; ++j) {
+                            if (j < n) *at = pair_at(left[m][j / 2], j & 1);
                             at += p.yt;
                         }
                     }
                 } else {
-                    const size_t tile_floats = (size_t)bn * 128 * MH, place0 = (size_t)col0 * 128 * MH + half0 * 128 + r0;
-                    const Deal deal(p.share, p.rest_tiles, p.units);
-                    const int t = tile - p.whole * (int)gridDim.x;
+                    // (where a CTA leaves its sums, Deal::place: the tile's first CTA began in an earlier tile or where this one does, the others in it)
+                    const size_t tile_floats = (size_t)bn * 128 * MH, place0 = (size_t)from * 128 * MH + half0 * 128 + r0;
+                    auto piece_of = [&](int c) { return p.partial + (size_t)(2 * c + (c == c0 ? 1 : 0)) * tile_floats + place0; };
 #pragma unroll
                     for (int m = 0; m < kRows; ++m) {
                         const int n = live(m);
-                        float* at = p.partial + (size_t)deal.place(t, (int)blockIdx.x) * tile_floats + place0 + 128 * m;
+                        float* at = piece_of((int)blockIdx.x) + 128 * m;
 #pragma unroll
-                        for (int j = 0; j < kMine; ++j)
-                            if (j < n) at[j * 128 * MH] = pair_at(sum[m][j / 2], j & 1);
+                        for (int j = 0; j < kLeave; ++j)
+                            if (j < n) at[j * 128 * MH] = pair_at(left[m][j / 2], j & 1);
                     }
-                    // the CTAs that share this tile, in unit order
-                    const int c0 = deal.first(t), c1 = deal.last(t, (int)blockIdx.x);
                     __threadfence();
-                    asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
+                    asm volatile("bar.sync 2, %0;" ::"n"(kDrainWarps * 32) : "memory");
                     if (tid == 0) {
                         asm volatile("griddepcontrol.wait;" ::: "memory");  // the counters were zeroed by the kernel before this one
                         last_piece = atomicAdd(p.arrived + t, 1) == c1 - c0;
                     }
-                    asm volatile("bar.sync 2, %0;" ::"n"(kLeave) : "memory");
+                    asm volatile("bar.sync 2, %0;" ::"n"(kDrainWarps * 32) : "memory");
                     if (last_piece) {
                         __threadfence();
                         // A few tokens at a time, two pieces at a time: 64 loads in flight, in the registers that the sums have left (a branch for each
                         // load would make each wait for the one before; the padding tokens' places exist and hold nothing that is used).
-                        constexpr int kAtOnce = kMine % 32 ? 16 : 32;
+                        constexpr int kAtOnce = kLeave % 32 == 0 ? 32 : (kLeave % 16 == 0 ? 16 : 8);
 #pragma unroll 1
                         for (int m = 0; m < kRows; ++m) {
                             const int n = live(m);
 #pragma unroll 1
                             for (int j0 = 0; j0 < n; j0 += kAtOnce) {
-                                const float* const first = p.partial + place0 + 128 * m + (size_t)j0 * 128 * MH;
                                 Pair total[kAtOnce / 2];
 #pragma unroll
                                 for (int q = 0; q < kAtOnce / 2; ++q) total[q] = 0;
 #pragma unroll 1
                                 for (int c = c0; c <= c1; c += 2) {
                                     const bool two = c < c1;
-                                    const float* piece = first + (size_t)deal.place(t, c) * tile_floats;
-                                    const float* other = two ? first + (size_t)deal.place(t, c + 1) * tile_floats : piece;
+                                    const float* piece = piece_of(c) + 128 * m + (size_t)j0 * 128 * MH;
+                                    const float* other = two ? piece_of(c + 1) + 128 * m + (size_t)j0 * 128 * MH : piece;
                                     float v[kAtOnce], w[kAtOnce];
 #pragma unroll
                                     for (int q = 0; q < kAtOnce; ++q) {
