@@ -7,6 +7,7 @@
 // them to Q8_0 at load (rq_weight_requantize), and that weight takes the streaming kernel. `.int(4)` stores Q4_1 and dots it
 // with int8 activation records: rq_gemv_q41_int8_kernel below.
 #include "rq_decode.cuh"
+#include "rq_mma.cuh"
 #include "rq_pairs.cuh"
 
 namespace {
@@ -18,24 +19,30 @@ constexpr int kGroupFloats = 36;           // a group's 32 inputs, padded: 144 b
 
 // N words from a 2-byte aligned address (blocks of 18, 22 and 110 bytes): the aligned words around it, shifted together. Nothing past
 // the last wanted byte's word is touched.
-template <int N>
+// RING: the bytes lie in shared memory
+template <bool RING, typename T> __device__ __forceinline__ T fetch(const T* p) {
+    if constexpr (RING) return *p;
+    else return __ldg(p);
+}
+template <int N, bool RING>
 __device__ __forceinline__ void load_words2(const uint8_t* p, uint32_t* w) {
     const uintptr_t a = (uintptr_t)p;
     const uint32_t* q = (const uint32_t*)(a & ~(uintptr_t)3);
     const uint32_t shift = (a & 2) ? 16u : 0u;
 #pragma unroll
-    for (int i = 0; i < N; ++i) w[i] = __ldg(q + i);
-    const uint32_t last = shift ? __ldg(q + N) : 0u;
+    for (int i = 0; i < N; ++i) w[i] = fetch<RING>(q + i);
+    const uint32_t last = shift ? fetch<RING>(q + N) : 0u;
 #pragma unroll
     for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(w[i], i + 1 < N ? w[i + 1] : last, shift);
 }
-template <int N>
+template <int N, bool RING>
 __device__ __forceinline__ void load_words4(const uint8_t* p, uint32_t* w) {
 #pragma unroll
-    for (int i = 0; i < N; ++i) w[i] = __ldg((const uint32_t*)p + i);
+    for (int i = 0; i < N; ++i) w[i] = fetch<RING>((const uint32_t*)p + i);
 }
+template <bool RING>
 __device__ __forceinline__ void load_line(const uint8_t* p, uint32_t* w) {
-    const uint4 v = __ldg((const uint4*)p);
+    const uint4 v = fetch<RING>((const uint4*)p);
     w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
 }
 
@@ -63,7 +70,7 @@ template <int TYPE> struct GroupBytes;
 template <> struct GroupBytes<RQ_Q4_1> {
     static constexpr int bias = 0;
     uint32_t w[5];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<5>(row + (int64_t)g * 20, w); }
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<5, RING>(row + (int64_t)g * 20, w); }
     __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         scale[0] = scale[1] = rq_h2f((uint16_t)(w[0] & 0xffff));
         offset[0] = offset[1] = rq_h2f((uint16_t)(w[0] >> 16));
@@ -74,10 +81,10 @@ template <> struct GroupBytes<RQ_Q4_1> {
 template <> struct GroupBytes<RQ_Q5_0> {
     static constexpr int bias = 16;
     uint32_t w[6];  // d | high bits 0..15, high bits 16..31 | nibbles, ..: the fields straddle words
-    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) {
         const uint8_t* blk = row + (int64_t)g * 22;
         w[0] = *(const uint16_t*)blk;
-        load_words2<5>(blk + 2, w + 1);
+        load_words2<5, RING>(blk + 2, w + 1);
     }
     __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         scale[0] = scale[1] = rq_h2f((uint16_t)w[0]);
@@ -92,7 +99,7 @@ template <> struct GroupBytes<RQ_Q5_0> {
 template <> struct GroupBytes<RQ_Q5_1> {
     static constexpr int bias = 0;
     uint32_t w[6];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<6>(row + (int64_t)g * 24, w); }
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<6, RING>(row + (int64_t)g * 24, w); }
     __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         scale[0] = scale[1] = rq_h2f((uint16_t)(w[0] & 0xffff));
         offset[0] = offset[1] = rq_h2f((uint16_t)(w[0] >> 16));
@@ -106,13 +113,13 @@ template <> struct GroupBytes<RQ_Q5_1> {
 template <> struct GroupBytes<RQ_Q5_K> {
     static constexpr int bias = 0;
     uint32_t hdr[4], qh[8], qs[8];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) {
         const uint8_t* blk = row + (int64_t)(g >> 3) * 176;  // eleven lines of sixteen bytes
-        load_line(blk, hdr);
-        load_line(blk + 16, qh);
-        load_line(blk + 32, qh + 4);
-        load_line(blk + 48 + 32 * ((g & 7) >> 1), qs);
-        load_line(blk + 64 + 32 * ((g & 7) >> 1), qs + 4);
+        load_line<RING>(blk, hdr);
+        load_line<RING>(blk + 16, qh);
+        load_line<RING>(blk + 32, qh + 4);
+        load_line<RING>(blk + 48 + 32 * ((g & 7) >> 1), qs);
+        load_line<RING>(blk + 64 + 32 * ((g & 7) >> 1), qs + 4);
     }
     __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         const int sub = g & 7;
@@ -127,10 +134,10 @@ template <> struct GroupBytes<RQ_Q5_K> {
 template <> struct GroupBytes<RQ_IQ4_NL> {
     static constexpr int bias = 128;
     uint32_t d, w[4];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) {
         const uint8_t* blk = row + (int64_t)g * 18;
         d = *(const uint16_t*)blk;
-        load_words2<4>(blk + 2, w);
+        load_words2<4, RING>(blk + 2, w);
     }
     __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         scale[0] = scale[1] = rq_h2f((uint16_t)d);
@@ -142,10 +149,10 @@ template <> struct GroupBytes<RQ_IQ4_NL> {
 template <> struct GroupBytes<RQ_IQ4_XS> {
     static constexpr int bias = 128;
     uint32_t hdr[2], w[4];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) {
         const uint8_t* blk = row + (int64_t)(g >> 3) * 136;
-        load_words4<2>(blk, hdr);
-        load_words4<4>(blk + 8 + 16 * (g & 7), w);
+        load_words4<2, RING>(blk, hdr);
+        load_words4<4, RING>(blk + 8 + 16 * (g & 7), w);
     }
     __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         const int b = g & 7, high = (hdr[0] >> (16 + 2 * b)) & 3, low = (hdr[1] >> (4 * b)) & 15;
@@ -158,7 +165,7 @@ template <> struct GroupBytes<RQ_IQ4_XS> {
 template <> struct GroupBytes<RQ_Q8_1> {
     static constexpr int bias = 128;
     uint32_t w[9];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<9>(row + (int64_t)g * 36, w); }
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) { load_words4<9, RING>(row + (int64_t)g * 36, w); }
     __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         scale[0] = scale[1] = rq_h2f((uint16_t)(w[0] & 0xffff));
         offset[0] = offset[1] = 0.f;
@@ -169,10 +176,10 @@ template <> struct GroupBytes<RQ_Q8_1> {
 template <> struct GroupBytes<RQ_Q8_K> {
     static constexpr int bias = 128;
     uint32_t d, w[8];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) {
         const uint8_t* blk = row + (int64_t)(g >> 3) * 292;
-        d = __ldg((const uint32_t*)blk);
-        load_words4<8>(blk + 4 + 32 * (g & 7), w);
+        d = fetch<RING>((const uint32_t*)blk);
+        load_words4<8, RING>(blk + 4 + 32 * (g & 7), w);
     }
     __device__ __forceinline__ void decode(int, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         scale[0] = scale[1] = __uint_as_float(d);
@@ -184,11 +191,11 @@ template <> struct GroupBytes<RQ_Q8_K> {
 template <> struct GroupBytes<RQ_Q2_K> {
     static constexpr int bias = 0;
     uint32_t meta, dd, w[8];
-    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) {
         const uint8_t* blk = row + (int64_t)(g >> 3) * 84;
         meta = *(const uint16_t*)(blk + 2 * (g & 7));
-        load_words4<8>(blk + 16 + 32 * ((g & 7) >> 2), w);
-        dd = __ldg((const uint32_t*)(blk + 80));
+        load_words4<8, RING>(blk + 16 + 32 * ((g & 7) >> 2), w);
+        dd = fetch<RING>((const uint32_t*)(blk + 80));
     }
     __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
         const float d = rq_h2f((uint16_t)(dd & 0xffff)), dmin = rq_h2f((uint16_t)(dd >> 16));
@@ -205,11 +212,11 @@ template <> struct GroupBytes<RQ_Q2_K> {
 template <> struct GroupBytes<RQ_Q3_K> {
     static constexpr int bias = 4;  // a clear mask bit takes four off the code
     uint32_t mask[8], w[8], sc[3], d;
-    __device__ __forceinline__ void load(const uint8_t* row, int g) {
+    template <bool RING> __device__ __forceinline__ void load(const uint8_t* row, int g) {
         const uint8_t* blk = row + (int64_t)(g >> 3) * 110;
-        load_words2<8>(blk, mask);
-        load_words2<8>(blk + 32 + 32 * ((g & 7) >> 2), w);
-        load_words2<3>(blk + 96, sc);
+        load_words2<8, RING>(blk, mask);
+        load_words2<8, RING>(blk + 32 + 32 * ((g & 7) >> 2), w);
+        load_words2<3, RING>(blk + 96, sc);
         d = *(const uint16_t*)(blk + 108);
     }
     __device__ __forceinline__ void decode(int g, uint32_t (&c)[8], float (&scale)[2], float (&offset)[2]) const {
@@ -227,6 +234,30 @@ template <> struct GroupBytes<RQ_Q3_K> {
     }
 };
 
+// A group's weights, each put together whole, against its 32 inputs (v).
+template <int TYPE>
+__device__ __forceinline__ float dot_group(const GroupBytes<TYPE>& raw, int g, const Pair (&v)[16]) {
+    constexpr bool kOffset = TYPE == RQ_Q4_1 || TYPE == RQ_Q5_1 || TYPE == RQ_Q5_K || TYPE == RQ_Q2_K;
+    uint32_t c[8];
+    float scale[2], offset[2];
+    raw.decode(g, c, scale, offset);
+    Pair acc[2][2];  // per sixteen: inputs 0, 1 and 2, 3 of every four
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const Pair by = pair_of(scale[j >> 2], scale[j >> 2]), plus = pair_of(offset[j >> 2], offset[j >> 2]);
+        // 0x4B0000cc is 2^23 + code: the subtraction leaves the code less its bias, exactly
+        constexpr float kOff = -8388608.0f - (float)GroupBytes<TYPE>::bias;
+        Pair lo = pair_add(pair_of(__byte_perm(c[j], 0x4B000000u, 0x7650), __byte_perm(c[j], 0x4B000000u, 0x7651)), pair_of(kOff, kOff));
+        Pair hi = pair_add(pair_of(__byte_perm(c[j], 0x4B000000u, 0x7652), __byte_perm(c[j], 0x4B000000u, 0x7653)), pair_of(kOff, kOff));
+        lo = kOffset ? pair_fma(lo, by, plus) : pair_mul(lo, by);
+        hi = kOffset ? pair_fma(hi, by, plus) : pair_mul(hi, by);
+        acc[j >> 2][0] = j & 3 ? pair_fma(lo, v[2 * j], acc[j >> 2][0]) : pair_mul(lo, v[2 * j]);
+        acc[j >> 2][1] = j & 3 ? pair_fma(hi, v[2 * j + 1], acc[j >> 2][1]) : pair_mul(hi, v[2 * j + 1]);
+    }
+    const Pair both = pair_add(pair_add(acc[0][0], acc[0][1]), pair_add(acc[1][0], acc[1][1]));
+    return pair_at(both, 0) + pair_at(both, 1);
+}
+
 // CTAs the registers are cut for: what is in flight per SM counts more than what a warp has in flight by itself, until the formats of many
 // words a group begin to spill with four rows. (4096 x 4096, a row a warp, four CTAs: Q4_1 6.8 us, Q5_0 7.5, Q2_K 7.3; left to the
 // compiler 8.6, 9.7, 9.8. Q5_K 14336 x 4096, four rows: two CTAs 22.9, three 35.6.)
@@ -240,14 +271,13 @@ constexpr int ctas_per_sm() {
 // for all of its rows, whose bytes are all in flight before the first is decoded. A weight is put together whole (scale * code + offset,
 // rounded once, as the decoders do) before it meets its input: scaled and offset sums kept apart cost two multiplies less per four weights,
 // but cancel against each other (2.3e-7 against 64 bits where decoding value by value has 1.0e-7, Q5_K over 512 inputs), and a code
-// times a large input can leave the range that the weight's own product stays in. What bounds it is instruction issue (per four
-// weights: two or three to isolate the codes, four to place them, six packed ones). Measured, Q5_K 14336 x 4096, one token: 26.5 us (28.2 with the sums kept apart); decoding value by
-// value, every header field once per value, took 175.6.
+// times a large input can leave the range that the weight's own product stays in. Per four
+// weights: two or three instructions to isolate the codes, four to place them, six packed ones. Measured, Q5_K 14336 x 4096, one token: 26.5 us (28.2 with the sums kept apart; with a ring,
+// below, 20.9); decoding value by value, every header field once per value, took 175.6.
 template <int TYPE, int ROWS>
 __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* x,
                                                                         int64_t sk, int64_t st, float* __restrict__ y, int64_t yn, int64_t yt) {
     extern __shared__ __align__(16) float xs[];
-    constexpr bool kOffset = TYPE == RQ_Q4_1 || TYPE == RQ_Q5_1 || TYPE == RQ_Q5_K || TYPE == RQ_Q2_K;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, token = blockIdx.y;
     const float* xt = x + (int64_t)token * st;
@@ -269,7 +299,7 @@ __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gem
             const int g = g0 + i;
             GroupBytes<TYPE> raw[ROWS];
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r) raw[r].load(base[r], g);
+            for (int r = 0; r < ROWS; ++r) raw[r].template load<false>(base[r], g);
             Pair v[16];  // the group's inputs
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -279,24 +309,7 @@ __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gem
             }
 #pragma unroll
             for (int r = 0; r < ROWS; ++r) {
-                uint32_t c[8];
-                float scale[2], offset[2];
-                raw[r].decode(g, c, scale, offset);
-                Pair acc[2][2];  // per sixteen: inputs 0, 1 and 2, 3 of every four
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const Pair by = pair_of(scale[j >> 2], scale[j >> 2]), plus = pair_of(offset[j >> 2], offset[j >> 2]);
-                    // 0x4B0000cc is 2^23 + code: the subtraction leaves the code less its bias, exactly
-                    constexpr float kOff = -8388608.0f - (float)GroupBytes<TYPE>::bias;
-                    Pair lo = pair_add(pair_of(__byte_perm(c[j], 0x4B000000u, 0x7650), __byte_perm(c[j], 0x4B000000u, 0x7651)), pair_of(kOff, kOff));
-                    Pair hi = pair_add(pair_of(__byte_perm(c[j], 0x4B000000u, 0x7652), __byte_perm(c[j], 0x4B000000u, 0x7653)), pair_of(kOff, kOff));
-                    lo = kOffset ? pair_fma(lo, by, plus) : pair_mul(lo, by);
-                    hi = kOffset ? pair_fma(hi, by, plus) : pair_mul(hi, by);
-                    acc[j >> 2][0] = j & 3 ? pair_fma(lo, v[2 * j], acc[j >> 2][0]) : pair_mul(lo, v[2 * j]);
-                    acc[j >> 2][1] = j & 3 ? pair_fma(hi, v[2 * j + 1], acc[j >> 2][1]) : pair_mul(hi, v[2 * j + 1]);
-                }
-                const Pair both = pair_add(pair_add(acc[0][0], acc[0][1]), pair_add(acc[1][0], acc[1][1]));
-                sum[r] += pair_at(both, 0) + pair_at(both, 1);
+                sum[r] += dot_group<TYPE>(raw[r], g, v);
             }
         }
     }
@@ -306,6 +319,94 @@ __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gem
         for (int off = 16; off > 0; off >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], off);
         if (lane == 0 && row0 + r < rows) y[(row0 + r) * yn + (int64_t)token * yt] = sum[r];
     }
+}
+
+// The same product where a row and 32 of its groups are whole 16-byte lines: a warp owns a range of rows (an equal share, to one row) and
+// brings up to four of them at a time, 32 groups of each, into a ring of its own in shared memory with bulk copies, which start before the wait
+// for the kernel before. The kernel above leaves a warp waiting for memory between its dots (a quarter of the issue slots used): its registers hold
+// one round's bytes, and 448 CTAs of 296 at a time are two rounds where one and a half would do. The same additions in the same order. What
+// bounds it is instruction issue (codes turned into fp32 by conversions instead of byte permutes: 22.9). us before / now: Q5_K 14336 x 4096 26.5 / 20.9,
+// 60000 x 2560 63.6 / 54.3; Q4_1 14336 x 4096 19.5 / 15.6; Q8_1 20.5 / 16.2.
+constexpr int kRingRows = 4, kRingMax = 4;
+template <int TYPE>
+__global__ void __launch_bounds__(kWarps * 32, 2) rq_gemv_ring_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int row_bytes, int chunk_bytes, int stages, int groups, const float* x, int64_t sk,
+                                                                    int64_t st, float* __restrict__ y, int64_t yn, int64_t yt, int* error_flag, unsigned long long wait_ns) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    __shared__ __align__(8) uint64_t full[kWarps][kRingMax];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, token = blockIdx.y;
+    float* const xs = (float*)smem;
+    const int slot_bytes = kRingRows * chunk_bytes;
+    uint8_t* const ring = smem + ((groups * kGroupFloats * 4 + 127) & ~127) + warp * stages * slot_bytes;
+    const int64_t warps = (int64_t)gridDim.x * kWarps, me = (int64_t)blockIdx.x * kWarps + warp;
+    const int64_t row_end = rows * (me + 1) / warps;
+    int64_t next_row = rows * me / warps, row = next_row;  // of the copies; of the dots
+    const int chunks = (groups + 31) >> 5;
+    int next_chunk = 0;
+    if (lane == 0) {
+        for (int i = 0; i < stages; ++i) rqmma::mbar_init(&full[warp][i], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    // the next four rows' next 32 groups into `slot`: a lane a row
+    auto issue = [&](int slot) {
+        if (next_row >= row_end) return;
+        const int n = (int)min((int64_t)kRingRows, row_end - next_row), at = next_chunk * chunk_bytes, bytes = min(chunk_bytes, row_bytes - at);
+        if (lane == 0) rqmma::mbar_expect_tx(&full[warp][slot], (uint32_t)(n * bytes));
+        __syncwarp();
+        if (lane < n) rqmma::bulk_g2s(ring + slot * slot_bytes + lane * chunk_bytes, main_plane + (next_row + lane) * row_bytes + at, (uint32_t)bytes, &full[warp][slot]);
+        if (++next_chunk == chunks) { next_chunk = 0; next_row += n; }
+    };
+    for (int i = 0; i < stages; ++i) issue(i);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const float* const xt = x + (int64_t)token * st;
+    for (int k = threadIdx.x; k < groups * 32; k += kWarps * 32) xs[(k >> 5) * kGroupFloats + (k & 31)] = __ldcg(xt + (int64_t)k * sk);
+    __syncthreads();
+    int slot = 0;
+    uint32_t phase = 0;
+    bool dead = false;
+    while (row < row_end) {
+        const int n = (int)min((int64_t)kRingRows, row_end - row);
+        float sum[kRingRows];
+#pragma unroll
+        for (int r = 0; r < kRingRows; ++r) sum[r] = 0.f;
+        for (int g0 = 0; g0 < groups; g0 += 32) {
+            if (!rqmma::mbar_wait_warp(&full[warp][slot], phase, wait_ns, dead)) atomicExch(error_flag, 22);
+            const uint8_t* const from = ring + slot * slot_bytes;
+            if (g0 + lane < groups) {
+                Pair v[16];  // the group's inputs
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const ulonglong2 four = *(const ulonglong2*)(xs + (g0 + lane) * kGroupFloats + 4 * j);
+                    v[2 * j] = four.x;
+                    v[2 * j + 1] = four.y;
+                }
+#pragma unroll
+                for (int r = 0; r < kRingRows; ++r) {
+                    if (r < n) {
+                        GroupBytes<TYPE> raw;
+                        raw.template load<true>(from + r * chunk_bytes, lane);
+                        sum[r] += dot_group<TYPE>(raw, lane, v);
+                    }
+                }
+            }
+            // the slot's bytes have met their inputs: it may be filled again, once the reads are in order before the copies
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            issue(slot);
+            if (++slot == stages) { slot = 0; phase ^= 1; }
+        }
+#pragma unroll
+        for (int r = 0; r < kRingRows; ++r) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], off);
+            if (lane == 0 && r < n) y[(row + r) * yn + (int64_t)token * yt] = sum[r];
+        }
+        row += n;
+    }
+    // (every copy that was issued has been waited for, unless a wait ran out: then once more, so that none lands after the CTA has left)
+    if (dead)
+        for (int i = 0; i < stages; ++i) rqmma::mbar_wait(&full[warp][i], phase ^ (i < slot ? 1 : 0), wait_ns);
 }
 
 // `.int(4)`: int8 activation records against Q4_1 blocks (block32 slice kind 3, build.rs:777-796). Per 16-value slice
@@ -395,8 +496,49 @@ int launch_generic_rows(const rq_weight* w, const float* x, int64_t sk, int64_t 
     RQ_CUDA(cudaLaunchKernelEx(&cfg, rq_gemv_generic_kernel<TYPE, ROWS>, (const uint8_t*)w->main, w->rows, row_bytes, groups, x, sk, st, y, yn, yt));
     return RQ_OK;
 }
+// RQ_ERR_UNSUPPORTED, the kernel without a ring: rows or 32 groups that are not whole lines (Q3_K, odd widths); more inputs than lie in shared
+// memory at once; fewer rows than four a warp, or several tokens, which have warps enough to hide each other's waits (Q4_1, us without / with
+// the ring: 1000 x 8192 6.9 / 9.2, 4096 x 4096 6.8 / 7.1, four tokens of 9000 x 3072 24.9 / 30.6; 14336 x 4096 20.5 / 16.6); blocks whose words
+// straddle the ring's banks worst (18, 22 and 24 bytes), where a row's last round is part-filled or the inputs leave the ring few slots (Q5_1
+// 60000 x 2560 44.7 / 46.7, 12000 x 7168 25.1 / 25.5, 14336 x 4096 20.8 / 17.4; Q5_0 50.6 / 52.2, 27.7 / 28.4, 23.9 / 19.2).
 template <int TYPE>
-int launch_generic(const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, int sm_count, cudaStream_t s) {
+int launch_ring(const rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s) {
+    const int groups = (int)(w->cols >> 5);
+    const int64_t row_bytes = w->cols / rq_block_values(TYPE) * rq_block_bytes(TYPE);
+    const int chunk_bytes = 1024 / rq_block_values(TYPE) * rq_block_bytes(TYPE);
+    constexpr bool kShortBlocks = TYPE == RQ_Q5_0 || TYPE == RQ_Q5_1 || TYPE == RQ_IQ4_NL;
+    if (tokens > 1 || w->rows < (int64_t)ctx->sm_count * 2 * kWarps * kRingRows || (kShortBlocks && (groups % 32 || w->cols > 4096))) return RQ_ERR_UNSUPPORTED;
+    if (w->cols > 32 * kChunkGroups || row_bytes % 16 || chunk_bytes % 16 || ((uintptr_t)w->main & 15)) return RQ_ERR_UNSUPPORTED;
+    // two CTAs an SM: as many slots as fit half of its shared memory beside the inputs
+    const size_t inputs = ((size_t)groups * kGroupFloats * 4 + 127) & ~(size_t)127, slot = (size_t)kWarps * kRingRows * chunk_bytes;
+    int stages = (int)((112 * 1024 - inputs) / slot);
+    if (stages < 2) return RQ_ERR_UNSUPPORTED;
+    if (stages > kRingMax) stages = kRingMax;
+    auto kernel = rq_gemv_ring_kernel<TYPE>;
+    static bool configured[64] = {};
+    if (ctx->device >= 64 || !configured[ctx->device]) {
+        RQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+        if (ctx->device < 64) configured[ctx->device] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    const int64_t ctas = (w->rows + kWarps - 1) / kWarps, most = (int64_t)ctx->sm_count * 2;
+    cfg.gridDim = dim3((unsigned)(ctas < most ? ctas : most), (unsigned)tokens);
+    cfg.blockDim = dim3(kWarps * 32);
+    cfg.dynamicSmemBytes = inputs + stages * slot;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    RQ_CUDA(cudaLaunchKernelEx(&cfg, kernel, (const uint8_t*)w->main, w->rows, (int)row_bytes, chunk_bytes, stages, groups, x, sk, st, y, yn, yt, ctx->error_flag, ctx->wait_limit_ns));
+    return RQ_OK;
+}
+template <int TYPE>
+int launch_generic(const rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s) {
+    const int rc = launch_ring<TYPE>(ctx, w, x, sk, st, tokens, y, yn, yt, s);
+    if (rc != RQ_ERR_UNSUPPORTED) return rc;
+    const int sm_count = ctx->sm_count;
     // rows per warp: as many as leave every SM two CTAs (a row's sums do not depend on it)
     const int64_t warps = (int64_t)sm_count * 2 * kWarps / (tokens < 8 ? tokens : 8);
     if (w->rows >= 4 * warps) return launch_generic_rows<TYPE, 4>(w, x, sk, st, tokens, y, yn, yt, s);
@@ -409,7 +551,7 @@ int launch_generic(const rq_weight* w, const float* x, int64_t sk, int64_t st, i
 int rq_launch_gemv_generic(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s) {
     if (tokens > 65535) return rq_fail(RQ_ERR_LIMIT, "matvec: %d tokens over a %d-type weight, at most 65535 per call", tokens, w->type);
     switch (w->type) {
-#define RQ_CASE(T) case T: return launch_generic<T>(w, x, sk, st, tokens, y, yn, yt, ctx->sm_count, s);
+#define RQ_CASE(T) case T: return launch_generic<T>(ctx, w, x, sk, st, tokens, y, yn, yt, s);
         RQ_DECODE_ONLY_TYPES(RQ_CASE)
 #undef RQ_CASE
         default: return rq_fail(RQ_ERR_INVALID, "matvec: type %d", w->type);
