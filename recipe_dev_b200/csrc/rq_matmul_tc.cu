@@ -168,7 +168,7 @@ template <int TYPE> struct Stored {
             for (int j = 0; j < 8; ++j) {
                 const __half2 s2 = j < 4 ? s_first : s_second;
                 const uint32_t q4 = ((lw[j] >> (4 * sel)) & 0x0F0F0F0Fu) | (((hw[j] >> (2 * g)) & 0x03030303u) << 4);  // four six-bit codes
-                const uint32_t a = (q4 & 0x00FF00FFu) | 0x64006400u, b = ((q4 >> 8) & 0x00FF00FFu) | 0x64006400u;
+                const uint32_t a = __byte_perm(q4, 0x64646464u, 0x4240), b = __byte_perm(q4, 0x64646464u, 0x4341);  // bytes 0, 2 and 1, 3 under 0x64
                 const __half2 ca = __hsub2(as_half2(a), k1056), cb = __hsub2(as_half2(b), k1056);  // q - 32
                 const __half2 ha = __hmul2(ca, s2), hb = __hmul2(cb, s2);
                 o[2 * j] = as_u32(ha);
@@ -183,8 +183,8 @@ template <int TYPE> struct Stored {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const uint32_t c = w[j] ^ 0x80808080u;  // code + 128
-                o[2 * j] = as_u32(__hsub2(as_half2((c & 0x00FF00FFu) | 0x64006400u), k1152));
-                o[2 * j + 1] = as_u32(__hsub2(as_half2(((c >> 8) & 0x00FF00FFu) | 0x64006400u), k1152));
+                o[2 * j] = as_u32(__hsub2(as_half2(__byte_perm(c, 0x64646464u, 0x4240)), k1152));  // bytes 0, 2 under 0x64; then 1, 3
+                o[2 * j + 1] = as_u32(__hsub2(as_half2(__byte_perm(c, 0x64646464u, 0x4341)), k1152));
             }
         } else {
             const uint4& q = v[half];
