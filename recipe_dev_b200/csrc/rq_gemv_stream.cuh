@@ -115,6 +115,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
     }
     return true;
 }
+// A whole warp waits: every lane has seen the phase, or (the limit ran out in one) every lane is told that it did not. The vote is what a
+// warp needs in which one lane then acts on the slot: a parity says odd or even, so a slot refilled while a lane has yet to look would
+// show that lane a phase it takes for the old one.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned long long limit_ns) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit_ns));
+}
 // Weights are read once per launch: the copies carry an evict-first L2 policy, so the stream does not push
 // the activations, the outputs and the kernel's own code out of L2 between launches.
 __device__ __forceinline__ uint64_t evict_first_policy() {
@@ -1226,7 +1232,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     r = stop;
                 }
                 const RqSegment& sg = segs[seg];
-                if (st >= p.stages && !mbar_wait(&empty_bar[slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 1); failed = true; break; }
+                if (st >= p.stages && !mbar_wait_warp(&empty_bar[slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 1); failed = true; break; }
                 uint8_t* dst = ring + (size_t)slot * p.stage_bytes;
                 if (leader)
                     stage_info[slot] = make_int4(nr, seg, (int)lr0,
@@ -1235,7 +1241,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     // at most `window` pieces in flight: wait for the one issued `window` pieces ago
                     if (n_pieces >= p.window) {
                         const int old_piece = n_pieces - p.window, old_st = old_piece / p.pieces;
-                        if (!mbar_wait(&full_bar[2 * (old_st % p.stages) + (old_piece - old_st * p.pieces)], (old_st / p.stages) & 1, p.wait_ns)) { atomicExch(p.error_flag, 4); failed = true; break; }
+                        if (!mbar_wait_warp(&full_bar[2 * (old_st % p.stages) + (old_piece - old_st * p.pieces)], (old_st / p.stages) & 1, p.wait_ns)) { atomicExch(p.error_flag, 4); failed = true; break; }
                     }
                     ++n_pieces;
                     if (!leader) continue;
@@ -1316,7 +1322,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             issue(0x7fffffff);
             if (p.warp_rows && !failed) {
                 // the warp scheme's consumers read what each slot holds from stage_info: a stage of no rows ends their loop
-                if (st >= p.stages && !mbar_wait(&empty_bar[slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 1); failed = true; }
+                if (st >= p.stages && !mbar_wait_warp(&empty_bar[slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 1); failed = true; }
                 else {
                     if (leader) {
                         stage_info[slot] = make_int4(0, 0, 0, 0);
@@ -1329,7 +1335,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             // leave only after every copy this CTA issued has landed (bounded)
             for (int w = (issued > p.stages ? issued - p.stages : 0); w < issued; ++w)
                 for (int k = 0; k < p.pieces; ++k)
-                    if (!mbar_wait(&full_bar[2 * (w % p.stages) + k], (w / p.stages) & 1, p.wait_ns)) { atomicExch(p.error_flag, 2); break; }
+                    if (!mbar_wait_warp(&full_bar[2 * (w % p.stages) + k], (w / p.stages) & 1, p.wait_ns)) { atomicExch(p.error_flag, 2); break; }
         }
     } else {
         // ---------------------------------------------------------------- consumers
