@@ -25,6 +25,7 @@
 #include <string.h>
 
 #include "rq_internal.cuh"
+#include "rq_mma.cuh"
 
 namespace rqstream {
 
@@ -1193,14 +1194,21 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
         }
     };
 
-    if (tid >= kConsumers) {
+    // (the warp's number by a shuffle: visibly the same for the whole warp, so the producer's numbers stay in uniform registers)
+    if (__shfl_sync(0xffffffffu, tid >> 5, 0) >= NW) {
         // ---------------------------------------------------------------- producer warp
         // All lanes walk the stages and wait together, one lane acts: a look at a barrier by a lone lane is not suspended, it is repeated
-        // every 160 cycles, takes issue slots from the consumers and sees an arrival 100 to 200 cycles later than a whole warp does (Q8_0 4096 x 4096, calls back to
-        // back: 7.2 us so, 6.3 with the whole warp).
-        const bool leader = tid == kConsumers;
+        // every 160 cycles, takes issue slots from the consumers and sees an arrival 100 to 200 cycles later than a whole warp does. What
+        // lies between a slot that comes free and its copies is a chain that short rings do not hide, so it is kept short: the warp known as
+        // uniform and its leader elected, the piece `window` back counted along instead of found by divisions, addresses before the waits.
+        // us, launches back to back, lone lane / whole warp without these / with them: Q8_0 4096 x 4096 int8 6.8 / 6.0 / 5.5, 9000 x 8192
+        // int8 18.5 / 16.8 / 16.1, 14336 x 4096 fp32 16.4 / 16.8 / 16.2; Q4_K 4096 x 4096 fp32 7.6 / 7.9 / 7.5, eight positions of it 49.4 / 49.2 / 50.3;
+        // 64 Q6_K experts of 2560 x 1024, eight positions, 190 / 192 / 183.
+        const bool leader = rqmma::elect_one();  // (the same lane every time)
         int issued = 0, seg = 0, slot = 0, st = 0, n_pieces = 0;
         uint32_t phase = 1;  // parity of the slot's previous round: the first round of the ring waits for nothing
+        int back_slot = 0, back_piece = 0;  // the piece issued `window` pieces ago, counted along
+        uint32_t back_phase = 0;
         int64_t r = 0;
         const RqSegment* segs = p.inline_seg;
         bool failed = false;
@@ -1232,46 +1240,55 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     r = stop;
                 }
                 const RqSegment& sg = segs[seg];
+                // (where the stage's bytes are, before the waits: behind them it would be part of the chain)
+                const uint8_t* const main0 = sg.main[0] + lr0 * row_bytes;
+                const uintptr_t scales0 = TYPE != RQ_Q4_K ? (uintptr_t)sg.scale[0] + (uintptr_t)(lr0 * row_scales * 2) : 0;
                 if (st >= p.stages && !mbar_wait_warp(&empty_bar[slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 1); failed = true; break; }
                 uint8_t* dst = ring + (size_t)slot * p.stage_bytes;
                 if (leader)
                     stage_info[slot] = make_int4(nr, seg, (int)lr0,
-                                                 TYPE != RQ_Q4_K ? (int)(((uintptr_t)sg.scale[0] + (uintptr_t)(lr0 * row_scales * 2)) & 15) : 0);
+                                                 TYPE != RQ_Q4_K ? (int)(scales0 & 15) : 0);
                 for (int k = 0; k < p.pieces; ++k) {
                     // at most `window` pieces in flight: wait for the one issued `window` pieces ago
                     if (n_pieces >= p.window) {
-                        const int old_piece = n_pieces - p.window, old_st = old_piece / p.pieces;
-                        if (!mbar_wait_warp(&full_bar[2 * (old_st % p.stages) + (old_piece - old_st * p.pieces)], (old_st / p.stages) & 1, p.wait_ns)) { atomicExch(p.error_flag, 4); failed = true; break; }
+                        const bool there = mbar_wait_warp(&full_bar[2 * back_slot + back_piece], back_phase, p.wait_ns);
+                        if (++back_piece == p.pieces) {
+                            back_piece = 0;
+                            if (++back_slot == p.stages) { back_slot = 0; back_phase ^= 1; }
+                        }
+                        if (!there) { atomicExch(p.error_flag, 4); failed = true; break; }
                     }
                     ++n_pieces;
-                    if (!leader) continue;
-                    uint64_t* bar = &full_bar[2 * slot + k];
-                    int rows_k = nr - k * p.piece_rows;
-                    rows_k = rows_k < 0 ? 0 : (rows_k > p.piece_rows ? p.piece_rows : rows_k);
-                    if (p.pieces == 1) rows_k = nr;
-                    const uint32_t main_bytes = (uint32_t)(rows_k * row_bytes);
-                    // bytes first, then the copies: the barrier must expect them before any can complete.
-                    // The d values of the whole stage travel with its first piece.
-                    uint32_t total = main_bytes * subs;
-                    if (TYPE != RQ_Q4_K && k == 0) {
-                        for (int s = 0; s < subs; ++s) {
-                            // the rows' d values, widened to whole 16-byte lines (the plane has slack past its end)
-                            const uintptr_t first = (uintptr_t)sg.scale[s] + (uintptr_t)(lr0 * row_scales * 2);
-                            const uintptr_t last = first + (uintptr_t)nr * row_scales * 2;
-                            total += (uint32_t)(((last + 15) & ~(uintptr_t)15) - (first & ~(uintptr_t)15));
-                        }
-                    }
-                    mbar_expect_tx(bar, total);
-                    const int64_t piece_off = (int64_t)k * p.piece_rows * row_bytes;
-                    for (int s = 0; s < subs; ++s) {
-                        if (main_bytes) bulk_g2s(dst + (size_t)s * p.sub_main_bytes + piece_off, sg.main[s] + lr0 * row_bytes + piece_off, main_bytes, bar, policy);
+                    if (leader) {
+                        uint64_t* bar = &full_bar[2 * slot + k];
+                        int rows_k = nr - k * p.piece_rows;
+                        rows_k = rows_k < 0 ? 0 : (rows_k > p.piece_rows ? p.piece_rows : rows_k);
+                        if (p.pieces == 1) rows_k = nr;
+                        const uint32_t main_bytes = (uint32_t)(rows_k * row_bytes);
+                        // bytes first, then the copies: the barrier must expect them before any can complete.
+                        // The d values of the whole stage travel with its first piece.
+                        uint32_t total = main_bytes * subs;
                         if (TYPE != RQ_Q4_K && k == 0) {
-                            const uintptr_t first = (uintptr_t)sg.scale[s] + (uintptr_t)(lr0 * row_scales * 2);
-                            const uintptr_t last = first + (uintptr_t)nr * row_scales * 2;
-                            const uintptr_t a0 = first & ~(uintptr_t)15, a1 = (last + 15) & ~(uintptr_t)15;
-                            bulk_g2s(dst + (size_t)p.subs * p.sub_main_bytes + (size_t)s * p.sub_scale_bytes, (const void*)a0, (uint32_t)(a1 - a0), bar, policy);
+                            for (int s = 0; s < subs; ++s) {
+                                // the rows' d values, widened to whole 16-byte lines (the plane has slack past its end)
+                                const uintptr_t first = s == 0 ? scales0 : (uintptr_t)sg.scale[s] + (uintptr_t)(lr0 * row_scales * 2);
+                                const uintptr_t last = first + (uintptr_t)nr * row_scales * 2;
+                                total += (uint32_t)(((last + 15) & ~(uintptr_t)15) - (first & ~(uintptr_t)15));
+                            }
+                        }
+                        mbar_expect_tx(bar, total);
+                        const int64_t piece_off = (int64_t)k * p.piece_rows * row_bytes;
+                        for (int s = 0; s < subs; ++s) {
+                            if (main_bytes) bulk_g2s(dst + (size_t)s * p.sub_main_bytes + piece_off, (s == 0 ? main0 : sg.main[s] + lr0 * row_bytes) + piece_off, main_bytes, bar, policy);
+                            if (TYPE != RQ_Q4_K && k == 0) {
+                                const uintptr_t first = s == 0 ? scales0 : (uintptr_t)sg.scale[s] + (uintptr_t)(lr0 * row_scales * 2);
+                                const uintptr_t last = first + (uintptr_t)nr * row_scales * 2;
+                                const uintptr_t a0 = first & ~(uintptr_t)15, a1 = (last + 15) & ~(uintptr_t)15;
+                                bulk_g2s(dst + (size_t)p.subs * p.sub_main_bytes + (size_t)s * p.sub_scale_bytes, (const void*)a0, (uint32_t)(a1 - a0), bar, policy);
+                            }
                         }
                     }
+                    __syncwarp();
                 }
                 __syncwarp();
                 if (failed) break;
