@@ -60,8 +60,9 @@ struct Deal {
         while (c + 1 < share && begin(c + 1) < end) ++c;
         return c;
     }
-    // where CTA c leaves its sums of tile t: its first or its second place
-    RQ_HOST_DEVICE int place(int t, int c) const { return 2 * c + (begin(c) > (uint32_t)t * (uint32_t)units ? 0 : 1); }
+    // where CTA c leaves its sums of a tile whose pieces begin at CTA `first`: the tile's first CTA began in an earlier tile or where this
+    // one does and uses its second place, the others began in this tile and use their first
+    static RQ_HOST_DEVICE int place(int c, int first) { return 2 * c + (c == first ? 1 : 0); }
 };
 
 // The tiles and unit ranges of one CTA, in the order every role walks them.
@@ -89,7 +90,7 @@ struct Walk {
 
 struct TcCut {
     int mh, bn, n_tiles, tiles_m, units, image_tiles, windows, ctas, whole, rest_tiles, share;
-    int raw_slots, b_slots, a_slots, accs, accs_more;  // (accs_more: a last step's accumulators, where an odd number of steps fits)
+    int raw_slots, b_slots, a_slots, accs;
     size_t smem, records_bytes, xs_bytes, steps_bytes, partial_bytes;
 };
 struct FormatSizes { int raw_bytes, a_cols, raw_per_unit; };
@@ -134,8 +135,7 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     c.a_slots = type == RQ_Q6_K ? (c.mh == 1 ? 4 : 2) : (c.mh == 1 && 512 - 8 * f.a_cols - totals >= 2 * step_cols ? 8 : 4);
     int steps = (512 - c.a_slots * f.a_cols - totals) / step_cols;
     if (steps > kMaxAcc / halves) steps = kMaxAcc / halves;
-    c.accs = (steps & ~1) * halves;
-    c.accs_more = (steps & 1) * halves;
+    c.accs = steps * halves;
     // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window; codes, MH = 2: and the totals)
     const int kept = (c.mh == 1 ? c.bn * 128 * 4 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0) + (codes && c.mh == 2 ? c.bn * 256 * 4 : 0), budget = (codes ? 212 : 220) * 1024 - kept, b_bytes = c.bn * (codes ? 128 : 256);
     c.b_slots = c.mh == 1 || codes ? 4 : 3;

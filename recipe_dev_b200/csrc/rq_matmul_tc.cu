@@ -747,9 +747,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         }
                     }
                 } else {
-                    // (where a CTA leaves its sums, Deal::place: the tile's first CTA began in an earlier tile or where this one does, the others in it)
                     const size_t tile_floats = (size_t)bn * 128 * MH, place0 = (size_t)from * 128 * MH + half0 * 128 + r0;
-                    auto piece_of = [&](int c) { return p.partial + (size_t)(2 * c + (c == c0 ? 1 : 0)) * tile_floats + place0; };
+                    auto piece_of = [&](int c) { return p.partial + (size_t)Deal::place(c, c0) * tile_floats + place0; };
 #pragma unroll
                     for (int m = 0; m < kRows; ++m) {
                         const int n = live(m);
@@ -1131,7 +1130,7 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
     p.tiles_m = cut.tiles_m; p.whole = cut.whole; p.rest_tiles = cut.rest_tiles; p.share = cut.share;
     p.steps = (const float*)(xs + cut.xs_bytes);
     p.partial = partial; p.arrived = arrived;
-    p.raw_slots = cut.raw_slots; p.b_slots = cut.b_slots; p.a_slots = cut.a_slots; p.accs = cut.accs + cut.accs_more;
+    p.raw_slots = cut.raw_slots; p.b_slots = cut.b_slots; p.a_slots = cut.a_slots; p.accs = cut.accs;
     p.error_flag = ctx->error_flag; p.wait_ns = ctx->wait_limit_ns;
     switch (w->type) {
         case RQ_Q4_K: rc = launch_tc<RQ_Q4_K>(p, cut.mh, codes, cut.ctas, cut.smem, s); break;

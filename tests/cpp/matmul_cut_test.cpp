@@ -16,12 +16,23 @@ static int walk_call(int type, bool codes, int sms, int64_t rows, int64_t cols, 
     const TcCut c = tc_cut(type, codes, sms, rows, cols, tokens);
     const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles;
     if (c.tiles_m * 128LL * c.mh < rows || (int64_t)c.n_tiles * c.bn < tokens) return fail("outputs outside every tile", type, codes, sms, rows, cols, tokens);
-    // tensor memory: accumulators, totals of the codes' sums, operand slots; rings that alternate between two issuing threads; shared memory
+    // tensor memory, 512 columns: accumulators of at least two steps, (codes, one row half) two sets of totals, operand slots, found by a mask
     const bool k = type == RQ_Q4_K || type == RQ_Q6_K;
-    const int acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn;
-    if (c.accs * acc_cols + (codes ? 2 * c.bn : 0) + c.a_slots * format_sizes(type).a_cols > 512 || c.accs < (k ? 2 : 4) || c.accs > kMaxAcc || c.accs % (k ? 2 : 4) || c.a_slots < 2 || c.a_slots > kMaxA ||
-        c.a_slots % 2 || c.b_slots < 2 || c.b_slots > kMaxB || c.raw_slots < 2 || c.raw_slots > kMaxRaw || c.smem > (size_t)(codes ? 218 : 225) * 1024 || c.b_slots * c.mh * (k ? 1 : 2) >= 32)
+    const int acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn, totals = codes && c.mh == 1 ? 2 * c.bn : 0;
+    if (c.accs * acc_cols + totals + c.a_slots * format_sizes(type).a_cols > 512 || c.accs < (k ? 2 : 4) || c.accs > kMaxAcc || c.accs % (k ? 1 : 2) || c.a_slots < 2 || c.a_slots > kMaxA ||
+        (c.a_slots & (c.a_slots - 1)))
+        return fail("tensor memory", type, codes, sms, rows, cols, tokens);
+    // rings whose slots keep their waiters, and nobody as many steps ahead as there are step barriers (32)
+    const bool even_raw = c.mh == 2 || type == RQ_Q8_0;
+    if (c.b_slots < 2 || c.b_slots > kMaxB || (c.mh == 1 && c.b_slots % 2) || c.raw_slots < 2 || c.raw_slots > kMaxRaw || (even_raw && c.raw_slots % 2) || c.b_slots * c.mh * (k ? 1 : 2) >= 32)
         return fail("rings", type, codes, sms, rows, cols, tokens);
+    // shared memory: the rings, what the drain and staging warps keep behind them, and room to align
+    const size_t b_bytes = (size_t)c.bn * (codes ? 128 : 256), kept = (c.mh == 1 ? c.bn * 512 : (codes ? c.bn * 1024 : 0)) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0);
+    if (c.b_slots * b_bytes + (size_t)c.raw_slots * format_sizes(type).raw_bytes + kept + 1024 > c.smem || c.smem > (size_t)(codes ? 218 : 225) * 1024)
+        return fail("shared memory", type, codes, sms, rows, cols, tokens);
+    // token tiles of a width that the drain loops are instantiated for
+    const bool width = c.mh == 1 ? c.bn == 16 || c.bn == 32 || c.bn == 48 || c.bn == 64 : (codes ? c.bn == 64 : (k ? c.bn == 96 || c.bn == 128 : c.bn == 64 || c.bn == 96));
+    if (!width) return fail("a tile of another width", type, codes, sms, rows, cols, tokens);
     std::vector<int> next_unit(tiles, 0), arrivals(c.rest_tiles, 0), summed(c.rest_tiles, 0);
     std::vector<char> place_used((size_t)2 * c.share, 0);
     for (int cta = 0; cta < c.ctas; ++cta) {  // in CTA order, a tile's pieces come in unit order
@@ -36,13 +47,13 @@ static int walk_call(int type, bool codes, int sms, int64_t rows, int64_t cols, 
             const int t = (int)(tile - (int64_t)c.whole * c.ctas);
             if (t < 0 || t >= c.rest_tiles) return fail("a whole tile cut in pieces", type, codes, sms, rows, cols, tokens);
             const Deal deal(c.share, c.rest_tiles, c.units);
-            const int first = deal.first(t), last = deal.last(t, cta), place = deal.place(t, cta);
+            const int first = deal.first(t), last = deal.last(t, cta), place = Deal::place(cta, first);
             if (cta < first || cta > last || place < 0 || place >= 2 * c.share || place_used[place]) return fail("a piece's place", type, codes, sms, rows, cols, tokens);
             place_used[place] = 1;
             if (arrivals[t]++ == last - first) {  // the last one to arrive adds the pieces first .. last
                 ++summed[t];
                 for (int p = first; p <= last; ++p)
-                    if (!place_used[deal.place(t, p)]) return fail("a sum over a piece nobody left", type, codes, sms, rows, cols, tokens);
+                    if (!place_used[Deal::place(p, first)]) return fail("a sum over a piece nobody left", type, codes, sms, rows, cols, tokens);
             }
         }
         if (segments > c.whole + 2) return fail("more than two pieces", type, codes, sms, rows, cols, tokens);
