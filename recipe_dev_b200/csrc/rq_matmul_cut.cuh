@@ -102,6 +102,52 @@ inline FormatSizes format_sizes(int type) {
         default: return {Format<RQ_Q4_0>::raw_bytes, Format<RQ_Q4_0>::a_cols, 1};
     }
 }
+// Tokens per tile and token tiles, of tiles of at most `widest` tokens in steps of `grain`.
+struct TokenTiles { int n, bn; };
+inline TokenTiles token_tiles(int tokens, int widest, int grain) {
+    TokenTiles t;
+    t.n = (tokens + widest - 1) / widest;
+    t.bn = ((tokens + t.n - 1) / t.n + grain - 1) / grain * grain;
+    return t;
+}
+// Whole tiles per CTA, and the tiles that are left with the number of CTAs that share them out. Few tiles to share: more CTAs to a tile shorten its
+// products (some two microseconds a unit) and lengthen the last one's sum (most of a microsecond a piece, a trip to L2 each), so about
+// the square root of twice its units share one, at most (never more than it has).
+struct TileShare { int ctas, whole, rest_tiles, share; };
+inline TileShare share_out(int64_t tiles, int units, int sm_count) {
+    TileShare s;
+    s.ctas = tiles * units < sm_count ? (int)(tiles * units) : sm_count;
+    int pieces = 1;
+    while ((pieces + 1) * (pieces + 1) <= 2 * units) ++pieces;
+    if (tiles * pieces < s.ctas) s.ctas = (int)(tiles * pieces);
+    s.whole = (int)(tiles / s.ctas);
+    s.rest_tiles = (int)(tiles - (int64_t)s.whole * s.ctas);
+    s.share = (int64_t)s.rest_tiles * pieces < s.ctas ? s.rest_tiles * pieces : s.ctas;
+    return s;
+}
+// What the CTA with the most to do needs for a K-quant call of two row halves, roughly (one is some five nanoseconds): its units, each three hundred columns' worth of
+// staging and hand-offs besides its columns, and a shared tile's way out (two of them where the ranges do not end with the
+// tiles) with the sum over its pieces, both by the column. 312 calls (both K-quants, thirteen shapes, 65 to 509 tokens) timed with tiles of up to 96 and of up to 128
+// tokens: the lower estimate is the faster one, or within 7 % of it; where 128 had replaced 96 for every call, the few tiles of small weights and short rows took up to
+// 1.38 times as long (Q6_K, us, 96 / 128: 2000 x 1536 with 128 tokens 18.6 / 25.7, 12000 x 1024 with 256 35.1 / 44.5; 14336 x 4096 with 509 180 / 150).
+inline int64_t call_cost(int64_t row_tiles, int units, int tokens, int widest, int grain, int sm_count) {
+    const TokenTiles t = token_tiles(tokens, widest, grain);
+    const TileShare s = share_out(row_tiles * t.n, units, sm_count);
+    int64_t own = (int64_t)s.whole * units, ways = 0, pieces = 0;
+    if (s.share) {
+        const int64_t shared = (int64_t)s.rest_tiles * units;
+        own += (shared + s.share - 1) / s.share;
+        if (s.share % s.rest_tiles) {
+            const int64_t least = shared / s.share;
+            ways = 2;
+            pieces = (units + least - 1) / least + 1;
+        } else if (s.share > s.rest_tiles) {
+            ways = 1;
+            pieces = s.share / s.rest_tiles;
+        }
+    }
+    return 2 * own * (300 + t.bn) + t.bn * (10 * ways + pieces);
+}
 inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t cols, int tokens) {
     TcCut c;
     const FormatSizes f = format_sizes(type);
@@ -109,23 +155,18 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     // (fp32 activations over the 32-value formats: two accumulators a slice, of hi and lo columns each, twice; 48 tokens fit, 96 of two row halves)
     const int widest_1 = !codes && !kquant ? 48 : Shape<1, false>::cols;
     c.mh = tokens <= widest_1 ? 1 : 2;
-    const int widest = c.mh == 1 ? widest_1 : (codes ? Shape<2, true>::cols : (kquant ? Shape<2, false>::cols : 96)), grain = c.mh == 2 ? 32 : 16;
-    c.n_tiles = (tokens + widest - 1) / widest;
-    c.bn = ((tokens + c.n_tiles - 1) / c.n_tiles + grain - 1) / grain * grain;
     c.tiles_m = (int)((rows + 128 * c.mh - 1) / (128 * c.mh));
     c.units = (int)((cols + 255) / 256);
+    const int grain = c.mh == 2 ? 32 : 16;
+    int widest = c.mh == 1 ? widest_1 : (codes ? Shape<2, true>::cols : 96);
+    if (c.mh == 2 && kquant && call_cost(c.tiles_m, c.units, tokens, Shape<2, false>::cols, grain, sm_count) <= call_cost(c.tiles_m, c.units, tokens, widest, grain, sm_count)) widest = Shape<2, false>::cols;
+    const TokenTiles t = token_tiles(tokens, widest, grain);
+    c.n_tiles = t.n;
+    c.bn = t.bn;
     c.windows = type == RQ_Q4_K ? (c.units + 3) / 4 : 0;
     c.image_tiles = 4 * c.units + c.windows;
-    const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles, work = tiles * c.units;
-    c.ctas = work < sm_count ? (int)work : sm_count;
-    // Few tiles to share: more CTAs to a tile shorten its products (some two microseconds a unit) and lengthen the last one's sum (most of
-    // a microsecond a piece, a trip to L2 each), so about the square root of twice its units share one, at most (never more than it has).
-    int pieces = 1;
-    while ((pieces + 1) * (pieces + 1) <= 2 * c.units) ++pieces;
-    if (tiles * pieces < c.ctas) c.ctas = (int)(tiles * pieces);
-    c.whole = (int)(tiles / c.ctas);
-    c.rest_tiles = (int)(tiles - (int64_t)c.whole * c.ctas);
-    c.share = (int64_t)c.rest_tiles * pieces < c.ctas ? c.rest_tiles * pieces : c.ctas;
+    const TileShare sh = share_out((int64_t)c.tiles_m * c.n_tiles, c.units, sm_count);
+    c.ctas = sh.ctas; c.whole = sh.whole; c.rest_tiles = sh.rest_tiles; c.share = sh.share;
     // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: MH = 1, the issuing warps
     // take alternate activation slots, and Q8_0's staging groups every second tile of stored bytes; MH = 2, a staging group every second
     // tile: even numbers of each. (The steps' own barriers are indexed by the step.)

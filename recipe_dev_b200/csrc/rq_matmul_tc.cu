@@ -32,8 +32,8 @@
 // formats whose scale changes there) and the small cross terms go first or into columns of their own.
 //
 // Two forms. MH = 1 (token tiles of up to 64): B_hi and B_lo are one operand of 2 * bn columns, so a slice is four (Q6_K:
-// eight) instructions and the low products have accumulators of their own. MH = 2 (token tiles of up to 128, of 96 over the 32-value
-// formats, whose two sums a slice take the columns): two row halves share each activation tile, which halves the activation bytes a
+// eight) instructions and the low products have accumulators of their own. MH = 2 (token tiles of up to 128 or, where that leaves few tiles to
+// many CTAs, of up to 96: rq_matmul_cut.cuh; of 96 over the 32-value formats, whose two sums a slice take the columns): two row halves share each activation tile, which halves the activation bytes a
 // CTA pulls from L2 (they, at 4 bytes per input and token, are what the large shapes would be bound by); products of hi and lo
 // share an accumulator, a row half has four drain warps with up to 128 fp32 sums a thread (setmaxnreg; CODES: tiles of up to 64).
 //
@@ -809,7 +809,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             run_tiles(Columns<S::cols / 2>());  // (windows of more than 64 tokens are cut into tiles of 33 to 64)
         } else if constexpr (MH == 2) {
             if (bn == 96) run_tiles(Columns<96>());
-            else run_tiles(Columns<F::kquant ? S::cols : 64>());
+            else if (F::kquant && bn == 128) run_tiles(Columns<F::kquant ? 128 : 64>());
+            else run_tiles(Columns<64>());
         } else {
             switch (bn) {
                 case 16: run_tiles(Columns<16>()); break;

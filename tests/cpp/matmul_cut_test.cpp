@@ -31,7 +31,7 @@ static int walk_call(int type, bool codes, int sms, int64_t rows, int64_t cols, 
     if (c.b_slots * b_bytes + (size_t)c.raw_slots * format_sizes(type).raw_bytes + kept + 1024 > c.smem || c.smem > (size_t)(codes ? 218 : 225) * 1024)
         return fail("shared memory", type, codes, sms, rows, cols, tokens);
     // token tiles of a width that the drain loops are instantiated for
-    const bool width = c.mh == 1 ? c.bn == 16 || c.bn == 32 || c.bn == 48 || c.bn == 64 : (codes ? c.bn == 64 : (k ? c.bn == 96 || c.bn == 128 : c.bn == 64 || c.bn == 96));
+    const bool width = c.mh == 1 ? c.bn == 16 || c.bn == 32 || c.bn == 48 || c.bn == 64 : (codes ? c.bn == 64 : c.bn == 64 || c.bn == 96 || (k && c.bn == 128));
     if (!width) return fail("a tile of another width", type, codes, sms, rows, cols, tokens);
     std::vector<int> next_unit(tiles, 0), arrivals(c.rest_tiles, 0), summed(c.rest_tiles, 0);
     std::vector<char> place_used((size_t)2 * c.share, 0);
@@ -69,6 +69,11 @@ int main() {
     const int types[4] = {RQ_Q4_K, RQ_Q6_K, RQ_Q8_0, RQ_Q4_0};
     const int64_t named[][3] = {{14336, 4096, 673}, {14336, 4096, 700}, {14336, 4096, 768}, {28672, 8192, 300}, {151936, 4096, 1}, {151936, 2560, 16}, {152064, 3584, 16}, {11008, 4096, 600},
                                 {8192, 2048, 400}, {25600, 5120, 200}, {19072, 512, 16}, {19200, 4096, 16}, {19072, 4096, 100}, {1, 256, 12}, {300, 16777216, 9}};
+    // how wide a K-quant's token tile is: where there are tiles enough a wide one, where few are shared by many CTAs a narrower one
+    const int64_t widths[][4] = {{14336, 4096, 509, 128}, {4096, 14336, 256, 128}, {8192, 1024, 256, 128}, {14336, 4096, 80, 96}, {12000, 1024, 256, 96}, {8192, 1024, 300, 96}, {2000, 1536, 128, 64}, {512, 14336, 128, 64}};
+    for (int type : {RQ_Q4_K, RQ_Q6_K})
+        for (const auto& w : widths)
+            if (tc_cut(type, false, 148, w[0], w[1], (int)w[2]).bn != w[3]) return fail("another tile width than the measured one", type, false, 148, w[0], w[1], (int)w[2]);
     for (int type : types)
         for (int codes = 0; codes < (type == RQ_Q8_0 || type == RQ_Q4_0 ? 2 : 1); ++codes) {
             for (const auto& n : named)
