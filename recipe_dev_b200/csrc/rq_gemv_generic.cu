@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) rq_gemv_ring_kernel(const uint
     const int64_t row_end = rows * (me + 1) / warps;
     int64_t next_row = rows * me / warps, row = next_row;  // of the copies; of the dots
     const int chunks = (groups + 31) >> 5;
-    int next_chunk = 0;
+    int next_chunk = 0, in_flight = 0;  // in_flight: slots issued and not yet waited for
     if (lane == 0) {
         for (int i = 0; i < stages; ++i) rqmma::mbar_init(&full[warp][i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -356,6 +356,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) rq_gemv_ring_kernel(const uint
         __syncwarp();
         if (lane < n) rqmma::bulk_g2s(ring + slot * slot_bytes + lane * chunk_bytes, main_plane + (next_row + lane) * row_bytes + at, (uint32_t)bytes, &full[warp][slot]);
         if (++next_chunk == chunks) { next_chunk = 0; next_row += n; }
+        ++in_flight;
     };
     for (int i = 0; i < stages; ++i) issue(i);
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -371,7 +372,11 @@ __global__ void __launch_bounds__(kWarps * 32, 2) rq_gemv_ring_kernel(const uint
 #pragma unroll
         for (int r = 0; r < kRingRows; ++r) sum[r] = 0.f;
         for (int g0 = 0; g0 < groups; g0 += 32) {
-            if (!rqmma::mbar_wait_warp(&full[warp][slot], phase, wait_ns, dead)) atomicExch(error_flag, 22);
+            if (!rqmma::mbar_wait_warp(&full[warp][slot], phase, wait_ns, dead)) {  // the slot is still being written: nothing more goes into it, or out of it
+                atomicExch(error_flag, 22);
+                break;
+            }
+            --in_flight;
             const uint8_t* const from = ring + slot * slot_bytes;
             if (g0 + lane < groups) {
                 Pair v[16];  // the group's inputs
@@ -396,6 +401,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) rq_gemv_ring_kernel(const uint
             issue(slot);
             if (++slot == stages) { slot = 0; phase ^= 1; }
         }
+        if (dead) break;
 #pragma unroll
         for (int r = 0; r < kRingRows; ++r) {
 #pragma unroll
@@ -404,9 +410,11 @@ __global__ void __launch_bounds__(kWarps * 32, 2) rq_gemv_ring_kernel(const uint
         }
         row += n;
     }
-    // (every copy that was issued has been waited for, unless a wait ran out: then once more, so that none lands after the CTA has left)
-    if (dead)
-        for (int i = 0; i < stages; ++i) rqmma::mbar_wait(&full[warp][i], phase ^ (i < slot ? 1 : 0), wait_ns);
+    // every copy that was issued has been waited for, unless a wait ran out: then once more, so that none lands after the CTA has left
+    for (; in_flight > 0; --in_flight) {
+        if (!rqmma::mbar_wait(&full[warp][slot], phase, wait_ns)) break;
+        if (++slot == stages) { slot = 0; phase ^= 1; }
+    }
 }
 
 // `.int(4)`: int8 activation records against Q4_1 blocks (block32 slice kind 3, build.rs:777-796). Per 16-value slice
