@@ -9,13 +9,13 @@
 #include "rq_decode.cuh"
 #include "rq_mma.cuh"
 #include "rq_pairs.cuh"
+#include "rq_ring_rule.cuh"
 
 namespace {
 
-constexpr int kWarps = 8;  // rows per CTA
-
-constexpr int kChunkGroups = 256;          // 32-value groups of x in shared memory at a time: 8192 inputs
-constexpr int kGroupFloats = 36;           // a group's 32 inputs, padded: 144 bytes, so that eight lanes on adjacent groups read eight bank groups
+using rqring::kChunkGroups;
+using rqring::kGroupFloats;
+using rqring::kWarps;
 
 // N words from a 2-byte aligned address (blocks of 18, 22 and 110 bytes): the aligned words around it, shifted together. Nothing past
 // the last wanted byte's word is touched.
@@ -263,8 +263,7 @@ __device__ __forceinline__ float dot_group(const GroupBytes<TYPE>& raw, int g, c
 // compiler 8.6, 9.7, 9.8. Q5_K 14336 x 4096, four rows: two CTAs 22.9, three 35.6.)
 template <int TYPE, int ROWS>
 constexpr int ctas_per_sm() {
-    constexpr bool many = TYPE == RQ_Q5_K || TYPE == RQ_Q3_K || TYPE == RQ_Q8_1 || TYPE == RQ_Q8_K || TYPE == RQ_IQ4_XS;
-    return ROWS == 1 ? 4 : (ROWS == 4 && many ? 2 : 3);
+    return ROWS == 1 ? 4 : (ROWS == 4 && rqring::many_words(TYPE) ? 2 : 3);
 }
 
 // A warp owns ROWS rows, its lanes the groups g, g + 32, ..: a lane reads its group's 32 inputs from shared memory once and uses them
@@ -324,12 +323,12 @@ __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gem
 // The same product where a row and 32 of its groups are whole 16-byte lines: a warp owns a range of rows (an equal share, to one row) and
 // brings up to four of them at a time, 32 groups of each, into a ring of its own in shared memory with bulk copies, which start before the wait
 // for the kernel before. The kernel above leaves a warp waiting for memory between its dots (a quarter of the issue slots used): its registers hold
-// one round's bytes, and 448 CTAs of 296 at a time are two rounds where one and a half would do. The same additions in the same order. What
+// one round's bytes, and its CTAs come to an SM in whole numbers (448 of them to 148). The same additions in the same order. What
 // bounds it is instruction issue (codes turned into fp32 by conversions instead of byte permutes: 22.9). us before / now: Q5_K 14336 x 4096 26.5 / 20.9,
 // 60000 x 2560 63.6 / 54.3; Q4_1 14336 x 4096 19.5 / 15.6; Q8_1 20.5 / 16.2.
-constexpr int kRingRows = 4, kRingMax = 4;
+constexpr int kRingRows = rqring::kRows, kRingMax = rqring::kMaxStages;
 template <int TYPE>
-__global__ void __launch_bounds__(kWarps * 32, 2) rq_gemv_ring_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int row_bytes, int chunk_bytes, int stages, int groups, const float* x, int64_t sk,
+__global__ void __launch_bounds__(kWarps * 32, rqring::kCtas) rq_gemv_ring_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int row_bytes, int chunk_bytes, int stages, int groups, const float* x, int64_t sk,
                                                                     int64_t st, float* __restrict__ y, int64_t yn, int64_t yt, int* error_flag, unsigned long long wait_ns) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[kWarps][kRingMax];
@@ -504,32 +503,23 @@ int launch_generic_rows(const rq_weight* w, const float* x, int64_t sk, int64_t 
     RQ_CUDA(cudaLaunchKernelEx(&cfg, rq_gemv_generic_kernel<TYPE, ROWS>, (const uint8_t*)w->main, w->rows, row_bytes, groups, x, sk, st, y, yn, yt));
     return RQ_OK;
 }
-// RQ_ERR_UNSUPPORTED, the kernel without a ring: rows or 32 groups that are not whole lines (Q3_K, odd widths); more inputs than lie in shared
-// memory at once; fewer rows than four a warp, or several tokens, which have warps enough to hide each other's waits (Q4_1, us without / with
-// the ring: 1000 x 8192 6.9 / 9.2, 4096 x 4096 6.8 / 7.1, four tokens of 9000 x 3072 24.9 / 30.6; 14336 x 4096 20.5 / 16.6); blocks whose words
-// straddle the ring's banks worst (18, 22 and 24 bytes), where a row's last round is part-filled or the inputs leave the ring few slots (Q5_1
-// 60000 x 2560 44.7 / 46.7, 12000 x 7168 25.1 / 25.5, 14336 x 4096 20.8 / 17.4; Q5_0 50.6 / 52.2, 27.7 / 28.4, 23.9 / 19.2).
+// RQ_ERR_UNSUPPORTED: the kernel without a ring (rq_ring_rule.cuh says which calls, and why).
 template <int TYPE>
 int launch_ring(const rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s) {
+    const int stages = rqring::stages(TYPE, ctx->sm_count, w->rows, w->cols, tokens);
+    if (!stages || ((uintptr_t)w->main & 15)) return RQ_ERR_UNSUPPORTED;
     const int groups = (int)(w->cols >> 5);
-    const int64_t row_bytes = w->cols / rq_block_values(TYPE) * rq_block_bytes(TYPE);
-    const int chunk_bytes = 1024 / rq_block_values(TYPE) * rq_block_bytes(TYPE);
-    constexpr bool kShortBlocks = TYPE == RQ_Q5_0 || TYPE == RQ_Q5_1 || TYPE == RQ_IQ4_NL;
-    if (tokens > 1 || w->rows < (int64_t)ctx->sm_count * 2 * kWarps * kRingRows || (kShortBlocks && (groups % 32 || w->cols > 4096))) return RQ_ERR_UNSUPPORTED;
-    if (w->cols > 32 * kChunkGroups || row_bytes % 16 || chunk_bytes % 16 || ((uintptr_t)w->main & 15)) return RQ_ERR_UNSUPPORTED;
-    // two CTAs an SM: as many slots as fit half of its shared memory beside the inputs
-    const size_t inputs = ((size_t)groups * kGroupFloats * 4 + 127) & ~(size_t)127, slot = (size_t)kWarps * kRingRows * chunk_bytes;
-    int stages = (int)((112 * 1024 - inputs) / slot);
-    if (stages < 2) return RQ_ERR_UNSUPPORTED;
-    if (stages > kRingMax) stages = kRingMax;
+    const int64_t row_bytes = w->cols / rqring::block_values(TYPE) * rqring::block_bytes(TYPE);
+    constexpr int chunk_bytes = rqring::chunk_bytes(TYPE);
+    const size_t inputs = rqring::input_bytes(w->cols), slot = (size_t)kWarps * rqring::kRows * chunk_bytes;
     auto kernel = rq_gemv_ring_kernel<TYPE>;
     static bool configured[64] = {};
     if (ctx->device >= 64 || !configured[ctx->device]) {
-        RQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
+        RQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rqring::kSmem));
         if (ctx->device < 64) configured[ctx->device] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    const int64_t ctas = (w->rows + kWarps - 1) / kWarps, most = (int64_t)ctx->sm_count * 2;
+    const int64_t ctas = (w->rows + kWarps - 1) / kWarps, most = (int64_t)ctx->sm_count * rqring::kCtas;
     cfg.gridDim = dim3((unsigned)(ctas < most ? ctas : most), (unsigned)tokens);
     cfg.blockDim = dim3(kWarps * 32);
     cfg.dynamicSmemBytes = inputs + stages * slot;
@@ -544,8 +534,10 @@ int launch_ring(const rq_ctx* ctx, const rq_weight* w, const float* x, int64_t s
 }
 template <int TYPE>
 int launch_generic(const rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk, int64_t st, int tokens, float* y, int64_t yn, int64_t yt, cudaStream_t s) {
-    const int rc = launch_ring<TYPE>(ctx, w, x, sk, st, tokens, y, yn, yt, s);
-    if (rc != RQ_ERR_UNSUPPORTED) return rc;
+    if constexpr (rqring::whole_lines(TYPE)) {
+        const int rc = launch_ring<TYPE>(ctx, w, x, sk, st, tokens, y, yn, yt, s);
+        if (rc != RQ_ERR_UNSUPPORTED) return rc;
+    }
     const int sm_count = ctx->sm_count;
     // rows per warp: as many as leave every SM two CTAs (a row's sums do not depend on it)
     const int64_t warps = (int64_t)sm_count * 2 * kWarps / (tokens < 8 ? tokens : 8);
