@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gem
 
 // The same product where a row and 32 of its groups are whole 16-byte lines: a warp owns a range of rows (an equal share, to one row) and
 // brings up to four of them at a time, 32 groups of each, into a ring of its own in shared memory with bulk copies, which start before the wait
-// for the kernel before. The kernel above leaves a warp waiting for memory between its dots (a quarter of the issue slots used): its registers hold
+// for the kernel before (the kernels that write weights let nothing behind them start early: rq_layout.cu, rq_requant.cu). The kernel above leaves a warp waiting for memory between its dots (a quarter of the issue slots used): its registers hold
 // one round's bytes, and its CTAs come to an SM in whole numbers (448 of them to 148). The same additions in the same order. What
 // bounds it is instruction issue (codes turned into fp32 by conversions instead of byte permutes: 22.9). us before / now: Q5_K 14336 x 4096 26.5 / 20.9,
 // 60000 x 2560 63.6 / 54.3; Q4_1 14336 x 4096 19.5 / 15.6; Q8_1 20.5 / 16.2.

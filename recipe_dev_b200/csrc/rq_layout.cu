@@ -1,4 +1,7 @@
 // Load-time layout kernels (GGUF blocks <-> device planes) and the bit-exact dequantiser.
+//
+// A kernel that writes weights never issues griddepcontrol.launch_dependents: the products read weights before their
+// griddepcontrol.wait, so that wait orders nothing for them, only the launch behind a writer that has ended does.
 #include "rq_decode.cuh"
 #include "rq_internal.cuh"
 

@@ -11,6 +11,9 @@
 // fptosi(q + 0.5) or fptosi(q - 0.5) by the sign of q (half away from zero by truncation; f32::round
 // differs when q + 0.5 itself rounds up), the scale is narrowed to fp16 with round to nearest even.
 //
+// No kernel here issues griddepcontrol.launch_dependents: a product over the new weight may be the next launch, and products read weights
+// before their griddepcontrol.wait.
+//
 // One warp takes one 32-value block: lane i decodes value i from the source planes, the lanes agree
 // on the extreme by shuffles, and every lane writes its code straight into the Q8_0 planes of the
 // new weight (permuted chunks and all), so no staging buffer of GGUF blocks or fp32 values exists.
