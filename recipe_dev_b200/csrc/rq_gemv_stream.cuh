@@ -1205,7 +1205,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
         // int8 18.5 / 16.8 / 16.1, 14336 x 4096 fp32 16.4 / 16.8 / 16.2; Q4_K 4096 x 4096 fp32 7.6 / 7.9 / 7.5, eight positions of it 49.4 / 49.2 / 50.3;
         // 64 Q6_K experts of 2560 x 1024, eight positions, 190 / 192 / 183.
         const bool leader = rqmma::elect_one();  // (the same lane every time)
-        int issued = 0, seg = 0, slot = 0, st = 0, n_pieces = 0;
+        int seg = 0, slot = 0, st = 0, n_pieces = 0;
         uint32_t phase = 1;  // parity of the slot's previous round: the first round of the ring waits for nothing
         int back_slot = 0, back_piece = 0;  // the piece issued `window` pieces ago, counted along
         uint32_t back_phase = 0;
@@ -1292,7 +1292,6 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                 }
                 __syncwarp();
                 if (failed) break;
-                issued = st + 1;
                 if (++slot == p.stages) { slot = 0; phase ^= 1; }
             }
         };
@@ -1346,13 +1345,15 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                         for (int k = 0; k < p.pieces; ++k) mbar_expect_tx(&full_bar[2 * slot + k], 0);
                     }
                     __syncwarp();
-                    issued = ++st;
+                    n_pieces += p.pieces;
+                    ++st;
                 }
             }
-            // leave only after every copy this CTA issued has landed (bounded)
-            for (int w = (issued > p.stages ? issued - p.stages : 0); w < issued; ++w)
-                for (int k = 0; k < p.pieces; ++k)
-                    if (!mbar_wait_warp(&full_bar[2 * (w % p.stages) + k], (w / p.stages) & 1, p.wait_ns)) { atomicExch(p.error_flag, 2); break; }
+            // leave only after every copy this CTA issued has landed (bounded), the first piece of a stage whose second one was given up among them
+            for (int q = max(0, n_pieces - p.stages * p.pieces); q < n_pieces; ++q) {
+                const int w = q / p.pieces;
+                if (!mbar_wait_warp(&full_bar[2 * (w % p.stages) + q - w * p.pieces], (w / p.stages) & 1, p.wait_ns)) { atomicExch(p.error_flag, 2); break; }
+            }
         }
     } else {
         // ---------------------------------------------------------------- consumers

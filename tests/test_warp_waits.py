@@ -24,3 +24,12 @@ def test_the_ring_leaves_a_slot_alone_that_never_filled():
     rest = loop.split("issue(slot)")[1]
     assert rest.index("if (dead) break;") < rest.index("y[(row + r)")
     assert "in_flight > 0" in rest and "rqmma::mbar_wait(&full[warp][slot]" in rest
+
+
+def test_the_streaming_producer_waits_for_every_piece_it_issued():
+    """Counted by stages, a stage given up between its two pieces left the first one in flight when the CTA ended."""
+    producer = (CSRC / "rq_gemv_stream.cuh").read_text().split("- producer warp")[1].split("- consumers")[0]
+    last = producer.split("leave only after every copy")[1]
+    assert re.search(r"for \(int q = max\(0, n_pieces - p\.stages \* p\.pieces\); q < n_pieces; \+\+q\)", last) and "mbar_wait_warp(" in last
+    # every barrier that is armed is counted: a piece where its copies go out, and the empty stage that ends the warp scheme
+    assert producer.count("mbar_expect_tx(") == 2 and producer.count("++n_pieces;") == 1 and producer.count("n_pieces += p.pieces;") == 1
