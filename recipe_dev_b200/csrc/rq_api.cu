@@ -164,6 +164,8 @@ static const char* wait_code_text(int code) {
         case 18: return "batched product, staging warps: the stored bytes never arrived";
         case 19: return "batched product, copies of stored bytes: a slot never came free";
         case 20: return "batched product, drain warps: the activations' steps never arrived";
+        case 23: return "batched product, issuing warps: the products never completed";
+        case 24: return "batched product, copies: some never landed";
         case 22: return "matvec over a decode-only format: a row's bytes never arrived";
         case 21: return "wait self-test: the barrier nothing arrives on";
         case 31: return "exchange: a peer's arrival flag never came";

@@ -52,8 +52,8 @@
 // window of four superblocks one more slice (the terms' fp16 values and, behind them, their residuals) whose "activations" are the group
 // sums, twice.
 //
-// Every wait is bounded; a wait that runs out records a code in the context's error word, the thread stops waiting and the CTA
-// still frees its tensor memory before it exits.
+// Every wait is bounded; a wait that runs out records a code in the context's error word and the thread stops waiting. Before the CTA frees its
+// tensor memory and exits, the issuing and copying warps wait once more, within the same limit, for the products and copies that they have under way.
 #include "rq_internal.cuh"
 #include "rq_matmul_cut.cuh"
 #include "rq_mma.cuh"
@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
     // Indexing by step keeps every parity wait within one phase whatever the rings' lengths: no thread is ever kDone steps ahead
     // of anyone (activation slots x steps per slot < kDone).
     __shared__ __align__(8) uint64_t done[kDone], drained[kDone], a_full[kDone], raw_full[kMaxRaw], raw_empty[kMaxRaw], b_full[kMaxB];
+    __shared__ __align__(8) uint64_t ended[kIssuers];  // an issuing warp's products are all complete
     __shared__ uint32_t tmem_base_slot;
     __shared__ int last_piece;
     // CODES: the activations' steps of a few slices, a ring of its own (the drain warps read it, well after the products are done)
@@ -418,6 +419,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
         for (int s = 0; s < kDone; ++s) { mbar_init(&done[s], kBoth ? kIssuers : 1); mbar_init(&drained[s], kBoth ? kDrainWarps : 4); mbar_init(&a_full[s], 4); }
         for (int s = 0; s < kMaxRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], MH == 1 ? 4 * F::raw_slices : 4); }
         for (int s = 0; s < kMaxB; ++s) mbar_init(&b_full[s], 1);
+        for (int s = 0; s < kIssuers; ++s) mbar_init(&ended[s], 1);
         for (int s = 0; s < kStepSlots; ++s) { mbar_init(&steps_full[s], 1); mbar_init(&steps_empty[s], MH == 1 ? 4 : kDrainWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -925,6 +927,12 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
         // These warps wait as a whole and one lane acts: a look at a barrier by a lone lane is not suspended, it is repeated every 160 cycles, and
         // sees an arrival 100 to 200 cycles later than a whole warp does (Q4_K 14336 x 4096, 512 tokens: 154 us so, 135 with whole warps).
         const bool leader = elect_one();  // (the same lane every time)
+        // The copying warps leave only after every copy that they issued has landed: the last `slots` of n on a ring of barriers (bounded).
+        auto landed = [&](uint64_t* full, int slots, int n) {
+            bool dead = false;
+            for (int i = max(0, n - slots); i < n && !dead; ++i)
+                if (!mbar_wait_warp(&full[i % slots], (i / slots) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 24);
+        };
         if (warp < kMiscFirst + kIssuers) {
             // ------------------------------------------------------------ the issuing warps
             const int me = warp - kMiscFirst;
@@ -991,12 +999,16 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     __syncwarp();
                 }
             }
-            // nothing may be in flight when tensor memory is freed: the drain warps have waited for every step by then
+            // nothing may be in flight when tensor memory is freed. (The drain warps have waited for every step by then, unless one of their waits ran out.)
+            if (leader) mma_commit(&ended[me]);
+            __syncwarp();
+            dead = false;
+            if (!mbar_wait_warp(&ended[me], 0, p.wait_ns, dead)) atomicExch(p.error_flag, 23);
         } else if (warp == kMiscFirst + kIssuers) {
             // ------------------------------------------------------------ activation copies (the images were written by the kernel before this one)
             asm volatile("griddepcontrol.wait;" ::: "memory");
             Ring b_at(p.b_slots), steps_at(kStepSlots);
-            int ks_all = 0;
+            int ks_all = 0, images = 0;
             bool dead = false;
             while (!dead && walk.next(tile, u0, u1)) {
                 const uint8_t* src = p.xs + (size_t)(tile / p.tiles_m) * p.image_tiles * b_bytes;
@@ -1018,6 +1030,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         bulk_g2s(smem + (size_t)b_at.slot * b_bytes, src + (size_t)image * b_bytes, (uint32_t)b_bytes, &b_full[b_at.slot]);
                     }
                     b_at.next();
+                    ++images;
                     if (CODES) {
                         if (ks_all >= kStepSlots && !mbar_wait_warp(&steps_empty[steps_at.slot], steps_at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 16); break; }
                         if (leader) {
@@ -1028,6 +1041,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     }
                 }
             }
+            landed(b_full, p.b_slots, images);
+            if (CODES) landed(steps_full, kStepSlots, ks_all);
         } else {
             // ------------------------------------------------------------ stored bytes: constants of the model, nothing to wait for before the first fetches
             Ring at(p.raw_slots);
@@ -1046,6 +1061,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         at.next();
                     }
             }
+            landed(raw_full, p.raw_slots, n);
         }
         __syncwarp();
     }

@@ -33,3 +33,13 @@ def test_the_streaming_producer_waits_for_every_piece_it_issued():
     assert re.search(r"for \(int q = max\(0, n_pieces - p\.stages \* p\.pieces\); q < n_pieces; \+\+q\)", last) and "mbar_wait_warp(" in last
     # every barrier that is armed is counted: a piece where its copies go out, and the empty stage that ends the warp scheme
     assert producer.count("mbar_expect_tx(") == 2 and producer.count("++n_pieces;") == 1 and producer.count("n_pieces += p.pieces;") == 1
+
+
+def test_the_batched_product_ends_with_nothing_under_way():
+    """The drain and staging warps wait for every product and copy, but not once one of their waits has run out."""
+    misc = (CSRC / "rq_matmul_tc.cu").read_text().split("auto landed = [&]")[1].split("free the tensor memory")[0]
+    issuing, rest = misc.split("- activation copies")
+    activations, stored = rest.split("- stored bytes:")
+    assert issuing.index("mma_commit(&ended[me]);") < issuing.index("mbar_wait_warp(&ended[me], 0,")
+    assert "landed(b_full, p.b_slots, images);" in activations and "landed(steps_full, kStepSlots, ks_all);" in activations
+    assert "landed(raw_full, p.raw_slots, n);" in stored
