@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(kWarps * 32, rqring::kCtas) rq_gemv_ring_kerne
     const int64_t row_end = rows * (me + 1) / warps;
     int64_t next_row = rows * me / warps, row = next_row;  // of the copies; of the dots
     const int chunks = (groups + 31) >> 5;
-    int next_chunk = 0, in_flight = 0;  // in_flight: slots issued and not yet waited for
+    int next_chunk = 0;
     if (lane == 0) {
         for (int i = 0; i < stages; ++i) rqmma::mbar_init(&full[warp][i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -355,7 +355,6 @@ __global__ void __launch_bounds__(kWarps * 32, rqring::kCtas) rq_gemv_ring_kerne
         __syncwarp();
         if (lane < n) rqmma::bulk_g2s(ring + slot * slot_bytes + lane * chunk_bytes, main_plane + (next_row + lane) * row_bytes + at, (uint32_t)bytes, &full[warp][slot]);
         if (++next_chunk == chunks) { next_chunk = 0; next_row += n; }
-        ++in_flight;
     };
     for (int i = 0; i < stages; ++i) issue(i);
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -371,11 +370,16 @@ __global__ void __launch_bounds__(kWarps * 32, rqring::kCtas) rq_gemv_ring_kerne
 #pragma unroll
         for (int r = 0; r < kRingRows; ++r) sum[r] = 0.f;
         for (int g0 = 0; g0 < groups; g0 += 32) {
-            if (!rqmma::mbar_wait_warp(&full[warp][slot], phase, wait_ns, dead)) {  // the slot is still being written: nothing more goes into it, or out of it
+            if (!rqmma::mbar_wait_warp(&full[warp][slot], phase, wait_ns, dead)) {
+                // The slot is still being written: nothing more goes into a slot or out to y, and the warp leaves once the copies it has under way
+                // have landed (within the limit again).
                 atomicExch(error_flag, 22);
-                break;
+                const int64_t begin = rows * me / warps;
+                const int issued = (int)((next_row - begin + kRingRows - 1) / kRingRows) * chunks + next_chunk, used = (int)((row - begin) / kRingRows) * chunks + g0 / 32;
+                for (int in_flight = issued - used; in_flight > 0 && rqmma::mbar_wait(&full[warp][slot], phase, wait_ns); --in_flight)
+                    if (++slot == stages) { slot = 0; phase ^= 1; }
+                return;
             }
-            --in_flight;
             const uint8_t* const from = ring + slot * slot_bytes;
             if (g0 + lane < groups) {
                 Pair v[16];  // the group's inputs
@@ -400,7 +404,6 @@ __global__ void __launch_bounds__(kWarps * 32, rqring::kCtas) rq_gemv_ring_kerne
             issue(slot);
             if (++slot == stages) { slot = 0; phase ^= 1; }
         }
-        if (dead) break;
 #pragma unroll
         for (int r = 0; r < kRingRows; ++r) {
 #pragma unroll
@@ -408,11 +411,6 @@ __global__ void __launch_bounds__(kWarps * 32, rqring::kCtas) rq_gemv_ring_kerne
             if (lane == 0 && r < n) y[(row + r) * yn + (int64_t)token * yt] = sum[r];
         }
         row += n;
-    }
-    // every copy that was issued has been waited for, unless a wait ran out: then once more, so that none lands after the CTA has left
-    for (; in_flight > 0; --in_flight) {
-        if (!rqmma::mbar_wait(&full[warp][slot], phase, wait_ns)) break;
-        if (++slot == stages) { slot = 0; phase ^= 1; }
     }
 }
 

@@ -18,12 +18,9 @@ def test_the_ring_leaves_a_slot_alone_that_never_filled():
     """Armed a second time while its copies are in flight, a slot's barrier would count arrivals that it does not expect."""
     text = (CSRC / "rq_gemv_generic.cu").read_text()
     kernel = text.split("rq_gemv_ring_kernel(")[1].split("\ntemplate")[0]
-    loop = kernel.split("while (row < row_end) {")[1]
-    gave_up = loop.split("mbar_wait_warp(")[1].split("issue(slot)")[0]
-    assert re.search(r"error_flag, 22\);\s*break;", gave_up)
-    rest = loop.split("issue(slot)")[1]
-    assert rest.index("if (dead) break;") < rest.index("y[(row + r)")
-    assert "in_flight > 0" in rest and "rqmma::mbar_wait(&full[warp][slot]" in rest
+    gave_up, rest = kernel.split("while (row < row_end) {")[1].split("mbar_wait_warp(")[1].split("return;")
+    assert re.search(r"error_flag, 22\);", gave_up) and "in_flight > 0 && rqmma::mbar_wait(&full[warp][slot]" in gave_up
+    assert "issue(" not in gave_up and "y[" not in gave_up and "issue(slot)" in rest and "y[(row + r)" in rest
 
 
 def test_the_streaming_producer_waits_for_every_piece_it_issued():
