@@ -18,8 +18,7 @@ using rqring::kGroupFloats;
 using rqring::kWarps;
 
 // N words from a 2-byte aligned address (blocks of 18, 22 and 110 bytes): the aligned words around it, shifted together. Nothing past
-// the last wanted byte's word is touched.
-// RING: the bytes lie in shared memory
+// the last wanted byte's word is touched. RING: the bytes lie in shared memory.
 template <bool RING, typename T> __device__ __forceinline__ T fetch(const T* p) {
     if constexpr (RING) return *p;
     else return __ldg(p);
@@ -272,7 +271,7 @@ constexpr int ctas_per_sm() {
 // but cancel against each other (2.3e-7 against 64 bits where decoding value by value has 1.0e-7, Q5_K over 512 inputs), and a code
 // times a large input can leave the range that the weight's own product stays in. Per four
 // weights: two or three instructions to isolate the codes, four to place them, six packed ones. Measured, Q5_K 14336 x 4096, one token: 26.5 us (28.2 with the sums kept apart; with a ring,
-// below, 20.9); decoding value by value, every header field once per value, took 175.6.
+// below, 21.2); decoding value by value, every header field once per value, took 175.6.
 template <int TYPE, int ROWS>
 __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gemv_generic_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int64_t row_bytes, int groups, const float* x,
                                                                         int64_t sk, int64_t st, float* __restrict__ y, int64_t yn, int64_t yt) {
@@ -322,10 +321,11 @@ __global__ void __launch_bounds__(kWarps * 32, ctas_per_sm<TYPE, ROWS>()) rq_gem
 
 // The same product where a row and 32 of its groups are whole 16-byte lines: a warp owns a range of rows (an equal share, to one row) and
 // brings up to four of them at a time, 32 groups of each, into a ring of its own in shared memory with bulk copies, which start before the wait
-// for the kernel before (the kernels that write weights let nothing behind them start early: rq_layout.cu, rq_requant.cu). The kernel above leaves a warp waiting for memory between its dots (a quarter of the issue slots used): its registers hold
-// one round's bytes, and its CTAs come to an SM in whole numbers (448 of them to 148). The same additions in the same order. What
-// bounds it is instruction issue (codes turned into fp32 by conversions instead of byte permutes: 22.9). us before / now: Q5_K 14336 x 4096 26.5 / 20.9,
-// 60000 x 2560 63.6 / 54.3; Q4_1 14336 x 4096 19.5 / 15.6; Q8_1 20.5 / 16.2.
+// for the kernel before (the kernels that write weights let nothing behind them start early: rq_layout.cu, rq_requant.cu). The kernel above
+// leaves a warp waiting for memory between its dots (a quarter of the issue slots used): its registers hold one round's bytes, and its CTAs
+// come to an SM in whole numbers (448 of them to 148). The same additions in the same order. What bounds it is instruction issue (codes
+// turned into fp32 by conversions instead of byte permutes: 22.9). us without / with it: Q5_K 14336 x 4096 26.5 / 21.2, 60000 x 2560 64.4 / 55.4; Q4_1 14336 x 4096
+// 19.8 / 16.7; Q8_1 21.5 / 17.4. Which calls take it: rq_ring_rule.cuh.
 constexpr int kRingRows = rqring::kRows, kRingMax = rqring::kMaxStages;
 template <int TYPE>
 __global__ void __launch_bounds__(kWarps * 32, rqring::kCtas) rq_gemv_ring_kernel(const uint8_t* __restrict__ main_plane, int64_t rows, int row_bytes, int chunk_bytes, int stages, int groups, const float* x, int64_t sk,

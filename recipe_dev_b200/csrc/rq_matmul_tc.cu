@@ -43,7 +43,7 @@
 // 256 rows x 64 tokens x 64 inputs, a quarter of them the scaling, issued in 57 % of the cycles). Measured on one B200, calls back to back,
 // before (staging groups took slices in turn; a lone lane looked at barriers; columns were tested for in sixteens; tiles of 96;
 // the minimum terms read their headers again; CODES drained a row half by four warps, from one slice's accumulators, and kept totals in tensor memory) and
-// now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 27.7 / 41.2 / 45.9 / 118; Q6_K 4096 x 14336 int8 64
+// now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 27.7 / 41.2 / 45.9 / 118 (a burst; 199 -> 139 under load, where clocks fall); Q6_K 4096 x 14336 int8 64
 // tokens 50.8 -> 44.3; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 35.4, 4096 x 8192 fp32 200 tokens 84.3 -> 61.2, 4096 x 14336 int8 509 tokens
 // 332 -> 278. The shared tiles' sums as the last thing a CTA does, by drain and staging warps together, were slower (64 tokens 48.8): a CTA is
 // then the last of both of its tiles more often.
