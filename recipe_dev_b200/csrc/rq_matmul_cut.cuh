@@ -14,12 +14,12 @@ constexpr int kStashBytes = 4 * 128 * 16;  // Q4_K, a row half: the headers of a
 
 // drain_warps; groups: staging groups of four warps; cols: tokens per tile at most; registers of the drain, staging and other
 // warps, which together may not exceed the launch's (threads x the registers a thread is compiled for: 896 x 72, 640 x 96).
-// CODES: int8 activations over the 32-value formats.
+// CODES: int8 activations over the 32-value formats, up to 64 tokens (beyond: rq_matmul_int8.cu).
 template <int MH, bool CODES> struct Shape;
 template <> struct Shape<1, false> { static constexpr int drain_warps = 8, groups = 4, cols = 64, drain_regs = 120, stage_regs = 56, other_regs = 40, launch_regs = 72; };
 template <> struct Shape<2, false> { static constexpr int drain_warps = 8, groups = 2, cols = 128, drain_regs = 168, stage_regs = 56, other_regs = 32, launch_regs = 96; };
 template <> struct Shape<1, true> { static constexpr int drain_warps = 8, groups = 4, cols = 64, drain_regs = 128, stage_regs = 48, other_regs = 40, launch_regs = 72; };
-template <> struct Shape<2, true> { static constexpr int drain_warps = 8, groups = 2, cols = 64, drain_regs = 152, stage_regs = 64, other_regs = 48, launch_regs = 96; };
+constexpr int kInt8Tokens = 64;              // tokens of a tile of codes with two row halves
 
 template <int TYPE> struct Format {
     static constexpr bool kquant = TYPE == RQ_Q4_K || TYPE == RQ_Q6_K;
@@ -29,6 +29,14 @@ template <int TYPE> struct Format {
     static constexpr int raw_slices = TYPE == RQ_Q8_0 ? 2 : 4;   // slices in one TMA tile
     static constexpr int raw_bytes = 128 * box_bytes;
     static constexpr int a_cols = residual ? 64 : 32;            // tensor-memory columns of an operand slot
+};
+
+// The rings of the kernel of int8 activations over Q8_0 / Q4_0 and more than 64 tokens (rq_matmul_int8.cu; of a TcCut it takes the tiles, the deal and the
+// scratch), in half units of 256 rows x 64 tokens: activations, operands (Q8_0: the stored bytes as they land), Q4_0's stored bytes (slots of a unit of 128
+// rows), the steps and stored scales of a unit; behind them the totals, and room to align.
+template <int TYPE> struct Int8Rings {
+    static constexpr int b_slots = TYPE == RQ_Q8_0 ? 4 : 3, a_slots = TYPE == RQ_Q8_0 ? 3 : 2, raw_slots = TYPE == RQ_Q8_0 ? 0 : 3, scale_slots = 3;
+    static constexpr size_t bytes = b_slots * 8192 + a_slots * 32768 + raw_slots * 16384 + scale_slots * 6144 + 65536 + 1024;
 };
 
 // The slices of a segment (units u0 .. u1 - 1 of a tile) in the order every role takes them: four a unit and, over Q4_K, behind the last unit of every
@@ -158,13 +166,13 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     c.tiles_m = (int)((rows + 128 * c.mh - 1) / (128 * c.mh));
     c.units = (int)((cols + 255) / 256);
     const int grain = c.mh == 2 ? 32 : 16;
-    int widest = c.mh == 1 ? widest_1 : (codes ? Shape<2, true>::cols : 96);
+    int widest = c.mh == 1 ? widest_1 : (codes ? kInt8Tokens : 96);
     if (c.mh == 2 && kquant && call_cost(c.tiles_m, c.units, tokens, Shape<2, false>::cols, grain, sm_count) <= call_cost(c.tiles_m, c.units, tokens, widest, grain, sm_count)) widest = Shape<2, false>::cols;
     const TokenTiles t = token_tiles(tokens, widest, grain);
     c.n_tiles = t.n;
     c.bn = t.bn;
     c.windows = type == RQ_Q4_K ? (c.units + 3) / 4 : 0;
-    c.image_tiles = 4 * c.units + c.windows;
+    c.image_tiles = codes && c.mh == 2 ? 2 * c.units : 4 * c.units + c.windows;  // (of 64 inputs a row; codes of two row halves: bytes, of 128)
     const TileShare sh = share_out((int64_t)c.tiles_m * c.n_tiles, c.units, sm_count);
     c.ctas = sh.ctas; c.whole = sh.whole; c.rest_tiles = sh.rest_tiles; c.share = sh.share;
     // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: MH = 1, the issuing warps
@@ -183,14 +191,12 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
     const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 || f.raw_per_unit == 2 ? 2 : 1;
     c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
-    // codes, two row halves: four slots of each are enough beside the totals
-    if (codes && c.mh == 2) c.raw_slots = 4;
     const int b_max = c.mh == 1 ? kMaxB : (codes ? 4 : 6), b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
     while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
     c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + kept + 1024;
     c.records_bytes = codes ? (rq_act_token_bytes(cols) * (size_t)tokens + 255) & ~(size_t)255 : 0;
     c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
-    c.steps_bytes = codes ? (size_t)c.n_tiles * c.image_tiles * 2 * c.bn * 4 : 0;
+    c.steps_bytes = codes ? (size_t)c.n_tiles * c.units * 8 * c.bn * 4 : 0;
     c.partial_bytes = (size_t)2 * c.share * c.bn * 128 * c.mh * 4;
     return c;
 }

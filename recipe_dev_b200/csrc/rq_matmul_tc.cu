@@ -12,7 +12,7 @@
 // tensor core's 128-byte-swizzled K-major image; INT8 calls over the K-quants feed code * step through the same path. INT8 calls
 // over Q8_0 and Q4_0 (CODES) feed the codes themselves: their scale changes every 32 inputs anyway, as the activations' step does,
 // so a sum of 32 products is an exact integer that both scale on its way out -- half the products, half the activation bytes,
-// the matvec kernel's arithmetic, and no fp16 range to stay in.
+// the matvec kernel's arithmetic, and no fp16 range to stay in. Beyond 64 tokens they have a kernel of 8-bit products (rq_matmul_int8.cu), which this file prepares.
 //
 // One CTA per SM, persistent. Work is counted in UNITS, 256 inputs of one row tile (128 * MH rows) x one token tile: every CTA
 // takes the same number of whole tiles and then an equal share of the units that are left, whatever tile they fall in (where few are
@@ -35,17 +35,15 @@
 // eight) instructions and the low products have accumulators of their own. MH = 2 (token tiles of up to 128 or, where that leaves few tiles to
 // many CTAs, of up to 96: rq_matmul_cut.cuh; of 96 over the 32-value formats, whose two sums a slice take the columns): two row halves share each activation tile, which halves the activation bytes a
 // CTA pulls from L2 (they, at 4 bytes per input and token, are what the large shapes would be bound by); products of hi and lo
-// share an accumulator, a row half has four drain warps with up to 128 fp32 sums a thread (setmaxnreg; CODES: tiles of up to 64).
+// share an accumulator, a row half has four drain warps with up to 128 fp32 sums a thread (setmaxnreg).
 //
 // What bounds it, from cycles counted around every wait: 512 tokens, the tensor cores are busy for half of the time and the rest is
 // accumulators being drained (three of 128 columns are what tensor memory holds); a few tokens, a third is the wait for the
-// activation image, the rest the chain staging -> products -> drain of a slice; CODES with two row halves, instructions (5700 a slice of
-// 256 rows x 64 tokens x 64 inputs, a quarter of them the scaling, issued in 57 % of the cycles). Measured on one B200, calls back to back,
+// activation image, the rest the chain staging -> products -> drain of a slice. Measured on one B200, calls back to back,
 // before (staging groups took slices in turn; a lone lane looked at barriers; columns were tested for in sixteens; tiles of 96;
-// the minimum terms read their headers again; CODES drained a row half by four warps, from one slice's accumulators, and kept totals in tensor memory) and
+// the minimum terms read their headers again) and
 // now: Q4_K 14336 x 4096 16 / 64 / 90 / 512 tokens 34.2 / 49.4 / 55.6 / 188 us -> 27.7 / 41.2 / 45.9 / 118 (a burst; 199 -> 139 under load, where clocks fall); Q6_K 4096 x 14336 int8 64
-// tokens 50.8 -> 44.3; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 35.4, 4096 x 8192 fp32 200 tokens 84.3 -> 61.2, 4096 x 14336 int8 509 tokens
-// 332 -> 278. The shared tiles' sums as the last thing a CTA does, by drain and staging warps together, were slower (64 tokens 48.8): a CTA is
+// tokens 50.8 -> 44.3; Q8_0 14336 x 4096 int8 20 tokens 49.0 -> 35.4, 4096 x 8192 fp32 200 tokens 84.3 -> 61.2. The shared tiles' sums as the last thing a CTA does, by drain and staging warps together, were slower (64 tokens 48.8): a CTA is
 // then the last of both of its tiles more often.
 //
 // The Q4_K minimum term, sum_g (8 * d * sc_g - dmin * m_g) * (sum of x over group g), is a second, 32 times smaller product: per
@@ -56,6 +54,7 @@
 // tensor memory and exits, the issuing and copying warps wait once more, within the same limit, for the products and copies that they have under way.
 #include "rq_internal.cuh"
 #include "rq_matmul_cut.cuh"
+#include "rq_matmul_int8.cuh"
 #include "rq_mma.cuh"
 #include "rq_pairs.cuh"
 
@@ -229,21 +228,26 @@ __device__ __forceinline__ void minimum_terms(const uint4& hdr, uint32_t (&hi)[4
 // matvec kernels' records of the same inputs are left beside it for INT8_CACHED calls; STEP -1 reads those records instead of x. Rows
 // past the last token and inputs past the last column are zeros.
 // ------------------------------------------------------------------------------------------
-template <int STEP, bool CODES>
+enum Image { kPairs, kCodes, kBytes };  // fp16 hi | lo; the codes as fp16; the codes as bytes (rq_matmul_int8.cu), half a unit a tile
+template <int STEP, Image IMAGE>
 __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t sk, int64_t st, int cols, int units, int tokens, int padded, int bn, int image_tiles,
-                                                          int windows, uint8_t* records, uint8_t* xs, float* steps,
+                                                          int windows, int permuted, uint8_t* records, uint8_t* xs, float* steps,
                                                           int* arrived, int shared_tiles) {
+    constexpr bool CODES = IMAGE != kPairs;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31, unit = blockIdx.x;
     const int row = (blockIdx.z * gridDim.y + blockIdx.y) * 8 + (threadIdx.x >> 5);  // the padded rows are a multiple of sixteen
     if (row >= padded) return;  // a last layer of the grid that is not full (more rows than one layer takes)
     const int nt = row / bn, r = row - nt * bn, k0 = unit * 256 + 8 * lane;
     const bool vec = sk == 1 && (st & 3) == 0 && ((uintptr_t)x & 15) == 0;
-    uint8_t* hi = xs + ((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * (CODES ? 1 : 2) * (size_t)bn * 128 + swizzled(r, lane & 7);
+    // eight inputs: a 16-byte chunk of the image, or half of one (chunks in the order that the weight's plane has them in)
+    uint8_t* hi = IMAGE == kBytes ? xs + ((size_t)nt * image_tiles + 2 * unit + (lane >> 4)) * (size_t)bn * 128 + swizzled(r, ((lane >> 1) ^ (permuted ? unit : 0)) & 7) + 8 * (lane & 1)
+                                  : xs + ((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * (CODES ? 1 : 2) * (size_t)bn * 128 + swizzled(r, lane & 7);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (blockIdx.x == 0 && row < 8)
         for (int i = threadIdx.x; i < shared_tiles; i += 256) arrived[i] = 0;
     float v[8], d = 0.f;
+    uint32_t packed[2] = {0, 0};
     // CODES: where this lane's eight codes, their group's step and the sums lie in the token's records
     const bool inside = row < tokens && k0 < cols;
     uint8_t *rec_codes = nullptr, *rec_step = nullptr, *rec_sum16 = nullptr;
@@ -261,6 +265,8 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t
         for (int j = 0; j < 8; ++j) v[j] = 0.f;
         if (inside) {
             const uint2 c = __ldcg((const uint2*)rec_codes);
+            packed[0] = c.x;
+            packed[1] = c.y;
 #pragma unroll
             for (int j = 0; j < 8; ++j) v[j] = (float)(int8_t)((j < 4 ? c.x : c.y) >> (8 * (j & 3)));
             d = __ldcg((const float*)rec_step);
@@ -292,7 +298,6 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t
         const bool nonzero = fabsf(best) > 0.f;
         const float inverse = nonzero ? __fdiv_rn(-127.0f, best) : 0.f;
         d = nonzero ? __fdiv_rn(1.0f, inverse) : 0.f;
-        uint32_t packed[2] = {0, 0};
         int sum = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -315,7 +320,11 @@ __global__ void __launch_bounds__(256) rq_tc_prep_kernel(const float* x, int64_t
         }
     }
     if (CODES) {
-        if ((lane & 3) == 0) steps[(((size_t)nt * image_tiles + 4 * unit + (lane >> 3)) * 2 + ((lane >> 2) & 1)) * bn + r] = d;
+        if ((lane & 3) == 0) steps[(((size_t)nt * units + unit) * 8 + (lane >> 2)) * bn + r] = d;
+    }
+    if (IMAGE == kBytes) {
+        *(uint2*)hi = make_uint2(packed[0], packed[1]);
+        return;
     }
     uint32_t hw[4], lw[4];
     split2(v[0], v[2], hw[0], lw[0]);  // the order the weights' nibble pairs come in
@@ -365,6 +374,7 @@ __device__ __forceinline__ void tmem_ld16_pair(uint32_t a, uint32_t b, uint32_t 
 }
 
 template <int N> struct Columns { static constexpr int value = N; };
+template <Image I> struct ImageOf { static constexpr Image value = I; };
 
 // A ring position: slot index and the parity of its current use. (Kept by counting: a division by a ring's length, known at run time
 // only, is some thirty instructions.)
@@ -385,17 +395,13 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
     static_assert(32 * kDrainWarps * S::drain_regs + 128 * kGroups * S::stage_regs + 128 * S::other_regs <= tc_threads<MH, CODES>() * S::launch_regs, "more registers than the launch has: the increase would wait forever");
     static_assert(kDrainWarps == 8 && kGroups == (MH == 1 ? 4 : 2), "a staging group has one slice of every unit (MH = 1) or one row half (MH = 2)");
     constexpr int kHalves = F::halves;
-    // What a drain thread holds: MH = 1, a row of the even or of the odd slices; MH = 2, a row of its row half, or (kBoth) two rows, one of each
-    // half, of half the tokens: a token's step, read from shared memory, then serves two sums (a step is as many bytes
-    // as a sum, at a quarter of tensor memory's rate).
-    constexpr bool kBoth = MH == 2 && CODES;
-    constexpr int kRows = kBoth ? 2 : 1;
+    static_assert(MH == 1 || !CODES, "codes and two row halves: rq_matmul_int8.cu");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);  // swizzled tiles want 1024-byte alignment
-    // A STEP is one operand tile's products: (slice, row half), numbered in issue order; with kBoth a slice's, two commits. A step's commit
+    // A STEP is one operand tile's products: (slice, row half), numbered in issue order. A step's commit
     // arrives on done[step % kDone]: the drain warps wait for it (the sums are complete), the staging warps for the step that read
     // their operand slot, the activation copies for the last step that read theirs. What the drain warps have read they say on
-    // drained[step % kDone] (kBoth: of every half slice), and a staged tile (slice, row half) is announced on a_full[tile % kDone].
+    // drained[step % kDone], and a staged tile (slice, row half) is announced on a_full[tile % kDone].
     // Indexing by step keeps every parity wait within one phase whatever the rings' lengths: no thread is ever kDone steps ahead
     // of anyone (activation slots x steps per slot < kDone).
     __shared__ __align__(8) uint64_t done[kDone], drained[kDone], a_full[kDone], raw_full[kMaxRaw], raw_empty[kMaxRaw], b_full[kMaxB];
@@ -416,11 +422,11 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
     uint4* const stash = (uint4*)(raw + (size_t)p.raw_slots * F::raw_bytes + (MH == 1 ? (size_t)bn * 512 : 0));
 
     if (tid == 0) {
-        for (int s = 0; s < kDone; ++s) { mbar_init(&done[s], kBoth ? kIssuers : 1); mbar_init(&drained[s], kBoth ? kDrainWarps : 4); mbar_init(&a_full[s], 4); }
+        for (int s = 0; s < kDone; ++s) { mbar_init(&done[s], 1); mbar_init(&drained[s], 4); mbar_init(&a_full[s], 4); }
         for (int s = 0; s < kMaxRaw; ++s) { mbar_init(&raw_full[s], 1); mbar_init(&raw_empty[s], MH == 1 ? 4 * F::raw_slices : 4); }
         for (int s = 0; s < kMaxB; ++s) mbar_init(&b_full[s], 1);
         for (int s = 0; s < kIssuers; ++s) mbar_init(&ended[s], 1);
-        for (int s = 0; s < kStepSlots; ++s) { mbar_init(&steps_full[s], 1); mbar_init(&steps_empty[s], MH == 1 ? 4 : kDrainWarps); }
+        for (int s = 0; s < kStepSlots; ++s) { mbar_init(&steps_full[s], 1); mbar_init(&steps_empty[s], 4); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMiscFirst) {
@@ -439,13 +445,12 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
         // ------------------------------------------------------------ drain warps
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::drain_regs));
         // Warp w may read accumulator rows 32 (w % 4) .., so four warps, a SET, drain a sum's columns. MH = 1: the even and the odd slices, joined at
-        // the end of the tile; MH = 2: a row half each, or (kBoth) half the columns of both.
-        const int quarter = warp & 3, set = warp >> 2, half0 = MH == 2 && !kBoth ? set : 0;
-        const int col0 = kBoth ? set * (bn / 2) : 0;
+        // the end of the tile; MH = 2: a row half each.
+        const int quarter = warp & 3, set = warp >> 2, half0 = MH == 2 ? set : 0;
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         float* const joined = (float*)(raw + (size_t)p.raw_slots * F::raw_bytes);  // MH = 1: [bn][128]
         int slice_base = 0;  // slices of the segments before this one
-        Ring acc_at(sums, kBoth ? 0 : set);  // the accumulators of this set's next slice
+        Ring acc_at(sums, set);  // the accumulators of this set's next slice
         bool dead = false;
         // The number of columns is known where the loops are unrolled: with a test for each sixteen of them the sums went through copies, and a
         // drain of 128 columns took 1340 cycles instead of 550 (512 tokens: 135 us).
@@ -462,23 +467,20 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     c0 = deal.first(t);
                     c1 = deal.last(t, (int)blockIdx.x);
                 }
-                Pair sum[kRows][kMine / 2];
+                Pair sum[kMine / 2];
 #pragma unroll
-                for (int m = 0; m < kRows; ++m)
-#pragma unroll
-                    for (int i = 0; i < kMine / 2; ++i) sum[m][i] = 0;
+                for (int i = 0; i < kMine / 2; ++i) sum[i] = 0;
                 // CODES: the products are exact, so what a sum loses it loses where its terms (32 inputs each) are added up, and up to 448 of them one
                 // after another in one fp32 register lose more than the matvec kernel's tree does. Every few slices the sums go into totals,
                 // and what that addition rounds off stays in the register as the start of the next run (the shorter the segment, the more the
                 // additions inside a run weigh). Error against 64 bits, 4096 x 14336 and 509 tokens: 2.0e-7 without, 0.75e-7 so, the matvec
-                // kernel 0.90e-7. The totals lie in tensor memory (MH = 1) or, where its columns are better spent on accumulators, in shared
-                // memory, a thread's own. (In registers they spill; a compensated sum at every slice is slower than either.)
-                const int own = (MH == 1 ? 2 : 4) * (u1 - u0);  // (a set's slices of this segment)
-                const int run_length = own <= 16 ? 2 : (own <= 64 ? (kBoth ? 3 : 4) : (kBoth ? 5 : 8));
+                // kernel 0.90e-7. The totals lie in tensor memory. (In registers they
+                // spill; a compensated sum at every slice is slower.)
+                const int own = 2 * (u1 - u0);  // (a set's slices of this segment)
+                const int run_length = own <= 16 ? 2 : (own <= 64 ? 4 : 8);
                 int run = 0;
                 bool flushed = false;
                 [[maybe_unused]] const uint32_t totals = tmem_base + lane_base + (uint32_t)(p.accs * acc_cols + set * bn);
-                [[maybe_unused]] Pair* const totals_both = (Pair*)(raw + (size_t)p.raw_slots * F::raw_bytes) + tid;  // [row half][columns / 2][256]
                 const Pair minus = pair_of(-1.0f, -1.0f);
                 auto flush = [&]() {
                     run = 0;
@@ -489,91 +491,37 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         lost = pair_add(lost, s);
                         return t;
                     };
-                    if constexpr (kBoth) {
 #pragma unroll
-                        for (int m = 0; m < kRows; ++m) {
-                            Pair* const at = totals_both + m * (kMine / 2) * (32 * kDrainWarps);
-                            Pair total[kMine / 2];
+                    for (int c = 0; c < kMine; c += 16) {
+                        uint32_t v[16];
+                        if (flushed) {
+                            tmem_ld16(totals + c, v);
 #pragma unroll
-                            for (int i = 0; i < kMine / 2; ++i) total[i] = flushed ? at[i * (32 * kDrainWarps)] : 0;
-#pragma unroll
-                            for (int i = 0; i < kMine / 2; ++i) at[i * (32 * kDrainWarps)] = into(total[i], sum[m][i]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < kMine; c += 16) {
-                            uint32_t v[16];
-                            if (flushed) {
-                                tmem_ld16(totals + c, v);
-#pragma unroll
-                                for (int j = 0; j < 16; j += 2) {
-                                    const Pair t = into(pair_of(v[j], v[j + 1]), sum[0][(c + j) / 2]);
-                                    v[j] = __float_as_uint(pair_at(t, 0));
-                                    v[j + 1] = __float_as_uint(pair_at(t, 1));
-                                }
-                            } else {
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(pair_at(sum[0][(c + j) / 2], j & 1));
-#pragma unroll
-                                for (int j = 0; j < 8; ++j) sum[0][c / 2 + j] = 0;
+                            for (int j = 0; j < 16; j += 2) {
+                                const Pair t = into(pair_of(v[j], v[j + 1]), sum[(c + j) / 2]);
+                                v[j] = __float_as_uint(pair_at(t, 0));
+                                v[j + 1] = __float_as_uint(pair_at(t, 1));
                             }
-                            tmem_st16(totals + c, v);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(pair_at(sum[(c + j) / 2], j & 1));
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) sum[c / 2 + j] = 0;
                         }
-                        tmem_st_wait();
+                        tmem_st16(totals + c, v);
                     }
+                    tmem_st_wait();
                     flushed = true;
                     // an infinite total has no rounding error to carry on
                     if (!(fabsf(pair_at(lost, 0) + pair_at(lost, 1)) <= 3.402823466e38f)) {
 #pragma unroll
-                        for (int m = 0; m < kRows; ++m)
-#pragma unroll
-                            for (int i = 0; i < kMine / 2; ++i) {
-                                const float e0 = pair_at(sum[m][i], 0), e1 = pair_at(sum[m][i], 1);
-                                sum[m][i] = pair_of(fabsf(e0) <= 3.402823466e38f ? e0 : 0.f, fabsf(e1) <= 3.402823466e38f ? e1 : 0.f);
-                            }
+                        for (int i = 0; i < kMine / 2; ++i) {
+                            const float e0 = pair_at(sum[i], 0), e1 = pair_at(sum[i], 1);
+                            sum[i] = pair_of(fabsf(e0) <= 3.402823466e38f ? e0 : 0.f, fabsf(e1) <= 3.402823466e38f ? e1 : 0.f);
+                        }
                     }
                 };
-                // this lane's row (of row half half0 + m), kept inside the weight for the scale loads
-                auto row_at = [&](int m) -> int64_t { return min((int64_t)(mt * MH + half0 + m) * 128 + quarter * 32 + lane, p.rows - 1); };
-                // kBoth: slice `all` of the CTA's, d[m] holds the two fp16 scales of row half m's row
-                auto drain_both = [&](int all, const uint32_t (&d)[2]) {
-                    if (!mbar_wait_warp(&done[all % kDone], (all / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 14);
-                    const int slot = all % kStepSlots;
-                    if (!mbar_wait_warp(&steps_full[slot], (all / kStepSlots) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 20);
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const float* const d8 = &step_ring[slot][0][0] + col0;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const uint32_t acc = tmem_base + lane_base + (uint32_t)(acc_at.slot * 2 * acc_cols + col0);
-                        const float d0 = rq_h2f((uint16_t)(d[0] >> (16 * h))), d1 = rq_h2f((uint16_t)(d[1] >> (16 * h)));
-                        const Pair scale[2] = {pair_of(d0, d0), pair_of(d1, d1)};
-#pragma unroll
-                        for (int c = 0; c < kMine; c += 16) {
-                            uint32_t t[2][16];
-                            tmem_ld16_pair(acc + c, acc + acc_cols + c, t[0], t[1]);
-#pragma unroll
-                            for (int j = 0; j < 16; j += 4) {
-                                const float4 s4 = *(const float4*)(d8 + h * S::cols + c + j);
-                                const Pair sv[2] = {pair_of(s4.x, s4.y), pair_of(s4.z, s4.w)};
-#pragma unroll
-                                for (int m = 0; m < 2; ++m)
-#pragma unroll
-                                    for (int q = 0; q < 2; ++q) {
-                                        Pair& to = sum[m % kRows][(c + j) / 2 + q];
-                                        to = pair_fma(pair_mul(sv[q], scale[m]), pair_of(t[m][j + 2 * q], t[m][j + 2 * q + 1]), to);
-                                    }
-                            }
-                        }
-                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) {
-                            mbar_arrive(&drained[(2 * all + h) % kDone]);
-                            if (h) mbar_arrive(&steps_empty[slot]);
-                        }
-                        acc_at.next();
-                    }
-                    if (++run == run_length) flush();
-                };
+                const int64_t my_row = min((int64_t)(mt * MH + half0) * 128 + quarter * 32 + lane, p.rows - 1);  // kept inside the weight for the scale loads
                 // Slice `all` of the CTA's: d[0] (and d[1]: the second half slice's) scale its sums
                 auto drain = [&](int all, const float (&d)[2]) {
                     const int step = MH == 1 ? all : 2 * all + half0;
@@ -596,7 +544,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
 #pragma unroll
                                 for (int q = 0; q < 2; ++q) {
                                     const Pair even = pair_mul(pair_mul(sv[q], scale0), pair_of(t[j + 2 * q], t[j + 2 * q + 1]));
-                                    Pair& to = sum[0][(c + j) / 2 + q];
+                                    Pair& to = sum[(c + j) / 2 + q];
                                     to = pair_add(to, pair_fma(pair_mul(rv[q], scale1), pair_of(u[j + 2 * q], u[j + 2 * q + 1]), even));
                                 }
                             }
@@ -616,11 +564,11 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                                         uint32_t u[16];
                                         tmem_ld16_pair(at + c, at + bn + c, t, u);
 #pragma unroll
-                                        for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_fma(scale, pair_add(pair_of(t[j], t[j + 1]), pair_of(u[j], u[j + 1])), sum[0][(c + j) / 2]);
+                                        for (int j = 0; j < 16; j += 2) sum[(c + j) / 2] = pair_fma(scale, pair_add(pair_of(t[j], t[j + 1]), pair_of(u[j], u[j + 1])), sum[(c + j) / 2]);
                                     } else {
                                         tmem_ld16(at + c, t);
 #pragma unroll
-                                        for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_fma(scale, pair_of(t[j], t[j + 1]), sum[0][(c + j) / 2]);
+                                        for (int j = 0; j < 16; j += 2) sum[(c + j) / 2] = pair_fma(scale, pair_of(t[j], t[j + 1]), sum[(c + j) / 2]);
                                     }
                                 }
                             }
@@ -635,8 +583,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 };
                 if constexpr (F::kquant) {
                     auto d_of = [&](int u) -> float {
-                        if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (row_at(0) * p.units + u) * 144)));
-                        return rq_h2f(__ldg(p.scale + row_at(0) * p.units + u));
+                        if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (my_row * p.units + u) * 144)));
+                        return rq_h2f(__ldg(p.scale + my_row * p.units + u));
                     };
                     float d_next = d_of(u0);
                     int all = slice_base;
@@ -656,8 +604,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     // a unit's eight fp16 scales, the next unit's on their way: one load where rows are whole units (a load of two bytes goes to
                     // 32 lines, as one of sixteen does)
                     const bool wide = (p.blocks32 & 7) == 0 && ((uintptr_t)p.scale & 15) == 0;
-                    auto d_of = [&](int m, int u) -> uint4 {
-                        const uint16_t* at = p.scale + row_at(m) * p.blocks32 + 8 * u;
+                    auto d_of = [&](int u) -> uint4 {
+                        const uint16_t* at = p.scale + my_row * p.blocks32 + 8 * u;
                         if (wide) return __ldg((const uint4*)at);
                         uint32_t w[4];
 #pragma unroll
@@ -667,98 +615,65 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         }
                         return make_uint4(w[0], w[1], w[2], w[3]);
                     };
-                    uint4 next[kRows];
-#pragma unroll
-                    for (int m = 0; m < kRows; ++m) next[m] = d_of(m, u0);
+                    uint4 next = d_of(u0);
                     int all = slice_base;  // (a multiple of four)
 #pragma unroll 1
                     for (int u = u0; u < u1; ++u, all += 4) {
-                        uint4 d[kRows];
-#pragma unroll
-                        for (int m = 0; m < kRows; ++m) {
-                            d[m] = next[m];
-                            if (u + 1 < u1) next[m] = d_of(m, u + 1);
-                        }
-                        if constexpr (kBoth) {
+                        const uint4 d = next;
+                        if (u + 1 < u1) next = d_of(u + 1);
 #pragma unroll 1
-                            for (int sl = 0; sl < 4; ++sl) {
-                                const uint32_t w[2] = {sl < 2 ? (sl == 0 ? d[0].x : d[0].y) : (sl == 2 ? d[0].z : d[0].w),
-                                                       sl < 2 ? (sl == 0 ? d[kRows - 1].x : d[kRows - 1].y) : (sl == 2 ? d[kRows - 1].z : d[kRows - 1].w)};
-                                drain_both(all + sl, w);
-                            }
-                        } else {
-#pragma unroll 1
-                            for (int sl = MH == 1 ? set : 0; sl < 4; sl += MH == 1 ? 2 : 1) {
-                                const uint32_t w = sl < 2 ? (sl == 0 ? d[0].x : d[0].y) : (sl == 2 ? d[0].z : d[0].w);
-                                const float scale[2] = {rq_h2f((uint16_t)(w & 0xffff)), rq_h2f((uint16_t)(w >> 16))};
-                                drain(all + sl, scale);
-                            }
+                        for (int sl = MH == 1 ? set : 0; sl < 4; sl += MH == 1 ? 2 : 1) {
+                            const uint32_t w = sl < 2 ? (sl == 0 ? d.x : d.y) : (sl == 2 ? d.z : d.w);
+                            const float scale[2] = {rq_h2f((uint16_t)(w & 0xffff)), rq_h2f((uint16_t)(w >> 16))};
+                            drain(all + sl, scale);
                         }
                     }
                 }
                 slice_base += Order::count(u0, u1);
                 const int r0 = quarter * 32 + lane;
                 if (CODES && flushed) {  // the totals and what is in the registers
-                    if constexpr (kBoth) {
 #pragma unroll
-                        for (int m = 0; m < kRows; ++m)
+                    for (int c = 0; c < kMine; c += 16) {
+                        uint32_t v[16];
+                        tmem_ld16(totals + c, v);
 #pragma unroll
-                            for (int i = 0; i < kMine / 2; ++i) sum[m][i] = pair_add(totals_both[(m * (kMine / 2) + i) * (32 * kDrainWarps)], sum[m][i]);
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < kMine; c += 16) {
-                            uint32_t v[16];
-                            tmem_ld16(totals + c, v);
-#pragma unroll
-                            for (int j = 0; j < 16; j += 2) sum[0][(c + j) / 2] = pair_add(pair_of(v[j], v[j + 1]), sum[0][(c + j) / 2]);
-                        }
+                        for (int j = 0; j < 16; j += 2) sum[(c + j) / 2] = pair_add(pair_of(v[j], v[j + 1]), sum[(c + j) / 2]);
                     }
                 }
                 // MH = 1: each set gives the other half of the columns and keeps the sums of the even and odd slices of its own half
-                constexpr int kLeave = MH == 1 ? kMine / 2 : kMine;  // tokens that a thread carries out, of each of its rows
-                Pair left[kRows][kLeave / 2];
+                constexpr int kLeave = MH == 1 ? kMine / 2 : kMine;  // tokens that a thread carries out
+                Pair left[kLeave / 2];
                 if (MH == 1) {
                     const int give = (1 - set) * kLeave, keep = set * kLeave;
 #pragma unroll
-                    for (int j = 0; j < kLeave; ++j) joined[(give + j) * 128 + r0] = pair_at(set ? sum[0][j / 2] : sum[0][(kLeave + j) / 2], j & 1);
+                    for (int j = 0; j < kLeave; ++j) joined[(give + j) * 128 + r0] = pair_at(set ? sum[j / 2] : sum[(kLeave + j) / 2], j & 1);
                     asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
 #pragma unroll
                     for (int j = 0; j < kLeave; j += 2)
-                        left[0][j / 2] = pair_add(set ? sum[0][(kLeave + j) / 2] : sum[0][j / 2], pair_of(joined[(keep + j) * 128 + r0], joined[(keep + j + 1) * 128 + r0]));
+                        left[j / 2] = pair_add(set ? sum[(kLeave + j) / 2] : sum[j / 2], pair_of(joined[(keep + j) * 128 + r0], joined[(keep + j + 1) * 128 + r0]));
                     asm volatile("bar.sync 3, %0;" ::"n"(kDrainWarps * 32) : "memory");
                 } else {
 #pragma unroll
-                    for (int m = 0; m < kRows; ++m)
-#pragma unroll
-                        for (int j = 0; j < kLeave / 2; ++j) left[m][j] = sum[m][j];
+                    for (int j = 0; j < kLeave / 2; ++j) left[j] = sum[j];
                 }
-                const int from = MH == 1 ? set * kLeave : col0;  // the first of them
-                const int tokens_here = dead ? 0 : min(kLeave, p.tokens - nt * bn - from);
-                // row half m's row of this thread: how many tokens of it count, and where they go
-                auto live = [&](int m) { return (int64_t)(mt * MH + half0 + m) * 128 + r0 < p.rows ? tokens_here : 0; };
-                auto out = [&](int m) { return p.y + ((int64_t)(mt * MH + half0 + m) * 128 + r0) * p.yn + (int64_t)(nt * bn + from) * p.yt; };
+                const int from = MH == 1 ? set * kLeave : 0;  // the first of them
+                const int64_t row = (int64_t)(mt * MH + half0) * 128 + r0;
+                const int n = dead || row >= p.rows ? 0 : min(kLeave, p.tokens - nt * bn - from);  // how many of them count
+                float* const out = p.y + row * p.yn + (int64_t)(nt * bn + from) * p.yt;
                 if (whole) {
+                    float* at = out;
 #pragma unroll
-                    for (int m = 0; m < kRows; ++m) {
-                        const int n = live(m);
-                        float* at = out(m);
-#pragma unroll
-                        for (int j = 0; j < kLeave; ++j) {
-                            if (j < n) *at = pair_at(left[m][j / 2], j & 1);
-                            at += p.yt;
-                        }
+                    for (int j = 0; j < kLeave; ++j) {
+                        if (j < n) *at = pair_at(left[j / 2], j & 1);
+                        at += p.yt;
                     }
                 } else {
                     const size_t tile_floats = (size_t)bn * 128 * MH, place0 = (size_t)from * 128 * MH + half0 * 128 + r0;
                     auto piece_of = [&](int c) { return p.partial + (size_t)Deal::place(c, c0) * tile_floats + place0; };
+                    float* const piece = piece_of((int)blockIdx.x);
 #pragma unroll
-                    for (int m = 0; m < kRows; ++m) {
-                        const int n = live(m);
-                        float* at = piece_of((int)blockIdx.x) + 128 * m;
-#pragma unroll
-                        for (int j = 0; j < kLeave; ++j)
-                            if (j < n) at[j * 128 * MH] = pair_at(left[m][j / 2], j & 1);
-                    }
+                    for (int j = 0; j < kLeave; ++j)
+                        if (j < n) piece[j * 128 * MH] = pair_at(left[j / 2], j & 1);
                     __threadfence();
                     asm volatile("bar.sync 2, %0;" ::"n"(kDrainWarps * 32) : "memory");
                     if (tid == 0) {
@@ -773,43 +688,37 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         // a thread: 12 at a time (Q6_K 8192 x 1024, 48 tokens, by 8 / 12 / 24: 13.0 / 11.6 / 11.9 us; 1670 x 12800, 34 tokens: 26.2 / 23.8 / 29.1).
                         constexpr int kAtOnce = kLeave % 32 == 0 ? 32 : (kLeave % 16 == 0 ? 16 : (kLeave % 12 == 0 ? 12 : 8));
 #pragma unroll 1
-                        for (int m = 0; m < kRows; ++m) {
-                            const int n = live(m);
+                        for (int j0 = 0; j0 < n; j0 += kAtOnce) {
+                            Pair total[kAtOnce / 2];
+#pragma unroll
+                            for (int q = 0; q < kAtOnce / 2; ++q) total[q] = 0;
 #pragma unroll 1
-                            for (int j0 = 0; j0 < n; j0 += kAtOnce) {
-                                Pair total[kAtOnce / 2];
-#pragma unroll
-                                for (int q = 0; q < kAtOnce / 2; ++q) total[q] = 0;
-#pragma unroll 1
-                                for (int c = c0; c <= c1; c += 2) {
-                                    const bool two = c < c1;
-                                    const float* piece = piece_of(c) + 128 * m + (size_t)j0 * 128 * MH;
-                                    const float* other = two ? piece_of(c + 1) + 128 * m + (size_t)j0 * 128 * MH : piece;
-                                    float v[kAtOnce], w[kAtOnce];
-#pragma unroll
-                                    for (int q = 0; q < kAtOnce; ++q) {
-                                        v[q] = __ldcg(piece + q * 128 * MH);
-                                        w[q] = __ldcg(other + q * 128 * MH);
-                                    }
-#pragma unroll
-                                    for (int q = 0; q < kAtOnce; q += 2)
-                                        total[q / 2] = pair_add(total[q / 2], two ? pair_add(pair_of(v[q], v[q + 1]), pair_of(w[q], w[q + 1])) : pair_of(v[q], v[q + 1]));
-                                }
-                                float* at = out(m) + (int64_t)j0 * p.yt;
+                            for (int c = c0; c <= c1; c += 2) {
+                                const bool two = c < c1;
+                                const float* one = piece_of(c) + (size_t)j0 * 128 * MH;
+                                const float* other = two ? piece_of(c + 1) + (size_t)j0 * 128 * MH : one;
+                                float v[kAtOnce], w[kAtOnce];
 #pragma unroll
                                 for (int q = 0; q < kAtOnce; ++q) {
-                                    if (j0 + q < n) *at = pair_at(total[q / 2], q & 1);
-                                    at += p.yt;
+                                    v[q] = __ldcg(one + q * 128 * MH);
+                                    w[q] = __ldcg(other + q * 128 * MH);
                                 }
+#pragma unroll
+                                for (int q = 0; q < kAtOnce; q += 2)
+                                    total[q / 2] = pair_add(total[q / 2], two ? pair_add(pair_of(v[q], v[q + 1]), pair_of(w[q], w[q + 1])) : pair_of(v[q], v[q + 1]));
+                            }
+                            float* at = out + (int64_t)j0 * p.yt;
+#pragma unroll
+                            for (int q = 0; q < kAtOnce; ++q) {
+                                if (j0 + q < n) *at = pair_at(total[q / 2], q & 1);
+                                at += p.yt;
                             }
                         }
                     }
                 }
             }
         };
-        if constexpr (kBoth) {
-            run_tiles(Columns<S::cols / 2>());  // (windows of more than 64 tokens are cut into tiles of 33 to 64)
-        } else if constexpr (MH == 2) {
+        if constexpr (MH == 2) {
             if (bn == 96) run_tiles(Columns<96>());
             else if (F::kquant && bn == 128) run_tiles(Columns<F::kquant ? 128 : 64>());
             else run_tiles(Columns<64>());
@@ -833,7 +742,6 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
         auto wait_slot = [&](int step) {
             int freed = step - p.a_slots;
             if (freed >= 0) {
-                if (kBoth) freed >>= 1;
                 if (!mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 11);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
@@ -938,34 +846,22 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
             const int me = warp - kMiscFirst;
             const uint32_t idesc = instr_desc(bn), idesc2 = instr_desc(acc_cols);
             constexpr int kSkip = MH == 1 ? kIssuers : 1;  // slices from one of this warp's to the next (steps: two)
-            Ring b_at(p.b_slots, MH == 1 ? me : 0), acc_at(sums, kBoth ? 0 : me);
+            Ring b_at(p.b_slots, MH == 1 ? me : 0), acc_at(sums, me);
             int ks = MH == 1 ? me : 0, end = 0;
             bool dead = false;
             while (walk.next(tile, u0, u1)) {
                 end += Order::count(u0, u1);
 #pragma unroll 1
-                for (; ks < end; ks += kSkip, b_at.skip(kSkip), acc_at.skip(kBoth ? 0 : 2)) {
+                for (; ks < end; ks += kSkip, b_at.skip(kSkip), acc_at.skip(2)) {
                     const int step = MH == 1 ? ks : 2 * ks + me, bslot = b_at.slot;
                     if (!mbar_wait_warp(&b_full[bslot], b_at.phase, p.wait_ns, dead)) atomicExch(p.error_flag, 17);
                     const uint32_t bbase = smem_u32(smem + (size_t)bslot * b_bytes);
                     const uint64_t b_hi = smem_desc(bbase), b_lo = smem_desc(bbase + bn * 128);
-                    if (!kBoth && step >= sums && !mbar_wait_warp(&drained[(step - sums) % kDone], ((step - sums) / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 15);
+                    if (step >= sums && !mbar_wait_warp(&drained[(step - sums) % kDone], ((step - sums) / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 15);
                     if (!mbar_wait_warp(&a_full[step % kDone], (step / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 13);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t a_hi = a_ring + (uint32_t)((step & a_mask) * F::a_cols), a_res = a_hi + 32;
-                    if constexpr (kBoth) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h, acc_at.next()) {
-                            const int at = 2 * ks + h;
-                            if (at >= sums && !mbar_wait_warp(&drained[(at - sums) % kDone], ((at - sums) / kDone) & 1, p.wait_ns, dead)) atomicExch(p.error_flag, 15);
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            if (leader && !dead) {
-#pragma unroll
-                                for (int k = 0; k < 2; ++k) mma_f16_ts(tmem_base + (uint32_t)((2 * acc_at.slot + me) * acc_cols), a_hi + 8 * (2 * h + k), b_hi + 2 * (2 * h + k), idesc, k ? 1u : 0u);
-                                if (h) mma_commit(&done[ks % kDone]);
-                            }
-                        }
-                    } else if (leader && !dead) {
+                    if (leader && !dead) {
 #pragma unroll
                         for (int h = 0; h < kHalves; ++h) {
                             const uint32_t acc = tmem_base + (uint32_t)((acc_at.slot * kHalves + h) * acc_cols);
@@ -1017,8 +913,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     if (ks_all >= p.b_slots) {
                         // the last steps that read the slot, one of each row half (they come from different warps)
 #pragma unroll
-                        for (int m = 0; m < (kBoth ? 1 : MH) && !dead; ++m) {
-                            const int freed = kBoth ? ks_all - p.b_slots : (ks_all - p.b_slots) * MH + m;
+                        for (int m = 0; m < MH && !dead; ++m) {
+                            const int freed = (ks_all - p.b_slots) * MH + m;
                             if (!mbar_wait_warp(&done[freed % kDone], (freed / kDone) & 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 16); }
                         }
                         if (dead) break;
@@ -1097,7 +993,7 @@ int launch_tc(const TcParams& p, int ctas, size_t smem, cudaStream_t s) {
 template <int TYPE>
 int launch_tc(const TcParams& p, int mh, bool codes, int ctas, size_t smem, cudaStream_t s) {
     if constexpr (!Format<TYPE>::kquant) {
-        if (codes) return mh == 1 ? launch_tc<TYPE, 1, true>(p, ctas, smem, s) : launch_tc<TYPE, 2, true>(p, ctas, smem, s);
+        if (codes) return launch_tc<TYPE, 1, true>(p, ctas, smem, s);
     }
     return mh == 1 ? launch_tc<TYPE, 1, false>(p, ctas, smem, s) : launch_tc<TYPE, 2, false>(p, ctas, smem, s);
 }
@@ -1114,6 +1010,7 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
     // fp32 activations over an odd number of 32-value blocks stay with the matvec kernel, as they were: it has no fp16 range to keep to
     if (!codes && w->cols % BK) return RQ_ERR_UNSUPPORTED;
     const TcCut cut = tc_cut(w->type, codes, ctx->sm_count, w->rows, w->cols, tokens);
+    const bool bytes = codes && cut.mh == 2;
     const bool cached = act_mode == RQ_ACT_INT8_CACHED;
     if (cached && (!codes || ctx->act_cols != w->cols || ctx->act_tokens != tokens || ctx->act_step != step || scratch_bytes(cut) > ctx->act_scratch_bytes)) return RQ_ERR_UNSUPPORTED;
     int rc = rq_ensure_act_scratch(ctx, scratch_bytes(cut), s);
@@ -1134,11 +1031,25 @@ int rq_launch_matmul(rq_ctx* ctx, const rq_weight* w, const float* x, int64_t sk
         cfg.stream = s;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        auto prep = act_mode == RQ_ACT_FLOAT ? rq_tc_prep_kernel<0, false>
-               : cached                    ? rq_tc_prep_kernel<-1, true>
-                                             : (codes ? (step == 256 ? rq_tc_prep_kernel<256, true> : rq_tc_prep_kernel<32, true>)
-                                                      : (step == 256 ? rq_tc_prep_kernel<256, false> : rq_tc_prep_kernel<32, false>));
-        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, padded, cut.bn, cut.image_tiles, cut.windows, ctx->act_scratch, xs, (float*)(xs + cut.xs_bytes), arrived, cut.rest_tiles));
+        auto prep_of = [&](auto image) {
+            constexpr Image kImage = decltype(image)::value;
+            if constexpr (kImage != kPairs)
+                if (cached) return rq_tc_prep_kernel<-1, kImage>;
+            return step == 256 ? rq_tc_prep_kernel<256, kImage> : rq_tc_prep_kernel<32, kImage>;
+        };
+        auto prep = act_mode == RQ_ACT_FLOAT ? rq_tc_prep_kernel<0, kPairs> : !codes ? prep_of(ImageOf<kPairs>()) : (bytes ? prep_of(ImageOf<kBytes>()) : prep_of(ImageOf<kCodes>()));
+        RQ_CUDA(cudaLaunchKernelEx(&cfg, prep, x, sk, st, (int)w->cols, cut.units, tokens, padded, cut.bn, cut.image_tiles, cut.windows, bytes && w->type == RQ_Q8_0 && rq_plane_permuted(w->type, w->cols) ? 1 : 0, ctx->act_scratch, xs, (float*)(xs + cut.xs_bytes), arrived, cut.rest_tiles));
+    }
+    if (bytes) {
+        RqInt8Params q;
+        q.tile_map = w->tile_map; q.scale = w->scale; q.rows = w->rows;
+        q.blocks32 = (int)(w->cols / 32); q.units = cut.units; q.permuted = rq_plane_permuted(w->type, w->cols) ? 1 : 0;
+        q.xs = xs; q.steps = (const float*)(xs + cut.xs_bytes); q.tokens = tokens; q.y = y; q.yn = yn; q.yt = yt;
+        q.tiles_m = cut.tiles_m; q.whole = cut.whole; q.rest_tiles = cut.rest_tiles; q.share = cut.share;
+        q.partial = partial; q.arrived = arrived; q.error_flag = ctx->error_flag; q.wait_ns = ctx->wait_limit_ns;
+        rc = rq_launch_tc_int8(w->type, q, cut.ctas, s);
+        if (rc == RQ_OK) { ctx->act_cols = w->cols; ctx->act_tokens = tokens; ctx->act_step = step; }
+        return rc;
     }
     TcParams p;
     p.tile_map = w->tile_map;
