@@ -71,6 +71,8 @@ struct StreamParams {
                                // bandwidth, not more -- a deeper queue only delays everything else that reads memory (the activations)
     int row_warps;             // warp scheme: 1 = a row lies inside one warp; NW = every warp holds 32 / warp_rows lanes' worth of
                                // each row of the pass, and the warps' sums meet in shared memory (the last warp to arrive adds them)
+    int bank_group;            // > 0: the warp scheme of an expert bank's down rows -- a sub-row's units are this many lanes (a power of two), a virtual
+                               // row p.subs times as many, side by side in each half of a warp (first and second halves of the units); warp_rows virtual rows a pass
     int sum_group, sum_chunks; // the order a row's item sums are added in when the shape has a warp scheme (so that a multi-token
                                // launch gives each token the bits a single-token launch gives it): chunks of sum_group items, an
                                // xor tree inside a chunk, chunks in order. sum_group = 0: items strided over eight lanes, then a tree
@@ -1139,8 +1141,8 @@ __device__ __forceinline__ float rq_sigmoid_portable(float x) { return __fmul_rn
 __device__ __forceinline__ float rq_silu_portable(float x) { return __fmul_rn(x, rq_sigmoid_portable(x)); }
 
 // R = rows a thread takes per stage in the warp scheme (its weight registers): 2 only where the launch uses two. GATED: the two are
-// the gate row and the up row of one virtual row
-template <int TYPE, int MODE, int T, int NW, int R, bool GATED>
+// the gate row and the up row of one virtual row. BANKED: a virtual row is an expert bank's down rows, one of each slot
+template <int TYPE, int MODE, int T, int NW, int R, bool GATED, bool BANKED>
 __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW <= 7 ? 2 : 1)) rq_gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr int kConsumers = NW * 32;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1600,7 +1602,70 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             }
         };
         constexpr int kSweep = kConsumers / 8;  // row tasks per sweep of the consumer threads
-        if ((T <= 2 || MODE == RQ_ACT_INT8) && p.warp_rows) {
+        if constexpr (BANKED) {
+            // ---- the warp scheme of an expert bank's down rows: a virtual row's sub-rows, one of each slot, are short (512 inputs: four items) and
+            // lie side by side in a warp, so their sums need neither shared memory nor a barrier of the CTA, and the two rows of a thread share
+            // the digits that it reads. An item per thread and barrier of the CTA was 675 instructions a warp and item, most of them around the dot; so 455, and the
+            // launch of sixteen tokens (top-8 of 256 experts, 2048 x 512) 38.5 -> 28.9 us under a profiler, the call 86.0 -> 75.8. With a row's lanes in item
+            // order, eight-way bank conflicts took all of that back (46.6).
+            // The additions are those of reduce_rows, in their order: the halves of a unit, a tree over the units (of eight, those that
+            // are not there add nothing), the slots' sums one after another.
+            // (Lanes 0 .. 15 take the units' first halves: eight neighbours are eight neighbouring units, whose lines lie in eight bank groups.)
+            const int group = p.bank_group, row_lanes = group * p.subs, h = lane >> 4;
+            const int row_in_warp = (lane & 15) / row_lanes, in_row = (lane & 15) - row_in_warp * row_lanes;
+            const int s = in_row / group, u = in_row - s * group;
+            const bool owner = row_in_warp < p.warp_rows && s < subs && u < p.units;
+            const int rows_per_pass = NW * p.warp_rows, row_in_pass = warp * p.warp_rows + row_in_warp;
+            const int my_off = (int)(s * p.sub_main_bytes) + row_in_pass * (int)row_bytes + u * p.unit_bytes, pass_bytes = rows_per_pass * (int)row_bytes;
+            const int from = min(row_in_warp * row_lanes, 16 - row_lanes) + (lane & 16);  // the lanes that hold the sums this one adds up: the first half's the first row's, the second half's the second's
+            while (true) {
+                if (!mbar_wait(&full_bar[2 * slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); break; }
+                const int4 info = stage_info[slot];  // rows, segment, first local row
+                if (info.x == 0) break;              // the producer has no more rows for this CTA
+                const RqSegment& sg = table[info.y];
+                const uint8_t* stage = ring + (size_t)slot * p.stage_bytes;
+                const uint8_t* rec = act_smem + (owner ? sg.act[s] * (int)p.act_bytes + u * kRecord : 0);
+                ItemRegs<TYPE> wr[R];
+                bool have[R], gone = false;
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    const int lr = row_in_pass + k * rows_per_pass;
+                    // the second pass's rows are the stage's second piece
+                    if (k == 1 && p.pieces == 2 && !mbar_wait(&full_bar[2 * slot + 1], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); gone = true; }
+                    have[k] = lr < info.x && owner;
+                    if (have[k]) {
+                        const uint16_t* sc = nullptr;
+                        if (TYPE != RQ_Q4_K) {
+                            const uintptr_t first = (uintptr_t)sg.scale[s] + (uintptr_t)((int64_t)info.z * row_scales * 2);
+                            sc = (const uint16_t*)(stage + (size_t)p.subs * p.sub_main_bytes + (size_t)s * p.sub_scale_bytes + (first & 15)) + ((size_t)lr * p.units + u) * p.scales_per_unit;
+                        }
+                        wr[k].load(stage + my_off + k * pass_bytes, sc, h, u);
+                    }
+                }
+                // the warp holds its weights in registers: the producer may refill the slot
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&empty_bar[slot]);
+                if (++slot == p.stages) { slot = 0; phase ^= 1; }
+                const uint32_t odd = owner ? *(const uint32_t*)(rec + 992 + 4 * h) : 0u;
+                float extra[R], v[R];
+#pragma unroll
+                for (int k = 0; k < R; ++k) extra[k] = 0.f;
+                if (__builtin_expect(odd != 0, 0)) add_odd_inputs<TYPE, R>(wr, have, odd, (const uint32_t*)(rec + 960 + 16 * h), xbase + (int64_t)sg.act[s] * p.st + (int64_t)(256 * u + 128 * h) * p.sk, p.sk, h, extra);
+                dot_regs_float<R>(wr, have, rec, h, v);
+#pragma unroll
+                for (int k = 0; k < R; ++k) {
+                    v[k] = __fadd_rn(v[k], extra[k]);
+                    v[k] += __shfl_xor_sync(0xffffffffu, v[k], 16);
+                    for (int off = group >> 1; off > 0; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);  // (units j and j + 4, then j + 2, then j + 1)
+                }
+                const float mine = h ? v[R - 1] : v[0];
+                float out = 0.f;
+                for (int q = 0; q < subs; ++q) out = fmaf(__shfl_sync(0xffffffffu, mine, (from + q * group) & 31), sg.coef[q], out);
+                const int lr = row_in_pass + h * rows_per_pass;
+                if (in_row == 0 && h < R && row_in_warp < p.warp_rows && lr < info.x && !gone) sg.y[(int64_t)(info.z + lr) * p.yn] = out;
+                if (gone) break;
+            }
+        } else if ((T <= 2 || MODE == RQ_ACT_INT8) && p.warp_rows) {
             // ---- the warp scheme: no partial sums in shared memory, no CTA-wide barrier. A row's items are
             // `group` adjacent lanes; a thread takes up to two rows of a stage (one per pass), holds their
             // weights in registers, releases the stage, and the lanes of a row join their sums by an xor tree.
@@ -1867,9 +1932,9 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
     }
 }
 
-template <int TYPE, int MODE, int T, int NW, int R, bool GATED = false>
+template <int TYPE, int MODE, int T, int NW, int R, bool GATED = false, bool BANKED = false>
 int launch_stream(const StreamParams& p, int grid_x, size_t smem, cudaStream_t s) {
-    auto kernel = rq_gemv_stream_kernel<TYPE, MODE, T, NW, R, GATED>;
+    auto kernel = rq_gemv_stream_kernel<TYPE, MODE, T, NW, R, GATED, BANKED>;
     static bool configured[64] = {};  // per instantiation and device: the opt-in to large dynamic shared memory
     int dev = 0;
     RQ_CUDA(cudaGetDevice(&dev));
@@ -1984,6 +2049,22 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
         p.rows_per_thread = gated_shape || ((int64_t)2 * p.warp_rows * row_bytes <= 34 * 1024 && rows_per_cta > p.warp_rows && 2 * p.warp_rows <= 8) ? 2 : 1;
         stage_rows = gated_shape ? p.warp_rows : p.warp_rows * p.rows_per_thread;
     }
+    // An expert bank's down rows: the slots' sub-rows side by side in a warp, where they fit one. (Of eight units and more a row's sums are strided over
+    // eight lanes instead; longer rows than a warp holds keep partial sums.)
+    p.bank_group = 0;
+    const bool banked_shape = MODE == RQ_ACT_FLOAT && NW == 7 && p.epilogue == RQ_EPI_WSUM && p.plan != nullptr && vectors_per_launch > 0 && p.units <= 8;
+    if (banked_shape) {
+        int group = 1;
+        while (group < p.units) group <<= 1;
+        if (group * p.subs <= 16) {
+            p.bank_group = group;
+            p.warp_rows = 16 / (group * p.subs);
+            p.act_bytes = (size_t)p.units * kRecord;  // a slot's records right behind the slot's before: neighbouring units in neighbouring bank groups
+            const int pass_rows = NW * p.warp_rows;
+            p.rows_per_thread = (int64_t)2 * pass_rows * row_bytes * p.subs <= 34 * 1024 && rows_per_cta > pass_rows ? 2 : 1;
+            stage_rows = pass_rows * p.rows_per_thread;
+        }
+    }
     if (token_pairs) {
         if (!p.warp_rows) return RQ_ERR_UNSUPPORTED;  // pairs run a warp scheme or not at all
         if (p.rows_per_thread == 2) { p.rows_per_thread = 1; stage_rows /= 2; }  // two tokens' records leave no registers for a second row
@@ -1998,10 +2079,14 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
         if (p.window < 2) p.window = 2;
     }
     p.sub_main_bytes = ((size_t)stage_rows * row_bytes + 127) & ~(size_t)127;
+    // (and the sub-rows' units likewise: as far apart, in lines of sixteen bytes modulo eight, as if one row's followed the other's. The 32-value formats'
+    // chunks are permuted by the unit: one line a unit does there.)
+    while (p.bank_group && (p.sub_main_bytes / 16 - (size_t)p.units * (p.scales_per_unit == 8 ? 1 : p.unit_bytes / 16)) % 8) p.sub_main_bytes += 16;
     p.sub_scale_bytes = p.scales_per_unit ? (((size_t)stage_rows * p.units * p.scales_per_unit * 2 + 32 + 127) & ~(size_t)127) : 0;
     p.stage_bytes = (p.sub_main_bytes + p.sub_scale_bytes) * p.subs;
     p.partial_bytes = ((size_t)2 * (t == 1 ? 2 : t) * stage_rows * ipr * 4 + 127) & ~(size_t)127;  // two buffers of T stages (of a pair of stages when T = 1)
     if (p.warp_rows) p.partial_bytes = 0;
+    if (p.bank_group) p.partial_bytes = (128 - p.act_bytes * p.act_vectors % 128) % 128;  // (none: what aligns the ring)
     const size_t fixed = p.act_bytes * p.act_vectors + p.partial_bytes;
     if (fixed + 2 * p.stage_bytes > kSmemBudget) return RQ_ERR_UNSUPPORTED;
     int stages = (int)((kSmemBudget - fixed) / p.stage_bytes);
@@ -2027,6 +2112,9 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
         if (t == 4 && p.warp_rows && p.rows_per_thread == 2) return launch_stream<TYPE, MODE, 4, NW, 2>(p, grid_x, smem, s);
     }
     if (t == 4) return launch_stream<TYPE, MODE, 4, NW, 1>(p, grid_x, smem, s);
+    if constexpr (NW == 7 && MODE == RQ_ACT_FLOAT) {
+        if (p.bank_group) return p.rows_per_thread == 2 ? launch_stream<TYPE, MODE, 1, NW, 2, false, true>(p, grid_x, smem, s) : launch_stream<TYPE, MODE, 1, NW, 1, false, true>(p, grid_x, smem, s);
+    }
     if constexpr (NW != 5) {
         if (p.warp_rows && gated_shape) return launch_stream<TYPE, MODE, 1, NW, 2, true>(p, grid_x, smem, s);
     }
