@@ -46,7 +46,7 @@ int rq_launch_stream(rq_ctx* ctx, int type, int64_t cols, const RqSegment* table
 // that many planned launches as the grid rows of one: row y reads plan[y * plan_stride] and x + y * x_plan_stride.
 int rq_launch_stream_plan(rq_ctx* ctx, int type, int64_t cols, const RqPlan* plan, int plan_count, int plan_stride, int max_segments, int max_subs,
                           int epilogue, int64_t max_rows, const float* x, int64_t x_plan_stride, int64_t sk, int64_t st, int vectors, int64_t yn, int64_t yt,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool side_by_side) {
     if (cols % 256 || max_subs < 1 || max_subs > RQ_MAX_SUB || max_segments < 1 || max_segments > RQ_MAX_SEGMENTS || vectors < 1) return RQ_ERR_UNSUPPORTED;
     StreamParams p;
     memset(&p, 0, sizeof(p));
@@ -54,6 +54,7 @@ int rq_launch_stream_plan(rq_ctx* ctx, int type, int64_t cols, const RqPlan* pla
     p.n_segments = max_segments; p.subs = max_subs; p.epilogue = epilogue;
     p.rows = max_rows; p.cols = (int)cols; p.units = (int)(cols / 256);
     p.x = x; p.sk = sk; p.st = st; p.yn = yn; p.yt = yt; p.tokens = 1;
+    p.side_by_side = side_by_side ? 1 : 0;
     p.error_flag = ctx->error_flag; p.wait_ns = ctx->wait_limit_ns;
     switch (type) {
         case RQ_Q4_K: p.unit_bytes = 144; p.scales_per_unit = 0; break;

@@ -71,6 +71,7 @@ struct StreamParams {
                                // bandwidth, not more -- a deeper queue only delays everything else that reads memory (the activations)
     int row_warps;             // warp scheme: 1 = a row lies inside one warp; NW = every warp holds 32 / warp_rows lanes' worth of
                                // each row of the pass, and the warps' sums meet in shared memory (the last warp to arrive adds them)
+    int side_by_side;          // the launch is meant for the scheme of an expert bank's down rows, or for nobody
     int bank_group;            // > 0: the warp scheme of an expert bank's down rows -- a sub-row's units are this many lanes (a power of two), a virtual
                                // row p.subs times as many, side by side in each half of a warp (first and second halves of the units); warp_rows virtual rows a pass
     int sum_group, sum_chunks; // the order a row's item sums are added in when the shape has a warp scheme (so that a multi-token
@@ -2049,22 +2050,29 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
         p.rows_per_thread = gated_shape || ((int64_t)2 * p.warp_rows * row_bytes <= 34 * 1024 && rows_per_cta > p.warp_rows && 2 * p.warp_rows <= 8) ? 2 : 1;
         stage_rows = gated_shape ? p.warp_rows : p.warp_rows * p.rows_per_thread;
     }
-    // An expert bank's down rows: the slots' sub-rows side by side in a warp, where they fit one. (Of eight units and more a row's sums are strided over
-    // eight lanes instead; longer rows than a warp holds keep partial sums.)
+    // An expert bank's down rows: the slots' sub-rows side by side in a warp, where they fit one. (Of more than eight units a row's sums are strided over
+    // eight lanes instead; longer rows than a warp holds keep partial sums. 32 experts, eight tokens, hidden 2048, of 256 to 1024 inputs a slot and one to eight slots, the
+    // four formats: 0.78 to 0.98 of the time with partial sums.)
     p.bank_group = 0;
-    const bool banked_shape = MODE == RQ_ACT_FLOAT && NW == 7 && p.epilogue == RQ_EPI_WSUM && p.plan != nullptr && vectors_per_launch > 0 && p.units <= 8;
-    if (banked_shape) {
+    if (p.side_by_side && MODE == RQ_ACT_FLOAT && NW == 7 && !one_per_sm && p.epilogue == RQ_EPI_WSUM && p.units <= 8) {
         int group = 1;
         while (group < p.units) group <<= 1;
-        if (group * p.subs <= 16) {
+        const int fit = 16 / (group * p.subs), pass_rows = NW * fit;  // virtual rows of a warp (a pass)
+        // Two rows a thread where a ring of two such stages fits beside the digits; where it does not, warps whose lanes are nearly all used (Q8_0, eight
+        // tokens of hidden 2048: eight slots of 512 inputs 66.8 -> 58.9 us with a row a thread, six of them 51.5 -> 52.6).
+        const int64_t two_rows = p.subs * (2 * pass_rows * (row_bytes + 2 * p.units * p.scales_per_unit) + 512);
+        const bool two = (int64_t)p.act_vectors * p.units * kRecord + 2 * two_rows <= (int64_t)kSmemBudget && rows_per_cta > pass_rows;
+        // (Few rows a CTA, one token's: not where they would take a second pass for which the partial sums' threads have room, 2304 rows of six slots 27.0 -> 27.7 us.)
+        const bool fewer_there = rows_per_cta > pass_rows && rows_per_cta <= kConsumers / ipr;
+        if (fit > 0 && !fewer_there && (two || rows_per_cta <= pass_rows || fit * p.subs * p.units >= 14)) {
             p.bank_group = group;
-            p.warp_rows = 16 / (group * p.subs);
+            p.warp_rows = fit;
             p.act_bytes = (size_t)p.units * kRecord;  // a slot's records right behind the slot's before: neighbouring units in neighbouring bank groups
-            const int pass_rows = NW * p.warp_rows;
-            p.rows_per_thread = (int64_t)2 * pass_rows * row_bytes * p.subs <= 34 * 1024 && rows_per_cta > pass_rows ? 2 : 1;
+            p.rows_per_thread = two ? 2 : 1;
             stage_rows = pass_rows * p.rows_per_thread;
         }
     }
+    if (p.side_by_side && !p.bank_group) return RQ_ERR_UNSUPPORTED;
     if (token_pairs) {
         if (!p.warp_rows) return RQ_ERR_UNSUPPORTED;  // pairs run a warp scheme or not at all
         if (p.rows_per_thread == 2) { p.rows_per_thread = 1; stage_rows /= 2; }  // two tokens' records leave no registers for a second row

@@ -663,8 +663,8 @@ extern "C" int rq_moe_forward(rq_ctx* ctx, rq_moe* m, const float* x, int64_t x_
 }
 
 static int launch_banks(rq_ctx* ctx, rq_moe* m, const float* x, int64_t x_k_stride, int64_t x_t_stride, int top_k, int tokens, int64_t y_n_stride, cudaStream_t s) {
-    const int apart = (top_k + (m->has_shared ? m->sh_count : 1)) * m->ffn;  // from one token's h to the next one's, as the plans have them
-    const int slots = top_k + (m->has_shared ? m->sh_count : 0);
+    const int shared_slots = m->has_shared ? m->sh_count : 1;
+    const int slots = top_k + shared_slots;
     int rc;
     // All tokens in two launches: grid row t of each reads token t's plan and activations.
     // expert gate and up rows against the token's x, h = silu(g) * u per slot
@@ -672,8 +672,13 @@ static int launch_banks(rq_ctx* ctx, rq_moe* m, const float* x, int64_t x_k_stri
                                    1, 1, 0, s);
     if (rc == RQ_ERR_UNSUPPORTED) return rq_fail(RQ_ERR_LIMIT, "rq_moe_forward: hidden=%d is beyond what the streaming kernel holds", m->hidden);
     if (rc) return rc;
-    // expert down rows, one sub-row per slot against that slot's h, summed with the routing weights
-    rc = rq_launch_stream_plan(ctx, m->type, m->ffn, m->plans + 1, tokens, 2, 1, slots, RQ_EPI_WSUM, m->hidden, m->h, apart, 1, m->ffn, slots,
+    // expert down rows, one sub-row per slot against that slot's h, summed with the routing weights: the slots that a token can have side by side in
+    // a warp, where they fit one; else partial sums (whose stages a spare slot makes no slower)
+    const int live = top_k + (m->has_shared ? m->sh_count : 0);
+    rc = rq_launch_stream_plan(ctx, m->type, m->ffn, m->plans + 1, tokens, 2, 1, live, RQ_EPI_WSUM, m->hidden, m->h, (int64_t)slots * m->ffn, 1, m->ffn, live,
+                               y_n_stride, 0, s, true);
+    if (rc != RQ_ERR_UNSUPPORTED) return rc;
+    rc = rq_launch_stream_plan(ctx, m->type, m->ffn, m->plans + 1, tokens, 2, 1, slots, RQ_EPI_WSUM, m->hidden, m->h, (int64_t)slots * m->ffn, 1, m->ffn, slots,
                                y_n_stride, 0, s);
     if (rc == RQ_ERR_UNSUPPORTED) return rq_fail(RQ_ERR_LIMIT, "rq_moe_forward: ffn=%d with %d slots is beyond what the streaming kernel holds", m->ffn, slots);
     if (rc) return rc;
