@@ -54,7 +54,7 @@ int rq_launch_stream_plan(rq_ctx* ctx, int type, int64_t cols, const RqPlan* pla
     p.n_segments = max_segments; p.subs = max_subs; p.epilogue = epilogue;
     p.rows = max_rows; p.cols = (int)cols; p.units = (int)(cols / 256);
     p.x = x; p.sk = sk; p.st = st; p.yn = yn; p.yt = yt; p.tokens = 1;
-    p.side_by_side = side_by_side ? 1 : 0;
+    p.bank_group = side_by_side ? -1 : 0;
     p.error_flag = ctx->error_flag; p.wait_ns = ctx->wait_limit_ns;
     switch (type) {
         case RQ_Q4_K: p.unit_bytes = 144; p.scales_per_unit = 0; break;

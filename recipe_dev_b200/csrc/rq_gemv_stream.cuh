@@ -47,6 +47,10 @@ struct StreamParams {
     int64_t x_plan_stride;
     RqSegment inline_seg[RQ_INLINE_SEGMENTS];
     int n_segments, subs, epilogue;
+    int bank_group;            // > 0: the warp scheme of an expert bank's down rows -- a sub-row's units are this many lanes (a power of two), a virtual row p.subs times
+                               // as many, side by side in each half of a warp (first and second halves of the units); warp_rows virtual rows a pass. -1 before the
+                               // launch is laid out: meant for that scheme, or for nobody
+                               // (In the hole behind three ints: eight bytes more of parameters cost every launch 0.2 us of the host's time.)
     int64_t rows;              // virtual rows of all segments
     int64_t rows_quot; int rows_rem;  // rows / CTAs and rows % CTAs (launches whose row count the host knows): CTA b takes
                                // rows_quot rows from b * rows_quot + min(b, rows_rem), one more when b < rows_rem
@@ -71,9 +75,6 @@ struct StreamParams {
                                // bandwidth, not more -- a deeper queue only delays everything else that reads memory (the activations)
     int row_warps;             // warp scheme: 1 = a row lies inside one warp; NW = every warp holds 32 / warp_rows lanes' worth of
                                // each row of the pass, and the warps' sums meet in shared memory (the last warp to arrive adds them)
-    int side_by_side;          // the launch is meant for the scheme of an expert bank's down rows, or for nobody
-    int bank_group;            // > 0: the warp scheme of an expert bank's down rows -- a sub-row's units are this many lanes (a power of two), a virtual
-                               // row p.subs times as many, side by side in each half of a warp (first and second halves of the units); warp_rows virtual rows a pass
     int sum_group, sum_chunks; // the order a row's item sums are added in when the shape has a warp scheme (so that a multi-token
                                // launch gives each token the bits a single-token launch gives it): chunks of sum_group items, an
                                // xor tree inside a chunk, chunks in order. sum_group = 0: items strided over eight lanes, then a tree
@@ -2053,8 +2054,9 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     // An expert bank's down rows: the slots' sub-rows side by side in a warp, where they fit one. (Of more than eight units a row's sums are strided over
     // eight lanes instead; longer rows than a warp holds keep partial sums. 32 experts, eight tokens, hidden 2048, of 256 to 1024 inputs a slot and one to eight slots, the
     // four formats: 0.78 to 0.98 of the time with partial sums.)
+    const bool side_by_side = p.bank_group < 0;
     p.bank_group = 0;
-    if (p.side_by_side && MODE == RQ_ACT_FLOAT && NW == 7 && !one_per_sm && p.epilogue == RQ_EPI_WSUM && p.units <= 8) {
+    if (side_by_side && MODE == RQ_ACT_FLOAT && NW == 7 && !one_per_sm && p.epilogue == RQ_EPI_WSUM && p.units <= 8) {
         int group = 1;
         while (group < p.units) group <<= 1;
         const int fit = 16 / (group * p.subs), pass_rows = NW * fit;  // virtual rows of a warp (a pass)
@@ -2072,7 +2074,7 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
             stage_rows = pass_rows * p.rows_per_thread;
         }
     }
-    if (p.side_by_side && !p.bank_group) return RQ_ERR_UNSUPPORTED;
+    if (side_by_side && !p.bank_group) { p.bank_group = -1; return RQ_ERR_UNSUPPORTED; }
     if (token_pairs) {
         if (!p.warp_rows) return RQ_ERR_UNSUPPORTED;  // pairs run a warp scheme or not at all
         if (p.rows_per_thread == 2) { p.rows_per_thread = 1; stage_rows /= 2; }  // two tokens' records leave no registers for a second row
@@ -2096,7 +2098,7 @@ int dispatch_stream_nw(StreamParams& p, int sm_count, int vectors_per_launch, cu
     if (p.warp_rows) p.partial_bytes = 0;
     if (p.bank_group) p.partial_bytes = (128 - p.act_bytes * p.act_vectors % 128) % 128;  // (none: what aligns the ring)
     const size_t fixed = p.act_bytes * p.act_vectors + p.partial_bytes;
-    if (fixed + 2 * p.stage_bytes > kSmemBudget) return RQ_ERR_UNSUPPORTED;
+    if (fixed + 2 * p.stage_bytes > kSmemBudget) { if (side_by_side) p.bank_group = -1; return RQ_ERR_UNSUPPORTED; }
     int stages = (int)((kSmemBudget - fixed) / p.stage_bytes);
     if (stages > kMaxStages) stages = kMaxStages;
     p.stages = stages;
