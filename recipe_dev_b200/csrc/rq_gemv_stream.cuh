@@ -1683,6 +1683,11 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             // Gated launches: the sums of a virtual row's gate and up rows wait in the warp's lanes, one virtual row a lane, until the
             // lanes are full or the rows are over: silu goes through double precision, a long chain that one lane would otherwise walk
             // for every row by itself.
+            // A row that is not there is loaded and dotted all the same (its slot has room for it) and its sum dropped: with a branch around each row's loads and
+            // another around its dot, a thread's two rows follow one another. Q6_K and Q8_0, int8, one token, us: Q6_K 262144 x 2560 97.9 -> 95.9, 4096 x
+            // 14336 12.7 -> 12.5, 30000 x 1024 7.5 -> 7.35; Q8_0 100000 x 2560 46.1 -> 45.5. Not the four-bit formats, whose dot is half as long (Q4_0 100000
+            // x 2560 31.8 -> 32.9).
+            constexpr bool kAlways = MODE == RQ_ACT_INT8 && T != 4 && (TYPE == RQ_Q6_K || TYPE == RQ_Q8_0);
             constexpr bool gated = GATED;
             int pending = 0;
             float held_gate = 0.f, held_up = 0.f;
@@ -1706,7 +1711,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     // the second pass's rows are the stage's second piece
                     if (k == 1 && p.pieces == 2 && !dead && !mbar_wait(&full_bar[2 * slot + 1], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); dead = true; }
                     have[k] = lr < info.x && act_owner;
-                    if (have[k]) {
+                    if (kAlways || have[k]) {
                         const uint16_t* sc = nullptr;
                         if (TYPE != RQ_Q4_K) {
                             const uint8_t* plane = stage + (gated ? 2 : 1) * p.sub_main_bytes + info.w;
@@ -1735,7 +1740,13 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
 #pragma unroll
                     for (int j = 0; j < TR; ++j)
 #pragma unroll
-                        for (int k = 0; k < R; ++k) v[j][k] = have[k] ? dot_regs(wr[k], areg[j], my_h) : 0.f;
+                        for (int k = 0; k < R; ++k) v[j][k] = kAlways || have[k] ? dot_regs(wr[k], areg[j], my_h) : 0.f;
+                    if (kAlways) {
+#pragma unroll
+                        for (int j = 0; j < TR; ++j)
+#pragma unroll
+                            for (int k = 0; k < R; ++k) v[j][k] = have[k] ? v[j][k] : 0.f;
+                    }
                 } else {
                     float extra[R];
 #pragma unroll
