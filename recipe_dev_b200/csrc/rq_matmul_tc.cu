@@ -521,7 +521,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         }
                     }
                 };
-                const int64_t my_row = min((int64_t)(mt * MH + half0) * 128 + quarter * 32 + lane, p.rows - 1);  // kept inside the weight for the scale loads
+                // this lane's row, kept inside the weight for the scale loads (found anew by each: held, it cost Q8_0 and Q4_0 4 % in spilled registers)
+                auto my_row = [&]() -> int64_t { return min((int64_t)(mt * MH + half0) * 128 + quarter * 32 + lane, p.rows - 1); };
                 // Slice `all` of the CTA's: d[0] (and d[1]: the second half slice's) scale its sums
                 auto drain = [&](int all, const float (&d)[2]) {
                     const int step = MH == 1 ? all : 2 * all + half0;
@@ -583,8 +584,8 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 };
                 if constexpr (F::kquant) {
                     auto d_of = [&](int u) -> float {
-                        if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (my_row * p.units + u) * 144)));
-                        return rq_h2f(__ldg(p.scale + my_row * p.units + u));
+                        if (TYPE == RQ_Q4_K) return rq_h2f(__ldg((const uint16_t*)(p.main + (my_row() * p.units + u) * 144)));
+                        return rq_h2f(__ldg(p.scale + my_row() * p.units + u));
                     };
                     float d_next = d_of(u0);
                     int all = slice_base;
@@ -605,7 +606,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     // 32 lines, as one of sixteen does)
                     const bool wide = (p.blocks32 & 7) == 0 && ((uintptr_t)p.scale & 15) == 0;
                     auto d_of = [&](int u) -> uint4 {
-                        const uint16_t* at = p.scale + my_row * p.blocks32 + 8 * u;
+                        const uint16_t* at = p.scale + my_row() * p.blocks32 + 8 * u;
                         if (wide) return __ldg((const uint4*)at);
                         uint32_t w[4];
 #pragma unroll
@@ -657,11 +658,13 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                     for (int j = 0; j < kLeave / 2; ++j) left[j] = sum[j];
                 }
                 const int from = MH == 1 ? set * kLeave : 0;  // the first of them
-                const int64_t row = (int64_t)(mt * MH + half0) * 128 + r0;
-                const int n = dead || row >= p.rows ? 0 : min(kLeave, p.tokens - nt * bn - from);  // how many of them count
-                float* const out = p.y + row * p.yn + (int64_t)(nt * bn + from) * p.yt;
+                const int tokens_here = dead ? 0 : min(kLeave, p.tokens - nt * bn - from);
+                // how many of this thread's tokens count, and where they go (found anew by each, as the row)
+                auto live = [&]() { return (int64_t)(mt * MH + half0) * 128 + r0 < p.rows ? tokens_here : 0; };
+                auto out = [&]() { return p.y + ((int64_t)(mt * MH + half0) * 128 + r0) * p.yn + (int64_t)(nt * bn + from) * p.yt; };
                 if (whole) {
-                    float* at = out;
+                    const int n = live();
+                    float* at = out();
 #pragma unroll
                     for (int j = 0; j < kLeave; ++j) {
                         if (j < n) *at = pair_at(left[j / 2], j & 1);
@@ -670,10 +673,13 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                 } else {
                     const size_t tile_floats = (size_t)bn * 128 * MH, place0 = (size_t)from * 128 * MH + half0 * 128 + r0;
                     auto piece_of = [&](int c) { return p.partial + (size_t)Deal::place(c, c0) * tile_floats + place0; };
-                    float* const piece = piece_of((int)blockIdx.x);
+                    {
+                        const int n = live();
+                        float* const piece = piece_of((int)blockIdx.x);
 #pragma unroll
-                    for (int j = 0; j < kLeave; ++j)
-                        if (j < n) piece[j * 128 * MH] = pair_at(left[j / 2], j & 1);
+                        for (int j = 0; j < kLeave; ++j)
+                            if (j < n) piece[j * 128 * MH] = pair_at(left[j / 2], j & 1);
+                    }
                     __threadfence();
                     asm volatile("bar.sync 2, %0;" ::"n"(kDrainWarps * 32) : "memory");
                     if (tid == 0) {
@@ -687,6 +693,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                         // load would make each wait for the one before; the padding tokens' places exist and hold nothing that is used). Tiles of 48 tokens, 24
                         // a thread: 12 at a time (Q6_K 8192 x 1024, 48 tokens, by 8 / 12 / 24: 13.0 / 11.6 / 11.9 us; 1670 x 12800, 34 tokens: 26.2 / 23.8 / 29.1).
                         constexpr int kAtOnce = kLeave % 32 == 0 ? 32 : (kLeave % 16 == 0 ? 16 : (kLeave % 12 == 0 ? 12 : 8));
+                        const int n = live();
 #pragma unroll 1
                         for (int j0 = 0; j0 < n; j0 += kAtOnce) {
                             Pair total[kAtOnce / 2];
@@ -707,7 +714,7 @@ __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const
                                 for (int q = 0; q < kAtOnce; q += 2)
                                     total[q / 2] = pair_add(total[q / 2], two ? pair_add(pair_of(v[q], v[q + 1]), pair_of(w[q], w[q + 1])) : pair_of(v[q], v[q + 1]));
                             }
-                            float* at = out + (int64_t)j0 * p.yt;
+                            float* at = out() + (int64_t)j0 * p.yt;
 #pragma unroll
                             for (int q = 0; q < kAtOnce; ++q) {
                                 if (j0 + q < n) *at = pair_at(total[q / 2], q & 1);
