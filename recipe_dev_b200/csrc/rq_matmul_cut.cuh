@@ -185,7 +185,8 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     int steps = (512 - c.a_slots * f.a_cols - totals) / step_cols;
     if (steps > kMaxAcc / halves) steps = kMaxAcc / halves;
     c.accs = steps * halves;
-    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window; codes, MH = 2: and the totals)
+    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window; codes, MH = 2: room as large as the sums,
+    // of which the kernel of bytes makes rings of its own, Int8Rings)
     const int kept = (c.mh == 1 ? c.bn * 128 * 4 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0) + (codes && c.mh == 2 ? c.bn * 256 * 4 : 0), budget = (codes ? 212 : 220) * 1024 - kept, b_bytes = c.bn * (codes ? 128 : 256);
     c.b_slots = c.mh == 1 || codes ? 4 : 3;
     c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
