@@ -1626,19 +1626,18 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             const int my_off = (int)(s * p.sub_main_bytes) + row_in_pass * (int)row_bytes + u * p.unit_bytes, pass_bytes = rows_per_pass * (int)row_bytes;
             const int from = min(row_in_warp * row_lanes, 16 - row_lanes) + (lane & 16);  // the lanes that hold the sums this one adds up: the first half's the first row's, the second half's the second's
             while (true) {
-                if (!mbar_wait(&full_bar[2 * slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); break; }
-                const int4 info = stage_info[slot];  // rows, segment, first local row
-                if (info.x == 0) break;              // the producer has no more rows for this CTA
+                bool there = mbar_wait(&full_bar[2 * slot], phase, p.wait_ns);
+                const int4 info = there ? stage_info[slot] : make_int4(0, 0, 0, 0);  // rows, segment, first local row
                 const RqSegment& sg = table[info.y];
                 const uint8_t* stage = ring + (size_t)slot * p.stage_bytes;
                 const uint8_t* rec = act_smem + (owner ? sg.act[s] * (int)p.act_bytes + u * kRecord : 0);
                 ItemRegs<TYPE> wr[R];
-                bool have[R], gone = false;
+                bool have[R];
 #pragma unroll
                 for (int k = 0; k < R; ++k) {
                     const int lr = row_in_pass + k * rows_per_pass;
                     // the second pass's rows are the stage's second piece
-                    if (k == 1 && p.pieces == 2 && !mbar_wait(&full_bar[2 * slot + 1], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); gone = true; }
+                    if (k == 1 && p.pieces == 2) there = mbar_wait(&full_bar[2 * slot + 1], phase, p.wait_ns) && there;
                     have[k] = lr < info.x && owner;
                     if (have[k]) {
                         const uint16_t* sc = nullptr;
@@ -1649,8 +1648,10 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                         wr[k].load(stage + my_off + k * pass_bytes, sc, h, u);
                     }
                 }
-                // the warp holds its weights in registers: the producer may refill the slot
-                __syncwarp();
+                // the warp holds its weights in registers: the producer may refill the slot. (A wait that ran out in one lane ends the whole warp's work:
+                // the sums below are joined by shuffles of all lanes.)
+                if (!__all_sync(0xffffffffu, there)) { atomicExch(p.error_flag, 3); break; }
+                if (info.x == 0) break;  // the producer has no more rows for this CTA
                 if (lane == 0) mbar_arrive(&empty_bar[slot]);
                 if (++slot == p.stages) { slot = 0; phase ^= 1; }
                 const uint32_t odd = owner ? *(const uint32_t*)(rec + 992 + 4 * h) : 0u;
@@ -1669,8 +1670,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                 float out = 0.f;
                 for (int q = 0; q < subs; ++q) out = fmaf(__shfl_sync(0xffffffffu, mine, (from + q * group) & 31), sg.coef[q], out);
                 const int lr = row_in_pass + h * rows_per_pass;
-                if (in_row == 0 && h < R && row_in_warp < p.warp_rows && lr < info.x && !gone) sg.y[(int64_t)(info.z + lr) * p.yn] = out;
-                if (gone) break;
+                if (in_row == 0 && h < R && row_in_warp < p.warp_rows && lr < info.x) sg.y[(int64_t)(info.z + lr) * p.yn] = out;
             }
         } else if ((T <= 2 || MODE == RQ_ACT_INT8) && p.warp_rows) {
             // ---- the warp scheme: no partial sums in shared memory, no CTA-wide barrier. A row's items are
@@ -1702,11 +1702,13 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                 held_y = nullptr;
                 pending = 0;
             };
+            // A stage's two looks at its barriers end in one vote, where the warp met anyway; a vote at each look took 0.8 % longer over 53 calls. Lanes that
+            // gave up used to leave one by one, and without that way out the loop is the shorter one. us, before / now: int8 Q6_K 262144 x 2560 96.4 / 91.2, two
+            // positions of 9000 x 2560 9.6 / 8.5, Q4_K 12000 x 5120 11.0 / 10.6; fp32 Q4_K 4096 x 14336 15.1 / 14.4; 64 Q8_0 experts of 2048 x 512, sixteen positions, 54.2 / 51.7;
+            // 83 calls 0.98, the slowest 1.015 (Q4_K 4096 x 4096 fp32 7.5 / 7.6).
             while (true) {
-                if (!mbar_wait(&full_bar[2 * slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); dead = true; }
-                if (dead) break;
-                const int4 info = stage_info[slot];  // rows, segment, first local row, offset of the first d
-                if (info.x == 0) break;               // the producer has no more rows for this CTA
+                bool there = mbar_wait(&full_bar[2 * slot], phase, p.wait_ns);
+                const int4 info = there ? stage_info[slot] : make_int4(0, 0, 0, 0);  // rows, segment, first local row, offset of the first d
                 const uint8_t* stage = ring + (size_t)slot * p.stage_bytes;
                 ItemRegs<TYPE> wr[R];
                 bool have[R];
@@ -1714,7 +1716,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                 for (int k = 0; k < R; ++k) {
                     const int lr = row_in_pass + (gated ? 0 : k * rows_per_pass);
                     // the second pass's rows are the stage's second piece
-                    if (k == 1 && p.pieces == 2 && !dead && !mbar_wait(&full_bar[2 * slot + 1], phase, p.wait_ns)) { atomicExch(p.error_flag, 3); dead = true; }
+                    if (k == 1 && p.pieces == 2) there = mbar_wait(&full_bar[2 * slot + 1], phase, p.wait_ns) && there;
                     have[k] = lr < info.x && act_owner;
                     if (kAlways || have[k]) {
                         const uint16_t* sc = nullptr;
@@ -1728,8 +1730,10 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                         wr[k].load(stage + my_off + (gated ? k * p.sub_main_bytes : k * pass_bytes), sc, my_h, my_u);
                     }
                 }
-                // the warp holds its weights in registers: the producer may refill the slot
-                __syncwarp();
+                // the warp holds its weights in registers: the producer may refill the slot. (A wait that ran out in one lane ends the whole warp's work:
+                // the sums below are joined by shuffles of all lanes.)
+                if (!__all_sync(0xffffffffu, there)) { atomicExch(p.error_flag, 3); break; }
+                if (info.x == 0) break;  // the producer has no more rows for this CTA
                 if (lane == 0) mbar_arrive(&empty_bar[slot]);
                 if (++slot == p.stages) { slot = 0; phase ^= 1; }
                 // v[j][k]: token tok0 + j (the tokens a thread holds in registers) against row k of the stage; every token's

@@ -32,6 +32,17 @@ def test_the_streaming_producer_waits_for_every_piece_it_issued():
     assert producer.count("mbar_expect_tx(") == 2 and producer.count("++n_pieces;") == 1 and producer.count("n_pieces += p.pieces;") == 1
 
 
+def test_the_streaming_consumers_that_join_sums_by_shuffles_stay_together():
+    """A lane that gave up and left alone would be missing from the others' shuffles, and a slot whose copies never landed must not be handed back."""
+    consumers = (CSRC / "rq_gemv_stream.cuh").read_text().split("- the warp scheme of an expert bank's down rows")[1].split("two-row instantiations serve")[0]
+    for scheme in consumers.split("- the warp scheme: no partial sums"):
+        before, after = scheme.split("while (true) {")[1].split("if (!__all_sync(0xffffffffu, there)) { atomicExch(p.error_flag, 3); break; }")
+        assert before.count("there = mbar_wait(") == scheme.count("mbar_wait(") == 2
+        assert "there ? stage_info[slot] : make_int4(0, 0, 0, 0)" in before  # what a slot that never filled says is not used
+        assert not re.search(r"_sync\(|break|continue|return|mbar_arrive", before)
+        assert after.index("if (info.x == 0) break;") < after.index("mbar_arrive(&empty_bar[slot])") < after.index("__shfl")
+
+
 def test_the_batched_product_ends_with_nothing_under_way():
     """The drain and staging warps wait for every product and copy, but not once one of their waits has run out."""
     misc = (CSRC / "rq_matmul_tc.cu").read_text().split("auto landed = [&]")[1].split("free the tensor memory")[0]
