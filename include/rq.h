@@ -241,7 +241,7 @@ typedef struct rq_moe rq_moe; /* the expert tables of one gguf_moe block residen
 /* Routing weights of `tokens` positions from their router scores: softmax or sigmoid scoring, the
  * top_k experts by score (ties to the lower index; with a selection bias, by probability + bias),
  * renormalised over the kept experts or not. Writes the dense plane the expert bodies read:
- * weights[e * weight_e_stride + t * weight_t_stride], zero for experts not taken.
+ * weights[e * weight_e_stride + t * weight_t_stride], zero for experts not taken. (It may be the scores' own plane, with the same strides.)
  * Replaces topk_forward_body (amd-nv-cpu.ll:4666-4716), same bits (its exp is build.rs:1079-1120). */
 int rq_moe_route(rq_ctx* ctx, const float* scores, int64_t score_e_stride, int64_t score_t_stride, int experts, int top_k, int scoring,
                  int renormalize, const float* selection_bias, int tokens, float* weights, int64_t weight_e_stride, int64_t weight_t_stride,

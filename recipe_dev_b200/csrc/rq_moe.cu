@@ -133,8 +133,10 @@ __device__ __forceinline__ float block_max(float v, float* scratch, int tid) {
     return m;
 }
 
-__device__ __forceinline__ void route_token(const float* __restrict__ scores, int64_t se, int64_t st, int experts, int top, int sigmoid, int renorm,
-                                            const float* __restrict__ bias, float* __restrict__ weights, int64_t we, int64_t wt) {
+// (Scores and weights may be one plane, so neither is declared __restrict__, here and below: a score read again behind the first weight
+// written, or through the read-only path, could be a weight.)
+__device__ __forceinline__ void route_token(const float* scores, int64_t se, int64_t st, int experts, int top, int sigmoid, int renorm,
+                                            const float* __restrict__ bias, float* weights, int64_t we, int64_t wt) {
     extern __shared__ float sm[];      // [experts] raw scores | [experts] values | [experts] keys | [experts] marks
     float* raw = sm;
     float* val = sm + experts;
@@ -343,9 +345,9 @@ __device__ __forceinline__ bool route_by_warp(const float* scores, int64_t se, i
     return experts <= 256 ? pick_by_warp<8>(scores, se, st, experts, top, sigmoid != 0, weights, we, wt, picks) : pick_by_warp<32>(scores, se, st, experts, top, sigmoid != 0, weights, we, wt, picks);
 }
 
-__global__ void __launch_bounds__(kRouteThreads) rq_route_kernel(const float* __restrict__ scores, int64_t se, int64_t st, int experts, int top,
+__global__ void __launch_bounds__(kRouteThreads) rq_route_kernel(const float* scores, int64_t se, int64_t st, int experts, int top,
                                                                 int sigmoid, int renorm, const float* __restrict__ bias,
-                                                                float* __restrict__ weights, int64_t we, int64_t wt) {
+                                                                float* weights, int64_t we, int64_t wt) {
     __shared__ Picks picks;
     if (route_by_warp(scores, se, st, experts, top, sigmoid, renorm, bias, weights, we, wt, &picks)) return;
     route_token(scores, se, st, experts, top, sigmoid, renorm, bias, weights, we, wt);
@@ -363,7 +365,7 @@ struct BankView {
     const float* sh_vector;
 };
 
-__device__ __forceinline__ void plan_token(const BankView& b, const float* __restrict__ routing, int64_t re, int64_t rt, const float* __restrict__ x, int64_t sk,
+__device__ __forceinline__ void plan_token(const BankView& b, const float* routing, int64_t re, int64_t rt, const float* __restrict__ x, int64_t sk,
                                            int64_t st, int top, int include_shared, RqPlan* __restrict__ plans, float* __restrict__ h, float* __restrict__ y,
                                            int64_t yn, int64_t yt, const Picks* picks = nullptr) {
     const int t = blockIdx.x, tid = threadIdx.x;
@@ -478,8 +480,8 @@ __global__ void __launch_bounds__(256) rq_moe_plan_kernel(BankView b, const floa
 // dense plane, which stays the block's visible result) reads them back after a barrier and writes the token's two segment
 // tables. One launch and one dependency less on the path of a decode step.
 static_assert(kRouteThreads == 256, "the fused launch runs both bodies with the same CTA");
-__global__ void __launch_bounds__(256) rq_moe_route_plan_kernel(BankView b, const float* __restrict__ scores, int64_t se, int64_t sst, int experts, int top, int sigmoid,
-                                                               int renorm, const float* __restrict__ bias, float* __restrict__ weights, int64_t we, int64_t wt,
+__global__ void __launch_bounds__(256) rq_moe_route_plan_kernel(BankView b, const float* scores, int64_t se, int64_t sst, int experts, int top, int sigmoid,
+                                                               int renorm, const float* __restrict__ bias, float* weights, int64_t we, int64_t wt,
                                                                const float* __restrict__ x, int64_t sk, int64_t st, int include_shared, RqPlan* __restrict__ plans,
                                                                float* __restrict__ h, float* __restrict__ y, int64_t yn, int64_t yt) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the gate and up launch may take its places on the SMs (it waits for this one's end)
