@@ -1142,6 +1142,10 @@ __device__ inline float rq_tanh_portable(float xf) {
 __device__ __forceinline__ float rq_sigmoid_portable(float x) { return __fmul_rn(0.5f, __fadd_rn(rq_tanh_portable(__fmul_rn(0.5f, x)), 1.0f)); }
 __device__ __forceinline__ float rq_silu_portable(float x) { return __fmul_rn(x, rq_sigmoid_portable(x)); }
 
+// Beside a stage's segment: the CTA's rows end with it. (An empty stage behind the last one, which every warp waited for, loaded of and voted on, was 0.3 us of a
+// short bank's call: 40 experts of 1536 x 256, one position, 15.4 -> 15.0 us; int8 Q4_0 4096 x 4096, two positions, 9.2 -> 8.9; fp32 Q8_0 1024 x 1024 4.27 -> 4.10.)
+constexpr int kLastStage = 1 << 30;
+
 // R = rows a thread takes per stage in the warp scheme (its weight registers): 2 only where the launch uses two. GATED: the two are
 // the gate row and the up row of one virtual row. BANKED: a virtual row is an expert bank's down rows, one of each slot.
 // ONE (fp32 activations): a slice of sixteen inputs a thread is enough; a straight line takes half a microsecond less than a loop with the next round's loads
@@ -1224,9 +1228,11 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
         // issues stages until `limit` have been issued or the rows run out
         const int grid = (int)gridDim.x;
         int my_stage = (int)blockIdx.x;  // interleaved launches: the stage to issue next
+        bool said = false;  // the last stage was among them
         auto issue = [&](int limit) {
             for (; st < limit && !failed; ++st) {
                 int nr;
+                bool last = false;
                 int64_t lr0;  // first row, local to the segment
                 if (p.interleaved) {
                     if (my_stage >= p.total_stages) break;
@@ -1236,6 +1242,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     const int64_t left = segs[seg].rows - lr0;
                     nr = (int)(left < p.stage_rows ? left : p.stage_rows);
                     my_stage += grid;
+                    last = my_stage >= p.total_stages;
                 } else {
                     if (r >= row_end) break;
                     while (seg + 1 < n_segments && r >= segs[seg].row_begin + segs[seg].rows) ++seg;
@@ -1246,7 +1253,9 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     nr = (int)(stop - r);
                     lr0 = r - segs[seg].row_begin;
                     r = stop;
+                    last = r >= row_end;
                 }
+                said = said || last;
                 const RqSegment& sg = segs[seg];
                 // (where the stage's bytes are, before the waits: behind them it would be part of the chain)
                 const uint8_t* const main0 = sg.main[0] + lr0 * row_bytes;
@@ -1254,7 +1263,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                 if (st >= p.stages && !mbar_wait_warp(&empty_bar[slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 1); failed = true; break; }
                 uint8_t* dst = ring + (size_t)slot * p.stage_bytes;
                 if (leader)
-                    stage_info[slot] = make_int4(nr, seg, (int)lr0,
+                    stage_info[slot] = make_int4(nr, last ? seg | kLastStage : seg, (int)lr0,
                                                  TYPE != RQ_Q4_K ? (int)(scales0 & 15) : 0);
                 for (int k = 0; k < p.pieces; ++k) {
                     // at most `window` pieces in flight: wait for the one issued `window` pieces ago
@@ -1344,8 +1353,9 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
         {
             if (!direct) segs = table;  // the same entries, now in shared memory
             issue(0x7fffffff);
-            if (p.warp_rows && !failed) {
-                // the warp scheme's consumers read what each slot holds from stage_info: a stage of no rows ends their loop
+            if (p.warp_rows && !failed && !said) {
+                // the warp scheme's consumers read what each slot holds from stage_info: where no stage was the last one (the CTA has none), one of no rows ends
+                // their loop
                 if (st >= p.stages && !mbar_wait_warp(&empty_bar[slot], phase, p.wait_ns)) { atomicExch(p.error_flag, 1); failed = true; }
                 else {
                     if (leader) {
@@ -1628,7 +1638,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             while (true) {
                 bool there = mbar_wait(&full_bar[2 * slot], phase, p.wait_ns);
                 const int4 info = there ? stage_info[slot] : make_int4(0, 0, 0, 0);  // rows, segment, first local row
-                const RqSegment& sg = table[info.y];
+                const RqSegment& sg = table[info.y & ~kLastStage];
                 const uint8_t* stage = ring + (size_t)slot * p.stage_bytes;
                 const uint8_t* rec = act_smem + (owner ? sg.act[s] * (int)p.act_bytes + u * kRecord : 0);
                 ItemRegs<TYPE> wr[R];
@@ -1671,6 +1681,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                 for (int q = 0; q < subs; ++q) out = fmaf(__shfl_sync(0xffffffffu, mine, (from + q * group) & 31), sg.coef[q], out);
                 const int lr = row_in_pass + h * rows_per_pass;
                 if (in_row == 0 && h < R && row_in_warp < p.warp_rows && lr < info.x) sg.y[(int64_t)(info.z + lr) * p.yn] = out;
+                if (info.y & kLastStage) break;
             }
         } else if ((T <= 2 || MODE == RQ_ACT_INT8) && p.warp_rows) {
             // ---- the warp scheme: no partial sums in shared memory, no CTA-wide barrier. A row's items are
@@ -1708,7 +1719,9 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             // 83 calls 0.98, the slowest 1.015 (Q4_K 4096 x 4096 fp32 7.5 / 7.6).
             while (true) {
                 bool there = mbar_wait(&full_bar[2 * slot], phase, p.wait_ns);
-                const int4 info = there ? stage_info[slot] : make_int4(0, 0, 0, 0);  // rows, segment, first local row, offset of the first d
+                int4 info = there ? stage_info[slot] : make_int4(0, 0, 0, 0);  // rows, segment, first local row, offset of the first d
+                const bool last = (info.y & kLastStage) != 0;
+                info.y &= ~kLastStage;
                 const uint8_t* stage = ring + (size_t)slot * p.stage_bytes;
                 ItemRegs<TYPE> wr[R];
                 bool have[R];
@@ -1831,6 +1844,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
                     }
                     if (++cross_buf > kMaxStages) cross_buf = 0;
                 }
+                if (last) break;
             }
             if (gated) flush();
         } else if (R == 2) {
