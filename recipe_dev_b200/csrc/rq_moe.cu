@@ -276,7 +276,7 @@ __device__ __forceinline__ void route_token(const float* scores, int64_t se, int
     for (int e = tid; e < experts; e += kRouteThreads) weights[e * we + t * wt] = mark[e] ? __fdiv_rn(val[e], denom) : 0.0f;
 }
 
-// The kept experts of a token in ascending order with their weights, in shared memory (how many: -1, not known this way).
+// The kept experts of a token in ascending order with their weights, in shared memory.
 struct Picks { int count, expert[32]; float weight[32]; };
 
 // The common case by one warp: no selection bias (the key is the raw score), weights over the kept experts only, no NaN. Each lane holds PER scores as
@@ -338,18 +338,20 @@ __device__ __forceinline__ bool pick_by_warp(const float* scores, int64_t se, in
     if (tid < top) weights[picks->expert[tid] * we + t * wt] = picks->weight[tid];
     return true;
 }
-// Whether it was that case (the same answer to every thread).
-__device__ __forceinline__ bool route_by_warp(const float* scores, int64_t se, int64_t st, int experts, int top, int sigmoid, int renorm, const float* bias, float* weights,
-                                              int64_t we, int64_t wt, Picks* picks) {
-    if (bias || renorm == 0 || experts > 1024 || top > 32) return false;
-    return experts <= 256 ? pick_by_warp<8>(scores, se, st, experts, top, sigmoid != 0, weights, we, wt, picks) : pick_by_warp<32>(scores, se, st, experts, top, sigmoid != 0, weights, we, wt, picks);
+// Scores a lane holds where one warp may pick, or 0: not its case.
+__host__ __device__ __forceinline__ int scores_per_lane(int experts, int top, int renorm, const float* bias) {
+    return bias || renorm == 0 || experts > 1024 || top > 32 ? 0 : (experts <= 256 ? 8 : 32);
 }
 
+// One way a kernel, chosen by the host (and counting for the tokens with a NaN): with all of them in one the calls that count took 0.1 us longer.
+template <int PER>
 __global__ void __launch_bounds__(kRouteThreads) rq_route_kernel(const float* scores, int64_t se, int64_t st, int experts, int top,
                                                                 int sigmoid, int renorm, const float* __restrict__ bias,
                                                                 float* weights, int64_t we, int64_t wt) {
-    __shared__ Picks picks;
-    if (route_by_warp(scores, se, st, experts, top, sigmoid, renorm, bias, weights, we, wt, &picks)) return;
+    if constexpr (PER != 0) {
+        __shared__ Picks picks;
+        if (pick_by_warp<PER>(scores, se, st, experts, top, sigmoid != 0, weights, we, wt, &picks)) return;
+    }
     route_token(scores, se, st, experts, top, sigmoid, renorm, bias, weights, we, wt);
 }
 
@@ -486,7 +488,9 @@ __global__ void __launch_bounds__(256) rq_moe_route_plan_kernel(BankView b, cons
                                                                float* __restrict__ h, float* __restrict__ y, int64_t yn, int64_t yt) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the gate and up launch may take its places on the SMs (it waits for this one's end)
     __shared__ Picks picks;
-    if (route_by_warp(scores, se, sst, experts, top, sigmoid, renorm, bias, weights, we, wt, &picks)) {
+    // (All ways in one kernel here: one for each took 0.5 to 0.9 us longer, 256 experts, one token, 19.1 -> 20.1.)
+    const int per = scores_per_lane(experts, top, renorm, bias);
+    if (per && (per == 8 ? pick_by_warp<8>(scores, se, sst, experts, top, sigmoid != 0, weights, we, wt, &picks) : pick_by_warp<32>(scores, se, sst, experts, top, sigmoid != 0, weights, we, wt, &picks))) {
         plan_token(b, weights, we, wt, x, sk, st, top, include_shared, plans, h, y, yn, yt, &picks);
         return;
     }
@@ -679,13 +683,17 @@ extern "C" int rq_moe_route(rq_ctx* ctx, const float* scores, int64_t score_e_st
         static bool configured[64] = {};
         int dev = ctx->device;
         if (dev < 0 || dev >= 64 || !configured[dev]) {
-            RQ_CUDA(cudaFuncSetAttribute(rq_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 16));
+            RQ_CUDA(cudaFuncSetAttribute(rq_route_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 16));
             if (dev >= 0 && dev < 64) configured[dev] = true;
         }
     }
-    rq_route_kernel<<<tokens, kRouteThreads, (size_t)experts * 16, (cudaStream_t)stream>>>(scores, score_e_stride, score_t_stride, experts, top_k, scoring,
-                                                                                        renormalize, selection_bias, weights, weight_e_stride,
-                                                                                        weight_t_stride);
+    // Many picks among few experts, one after another, are the longer way: us, by one warp / by counting: top 13 of 32 experts 2.9 / 2.8, 16 of 32 3.1 / 2.8, 16 of 64 3.2 / 3.3,
+    // 32 of 64 4.5 / 3.4, 25 of 128 4.0 / 4.4, 32 of 128 4.5 / 4.4, 32 of 191 4.6 / 6.4. (Not so where a plan is written behind it, which takes the picks
+    // over: banks of 16 to 64 experts, top 8 to 15, 33 to 44 us by counting, 31 to 39 by one warp.)
+    const int per = top_k <= 8 + experts / 6 ? scores_per_lane(experts, top_k, renormalize, selection_bias) : 0;
+    auto kernel = per == 8 ? rq_route_kernel<8> : (per == 32 ? rq_route_kernel<32> : rq_route_kernel<0>);
+    kernel<<<tokens, kRouteThreads, (size_t)experts * 16, (cudaStream_t)stream>>>(scores, score_e_stride, score_t_stride, experts, top_k, scoring, renormalize, selection_bias,
+                                                                               weights, weight_e_stride, weight_t_stride);
     RQ_CUDA(cudaGetLastError());
     return RQ_OK;
 }

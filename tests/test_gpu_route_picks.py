@@ -62,3 +62,14 @@ def test_a_ranks_experts_take_their_slots(rq_ctx, oracle, first, count):
         one, weights = rq_ctx.moe_route_forward(bank, scores, x, top)
         assert torch.equal(weights, routing) and torch.equal(one, two)
     rq_ctx.check()
+
+
+@pytest.mark.parametrize("experts,top", [(8, 8), (16, 10), (16, 11), (32, 13), (32, 14), (32, 32), (64, 18), (64, 19), (128, 29), (128, 30), (143, 31), (143, 32), (144, 32)])
+@pytest.mark.parametrize("scoring", [0, 1])
+def test_bits_on_both_sides_of_the_rule(rq_ctx, oracle, experts, top, scoring):
+    """One warp picks up to 8 + experts / 6; beyond, every thread counts its expert's place."""
+    rng = np.random.default_rng(experts + top)
+    scores = rng.normal(size=(experts, 3)).astype(np.float32)
+    scores[:, 1] = np.float32(rng.integers(-2, 3, size=experts))  # ties
+    assert same(rq_ctx.moe_route(cuda(scores), top, scoring, True).cpu().numpy(), oracle.topk(scores, top, scoring, True))
+    rq_ctx.check()

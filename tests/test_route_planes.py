@@ -7,7 +7,7 @@ CSRC = Path(__file__).resolve().parent.parent / "recipe_dev_b200" / "csrc"
 
 def test_planes_that_may_be_one_are_not_declared_apart():
     text = (CSRC / "rq_moe.cu").read_text()
-    for name in ("route_token", "rq_route_kernel", "pick_by_warp", "route_by_warp", "rq_moe_route_plan_kernel"):
+    for name in ("route_token", "rq_route_kernel", "pick_by_warp", "rq_moe_route_plan_kernel"):
         parameters = re.search(name + r"\(([^)]*)\) \{", text).group(1)
         assert "float* scores" in parameters and "float* weights" in parameters, name
     # within one kernel the plan reads the weights that the routing wrote
