@@ -156,16 +156,18 @@ static const char* wait_code_text(int code) {
         case 3: return "matvec consumer: a stage never arrived";
         case 4: return "matvec producer: an earlier copy of its window never landed";
         case 11: return "batched product, staging warps: an operand slot never came free";
-        case 13: return "batched product, issuing thread: an operand was never staged";
+        case 13: return "batched product, issuing warp: an operand was never there (staged, or copied as it is stored)";
         case 14: return "batched product, drain warps: a sum was never finished";
-        case 15: return "batched product, issuing thread: an accumulator never came free";
+        case 15: return "batched product, issuing warp: an accumulator never came free";
         case 16: return "batched product, activation copies: a slot never came free";
-        case 17: return "batched product, issuing thread: a slice of the activations never arrived";
+        case 17: return "batched product, issuing warp: a slice of the activations never arrived";
         case 18: return "batched product, staging warps: the stored bytes never arrived";
         case 19: return "batched product, copies of stored bytes: a slot never came free";
         case 20: return "batched product, drain warps: the activations' steps never arrived";
         case 23: return "batched product, issuing warps: the products never completed";
         case 24: return "batched product, copies: some never landed";
+        case 25: return "batched product, copies of steps and stored scales: a slot never came free";
+        case 26: return "batched product, drain warps: a unit's steps or stored scales never arrived";
         case 22: return "matvec over a decode-only format: a row's bytes never arrived";
         case 21: return "wait self-test: the barrier nothing arrives on";
         case 31: return "exchange: a peer's arrival flag never came";

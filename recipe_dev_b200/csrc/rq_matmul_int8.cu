@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(con
             };
 #pragma unroll 1
             for (int u = u0; u < u1; ++u, scale_at.next()) {
-                if (!mbar_wait_warp(&scales_full[scale_at.slot], scale_at.phase, p.wait_ns, dead)) atomicExch(p.error_flag, 20);
+                if (!mbar_wait_warp(&scales_full[scale_at.slot], scale_at.phase, p.wait_ns, dead)) atomicExch(p.error_flag, 26);
                 const uint8_t* const mine = scales + scale_at.slot * kScaleSlot;
                 const float* const steps = (const float*)mine + col0;
                 const uint32_t* const d = (const uint32_t*)(mine + 8 * kTokens * 4) + 4 * r0;
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(con
                         ++n;
                     }
                     if (dead) break;
-                    if (units >= R::scale_slots && !mbar_wait_warp(&scales_free[scale_at.slot], scale_at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 16); break; }
+                    if (units >= R::scale_slots && !mbar_wait_warp(&scales_free[scale_at.slot], scale_at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 25); break; }
                     if (leader) {
                         mbar_expect_tx(&scales_full[scale_at.slot], 8 * kTokens * 4);
                         bulk_g2s(scales + scale_at.slot * kScaleSlot, p.steps + (first + u) * (8 * kTokens), 8 * kTokens * 4, &scales_full[scale_at.slot]);
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(con
             while (!dead && walk.next(tile, u0, u1)) {
                 const int64_t row0 = (int64_t)(tile % p.tiles_m) * 256 + lane;
                 for (int u = u0; u < u1; ++u, ++n, at.next()) {
-                    if (n >= R::scale_slots && !mbar_wait_warp(&scales_free[at.slot], at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 19); break; }
+                    if (n >= R::scale_slots && !mbar_wait_warp(&scales_free[at.slot], at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 25); break; }
                     uint4* const to = (uint4*)(scales + at.slot * kScaleSlot + 8 * kTokens * 4) + lane;
 #pragma unroll 1
                     for (int i = 0; i < 256; i += 32) {
