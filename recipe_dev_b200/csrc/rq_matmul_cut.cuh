@@ -19,7 +19,10 @@ template <int MH, bool CODES> struct Shape;
 template <> struct Shape<1, false> { static constexpr int drain_warps = 8, groups = 4, cols = 64, drain_regs = 120, stage_regs = 56, other_regs = 40, launch_regs = 72; };
 template <> struct Shape<2, false> { static constexpr int drain_warps = 8, groups = 2, cols = 128, drain_regs = 168, stage_regs = 56, other_regs = 32, launch_regs = 96; };
 template <> struct Shape<1, true> { static constexpr int drain_warps = 8, groups = 4, cols = 64, drain_regs = 128, stage_regs = 48, other_regs = 40, launch_regs = 72; };
-constexpr int kInt8Tokens = 64;              // tokens of a tile of codes with two row halves
+// The kernel of int8 activations over Q8_0 / Q4_0 beyond that (rq_matmul_int8.cu): a tile is 128 * 2 rows x kInt8Tokens, a drain thread has two rows of a
+// quarter of the tokens; accumulators are stages of a 64-wide slice (two groups x two row halves).
+constexpr int kInt8Tokens = 64, kInt8DrainWarps = 16, kInt8Stages = 2, kInt8AccColumns = kInt8Stages * 2 * 2 * kInt8Tokens;
+static_assert(kInt8AccColumns == 512, "all of tensor memory, and no more");
 
 template <int TYPE> struct Format {
     static constexpr bool kquant = TYPE == RQ_Q4_K || TYPE == RQ_Q6_K;
@@ -31,12 +34,14 @@ template <int TYPE> struct Format {
     static constexpr int a_cols = residual ? 64 : 32;            // tensor-memory columns of an operand slot
 };
 
-// The rings of the kernel of int8 activations over Q8_0 / Q4_0 and more than 64 tokens (rq_matmul_int8.cu; of a TcCut it takes the tiles, the deal and the
-// scratch), in half units of 256 rows x 64 tokens: activations, operands (Q8_0: the stored bytes as they land), Q4_0's stored bytes (slots of a unit of 128
-// rows), the steps and stored scales of a unit; behind them the totals, and room to align.
+// The kernel of bytes' shared memory (of a TcCut it takes the tiles, the deal and the scratch), in half units: activations, operands of both row halves (Q8_0: the stored bytes as
+// they land), Q4_0's stored bytes (slots of a unit of 128 rows), the steps and the stored scales of a unit; behind them the drain threads' totals, and room to align.
 template <int TYPE> struct Int8Rings {
     static constexpr int b_slots = TYPE == RQ_Q8_0 ? 4 : 3, a_slots = TYPE == RQ_Q8_0 ? 3 : 2, raw_slots = TYPE == RQ_Q8_0 ? 0 : 3, scale_slots = 3;
-    static constexpr size_t bytes = b_slots * 8192 + a_slots * 32768 + raw_slots * 16384 + scale_slots * 6144 + 65536 + 1024;
+    static constexpr int b_bytes = kInt8Tokens * 128, half_bytes = 128 * 128, step_bytes = 8 * kInt8Tokens * 4, scale_bytes = step_bytes + 256 * 16;
+    static constexpr int totals_bytes = 32 * kInt8DrainWarps * 2 * (kInt8Tokens / 4) * 4;
+    static constexpr size_t bytes = b_slots * b_bytes + a_slots * 2 * half_bytes + raw_slots * half_bytes + scale_slots * scale_bytes + totals_bytes + 1024;
+    static_assert(bytes + 512 <= 227 * 1024, "the barriers want room too");
 };
 
 // The slices of a segment (units u0 .. u1 - 1 of a tile) in the order every role takes them: four a unit and, over Q4_K, behind the last unit of every
@@ -175,6 +180,16 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     c.image_tiles = codes && c.mh == 2 ? 2 * c.units : 4 * c.units + c.windows;  // (of 64 inputs a row; codes of two row halves: bytes, of 128)
     const TileShare sh = share_out((int64_t)c.tiles_m * c.n_tiles, c.units, sm_count);
     c.ctas = sh.ctas; c.whole = sh.whole; c.rest_tiles = sh.rest_tiles; c.share = sh.share;
+    const int b_bytes = c.bn * (codes ? 128 : 256);
+    c.records_bytes = codes ? (rq_act_token_bytes(cols) * (size_t)tokens + 255) & ~(size_t)255 : 0;
+    c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
+    c.steps_bytes = codes ? (size_t)c.n_tiles * c.units * 8 * c.bn * 4 : 0;
+    c.partial_bytes = (size_t)2 * c.share * c.bn * 128 * c.mh * 4;
+    if (codes && c.mh == 2) {  // rq_matmul_int8.cu: its rings are known beforehand
+        c.raw_slots = c.b_slots = c.a_slots = c.accs = 0;
+        c.smem = type == RQ_Q8_0 ? Int8Rings<RQ_Q8_0>::bytes : Int8Rings<RQ_Q4_0>::bytes;
+        return c;
+    }
     // A parity wait says no more than odd or even, so whoever waits on a slot must have seen its previous use: MH = 1, the issuing warps
     // take alternate activation slots, and Q8_0's staging groups every second tile of stored bytes; MH = 2, a staging group every second
     // tile: even numbers of each. (The steps' own barriers are indexed by the step.)
@@ -185,20 +200,15 @@ inline TcCut tc_cut(int type, bool codes, int sm_count, int64_t rows, int64_t co
     int steps = (512 - c.a_slots * f.a_cols - totals) / step_cols;
     if (steps > kMaxAcc / halves) steps = kMaxAcc / halves;
     c.accs = steps * halves;
-    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window; codes, MH = 2: room as large as the sums,
-    // of which the kernel of bytes makes rings of its own, Int8Rings)
-    const int kept = (c.mh == 1 ? c.bn * 128 * 4 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0) + (codes && c.mh == 2 ? c.bn * 256 * 4 : 0), budget = (codes ? 212 : 220) * 1024 - kept, b_bytes = c.bn * (codes ? 128 : 256);
-    c.b_slots = c.mh == 1 || codes ? 4 : 3;
+    // shared memory: activation slots, then as many slots of stored bytes as fit (MH = 1: and the odd slices' sums; Q4_K: and the headers of a window)
+    const int kept = (c.mh == 1 ? c.bn * 128 * 4 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0), budget = (codes ? 212 : 220) * 1024 - kept;
+    c.b_slots = c.mh == 1 ? 4 : 3;
     c.raw_slots = (budget - c.b_slots * b_bytes) / f.raw_bytes;
     const int raw_max = c.mh * 2 * f.raw_per_unit < kMaxRaw ? 6 : kMaxRaw, raw_grain = c.mh == 2 || f.raw_per_unit == 2 ? 2 : 1;
     c.raw_slots = (c.raw_slots < raw_max ? c.raw_slots : raw_max) / raw_grain * raw_grain;
-    const int b_max = c.mh == 1 ? kMaxB : (codes ? 4 : 6), b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
+    const int b_max = c.mh == 1 ? kMaxB : 6, b_more = c.mh == 1 ? 2 : 1;  // a slot is refilled over one trip to L2, some 1500 cycles, a few slices' worth of time
     while (c.b_slots + b_more <= b_max && (c.b_slots + b_more) * b_bytes + c.raw_slots * f.raw_bytes <= budget) c.b_slots += b_more;
     c.smem = (size_t)c.b_slots * b_bytes + (size_t)c.raw_slots * f.raw_bytes + kept + 1024;
-    c.records_bytes = codes ? (rq_act_token_bytes(cols) * (size_t)tokens + 255) & ~(size_t)255 : 0;
-    c.xs_bytes = (size_t)c.n_tiles * c.image_tiles * b_bytes;
-    c.steps_bytes = codes ? (size_t)c.n_tiles * c.units * 8 * c.bn * 4 : 0;
-    c.partial_bytes = (size_t)2 * c.share * c.bn * 128 * c.mh * 4;
     return c;
 }
 // Work area of a call: the records (where INT8_CACHED calls look for them), the image, its steps, the shared tiles' sums and a counter

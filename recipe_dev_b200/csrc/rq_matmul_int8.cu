@@ -39,7 +39,7 @@ using namespace rqcut;
 namespace {
 
 constexpr int kTokens = kInt8Tokens, kTile = 128 * 128;  // tokens of a tile; bytes of 128 rows x 128 inputs
-constexpr int kDrainWarps = 16, kStages = 2, kScaleSlot = 8 * kTokens * 4 + 256 * 16;
+constexpr int kDrainWarps = kInt8DrainWarps, kStages = kInt8Stages;
 template <int TYPE> __host__ __device__ constexpr int staging_warps() { return TYPE == RQ_Q4_0 ? 4 : 0; }
 template <int TYPE> __host__ __device__ constexpr int int8_threads() { return (kDrainWarps + staging_warps<TYPE>() + 4) * 32; }
 template <int TYPE> struct Regs;  // (of the launch: 384 x 168 and 512 x 128)
@@ -83,7 +83,8 @@ template <int TYPE>
 __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(const __grid_constant__ RqInt8Params p) {
     using R = Int8Rings<TYPE>;
     constexpr bool kStaged = TYPE == RQ_Q4_0;
-    constexpr int kRaw = kStaged ? R::raw_slots : 1;
+    constexpr int kRaw = kStaged ? R::raw_slots : 1, kScaleSlot = R::scale_bytes;
+    static_assert(R::half_bytes == kTile && R::b_bytes == kTokens * 128, "the rings' slots are what the copies fill");
     constexpr int kStaging = staging_warps<TYPE>(), kMiscFirst = kDrainWarps + kStaging;
     static_assert(32 * kDrainWarps * Regs<TYPE>::drain + 32 * (kStaging + 4) * Regs<TYPE>::other <= int8_threads<TYPE>() * (65536 / int8_threads<TYPE>() / 8 * 8), "more registers than the launch has: the increase would wait forever");
     extern __shared__ uint8_t smem_raw[];
@@ -187,7 +188,7 @@ __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(con
                 if (!mbar_wait_warp(&scales_full[scale_at.slot], scale_at.phase, p.wait_ns, dead)) atomicExch(p.error_flag, 26);
                 const uint8_t* const mine = scales + scale_at.slot * kScaleSlot;
                 const float* const steps = (const float*)mine + col0;
-                const uint32_t* const d = (const uint32_t*)(mine + 8 * kTokens * 4) + 4 * r0;
+                const uint32_t* const d = (const uint32_t*)(mine + R::step_bytes) + 4 * r0;
 #pragma unroll 1
                 for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -420,8 +421,8 @@ __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(con
                     if (dead) break;
                     if (units >= R::scale_slots && !mbar_wait_warp(&scales_free[scale_at.slot], scale_at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 25); break; }
                     if (leader) {
-                        mbar_expect_tx(&scales_full[scale_at.slot], 8 * kTokens * 4);
-                        bulk_g2s(scales + scale_at.slot * kScaleSlot, p.steps + (first + u) * (8 * kTokens), 8 * kTokens * 4, &scales_full[scale_at.slot]);
+                        mbar_expect_tx(&scales_full[scale_at.slot], R::step_bytes);
+                        bulk_g2s(scales + scale_at.slot * kScaleSlot, p.steps + (first + u) * (8 * kTokens), R::step_bytes, &scales_full[scale_at.slot]);
                     }
                     scale_at.next();
                     ++units;
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(con
                 const int64_t row0 = (int64_t)(tile % p.tiles_m) * 256 + lane;
                 for (int u = u0; u < u1; ++u, ++n, at.next()) {
                     if (n >= R::scale_slots && !mbar_wait_warp(&scales_free[at.slot], at.phase ^ 1, p.wait_ns, dead)) { atomicExch(p.error_flag, 25); break; }
-                    uint4* const to = (uint4*)(scales + at.slot * kScaleSlot + 8 * kTokens * 4) + lane;
+                    uint4* const to = (uint4*)(scales + at.slot * kScaleSlot + R::step_bytes) + lane;
 #pragma unroll 1
                     for (int i = 0; i < 256; i += 32) {
                         const uint16_t* from = p.scale + min(row0 + i, p.rows - 1) * p.blocks32 + 8 * u;  // (kept inside the weight)

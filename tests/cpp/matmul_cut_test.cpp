@@ -16,22 +16,33 @@ static int walk_call(int type, bool codes, int sms, int64_t rows, int64_t cols, 
     const TcCut c = tc_cut(type, codes, sms, rows, cols, tokens);
     const int64_t tiles = (int64_t)c.tiles_m * c.n_tiles;
     if (c.tiles_m * 128LL * c.mh < rows || (int64_t)c.n_tiles * c.bn < tokens) return fail("outputs outside every tile", type, codes, sms, rows, cols, tokens);
-    // tensor memory, 512 columns: accumulators of at least two steps, (codes, one row half) two sets of totals, operand slots, found by a mask
     const bool k = type == RQ_Q4_K || type == RQ_Q6_K;
-    const int acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn, totals = codes && c.mh == 1 ? 2 * c.bn : 0;
-    if (c.accs * acc_cols + totals + c.a_slots * format_sizes(type).a_cols > 512 || c.accs < (k ? 2 : 4) || c.accs > kMaxAcc || c.accs % (k ? 1 : 2) || c.a_slots < 2 || c.a_slots > kMaxA ||
-        (c.a_slots & (c.a_slots - 1)))
-        return fail("tensor memory", type, codes, sms, rows, cols, tokens);
-    // rings whose slots keep their waiters, and nobody as many steps ahead as there are step barriers (32)
-    const bool even_raw = c.mh == 2 || type == RQ_Q8_0;
-    if (c.b_slots < 2 || c.b_slots > kMaxB || (c.mh == 1 && c.b_slots % 2) || c.raw_slots < 2 || c.raw_slots > kMaxRaw || (even_raw && c.raw_slots % 2) || c.b_slots * c.mh * (k ? 1 : 2) >= 32)
-        return fail("rings", type, codes, sms, rows, cols, tokens);
-    // shared memory: the rings, what the drain and staging warps keep behind them, and room to align
-    const size_t b_bytes = (size_t)c.bn * (codes ? 128 : 256), kept = (c.mh == 1 ? c.bn * 512 : (codes ? c.bn * 1024 : 0)) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0);
-    if (c.b_slots * b_bytes + (size_t)c.raw_slots * format_sizes(type).raw_bytes + kept + 1024 > c.smem || c.smem > (size_t)(codes ? 218 : 225) * 1024)
-        return fail("shared memory", type, codes, sms, rows, cols, tokens);
+    if (codes && c.mh == 2) {
+        // the kernel of bytes: its own rings (how they fit is asserted where they are laid out), and every part of its shared memory in them
+        const bool q8 = type == RQ_Q8_0;
+        const int b = q8 ? 4 : 3, a = q8 ? 3 : 2, raw = q8 ? 0 : 3, scales = 3;
+        const size_t parts = (size_t)b * (64 * 128) + (size_t)a * (256 * 128) + (size_t)raw * (128 * 128) + (size_t)scales * (8 * 64 * 4 + 256 * 16) + 256 * 64 * 4;
+        if (c.smem != parts + 1024 || c.smem > 220 * 1024) return fail("shared memory of the kernel of bytes", type, codes, sms, rows, cols, tokens);
+        if (c.accs || c.a_slots || c.b_slots || c.raw_slots) return fail("rings that nobody reads", type, codes, sms, rows, cols, tokens);
+        if (c.xs_bytes != (size_t)c.n_tiles * c.units * 2 * (64 * 128) || c.steps_bytes != (size_t)c.n_tiles * c.units * 8 * 64 * 4 || c.partial_bytes != (size_t)2 * c.share * 64 * 256 * 4)
+            return fail("scratch of the kernel of bytes", type, codes, sms, rows, cols, tokens);
+    } else {
+        // tensor memory, 512 columns: accumulators of at least two steps, (codes, one row half) two sets of totals, operand slots, found by a mask
+        const int acc_cols = c.mh == 1 && !codes ? 2 * c.bn : c.bn, totals = codes ? 2 * c.bn : 0;
+        if (c.accs * acc_cols + totals + c.a_slots * format_sizes(type).a_cols > 512 || c.accs < (k ? 2 : 4) || c.accs > kMaxAcc || c.accs % (k ? 1 : 2) || c.a_slots < 2 || c.a_slots > kMaxA ||
+            (c.a_slots & (c.a_slots - 1)))
+            return fail("tensor memory", type, codes, sms, rows, cols, tokens);
+        // rings whose slots keep their waiters, and nobody as many steps ahead as there are step barriers (32)
+        const bool even_raw = c.mh == 2 || type == RQ_Q8_0;
+        if (c.b_slots < 2 || c.b_slots > kMaxB || (c.mh == 1 && c.b_slots % 2) || c.raw_slots < 2 || c.raw_slots > kMaxRaw || (even_raw && c.raw_slots % 2) || c.b_slots * c.mh * (k ? 1 : 2) >= 32)
+            return fail("rings", type, codes, sms, rows, cols, tokens);
+        // shared memory: the rings, what the drain and staging warps keep behind them, and room to align
+        const size_t b_bytes = (size_t)c.bn * (codes ? 128 : 256), kept = (c.mh == 1 ? c.bn * 512 : 0) + (type == RQ_Q4_K ? kStashBytes * c.mh : 0);
+        if (c.b_slots * b_bytes + (size_t)c.raw_slots * format_sizes(type).raw_bytes + kept + 1024 > c.smem || c.smem > (size_t)(codes ? 218 : 225) * 1024)
+            return fail("shared memory", type, codes, sms, rows, cols, tokens);
+    }
     // token tiles of a width that the drain loops are instantiated for
-    const bool width = c.mh == 1 ? c.bn == 16 || c.bn == 32 || c.bn == 48 || c.bn == 64 : (codes ? c.bn == 64 : c.bn == 64 || c.bn == 96 || (k && c.bn == 128));
+    const bool width = c.mh == 1 ? c.bn == 16 || c.bn == 32 || c.bn == 48 || c.bn == 64 : (codes ? c.bn == kInt8Tokens : c.bn == 64 || c.bn == 96 || (k && c.bn == 128));
     if (!width) return fail("a tile of another width", type, codes, sms, rows, cols, tokens);
     std::vector<int> next_unit(tiles, 0), arrivals(c.rest_tiles, 0), summed(c.rest_tiles, 0);
     std::vector<char> place_used((size_t)2 * c.share, 0);
