@@ -42,7 +42,7 @@ constexpr int kTokens = kInt8Tokens, kTile = 128 * 128;  // tokens of a tile; by
 constexpr int kDrainWarps = kInt8DrainWarps, kStages = kInt8Stages;
 template <int TYPE> __host__ __device__ constexpr int staging_warps() { return TYPE == RQ_Q4_0 ? 4 : 0; }
 template <int TYPE> __host__ __device__ constexpr int int8_threads() { return (kDrainWarps + staging_warps<TYPE>() + 4) * 32; }
-template <int TYPE> struct Regs;  // (of the launch: 384 x 168 and 512 x 128)
+template <int TYPE> struct Regs;  // of the launch's 640 x 96 and 768 x 80 (the kernels spill 68 and 166 bytes a thread)
 template <> struct Regs<RQ_Q8_0> { static constexpr int drain = 112, other = 32; };
 template <> struct Regs<RQ_Q4_0> { static constexpr int drain = 96, other = 40; };
 
@@ -56,8 +56,8 @@ __device__ __forceinline__ void mma_i8_ss(uint32_t tmem_d, uint64_t adesc, uint6
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(0u)
         : "memory");
 }
-// Sixteen columns at two places of this warp's 32 lanes, asked for; they are there behind tmem_landed (which has them as operands so
-// that nothing that uses them moves ahead of it).
+// Sixteen columns of this warp's 32 lanes, asked for; two such are there behind tmem_landed (which has them as operands so that nothing that uses
+// them moves ahead of it).
 __device__ __forceinline__ void tmem_ask(uint32_t a, uint32_t (&v)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
@@ -70,14 +70,6 @@ __device__ __forceinline__ void tmem_landed(uint32_t (&u)[16], uint32_t (&v)[16]
                    "+r"(u[13]), "+r"(u[14]), "+r"(u[15]), "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]),
                    "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]));
 }
-
-// A ring position: slot index and the parity of its current use.
-struct Ring {
-    int slot, n;
-    uint32_t phase;
-    __device__ __forceinline__ explicit Ring(int n_) : slot(0), n(n_), phase(0) {}
-    __device__ __forceinline__ void next() { if (++slot == n) { slot = 0; phase ^= 1; } }
-};
 
 template <int TYPE>
 __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(const __grid_constant__ RqInt8Params p) {
@@ -195,38 +187,41 @@ __global__ void __launch_bounds__(int8_threads<TYPE>(), 1) rq_tc_int8_kernel(con
                     for (int sl = 0; sl < 2; ++sl) {
                         static_assert(kStages == 2, "a half unit's slices take the stages in turn");
                         const uint32_t w[2] = {d[2 * h + sl], d[512 + 2 * h + sl]};
-                        // sixteen columns of both rows at a time, the next ones and their steps on their way meanwhile
+                        // a group's sixteen columns of both rows at a time; the first group's steps are asked for before the wait
                         constexpr int kItems = 2 * kMine / 16;
                         const uint32_t acc = acc0 + (uint32_t)(sl * 256);
                         const float* const st = steps + (4 * h + 2 * sl) * kTokens;
-                        uint32_t v[1][2][16];
-                        float4 s4[1][4];
-                        auto ask = [&](int i) {
-                            const uint32_t at = acc + (uint32_t)(i * 128);
-                            tmem_ask(at, v[0][0]);
-                            tmem_ask(at + kTokens, v[0][1]);
-                        };
+                        uint32_t v[2][16];
+                        float4 s4[4];
                         auto steps_of = [&](int i) {
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) s4[0][k] = *(const float4*)(st + i * kTokens + 4 * k);
+                            for (int k = 0; k < 4; ++k) s4[k] = *(const float4*)(st + i * kTokens + 4 * k);
                         };
                         steps_of(0);
                         if (!mbar_wait_warp(&done[sl], phase, p.wait_ns, dead)) atomicExch(p.error_flag, 14);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                         for (int i = 0; i < kItems; ++i) {
-                            ask(i); if (i) steps_of(i); tmem_landed(v[0][0], v[0][1]); if (i + 1 == kItems) { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); __syncwarp(); if (lane == 0) mbar_arrive(&drained[sl]); }
+                            tmem_ask(acc + (uint32_t)(i * 128), v[0]);
+                            tmem_ask(acc + (uint32_t)(i * 128) + kTokens, v[1]);
+                            if (i) steps_of(i);
+                            tmem_landed(v[0], v[1]);
+                            if (i + 1 == kItems) {  // the slice is in registers: its stage may be filled again
+                                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive(&drained[sl]);
+                            }
                             const float k = kStaged ? 0.0625f : 1.0f, d0 = k * rq_h2f((uint16_t)(w[0] >> (16 * i))), d1 = k * rq_h2f((uint16_t)(w[1] >> (16 * i)));
                             const Pair scale[2] = {pair_of(d0, d0), pair_of(d1, d1)};
 #pragma unroll
                             for (int j = 0; j < 16; j += 4) {
-                                const float4 sj = s4[0][j / 4];
+                                const float4 sj = s4[j / 4];
                                 const Pair sv[2] = {pair_of(sj.x, sj.y), pair_of(sj.z, sj.w)};
 #pragma unroll
                                 for (int m = 0; m < 2; ++m)
 #pragma unroll
                                     for (int q = 0; q < 2; ++q) {
-                                        const uint32_t* t = v[0][m] + j + 2 * q;
+                                        const uint32_t* t = v[m] + j + 2 * q;
                                         Pair& to = sum[m][j / 2 + q];
                                         to = pair_fma(pair_mul(sv[q], scale[m]), pair_of((float)(int)t[0], (float)(int)t[1]), to);
                                     }

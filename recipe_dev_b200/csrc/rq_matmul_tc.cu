@@ -376,16 +376,6 @@ __device__ __forceinline__ void tmem_ld16_pair(uint32_t a, uint32_t b, uint32_t 
 template <int N> struct Columns { static constexpr int value = N; };
 template <Image I> struct ImageOf { static constexpr Image value = I; };
 
-// A ring position: slot index and the parity of its current use. (Kept by counting: a division by a ring's length, known at run time
-// only, is some thirty instructions.)
-struct Ring {
-    int slot, n;
-    uint32_t phase;
-    __device__ __forceinline__ explicit Ring(int n_, int first = 0) : slot(0), n(n_), phase(0) { skip(first); }
-    __device__ __forceinline__ void next() { if (++slot == n) { slot = 0; phase ^= 1; } }
-    __device__ __forceinline__ void skip(int by) { for (slot += by; slot >= n;) { slot -= n; phase ^= 1; } }
-};
-
 template <int TYPE, int MH, bool CODES>
 __global__ void __launch_bounds__(tc_threads<MH, CODES>(), 1) rq_tc_kernel(const __grid_constant__ TcParams p) {
     using F = Format<TYPE>;

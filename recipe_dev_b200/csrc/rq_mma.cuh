@@ -45,6 +45,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
     else return true;
     return !dead;
 }
+// A ring position: slot index and the parity of its current use. (Kept by counting: a division by a ring's length, known at run time
+// only, is some thirty instructions.)
+struct Ring {
+    int slot, n;
+    uint32_t phase;
+    __device__ __forceinline__ explicit Ring(int n_, int first = 0) : slot(0), n(n_), phase(0) { skip(first); }
+    __device__ __forceinline__ void next() { if (++slot == n) { slot = 0; phase ^= 1; } }
+    __device__ __forceinline__ void skip(int by) { for (slot += by; slot >= n;) { slot -= n; phase ^= 1; } }
+};
 // True in one lane of a converged warp. The compiler knows that the code behind it runs in a single thread, so the operands of the
 // instructions that take uniform registers (tcgen05.mma, commits, copies) stay there.
 __device__ __forceinline__ bool elect_one() {

@@ -51,3 +51,17 @@ def test_the_batched_product_ends_with_nothing_under_way():
     assert issuing.index("mma_commit(&ended[me]);") < issuing.index("mbar_wait_warp(&ended[me], 0,")
     assert "landed(b_full, p.b_slots, images);" in activations and "landed(steps_full, kStepSlots, ks_all);" in activations
     assert "landed(raw_full, p.raw_slots, n);" in stored
+
+
+def test_the_product_of_bytes_ends_with_nothing_under_way():
+    """The same of the kernel of 8-bit products: its copies by barriers, the stored scales' also where they go by cp.async."""
+    text = (CSRC / "rq_matmul_int8.cu").read_text()
+    misc = text.split("auto landed = [&]")[1].split("free the tensor memory")[0]
+    issuing, rest = misc.split("- activation copies")
+    activations, rest = rest.split("- stored bytes:")
+    stored, scales = rest.split("- the stored scales:")
+    assert issuing.index("mma_commit(&ended);") < issuing.index("mbar_wait_warp(&ended, 0,")
+    assert "landed(b_full, R::b_slots, n);" in activations and "landed(scales_full, R::scale_slots, units);" in activations
+    assert "landed(full, kSlots, n);" in stored and "cp.async.wait_all;" in scales
+    # every copy's barrier is one of those
+    assert activations.count("bulk_g2s(") == 2 and stored.count("tma_load_2d(") == 1 and text.count("bulk_g2s(") == 2 and text.count("tma_load_2d(") == 1
