@@ -1148,10 +1148,10 @@ constexpr int kLastStage = 1 << 30;
 
 // R = rows a thread takes per stage in the warp scheme (its weight registers): 2 only where the launch uses two. GATED: the two are
 // the gate row and the up row of one virtual row. BANKED: a virtual row is an expert bank's down rows, one of each slot.
-// ONE (fp32 activations): a slice of sixteen inputs a thread is enough; a straight line takes half a microsecond less than a loop with the next round's loads
-// under way (8000 x 2048: Q4_K 5.98 -> 5.47 us, Q6_K 7.35 -> 6.84, Q8_0 7.86 -> 7.33; 256 experts, one token 22.5 -> 21.6). Side by side in one kernel the loop's
-// launches were slower for it (a decode layer of 4096 inputs 66.3 -> 67.2); up to 4096 inputs with the producer's threads too was (4096 x 4096 7.7 -> 8.7), and two
-// slices side by side in each round (900 x 10240 11.4 -> 13.9).
+// ONE (fp32 activations, launches of two rows a thread and of banks): a slice of sixteen inputs a thread is enough, so there is no loop (256 experts, one token 22.5 -> 21.6 us). Up to 4096 inputs with the
+// producer's threads too was slower (4096 x 4096 7.7 -> 8.7), and so were two slices side by side in each round (900 x 10240 11.4 -> 13.9). The launches of a row a thread, partial
+// sums among them, keep to the loop: a layer of 2560 inputs runs several of them on both sides of what a slice a thread holds, and two kernels that each fill the instruction cache took more
+// than the straight line gave (2560 inputs, 10240 in the feed-forward, us, a loop that fetched once too often / two kernels / this: Q6_K 62.0 / 65.0 / 60.5, Q4_0 60.4 / 62.1 / 58.5).
 template <int TYPE, int MODE, int T, int NW, int R, bool GATED, bool BANKED, bool ONE>
 __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW <= 7 ? 2 : 1)) rq_gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr int kConsumers = NW * 32;
@@ -1456,11 +1456,14 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             fetch(tid, v, s2, cur);
             if constexpr (ONE) odd = digits_to_smem(cur, act_smem + v * p.act_bytes + (size_t)(s2 >> 4) * kRecord, s2 & 15, tid < total, v < used);
 #pragma unroll 1
-            for (int base_i = 0; !ONE && base_i < total; base_i += kConsumers) {  // uniform: the two threads of a group exchange by shuffles
+            for (int base_i = 0; !ONE; base_i += kConsumers) {  // uniform: the two threads of a group exchange by shuffles
+                // (behind the last round nothing is fetched or handed on: with it, fp32 Q4_0 4096 x 4096 took 7.7 us instead of 7.0)
+                const bool more = base_i + kConsumers < total;
                 int nv = v + adv_v, ns = s2 + adv_s;
                 if (ns >= per_vec) { ns -= per_vec; ++nv; }
-                fetch(base_i + kConsumers + tid, nv, ns, nxt);
+                if (more) fetch(base_i + kConsumers + tid, nv, ns, nxt);
                 odd |= digits_to_smem(cur, act_smem + v * p.act_bytes + (size_t)(s2 >> 4) * kRecord, s2 & 15, base_i + tid < total, v < used);
+                if (!more) break;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) cur[j] = nxt[j];
                 v = nv; s2 = ns;
@@ -1970,7 +1973,7 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
 
 template <int TYPE, int MODE, int T, int NW, int R, bool GATED = false, bool BANKED = false, bool ONE = false>
 int launch_stream(const StreamParams& p, int grid_x, size_t smem, cudaStream_t s) {
-    if constexpr (MODE == RQ_ACT_FLOAT && T == 1 && NW == 7 && !ONE) {
+    if constexpr (MODE == RQ_ACT_FLOAT && T == 1 && NW == 7 && !ONE && (R == 2 || BANKED)) {
         if (p.act_vectors * (p.cols >> 4) <= NW * 32) return launch_stream<TYPE, MODE, T, NW, R, GATED, BANKED, true>(p, grid_x, smem, s);
     }
     auto kernel = rq_gemv_stream_kernel<TYPE, MODE, T, NW, R, GATED, BANKED, ONE>;
