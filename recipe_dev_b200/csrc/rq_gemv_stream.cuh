@@ -50,7 +50,7 @@ struct StreamParams {
     int bank_group;            // > 0: the warp scheme of an expert bank's down rows -- a sub-row's units are this many lanes (a power of two), a virtual row p.subs times
                                // as many, side by side in each half of a warp (first and second halves of the units); warp_rows virtual rows a pass. -1 before the
                                // launch is laid out: meant for that scheme, or for nobody
-                               // (In the hole behind three ints: eight bytes more of parameters cost every launch 0.2 us of the host's time.)
+                               // (In the hole behind three ints: with 1896 bytes of parameters eager calls of one shape took 0.2 us longer than with 1888; with 544 they took no less.)
     int64_t rows;              // virtual rows of all segments
     int64_t rows_quot; int rows_rem;  // rows / CTAs and rows % CTAs (launches whose row count the host knows): CTA b takes
                                // rows_quot rows from b * rows_quot + min(b, rows_rem), one more when b < rows_rem
@@ -1148,10 +1148,11 @@ constexpr int kLastStage = 1 << 30;
 
 // R = rows a thread takes per stage in the warp scheme (its weight registers): 2 only where the launch uses two. GATED: the two are
 // the gate row and the up row of one virtual row. BANKED: a virtual row is an expert bank's down rows, one of each slot.
-// ONE (fp32 activations, launches of two rows a thread and of banks): a slice of sixteen inputs a thread is enough, so there is no loop (256 experts, one token 22.5 -> 21.6 us). Up to 4096 inputs with the
-// producer's threads too was slower (4096 x 4096 7.7 -> 8.7), and so were two slices side by side in each round (900 x 10240 11.4 -> 13.9). The launches of a row a thread, partial
-// sums among them, keep to the loop: a layer of 2560 inputs runs several of them on both sides of what a slice a thread holds, and two kernels that each fill the instruction cache took more
-// than the straight line gave (2560 inputs, 10240 in the feed-forward, us, a loop that fetched once too often / two kernels / this: Q6_K 62.0 / 65.0 / 60.5, Q4_0 60.4 / 62.1 / 58.5).
+// ONE (fp32 activations, launches of two rows a thread and of banks): a slice of sixteen inputs a thread is enough, so there is no loop over rounds (256 experts,
+// one token, 22.5 -> 21.6 us). Up to 4096 inputs with the producer's threads too was slower (4096 x 4096 7.7 -> 8.7), and so were two slices side by side in
+// each round (900 x 10240 11.4 -> 13.9). The other launches of a row a thread, partial sums among them, keep to the loop: a layer of 2560 inputs runs several on
+// both sides of what a slice a thread holds, and two kernels that each fill the instruction cache took more than the straight line gave (2560 inputs, 10240 in the
+// feed-forward, us, a loop that fetched once too often / two kernels / this: Q6_K 61.8 / 65.0 / 60.6, Q4_0 60.2 / 62.0 / 58.1).
 template <int TYPE, int MODE, int T, int NW, int R, bool GATED, bool BANKED, bool ONE>
 __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW <= 7 ? 2 : 1)) rq_gemv_stream_kernel(const __grid_constant__ StreamParams p) {
     constexpr int kConsumers = NW * 32;
@@ -1703,9 +1704,9 @@ __global__ void __launch_bounds__(NW * 32 + 32, NW == 5 ? (T >= 2 ? 2 : 3) : (NW
             // lanes are full or the rows are over: silu goes through double precision, a long chain that one lane would otherwise walk
             // for every row by itself.
             // A row that is not there is loaded and dotted all the same (its slot has room for it) and its sum dropped: with a branch around each row's loads and
-            // another around its dot, a thread's two rows follow one another. Q6_K and Q8_0, int8, one token, us: Q6_K 262144 x 2560 97.9 -> 95.9, 4096 x
-            // 14336 12.7 -> 12.5, 30000 x 1024 7.5 -> 7.35; Q8_0 100000 x 2560 46.1 -> 45.5. Not the four-bit formats, whose dot is half as long (Q4_0 100000
-            // x 2560 31.8 -> 32.9).
+            // another around its dot, a thread's two rows follow one another. Q6_K and Q8_0, int8, us, with the branches / without: Q6_K 262144 x 2560 93.1 / 91.2, 4096 x
+            // 14336 12.0 / 11.7, 30000 x 1024 7.5 / 7.3, Q8_0 4096 x 4096 5.6 / 5.4; two positions 262144 x 2560 138.6 / 127.7, Q8_0 100000 x 2560 48.8 / 45.8. Not the four-bit
+            // formats, whose dot is half as long (Q4_0 100000 x 2560 31.8 / 32.9), nor windows of four positions, whose dots have no branches.
             constexpr bool kAlways = MODE == RQ_ACT_INT8 && T != 4 && (TYPE == RQ_Q6_K || TYPE == RQ_Q8_0);
             constexpr bool gated = GATED;
             int pending = 0;
